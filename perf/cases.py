@@ -6,6 +6,7 @@ over a key/value cache and stepwise translation decoding, in the data types that
     draw(rng)            one more case of the same ranges
     prepare(case, seed)  the model and the inputs, on the GPU, from the seed
     run(state)           one pass through the public entry points
+    exact(case, seed)    what that pass computes, in 64 bits and plain torch
     work(case)           the bytes and floating-point operations that one pass cannot do without
     tolerance(case)      how far two correct implementations at the case's precision may differ
 """
@@ -165,7 +166,8 @@ def _mask_lengths(case, seed):
     return _lengths(case["batch"], max(1, case["seq"] // 4), case["seq"], seed) if case["batch"] > 1 else [max(1, case["seq"] * 3 // 4)]
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """The torch module and the inputs of one pass."""
     g = torch.Generator(device=DEVICE).manual_seed(seed)
     dtype, kind, B = DTYPES[case["dtype"]], case["kind"], case["batch"]
     if kind == "nmt":
@@ -173,7 +175,7 @@ def prepare(case, seed):
             stack = _DecoderStack()
         S = case["source"]
         lens = torch.tensor(_lengths(B, max(1, S // 2), S, seed) if B > 1 else [S], device=DEVICE)
-        return {"kind": kind, "model": tt.TransformerDecoder.from_onmt(_weights(stack, g, dtype), DEVICE),
+        return {"kind": kind, "torch_model": _weights(stack, g, dtype),
                 "memory": torch.randn(S, B, NMT["hidden"], generator=g, device=DEVICE, dtype=dtype), "lengths": lens,
                 "source": torch.randint(2, NMT["vocab"], (S, B, 1), generator=g, device=DEVICE),
                 "targets": [torch.randint(2, NMT["vocab"], (1, B, 1), generator=g, device=DEVICE) for _ in range(case["steps"])]}
@@ -182,24 +184,29 @@ def prepare(case, seed):
     # the torch module stays with the state: the framework's layers alias some of its tensors
     state = {"kind": kind, "torch_model": torch_model}
     if kind == "bert":
-        loader = tt.QBertModel if case["dtype"] == "int8" else tt.BertModel
-        mask = None
+        state["mask"] = None
         if case["masked"]:
             kept = torch.tensor(_mask_lengths(case, seed), device=DEVICE)
-            mask = (torch.arange(case["seq"], device=DEVICE)[None] < kept[:, None]).to(torch.int64)
-        state.update(model=loader.from_torch(torch_model, DEVICE), mask=mask,
-                     ids=torch.randint(0, vocab, (B, case["seq"]), generator=g, device=DEVICE))
+            state["mask"] = (torch.arange(case["seq"], device=DEVICE)[None] < kept[:, None]).to(torch.int64)
+        state["ids"] = torch.randint(0, vocab, (B, case["seq"]), generator=g, device=DEVICE)
     elif kind == "packed":
-        lens = _lengths(B, case["low"], case["high"], seed)
-        state.update(model=tt.BertModelSmartBatch.from_torch(torch_model, DEVICE), lengths=lens,
-                     ids=[torch.randint(0, vocab, (n,), generator=g, device=DEVICE) for n in lens])
+        state["lengths"] = _lengths(B, case["low"], case["high"], seed)
+        state["ids"] = [torch.randint(0, vocab, (n,), generator=g, device=DEVICE) for n in state["lengths"]]
+    elif kind == "gpt2":
+        state["ids"] = torch.randint(0, vocab, (B, case["seq"]), generator=g, device=DEVICE)
     else:
-        state.update(model=tt.GPT2Model.from_torch(torch_model, DEVICE))
-        if kind == "gpt2":
-            state.update(ids=torch.randint(0, vocab, (B, case["seq"]), generator=g, device=DEVICE))
-        else:
-            state.update(prompt=torch.randint(0, vocab, (B, case["prompt"]), generator=g, device=DEVICE),
-                         tokens=[torch.randint(0, vocab, (B, 1), generator=g, device=DEVICE) for _ in range(case["steps"])])
+        state["prompt"] = torch.randint(0, vocab, (B, case["prompt"]), generator=g, device=DEVICE)
+        state["tokens"] = [torch.randint(0, vocab, (B, 1), generator=g, device=DEVICE) for _ in range(case["steps"])]
+    return state
+
+
+def prepare(case, seed):
+    state = _inputs(case, seed)
+    if state["kind"] == "nmt":
+        state["model"] = tt.TransformerDecoder.from_onmt(state["torch_model"], DEVICE)
+    else:
+        loader = {"bert": tt.QBertModel if case["dtype"] == "int8" else tt.BertModel, "packed": tt.BertModelSmartBatch}.get(state["kind"], tt.GPT2Model)
+        state["model"] = loader.from_torch(state["torch_model"], DEVICE)
     return state
 
 
@@ -226,6 +233,80 @@ def run(state):
             hidden, attention = model(token, state["memory"], step=step, memory_lengths=state["lengths"])
             outs += [hidden, attention["std"]]
         return outs
+
+
+# ---------------------------------------------------------------------------------------------------
+# the same passes in 64 bits
+# ---------------------------------------------------------------------------------------------------
+def _norm(x, ln):
+    return torch.nn.functional.layer_norm(x, ln.normalized_shape, ln.weight, ln.bias, ln.eps)
+
+
+def _gelu(x):
+    return torch.nn.functional.gelu(x, approximate="tanh")  # the form that the framework documents for every model
+
+
+def _attend(q, k, v, heads, keep=None):
+    """Rows [B, L, H] and keys and values [B, S, H] -> context [B, L, H] and probabilities [B, heads, L, S]; keep: what is seen."""
+    q, k, v = (t.unflatten(-1, (heads, -1)).transpose(1, 2) for t in (q, k, v))
+    scores = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+    probs = (scores if keep is None else scores.masked_fill(~keep, -math.inf)).softmax(-1)
+    return (probs @ v).transpose(1, 2).flatten(2), probs
+
+
+def _bert(m, ids, mask):
+    e, keep = m.embeddings, None if mask is None else mask.bool()[:, None, None]
+    x = e.word_embeddings(ids) + e.position_embeddings.weight[: ids.shape[1]] + e.token_type_embeddings.weight[0]
+    x = _norm(x, e.LayerNorm)
+    for layer in m.encoder.layer:
+        a = layer.attention
+        context, _ = _attend(a.self.query(x), a.self.key(x), a.self.value(x), m.config.num_attention_heads, keep)
+        x = _norm(x + a.output.dense(context), a.output.LayerNorm)
+        x = _norm(x + layer.output.dense(_gelu(layer.intermediate.dense(x))), layer.output.LayerNorm)
+    return x, torch.tanh(m.pooler.dense(x[:, 0]))
+
+
+def _gpt2(m, ids):
+    L = ids.shape[1]
+    x = m.wte(ids) + m.wpe.weight[:L]
+    seen = torch.ones(L, L, dtype=torch.bool, device=DEVICE).tril()
+    for b in m.h:
+        q, k, v = (_norm(x, b.ln_1) @ b.attn.c_attn.weight + b.attn.c_attn.bias).chunk(3, -1)
+        x = x + _attend(q, k, v, m.config.n_head, seen)[0] @ b.attn.c_proj.weight + b.attn.c_proj.bias
+        x = x + _gelu(_norm(x, b.ln_2) @ b.mlp.c_fc.weight + b.mlp.c_fc.bias) @ b.mlp.c_proj.weight + b.mlp.c_proj.bias
+    return _norm(x, m.ln_f)
+
+
+def exact(case, seed):
+    """The int8 models are compared with their unquantised weights: what is left is then mostly the quantisation."""
+    s = _inputs(case, seed)
+    kind, m = s["kind"], s["torch_model"].double()
+    with torch.no_grad():
+        if kind == "bert":
+            return list(_bert(m, s["ids"], s["mask"]))
+        if kind == "packed":
+            each = [_bert(m, ids[None], None) for ids in s["ids"]]
+            return [torch.cat([x for x, _ in each], 1), torch.cat([p for _, p in each], 0)]
+        if kind == "gpt2":
+            hidden = _gpt2(m, s["ids"])
+            return [hidden, hidden @ m.wte.weight.T]
+        if kind == "generate":
+            hidden = _gpt2(m, torch.cat([s["prompt"]] + s["tokens"], 1))[:, case["prompt"]:]
+            return [hidden[:, t: t + 1] @ m.wte.weight.T for t in range(case["steps"])]
+        # All steps at once, each row seeing the steps before it.
+        memory, T = s["memory"].double().transpose(0, 1), case["steps"]
+        x = m.embeddings(torch.cat(s["targets"])).transpose(0, 1)
+        seen = torch.ones(T, T, dtype=torch.bool, device=DEVICE).tril()
+        real = (torch.arange(case["source"], device=DEVICE)[None] < s["lengths"][:, None])[:, None, None]
+        for layer in m.transformer_layers:
+            a, f, y = layer.self_attn, layer.feed_forward, _norm(x, layer.layer_norm_1)
+            x = x + a.final_linear(_attend(a.linear_query(y), a.linear_keys(y), a.linear_values(y), a.head_count, seen)[0])
+            a, y = layer.context_attn, _norm(x, layer.layer_norm_2)
+            context, probs = _attend(a.linear_query(y), a.linear_keys(memory), a.linear_values(memory), a.head_count, real)
+            x = x + a.final_linear(context)
+            x = x + f.w_2(torch.relu(f.w_1(_norm(x, f.layer_norm))))
+        hidden = _norm(x, m.layer_norm)
+        return [out for t in range(T) for out in (hidden[:, t][None], probs[:, 0, t][None])]
 
 
 # ---------------------------------------------------------------------------------------------------
