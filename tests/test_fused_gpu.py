@@ -69,6 +69,32 @@ def test_linear_matches_unfused_reference(ctx, dt, M, N, K, epi):
     assert maxdiff(got, want) < tol
 
 
+# 128 x 32 tiles (one per block, then several), 128 x 64 and 128 x 128 tiles: one k-block, an odd count that leaves the ring of
+# slots in the middle between two tiles, a ragged last k-block, and split-K ranges of odd length (K = 1984: 31 k-blocks)
+@pytest.mark.parametrize("M,N", [(40, 96), (40, 9504), (1100, 700), (2500, 1200)])
+@pytest.mark.parametrize("K", [8, 64, 192, 584, 1984])
+def test_linear_counts_of_k_blocks_between_the_two_issuing_warps(ctx, M, N, K):
+    r = rng(M + N + K)
+    a = rounded(r.standard_normal((M, K)).astype(np.float32), "f16")
+    w = rounded(r.standard_normal((K, N)).astype(np.float32) * 0.05, "f16")
+    want = a @ w
+    Wp = prepack(ctx, w, "f16")
+    out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    ctx.call("linear", _capi.F16, dev(a, "f16"), K, Wp, None, None, 0, M, N, K, EPIS["none"], out, N)
+    assert ctx.device_status() == _capi.OK
+    # fp32 sums rounded once to fp16
+    assert maxdiff(host(out), want) < 2.0 ** -11 * float(np.abs(want).max()) + 1e-4 * math.sqrt(K)
+    aq, wq = r.integers(-127, 128, (M, 16 * ((K + 15) // 16))), r.integers(-127, 128, (N, 16 * ((K + 15) // 16)))
+    scale = np.full(M, 2.0 ** -16, np.float32)
+    outq = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    ctx.call("linear_int8", _capi.F16, dev(aq.astype(np.int8)), dev(scale), dev(wq.astype(np.int8)), dev(np.ones(1, np.float32)), None, None, 0,
+             M, N, aq.shape[1], EPIS["none"], outq, N)
+    # exact int32 sums (below 2^25: one fp32 rounding at most), then one rounding to fp16
+    wantq = (aq.astype(np.float64) @ wq.T.astype(np.float64)) * 2.0 ** -16
+    assert maxdiff(host(outq), wantq) < (2.0 ** -11 + 2.0 ** -24) * float(np.abs(wantq).max()) + 2.0 ** -24
+    assert ctx.device_status() == _capi.OK
+
+
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 def test_linear_plain_and_tanh_epilogues_and_strided_io(ctx, dt):
     r = rng(77)

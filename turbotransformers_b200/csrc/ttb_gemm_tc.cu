@@ -1,11 +1,12 @@
 // Tensor-core Linear for sm_100a: out[M,N] = epilogue(sum over passes of A_p[M,K] . W_p[N,K]^T).
 //
-// One persistent CTA (or CTA pair) per SM, 320 threads in three roles:
+// One persistent CTA (or CTA pair) per SM, 320 or 352 threads in three roles:
 //   warp 0      : TMA producer  - cp.async.bulk.tensor loads of 128-byte-swizzled K-major tiles into a
 //                 shared-memory ring, completion signalled on "full" mbarriers
 //   warp 1      : MMA issuer    - one elected thread issues tcgen05.mma (128 x BN x 32 bytes of K per instruction)
 //                 from shared-memory descriptors into a TMEM accumulator; tcgen05.commit releases ring
 //                 slots ("empty" mbarriers) and publishes finished accumulators ("tmem_full")
+//   warp 10     : second issuer on tiles of up to 128 columns, with an accumulator of its own (every other k-block)
 //   warps 2..9  : epilogue      - tcgen05.ld the accumulator (one row per thread), apply scale/bias/activation/
 //                 residual in fp32, convert, stage through a swizzled shared-memory tile and TMA-store it
 // Two accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the MMAs of tile i+1.
@@ -51,7 +52,11 @@ template <int BN, bool TWO = false, bool SK = false> struct Cfg {
   static constexpr int B_BYTES = (TWO ? BN / 2 : BN) * BK_BYTES;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = SK ? 4 : (TWO ? 6 : ((BN == 256) ? 4 : (BN == 128 ? 6 : 8)));
-  static constexpr int TMEM_COLS = (2 * BN < 32) ? 32 : 2 * BN;
+  // Two MMA-issuing warps with an accumulator each (even and odd k-blocks) wherever a k-block's MMAs are short: see the issuer.
+  static constexpr int ISSUERS = (!TWO && BN <= 128) ? 2 : 1;
+  static constexpr int THREADS = kThreads + 32 * (ISSUERS - 1);
+  static constexpr int TMEM_COLS = 2 * ISSUERS * BN;
+  static_assert(STAGES % ISSUERS == 0 && TMEM_COLS >= 32 && TMEM_COLS <= 512, "ring slots divide evenly among the issuers; TMEM allocation");
   // Epilogue staging: per epilogue warp one [32 rows x 128 B] swizzled tile that its TMA stores read (BN >= 64 only).
   static constexpr int STAGING_BYTES = (BN >= 64) ? 8 * 4096 : 0;
   static constexpr int REDUCE_BYTES = SK ? (kMaxSplit - 1) * BM * BN * 4 : 0;  // [slot][column][row] 32-bit words
@@ -85,12 +90,6 @@ struct GemmParams {
   int split_k;             // CTAs per cluster sharing one tile (SK kernels), else 1
   int* status;
 };
-
-// 32 lanes x 32 columns of 32-bit accumulators, issued and waited for.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  tmem_ld32_issue(taddr, r);
-  tmem_ld_wait();
-}
 
 // One 16-byte group of output elements <-> floats: 8 values for the 16-bit types, 4 for fp32.
 template <typename OutT> struct Per16 { static constexpr int value = 16 / (int)sizeof(OutT); };
@@ -166,7 +165,7 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2 };
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR, bool LN = false>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmO2, const GemmParams p) {
@@ -216,7 +215,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       mbar_init(empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
-      mbar_init(tfull_bar(a), 1);
+      mbar_init(tfull_bar(a), C::ISSUERS);
       mbar_init(tempty_bar(a), TWO ? 16 : 8);  // one arrival per epilogue warp (of both CTAs when paired)
     }
     mbar_init(reduce_bar, (SK && group > 1) ? (uint32_t)(group - 1) * 128u : 1u);  // every thread of the other CTAs' four working warps
@@ -285,26 +284,36 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
+  } else if (warp == 1 || (C::ISSUERS == 2 && warp == 10)) {
+    // ------------------------------------------------------------------ MMA issuer(s)
+    // A thread that has issued MMAs sees its next shared-memory read (the wait for the next slot) return only once they have
+    // drained: 508 cycles per k-block at N <= 128, where the MMAs themselves need 128 to 256. So the narrow tiles have two
+    // issuing warps: each takes every other k-block into its own accumulator, one's wait passes under the other's MMAs, and
+    // the epilogue adds the two accumulators (the order of the sums is fixed by the shape). One issuer -> two, replayed from a
+    // graph, us: 600 x 2304 x 768 fp16 9.7 -> 8.5, 792 x 768 x 3072 15.4 -> 12.9, 2048 x 768 x 3072 26.4 -> 21.8, 128 x 2304 x 768
+    // 5.9 -> 5.4; fp32 (three products) 520 x 768 x 3072 68.7 -> 55.6. What is left there is the SM's share of L2 bandwidth
+    // (24 KB a k-block at 64 bytes a cycle). The chains of additions are half as long, too: the tensor core truncates each partial
+    // sum, and whole fp32 models come out at half their distance from 64 bits (4.9e-5 -> 2.4e-5 on 8 ragged sequences).
+    const int issuer = (C::ISSUERS == 2 && warp == 10) ? 1 : 0;
     if (lane == 0 && (!TWO || rank == 0)) {
-      int stage = 0;
-      uint32_t phase = 0;
+      uint32_t first_kb = 0;  // k-blocks of the tiles before this one: the ring position of the tile's first
       int acc_iter = 0;
       bool ok = true;
       // Descriptors differ only in the start-address field of their low word, so the loop below advances that
       // word with one add per MMA instead of rebuilding 64-bit descriptors (this single thread's instruction
       // stream is what paces the tensor core).
       const uint32_t a_lo0 = desc_lo(tiles);
-      uint32_t a_lo = a_lo0;
-      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step, ++acc_iter) {
+      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step, ++acc_iter, first_kb += (uint32_t)(kb_end - kb_begin)) {
         const int acc = acc_iter & 1;
         const uint32_t acc_phase = (uint32_t)(acc_iter >> 1) & 1u;
+        int stage = (int)((first_kb + issuer) % C::STAGES);
+        uint32_t phase = ((first_kb + issuer) / C::STAGES) & 1u;
+        uint32_t a_lo = a_lo0 + (uint32_t)stage * (uint32_t)(C::STAGE_BYTES >> 4);
         if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+        const uint32_t d_tmem = tmem_base + (uint32_t)((acc * C::ISSUERS + issuer) * BN);
         uint32_t accumulate = 0;
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
+        for (int kb = kb_begin + issuer; kb < kb_end; kb += C::ISSUERS) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) { ok = false; break; }
           const uint32_t b_lo = a_lo + (uint32_t)(C::A_BYTES >> 4);
 #pragma unroll
@@ -315,8 +324,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           // the slot is free (in both CTAs when paired) once these MMAs have read it
           if (TWO) tc_commit_pair(empty_bar(stage));
           else tc_commit(empty_bar(stage));
-          a_lo += (uint32_t)(C::STAGE_BYTES >> 4);
-          if (++stage == C::STAGES) { stage = 0; phase ^= 1u; a_lo = a_lo0; }
+          a_lo += (uint32_t)(C::ISSUERS * (C::STAGE_BYTES >> 4));
+          stage += C::ISSUERS;
+          if (stage >= C::STAGES) { stage -= C::STAGES; phase ^= 1u; a_lo -= (uint32_t)(C::STAGES * (C::STAGE_BYTES >> 4)); }
         }
         if (ok) {  // accumulator complete: wake the epilogue warps (of both CTAs when paired)
           if (TWO) tc_commit_pair(tfull_bar(acc));
@@ -379,6 +389,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       if (TWO && rank != 0) mbar_arrive_remote(tempty_bar(a), 0);
       else mbar_arrive(tempty_bar(a));
     };
+    // 32 columns of the tile's sums: one accumulator, or the even and the odd k-blocks' (a tile of one k-block has no odd one)
+    const bool two_acc = C::ISSUERS == 2 && kb_end - kb_begin >= 2;
+    auto load_sums = [&](uint32_t addr, uint32_t (&r)[32]) {
+      tmem_ld32_issue(addr, r);
+      if (two_acc) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // 16 columns at a time: 48 live words instead of 64
+          uint32_t r1[16];
+          tmem_ld16_issue(addr + (uint32_t)(BN + 16 * h), r1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const uint32_t w = r[16 * h + j];
+            r[16 * h + j] = (KIND == KIND_I8) ? (uint32_t)((int)w + (int)r1[j]) : __float_as_uint(__uint_as_float(w) + __uint_as_float(r1[j]));
+          }
+        }
+      } else {
+        tmem_ld_wait();
+      }
+    };
     // accumulator word -> value before bias: int8 dequantised (symmetric per row, or affine per tensor), else as it is
     auto dequant = [&](uint32_t word, float rs, int colsum) -> float {
       if (KIND != KIND_I8) return __uint_as_float(word);
@@ -408,7 +438,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) break;
         tc_fence_after();
         prefetch_residual(tile + tile_step);
-        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN);
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * C::ISSUERS * BN);
         uint4 vp[2][2][4];  // [chunk][32-column half][16-byte group]: the values, packed
         float sum = 0.f, sq = 0.f;
 #pragma unroll
@@ -539,7 +569,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       tc_fence_after();
       if (!SK) prefetch_residual(tile + tile_step);  // the next tile's rows, a whole mainloop ahead
       const float rs = (KIND != KIND_I8) ? 1.0f : (affine ? act_scale * w_scale : (row < p.M ? p.row_scale[row] * w_scale : 1.0f));
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN);
+      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * C::ISSUERS * BN);
       if (use_tma || half == 1) {
         if (!staged_work) {  // nothing to do for this warp on this tile: just hand the accumulator back
           tc_fence_before();
@@ -581,8 +611,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                 bq[g % ((EB == 2) ? G16 : 1)] = (colh + g * P16 < p.N) ? __ldg(reinterpret_cast<const uint4*>(bias + colh + g * P16)) : make_uint4(0, 0, 0, 0);
             }
             uint32_t r0[32];
-            tmem_ld32_issue(taddr + (uint32_t)(cc * CH + hh * 32), r0);
-            tmem_ld_wait();
+            load_sums(taddr + (uint32_t)(cc * CH + hh * 32), r0);
             if (hh == HALVES - 1 && cc == c_end - 1) {  // this warp's share of the accumulator is in registers: hand it back now
               tc_fence_before();
               __syncwarp();
@@ -673,7 +702,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll 1
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
-        tmem_ld32(taddr + (uint32_t)(c * 32), r);
+        load_sums(taddr + (uint32_t)(c * 32), r);
         const int col0 = n_blk * BN + c * 32;
         if (SK && group > 1) {
           // Split-K: ranks > 0 hand their partial tile to rank 0's shared memory ([slot][column][row] words, so a warp's
@@ -877,7 +906,7 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
     if (TWO) {
       cudaLaunchConfig_t probe = {};
       probe.gridDim = dim3(2 * (unsigned)ctx->sm_count);
-      probe.blockDim = dim3(kThreads);
+      probe.blockDim = dim3(C::THREADS);
       probe.dynamicSmemBytes = C::SMEM_BYTES;
       cudaLaunchAttribute pa[1];
       pa[0].id = cudaLaunchAttributeClusterDimension;
@@ -895,7 +924,7 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   const int64_t num_tiles = ((p.M + TILE_M - 1) / TILE_M) * (int64_t)((p.N + BN - 1) / BN);
   if (!TWO && !SK) {
     const int grid = (int)(num_tiles < ctx->sm_count ? num_tiles : ctx->sm_count);
-    cudaError_t e = launch_pdl(kern, dim3((unsigned)grid), dim3(kThreads), C::SMEM_BYTES, ctx->stream, tmA0, tmA1, tmB0, tmB1, tmO, tmO2, q);
+    cudaError_t e = launch_pdl(kern, dim3((unsigned)grid), dim3(C::THREADS), C::SMEM_BYTES, ctx->stream, tmA0, tmA1, tmB0, tmB1, tmO, tmO2, q);
     if (e != cudaSuccess) return fail(ctx, TTB_ERR_CUDA, "launch of gemm_tc failed: %s", cudaGetErrorString(e));
     return launched(ctx, "gemm_tc");
   }
@@ -903,7 +932,7 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   const int clusters = SK ? (int)num_tiles : (int)(num_tiles < max_clusters[dev] ? num_tiles : max_clusters[dev]);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(group * clusters));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(C::THREADS);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[2];
@@ -1053,7 +1082,7 @@ int max_resident_clusters(ttb_ctx* ctx, int split) {
   }
   cudaLaunchConfig_t probe = {};
   probe.gridDim = dim3((unsigned)(split * ctx->sm_count));
-  probe.blockDim = dim3(kThreads);
+  probe.blockDim = dim3(C::THREADS);
   probe.dynamicSmemBytes = C::SMEM_BYTES;
   cudaLaunchAttribute pa[1];
   pa[0].id = cudaLaunchAttributeClusterDimension;
