@@ -43,6 +43,8 @@ constexpr int kThreads = 320;    // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue 
 constexpr int kMaxSplit = 4;     // CTAs of a cluster that may share one tile's K range (clusters of 6 pack badly into the GPCs:
                                  // 24 of them did not fit the chip at once and the launch took two waves)
 
+constexpr int kPrefetchBlocks = 16;  // k-blocks of the first tile's weights that are sent for ahead of the wait: K = 1024 in 16 bits
+
 // TWO = a pair of CTAs (one cluster of two SMs) computes a 256 x BN tile with cta_group::2 MMAs: each CTA stages its
 // own 128 rows of A and its own half (BN/2 rows) of W, so a k-block costs 32 KB of L2->SM traffic per CTA instead of 48.
 // SK = split-K over a cluster (BN = 32 only): a shorter ring, plus room for the partial tiles of the other CTAs.
@@ -218,7 +220,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       mbar_init(tfull_bar(a), C::ISSUERS);
       mbar_init(tempty_bar(a), TWO ? 16 : 8);  // one arrival per epilogue warp (of both CTAs when paired)
     }
-    mbar_init(reduce_bar, (SK && group > 1) ? (uint32_t)(group - 1) * 128u : 1u);  // every thread of the other CTAs' four working warps
+    mbar_init(reduce_bar, (SK && group > 1) ? (uint32_t)(group - 1) * 4u : 1u);  // the other CTAs' four working warps
     *abort_flag = 0;
     mbar_init_fence();
   }
@@ -237,7 +239,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   if (TWO || SK) cluster_sync_all();  // the peers' barriers are initialised before anything signals them remotely
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();  // everything above ran in the shadow of the previous kernel; its results are visible from here on
 
   const int num_m = (p.M + TILE_M - 1) / TILE_M, num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
@@ -246,6 +247,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   // this CTA's share of a tile's k-blocks: all of them, or (split-K) one contiguous range per cluster rank
   const int kb_begin = SK ? (int)(((long long)total_kb * rank) / group) : 0;
   const int kb_end = SK ? (int)(((long long)total_kb * (rank + 1)) / group) : total_kb;
+  // The first tile's weights start on their way to L2 while the previous kernel still runs. A prefetch into L2 is not a read:
+  // should that kernel write the weights, the loads below (after the wait) see what it wrote.
+  // With the bias and residual fetched ahead of the sums and one arrival per warp in the split-K exchange (below), one product
+  // in a row of them, us: 128 x 768 x 768 5.5 -> 5.0, 1 x 768 x 768 5.0 -> 4.8, 128 x 768 x 3072 10.1 -> 9.4; whole passes, whose
+  // weights are colder: BERT-base 1 x 17 476 -> 462, GPT-2 generation, one user, 24 steps, 14.3 -> 13.5 ms with the two issuers.
+  if (warp == 0 && lane == 0 && tile0 < num_tiles) {
+    const int n_row = (tile0 % num_n) * BN + (int)(TWO ? rank : 0u) * (BN / 2);
+    int pass = kb_begin / num_kb, kk = kb_begin % num_kb;
+    for (int kb = kb_begin; kb < min(kb_end, kb_begin + kPrefetchBlocks) && n_row < p.N; ++kb) {
+      tma_prefetch_2d(((p.pass_b >> pass) & 1) ? &tmB1 : &tmB0, kk * BK_ELEMS, n_row);
+      if (++kk == num_kb) { kk = 0; ++pass; }
+    }
+  }
+  pdl_wait();  // everything above ran in the shadow of the previous kernel; its results are visible from here on
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -565,10 +580,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       const bool staged_work = use_tma && c_beg < c_end;
       uint4 res[8];
       if (staged_work && p.epilogue == TTB_EPI_BIAS_RESIDUAL) load_residual(res, row_base, n_blk * BN + c_beg * CH);  // before the wait
+      // Narrow tiles (one 32-column chunk per row): bias and residual are fetched before the wait for the sums. Behind it they
+      // would add their round trip to a kernel of 5 us.
+      constexpr int QN = (BN == 32) ? 32 * EB / 16 : 1;
+      uint4 bias_q[QN], res_q[QN];
+      const bool fetched = BN == 32 && half == 0 && vec_ok && row < p.M && n_blk * BN + 32 <= p.N && !(SK && rank != 0);
+      if (fetched) {
+        if (p.epilogue != TTB_EPI_NONE) {
+          const uint4* bp = reinterpret_cast<const uint4*>(bias + n_blk * BN);
+#pragma unroll
+          for (int i = 0; i < QN; ++i) bias_q[i] = bp[i];
+        }
+        if (p.epilogue == TTB_EPI_BIAS_RESIDUAL) {
+          const uint4* rp = reinterpret_cast<const uint4*>(residual + (long long)row * p.ldr + n_blk * BN);
+#pragma unroll
+          for (int i = 0; i < QN; ++i) res_q[i] = rp[i];
+        }
+      }
+      const float rs = (KIND != KIND_I8) ? 1.0f : (affine ? act_scale * w_scale : (row < p.M ? p.row_scale[row] * w_scale : 1.0f));
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) break;
       tc_fence_after();
       if (!SK) prefetch_residual(tile + tile_step);  // the next tile's rows, a whole mainloop ahead
-      const float rs = (KIND != KIND_I8) ? 1.0f : (affine ? act_scale * w_scale : (row < p.M ? p.row_scale[row] * w_scale : 1.0f));
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * C::ISSUERS * BN);
       if (use_tma || half == 1) {
         if (!staged_work) {  // nothing to do for this warp on this tile: just hand the accumulator back
@@ -712,7 +744,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             const uint32_t dst = map_to_rank(smem_u32(reduce_buf), 0) + (uint32_t)((((int)rank - 1) * BN * BM + trow) * 4);
 #pragma unroll
             for (int j = 0; j < 32; ++j) st_cluster_f32(dst + (uint32_t)(j * BM * 4), __uint_as_float(r[j]));
-            mbar_arrive_remote(reduce_bar, 0);  // release at cluster scope: this thread's stores are visible to the waiter
+            __syncwarp();  // orders the other lanes' stores before lane 0's release at cluster scope (which is cumulative)
+            if (lane == 0) mbar_arrive_remote(reduce_bar, 0);  // one arrival per warp: 128 per CTA queued up on one barrier word
             continue;
           }
           if (!mbar_wait_cluster(reduce_bar, 0, abort_flag)) { gave_up = true; break; }
@@ -732,8 +765,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         const bool full = vec_ok && (col0 + 32 <= p.N);
         if (p.epilogue != TTB_EPI_NONE) {
           float b[32];
-          if (full) load32<OutT>(bias + col0, b);
-          else {
+          if (BN == 32 && full) {
+#pragma unroll
+            for (int i = 0; i < QN; ++i) unpack16<OutT>(bias_q[i], b + i * P16);
+          } else if (full) {
+            load32<OutT>(bias + col0, b);
+          } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) b[j] = (col0 + j < p.N) ? to_f(bias[col0 + j]) : 0.f;
           }
@@ -749,8 +786,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         } else if (p.epilogue == TTB_EPI_BIAS_RESIDUAL) {
           const OutT* rp = residual + (long long)row * p.ldr + col0;
           float q[32];
-          if (full) load32<OutT>(rp, q);
-          else {
+          if (BN == 32 && full) {
+#pragma unroll
+            for (int i = 0; i < QN; ++i) unpack16<OutT>(res_q[i], q + i * P16);
+          } else if (full) {
+            load32<OutT>(rp, q);
+          } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) q[j] = (col0 + j < p.N) ? to_f(rp[j]) : 0.f;
           }

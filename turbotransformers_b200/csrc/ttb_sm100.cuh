@@ -116,6 +116,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// The same tile brought as far as L2: no destination, nothing to wait for.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+
 // TMA store of a [rows x 128 B] swizzled shared-memory tile; rows / columns outside the tensor are clipped by the
 // hardware. Completion is tracked per issuing thread in bulk groups.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
