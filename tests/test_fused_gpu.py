@@ -95,6 +95,24 @@ def test_linear_counts_of_k_blocks_between_the_two_issuing_warps(ctx, M, N, K):
     assert ctx.device_status() == _capi.OK
 
 
+# One shape each at which the tile rule turns to another kernel: 32- and 64-column tiles, split K, 128 columns in one wave and in
+# several, 256 columns, CTA pairs
+@pytest.mark.parametrize("M,N,K", [(90, 768, 768), (300, 2304, 768), (120, 768, 3072), (792, 2304, 768), (2050, 768, 3072), (6500, 768, 768),
+                                   (1100, 3072, 768), (3200, 768, 3072)])
+@pytest.mark.parametrize("epi", ["bias", "bias_residual"])
+def test_linear_on_every_side_of_the_tile_rule(ctx, M, N, K, epi):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device="cuda").half()
+    w = (torch.randn(N, K, generator=g, device="cuda") * 0.05).half()
+    bias, res = (torch.randn(*s, generator=g, device="cuda").half() for s in ((N,), (M, N)))
+    want = a.double() @ w.double().T + bias.double() + (res.double() if epi == "bias_residual" else 0.0)
+    out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+    ctx.call("linear", _capi.F16, a, K, w, bias, res, N, M, N, K, EPIS[epi], out, N)
+    assert ctx.device_status() == _capi.OK
+    # fp32 sums, one rounding to fp16
+    assert float((out.double() - want).abs().max()) < 2.0 ** -11 * float(want.abs().max()) + 1e-4 * math.sqrt(K)
+
+
 @pytest.mark.parametrize("dt", ["f16", "bf16"])
 def test_linear_plain_and_tanh_epilogues_and_strided_io(ctx, dt):
     r = rng(77)

@@ -1143,42 +1143,65 @@ int max_resident_clusters(ttb_ctx* ctx, int split) {
 
 template <int KIND, typename OutT, int VAR = VAR_PLAIN>
 int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
-  // Large problems: CTA pairs on 256 x 256 tiles (less L2->SM traffic per flop). Otherwise the largest single-CTA
-  // N-tile that still gives every SM a tile; small problems use narrow tiles to spread over SMs.
+  // The shape decides between tiles by what each is expected to take: waves of tiles over the chip, each wave its k-blocks or,
+  // where that takes longer, its epilogue, plus what a launch costs around them. The constants are nanoseconds fitted to
+  // graph-replayed runs of M = 128 .. 8192 by (N, K) = (2304, 768), (768, 768), (3072, 768), (768, 3072) in fp16, int8, bf16
+  // as two products and fp32 as three: a k-block is 128 bytes of every row whatever the type, and costs the same.
+  // Against the fixed thresholds that came before (the widest tile that still gives every SM one), us: fp16 2048 x 768 x 3072
+  // 21.8 -> 16.6 (128-column tiles in one wave instead of 64-column ones in two), 792 x 2304 x 768 8.9 -> 7.4, 6500 x 768 x 768
+  // 18.2 -> 15.7, 3200 x 768 x 3072 25.8 -> 22.8 (pairs), fp32 3000 x 768 x 3072 124 -> 75, 520 x 2304 x 768 31 -> 22.
   constexpr int IN_BYTES = (KIND == KIND_I8) ? 1 : (KIND == KIND_TF32 ? 4 : 2);
   const int64_t num_m = (p.M + BM - 1) / BM;
   auto tiles = [&](int bn) { return num_m * ((p.N + bn - 1) / bn); };
   const int64_t pair_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((p.N + 255) / 256);
-  // Measured on B200 in back-to-back launches at M = 18424 (single CTA -> pair, TFLOP/s): N=2304 K=768 1097 -> 1228,
-  // N=3072 K=768 1088 -> 1165, N=768 K=3072 1171 -> 1273, but N=768 K=768 789 -> 756: pairs win unless both the
-  // mainloop and the row of tiles are short.
-  const int64_t k_bytes = (int64_t)p.K * IN_BYTES * p.npass;
-  // (same box, bias + residual epilogue: N = K = 768 25.7 us single against 26.3 paired; N = K = 1024, M = 16384 37.1 against 35.8)
-  const bool pair_pays = k_bytes >= 4096 || p.N >= 1536 || (k_bytes >= 2048 && p.N >= 1024);
-  p.split_k = 1;
-  if (pair_mode() && pair_tiles >= ctx->sm_count / 2 && (pair_pays || pair_mode() == 2)) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
-  if (tiles(256) >= ctx->sm_count) return launch_tc<256, KIND, OutT, false, false, VAR>(ctx, op, p);
-  if (tiles(128) >= ctx->sm_count) return launch_tc<128, KIND, OutT, false, false, VAR>(ctx, op, p);
-  if (tiles(64) >= ctx->sm_count / 2) return launch_tc<64, KIND, OutT, false, false, VAR>(ctx, op, p);
-  // Fewer 128 x 32 tiles than half the SMs and a mainloop of several k-blocks: share each tile's K range among the CTAs
-  // of a cluster so that the weights stream through (nearly) all SMs instead of a few.
-  const int64_t t32 = tiles(32);
   const int64_t total_kb = (((int64_t)p.K * IN_BYTES + BK_BYTES - 1) / BK_BYTES) * p.npass;
-  // Measured at M = 128 in a replayed graph: K = 3072 (48 k-blocks) 15.6 us in one CTA per tile, 9.0 us split four ways;
-  // K = 768 (12 k-blocks) 6.1 us unsplit and no faster split (the launch, the pipeline fill and the epilogue are what is left).
-  if (splitk_cap() > 1 && t32 * 2 <= ctx->sm_count && total_kb >= 24) {
-    int64_t s = ctx->sm_count / t32;
+  const int64_t sms = ctx->sm_count;
+  auto expect = [&](int64_t fixed, int64_t per_kb, int64_t epilogue, int64_t n, int64_t slots, int64_t kb) {
+    return fixed + (n + slots - 1) / slots * std::max(per_kb * kb, epilogue);
+  };
+  // Pairs lose where both the mainloop and the row of tiles are short (bias + residual epilogue: N = K = 768, M = 18424 25.7 us
+  // single against 26.3 paired; N = K = 1024, M = 16384 37.1 against 35.8) and where a tile is bound by its epilogue (int8,
+  // K = 768: 8000 x 3072 24.9 single, 27.5 paired).
+  const int64_t k_bytes = (int64_t)p.K * IN_BYTES * p.npass;
+  const bool pair_pays = k_bytes >= 4096 || (k_bytes >= 1536 && p.N >= 1536) || (k_bytes >= 2048 && p.N >= 1024);
+  p.split_k = 1;
+  if (pair_mode() == 2 && pair_tiles >= sms / 2) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
+  int best = 0;
+  int64_t best_ns = INT64_MAX;
+  auto consider = [&](int which, int64_t ns) {
+    if (ns < best_ns) { best = which; best_ns = ns; }
+  };
+  if (pair_mode() && pair_pays) consider(0, expect(7300, 310, 5400, pair_tiles, sms / 2, total_kb));
+  consider(256, expect(6300, 350, 6000, tiles(256), sms, total_kb));
+  consider(128, expect(3500, 235, 4300, tiles(128), sms, total_kb));
+  consider(64, expect(3800, 190, 3000, tiles(64), sms, total_kb));
+  consider(32, expect(3900, 165, 2000, tiles(32), sms, total_kb));
+  // Few 128 x 32 tiles and a mainloop of several k-blocks: the CTAs of a cluster may share each tile's K range, so that the
+  // weights stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per
+  // tile, 8.7 split four ways; 12 k-blocks are not worth the exchange.
+  const int64_t t32 = tiles(32);
+  if (splitk_cap() > 1 && t32 * 2 <= sms && total_kb >= 24) {
+    int64_t s = sms / t32;
     if (s > splitk_cap()) s = splitk_cap();
     if (s > total_kb / 2) s = total_kb / 2;  // at least two k-blocks per CTA
     // all clusters must be resident at once (one wave): how many clusters of s CTAs the device holds depends on how
     // they pack into its GPCs
     while (s >= 2 && t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, (int)s)) --s;
     if (s >= 2) {
-      p.split_k = (int)s;
-      return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
+      consider(1, expect(6900, 165, 2000, t32, t32, (total_kb + s - 1) / s));
+      if (best == 1) {
+        p.split_k = (int)s;
+        return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
+      }
     }
   }
-  return launch_tc<32, KIND, OutT, false, false, VAR>(ctx, op, p);
+  switch (best) {
+    case 0: return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
+    case 256: return launch_tc<256, KIND, OutT, false, false, VAR>(ctx, op, p);
+    case 128: return launch_tc<128, KIND, OutT, false, false, VAR>(ctx, op, p);
+    case 64: return launch_tc<64, KIND, OutT, false, false, VAR>(ctx, op, p);
+    default: return launch_tc<32, KIND, OutT, false, false, VAR>(ctx, op, p);
+  }
 }
 
 int check_linear(ttb_ctx* ctx, const char* what, const void* A, const void* W, const void* bias, const void* residual,
