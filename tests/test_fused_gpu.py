@@ -161,6 +161,30 @@ def test_linear_ragged_width_into_padded_rows_then_compacted(ctx, M, N, K):
     assert maxdiff(host(out), got[:, :N]) == 0.0
 
 
+# Ragged and misaligned rows stored word by word: odd and even widths, a width just past a tile, rows that start on odd elements
+# (an odd pitch, an odd offset), fewer rows than a tile. Everything around the product keeps its value.
+@pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("M,N,ldo,off", [(1, 50257, 50257, 0), (130, 1001, 1001, 0), (131, 9001, 9003, 1), (300, 4130, 4131, 0),
+                                         (600, 2305, 2305, 0), (2100, 5003, 5003, 0)])
+def test_linear_ragged_rows_straight_into_the_output(ctx, dt, M, N, ldo, off):
+    K = 136
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    a, w = (torch.randn(*s, generator=g, device="cuda").to(TORCH_DT[dt]) for s in ((M, K), (N, K)))
+    buf = torch.full((off + M * ldo + 8,), 7.0, dtype=TORCH_DT[dt], device="cuda")
+    out = buf[off:]
+    rows = out[: M * ldo].view(M, ldo)
+    if dt == "f32":
+        ctx.linear_ex(_capi.F32, _capi.F32, a, w, M, N, K, EPIS["none"], out, ldo=ldo)
+    else:
+        ctx.call("linear", code(dt), a, K, w, None, None, 0, M, N, K, EPIS["none"], out, ldo)
+    assert ctx.device_status() == _capi.OK
+    want = a.double() @ w.double().T
+    # one rounding to the output type; one product of fp32 operands cut off to tf32: 2 x 2^-10 of |a| |w| a term, sqrt(K) terms, 5 sigma
+    tol = {"f16": 2.0 ** -11, "bf16": 2.0 ** -8, "f32": 0.0}[dt] * float(want.abs().max()) + (2.0 ** -9 * 5 * math.sqrt(K) if dt == "f32" else 1e-3)
+    assert float((rows[:, :N].double() - want).abs().max()) < tol
+    assert bool((rows[:, N:] == 7.0).all()) and bool((buf[:off] == 7.0).all()) and bool((out[M * ldo:] == 7.0).all())
+
+
 def test_linear_weight_given_as_out_in(ctx):
     # is_trans_weight=True in the reference: the weight arrives as [N,K] and is only converted
     r = rng(5)

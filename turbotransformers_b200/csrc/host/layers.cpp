@@ -1051,10 +1051,10 @@ void Linear::operator()(const Tensor& input, Tensor* output) const {
   const int dt = core::ToTTBDtype(input.dtype());
   const int64_t N = dense_.out_dim(is_trans_), M = input.rows();
   output->Reshape(input.dtype(), WithLast(input, N), kDLCUDA, input.device_id(), "Linear/Reshape");
-  if (dt != TTB_F32 && N % 8 != 0) {
-    // An output row that is not a multiple of 16 bytes (e.g. a 50257-wide vocabulary) would force the GEMM onto scalar
-    // stores. Compute into a row-padded scratch with the fast epilogue, then compact: one extra pass over the output
-    // at copy bandwidth instead of a several-times slower GEMM.
+  if (dt != TTB_F32 && N % 8 != 0 && !dense_.bias().is_null()) {
+    // Output rows that are not a multiple of 16 bytes, with a bias: the GEMM would add it and store element by element.
+    // Compute into a row-padded scratch, then compact. (Without a bias, such as a 50257-wide tied vocabulary, the GEMM stores
+    // ragged rows itself.)
     const int64_t Np = (N + 7) / 8 * 8;
     ttb_ctx* c = DeviceContext(input.device_id());
     Tensor padded(nullptr);

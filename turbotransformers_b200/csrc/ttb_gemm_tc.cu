@@ -66,6 +66,11 @@ template <int BN, bool TWO = false, bool SK = false> struct Cfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + REDUCE_BYTES + BAR_BYTES + 1024;  // + slack for 1024-byte alignment
 };
 
+// Output of the wider tiles: STORE_DIRECT, each thread its own row from registers; STORE_TMA, through shared memory and TMA
+// stores (16-byte-aligned rows of a multiple of 16 bytes); STORE_WORDS, through shared memory and word stores, 128 consecutive
+// bytes of one row per instruction whatever the row's alignment.
+enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
+
 struct GemmParams {
   int M, N, K;             // K in elements, per pass
   int npass;               // 1..3 passes over K into one accumulator
@@ -88,7 +93,7 @@ struct GemmParams {
   int* ln_counters;          // LN kernels: per 128-row block {warps that have published, warps that have read}; all zero between launches
   long long ln_rows;         // rows of the partials array (M rounded up to whole tiles)
   int epilogue;
-  int tma_store;           // 1: the output tile goes through shared memory and TMA stores (needs aligned, 16-byte-multiple rows)
+  int staged;              // STORE_*: how the output tile leaves (BN >= 64)
   int split_k;             // CTAs per cluster sharing one tile (SK kernels), else 1
   int* status;
 };
@@ -209,7 +214,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       prefetch_tensormap(&tmA1);
       prefetch_tensormap(&tmB1);
     }
-    if (p.tma_store) prefetch_tensormap(&tmO);
+    if (p.staged == STORE_TMA) prefetch_tensormap(&tmO);
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -376,7 +381,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
                         ((reinterpret_cast<uintptr_t>(p.out_lo) & 15) == 0) &&
                         (!bias || (reinterpret_cast<uintptr_t>(bias) & 15) == 0) &&
                         (!residual || ((p.ldr % 8 == 0) && (reinterpret_cast<uintptr_t>(residual) & 15) == 0));
-    const bool use_tma = (BN >= 64) && p.tma_store;
+    const bool use_tma = (BN >= 64) && p.staged != STORE_DIRECT;
     uint8_t* buf = staging + (warp - 2) * 4096;  // this warp's [32 rows x 128 B] staging tile
     int acc_iter = 0;
     // Pulls a tile's residual rows towards L2 ahead of time, so the epilogue's loads do not each pay a DRAM
@@ -702,6 +707,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               for (int g = 0; g < G16; ++g) lo_pack[(hh * G16 + g) % LO_N] = pack16<OutT>(&v[g * P16]);
             }
           }
+          if (p.staged == STORE_WORDS) {
+            // A row whose address is not a multiple of 4 (every other row of an odd 16-bit width) is shifted by half a word on
+            // the way out, and its first and last elements go out alone: nothing beyond the row's own elements is written.
+            __syncwarp();
+            const int n_cols = min(CH, p.N - col0);
+#pragma unroll 4
+            for (int r = 0; r < 32; ++r) {
+              if (row_base + r >= p.M) break;
+              OutT* dst = out + (long long)(row_base + r) * p.ldo + col0;
+              const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+              if (EB == 4) {
+                if (lane < n_cols) reinterpret_cast<uint32_t*>(dst)[lane] = w;
+              } else if ((reinterpret_cast<uintptr_t>(dst) & 2) == 0) {
+                if (2 * lane + 1 < n_cols) reinterpret_cast<uint32_t*>(dst)[lane] = w;
+                else if (2 * lane < n_cols) reinterpret_cast<uint16_t*>(dst)[2 * lane] = (uint16_t)w;
+              } else {
+                const uint32_t shifted = __funnelshift_r(w, __shfl_down_sync(0xffffffffu, w, 1), 16);  // elements 2 lane + 1, 2 lane + 2
+                if (lane < 31 && 2 * lane + 2 < n_cols) *reinterpret_cast<uint32_t*>(dst + 2 * lane + 1) = shifted;
+                else if (2 * lane + 1 < n_cols) reinterpret_cast<uint16_t*>(dst)[2 * lane + 1] = (uint16_t)shifted;
+                if (lane == 0) reinterpret_cast<uint16_t*>(dst)[0] = (uint16_t)w;
+              }
+            }
+            continue;
+          }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
@@ -930,10 +959,13 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
                            reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.col_sum)) & 15) == 0;
   // The staged epilogue reads bias and residual one 16-byte group at a time, and a TMA store clips a row at 16-byte
   // granularity: with a ragged N it writes zeros into the columns up to the next multiple of 16 bytes. So a ragged N takes
-  // this route only without bias/residual and when the caller declared those columns scratch (p.tma_store on entry).
-  q.tma_store = (BN >= 64 && aligned16 && p.ldo % EA == 0 && (p.N % EA == 0 || (p.epilogue == TTB_EPI_NONE && p.tma_store && !p.out_lo)) &&
-                 (!p.residual || p.ldr % EA == 0)) ? 1 : 0;
-  if (q.tma_store) {
+  // this route only without bias/residual and when the caller declared those columns scratch (p.staged on entry).
+  const bool tma = BN >= 64 && aligned16 && p.ldo % EA == 0 && (p.N % EA == 0 || (p.epilogue == TTB_EPI_NONE && p.staged == STORE_TMA && !p.out_lo)) &&
+                   (!p.residual || p.ldr % EA == 0);
+  // Ragged or misaligned rows without bias, residual or second plane (a 50257-wide vocabulary): word stores.
+  const bool words = BN >= 64 && !tma && p.epilogue == TTB_EPI_NONE && !p.out_lo;
+  q.staged = tma ? STORE_TMA : (words ? STORE_WORDS : STORE_DIRECT);
+  if (tma) {
     s = make_map(ctx, &tmO, out_kind<OutT>(), p.out, p.M, p.N, p.ldo, 32);
     if (s) return s;
     if (p.out_lo && (s = make_map(ctx, &tmO2, out_kind<OutT>(), p.out_lo, p.M, p.N, p.ldo, 32))) return s;
@@ -1032,7 +1064,7 @@ int launch_tc_ln(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   if ((s = make_map(ctx, &tmB0, KIND, op.W, p.N, p.K, p.K, TWO ? BN / 2 : BN))) return s;
   if ((s = make_map(ctx, &tmO, out_kind<OutT>(), p.out, p.M, p.N, p.ldo, 32))) return s;
   GemmParams q = p;
-  q.tma_store = 1;
+  q.staged = STORE_TMA;
   q.ln_partials = static_cast<float2*>(ctx->ln_ws);
   q.ln_rows = (long long)ctx->ln_ws_rows;
   q.ln_counters = reinterpret_cast<int*>(static_cast<char*>(ctx->ln_ws) + 2 * kLnMaxTiles * ctx->ln_ws_rows * sizeof(float2));
@@ -1386,7 +1418,7 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   p.pass_b = a->W2 ? 4 : 0;
   p.out = a->out; p.ldo = a->ldo; p.out_lo = a->out_lo;
   p.bias = a->bias; p.residual = a->residual; p.ldr = a->ldr;
-  p.epilogue = epilogue; p.tma_store = pad_scratch; p.split_k = 1; p.status = ctx->d_status;
+  p.epilogue = epilogue; p.staged = pad_scratch ? STORE_TMA : STORE_DIRECT; p.split_k = 1; p.status = ctx->d_status;
   const Operands op{a->A, a->A2, a->lda, a->W, a->W2};
   if (dt == TTB_F32) return pick_tile<KIND_TF32, float>(ctx, op, p);
   if (dt == TTB_F16) return odt == TTB_F32 ? pick_tile<KIND_F16, float>(ctx, op, p) : pick_tile<KIND_F16, __half>(ctx, op, p);
