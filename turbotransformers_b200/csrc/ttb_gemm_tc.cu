@@ -1,12 +1,13 @@
 // Tensor-core Linear for sm_100a: out[M,N] = epilogue(sum over passes of A_p[M,K] . W_p[N,K]^T).
 //
-// One persistent CTA (or CTA pair) per SM, 320 or 352 threads in three roles:
+// One persistent CTA (or CTA pair) per SM, 320 to 384 threads in three roles:
 //   warp 0      : TMA producer  - cp.async.bulk.tensor loads of 128-byte-swizzled K-major tiles into a
 //                 shared-memory ring, completion signalled on "full" mbarriers
 //   warp 1      : MMA issuer    - one elected thread issues tcgen05.mma (128 x BN x 32 bytes of K per instruction)
 //                 from shared-memory descriptors into a TMEM accumulator; tcgen05.commit releases ring
 //                 slots ("empty" mbarriers) and publishes finished accumulators ("tmem_full")
 //   warp 10     : second issuer on tiles of up to 128 columns, with an accumulator of its own (every other k-block)
+//   warp 11     : second producer on tiles of up to 64 columns, which loads W while warp 0 loads A
 //   warps 2..9  : epilogue      - tcgen05.ld the accumulator (one row per thread), apply scale/bias/activation/
 //                 residual in fp32, convert, stage through a swizzled shared-memory tile and TMA-store it
 // Two accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the MMAs of tile i+1.
@@ -56,8 +57,11 @@ template <int BN, bool TWO = false, bool SK = false> struct Cfg {
   static constexpr int STAGES = SK ? 4 : (TWO ? 6 : ((BN == 256) ? 4 : (BN == 128 ? 6 : 8)));
   // Two MMA-issuing warps with an accumulator each (even and odd k-blocks) wherever a k-block's MMAs are short: see the issuer.
   static constexpr int ISSUERS = (!TWO && BN <= 128) ? 2 : 1;
-  static constexpr int THREADS = kThreads + 32 * (ISSUERS - 1);
+  // Two TMA-issuing warps, one per operand, on the narrowest tiles: see the producer.
+  static constexpr int PRODUCERS = (!TWO && BN <= 64) ? 2 : 1;
+  static constexpr int THREADS = kThreads + 32 * (ISSUERS - 1) + 32 * (PRODUCERS - 1);
   static constexpr int TMEM_COLS = 2 * ISSUERS * BN;
+  static_assert(PRODUCERS == 1 || ISSUERS == 2, "warp numbers: 10 issues, 11 loads");
   static_assert(STAGES % ISSUERS == 0 && TMEM_COLS >= 32 && TMEM_COLS <= 512, "ring slots divide evenly among the issuers; TMEM allocation");
   // Epilogue staging: per epilogue warp one [32 rows x 128 B] swizzled tile that its TMA stores read (BN >= 64 only).
   static constexpr int STAGING_BYTES = (BN >= 64) ? 8 * 4096 : 0;
@@ -73,6 +77,7 @@ enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
 
 struct GemmParams {
   int M, N, K;             // K in elements, per pass
+  int a_rows;              // single CTAs: rows of A that a tile's load brings (fewer than BM when M is smaller; the rest is never read back)
   int npass;               // 1..3 passes over K into one accumulator
   int pass_a, pass_b;      // bit p set: pass p reads the second A map / the second W map
   void* out;
@@ -218,7 +223,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   }
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
+      mbar_init(full_bar(s), C::PRODUCERS);
       mbar_init(empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -267,8 +272,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   }
   pdl_wait();  // everything above ran in the shadow of the previous kernel; its results are visible from here on
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp == 0 || (C::PRODUCERS == 2 && warp == 11)) {
+    // ------------------------------------------------------------------ TMA producer(s)
+    // One thread's wait, byte count and two loads take about 320 cycles a k-block, which is what paces tiles of up to 64
+    // columns (a deeper ring changes nothing). With a warp per operand, us: 792 x 768 x 3072 fp16 13.0 -> 12.3, 128 x 2304 x 768
+    // 5.3 -> 5.1, fp32 520 x 768 x 3072 56.2 -> 51.2. Tiles of 128 columns are slower that way (15.2 -> 15.6).
+    const bool load_a = warp == 0, load_b = C::PRODUCERS == 1 || warp != 0;
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
@@ -287,9 +296,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             tma_load_2d_pair(a_dst, ma, full_bar(stage), kk * BK_ELEMS, m_blk * TILE_M + (int)rank * BM);
             tma_load_2d_pair(a_dst + C::A_BYTES, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN + (int)rank * (BN / 2));
           } else {
-            mbar_expect_tx(full_bar(stage), (uint32_t)C::STAGE_BYTES);
-            tma_load_2d(a_dst, ma, full_bar(stage), kk * BK_ELEMS, m_blk * BM);
-            tma_load_2d(a_dst + C::A_BYTES, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN);
+            mbar_expect_tx(full_bar(stage), (load_a ? (uint32_t)(p.a_rows * BK_BYTES) : 0u) + (load_b ? (uint32_t)C::B_BYTES : 0u));
+            if (load_a) tma_load_2d(a_dst, ma, full_bar(stage), kk * BK_ELEMS, m_blk * BM);
+            if (load_b) tma_load_2d(a_dst + C::A_BYTES, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN);
           }
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
           if (++kk == num_kb) { kk = 0; ++pass; }
@@ -945,15 +954,18 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   constexpr int TILE_M = TWO ? 2 * BM : BM;
   constexpr int EA = (int)sizeof(OutT) == 4 ? 4 : 8;  // output elements per 16 bytes
   CUtensorMap tmA0, tmA1, tmB0, tmB1;
-  int s = make_map(ctx, &tmA0, KIND, op.A, p.M, p.K, op.lda, BM);
+  // a few rows (decoding): a box of 32 or 64 rows, so that a slot is not filled up with zeros first
+  const int a_rows = (TWO || p.M > 64) ? BM : (p.M > 32 ? 64 : 32);
+  int s = make_map(ctx, &tmA0, KIND, op.A, p.M, p.K, op.lda, a_rows);
   if (s) return s;
   tmA1 = tmA0;
-  if (op.A2 && (s = make_map(ctx, &tmA1, KIND, op.A2, p.M, p.K, op.lda, BM))) return s;
+  if (op.A2 && (s = make_map(ctx, &tmA1, KIND, op.A2, p.M, p.K, op.lda, a_rows))) return s;
   s = make_map(ctx, &tmB0, KIND, op.W, p.N, p.K, p.K, TWO ? BN / 2 : BN);
   if (s) return s;
   tmB1 = tmB0;
   if (op.W2 && (s = make_map(ctx, &tmB1, KIND, op.W2, p.N, p.K, p.K, TWO ? BN / 2 : BN))) return s;
   GemmParams q = p;
+  q.a_rows = a_rows;
   CUtensorMap tmO = tmA0, tmO2 = tmA0;  // placeholders when the direct-store epilogue is used
   const bool aligned16 = ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.out_lo) | reinterpret_cast<uintptr_t>(p.bias) |
                            reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.col_sum)) & 15) == 0;
@@ -1065,6 +1077,7 @@ int launch_tc_ln(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   if ((s = make_map(ctx, &tmO, out_kind<OutT>(), p.out, p.M, p.N, p.ldo, 32))) return s;
   GemmParams q = p;
   q.staged = STORE_TMA;
+  q.a_rows = BM;
   q.ln_partials = static_cast<float2*>(ctx->ln_ws);
   q.ln_rows = (long long)ctx->ln_ws_rows;
   q.ln_counters = reinterpret_cast<int*>(static_cast<char*>(ctx->ln_ws) + 2 * kLnMaxTiles * ctx->ln_ws_rows * sizeof(float2));
@@ -1206,8 +1219,8 @@ int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
   if (pair_mode() && pair_pays) consider(0, expect(7300, 310, 5400, pair_tiles, sms / 2, total_kb));
   consider(256, expect(6300, 350, 6000, tiles(256), sms, total_kb));
   consider(128, expect(3500, 235, 4300, tiles(128), sms, total_kb));
-  consider(64, expect(3800, 190, 3000, tiles(64), sms, total_kb));
-  consider(32, expect(3900, 165, 2000, tiles(32), sms, total_kb));
+  consider(64, expect(3800, 177, 3000, tiles(64), sms, total_kb));
+  consider(32, expect(3900, 155, 2000, tiles(32), sms, total_kb));
   // Few 128 x 32 tiles and a mainloop of several k-blocks: the CTAs of a cluster may share each tile's K range, so that the
   // weights stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per
   // tile, 8.7 split four ways; 12 k-blocks are not worth the exchange.
@@ -1220,7 +1233,7 @@ int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
     // they pack into its GPCs
     while (s >= 2 && t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, (int)s)) --s;
     if (s >= 2) {
-      consider(1, expect(6900, 165, 2000, t32, t32, (total_kb + s - 1) / s));
+      consider(1, expect(6900, 155, 2000, t32, t32, (total_kb + s - 1) / s));
       if (best == 1) {
         p.split_k = (int)s;
         return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
