@@ -56,6 +56,8 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float (&f)[8], const _
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 kv_append_kernel(const T* __restrict__ qkv, int B, int n_new, int H, T* __restrict__ kc, T* __restrict__ vc, int past_len) {
+  pdl_trigger();
+  pdl_wait();
   // one 16-byte chunk of one K row and of one V row per thread
   const int chunks = H / 8;
   const long long total = (long long)B * n_new * chunks;
@@ -77,6 +79,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 5)
 attention_decode_kernel(const T* __restrict__ qkv, int B, int n_new, int heads, T* __restrict__ kc, T* __restrict__ vc, int past_len,
                         float scale, T* __restrict__ out, float* __restrict__ partial, int splits) {
+  pdl_trigger();
+  pdl_wait();
   const int h = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
   const int H = heads * D;
   const int tid = threadIdx.x, lane = tid & 31, sub = lane & 7, group = tid >> 3;
@@ -198,6 +202,8 @@ attention_decode_kernel(const T* __restrict__ qkv, int B, int n_new, int heads, 
 template <typename T>
 __global__ void __launch_bounds__(128)
 decode_merge_kernel(const float* __restrict__ partial, int rows_heads, int splits, int heads, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= rows_heads) return;
   const float* p = partial + (long long)item * splits * kPartial;
@@ -241,10 +247,10 @@ extern "C" int ttb_kv_cache_append(ttb_ctx* ctx, int dtype, const void* qkv, int
   const long long total = B * n_new * (H / 8);
   const int grid = (int)std::min<long long>((total + kThreads - 1) / kThreads, (long long)ctx->sm_count * 16);
   if (dtype == TTB_F16)
-    kv_append_kernel<__half><<<grid, kThreads, 0, ctx->stream>>>((const __half*)qkv, (int)B, (int)n_new, H, (__half*)k_cache, (__half*)v_cache,
+    launch_pdl(kv_append_kernel<__half>, dim3(grid), dim3(kThreads), 0, ctx->stream, (const __half*)qkv, (int)B, (int)n_new, H, (__half*)k_cache, (__half*)v_cache,
                                                                   (int)past_len);
   else
-    kv_append_kernel<__nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16*)qkv, (int)B, (int)n_new, H, (__nv_bfloat16*)k_cache,
+    launch_pdl(kv_append_kernel<__nv_bfloat16>, dim3(grid), dim3(kThreads), 0, ctx->stream, (const __nv_bfloat16*)qkv, (int)B, (int)n_new, H, (__nv_bfloat16*)k_cache,
                                                                          (__nv_bfloat16*)v_cache, (int)past_len);
   return launched(ctx, "kv_cache_append");
 }
@@ -272,15 +278,15 @@ extern "C" int ttb_attention_decode(ttb_ctx* ctx, int dtype, const void* qkv, in
   dim3 grid((unsigned)heads, (unsigned)B, (unsigned)splits);
   const int items = (int)(B * n_new * heads);
   if (dtype == TTB_F16) {
-    attention_decode_kernel<__half><<<grid, kThreads, 0, ctx->stream>>>((const __half*)qkv, (int)B, (int)n_new, (int)heads, (__half*)k_cache,
+    launch_pdl(attention_decode_kernel<__half>, dim3(grid), dim3(kThreads), 0, ctx->stream, (const __half*)qkv, (int)B, (int)n_new, (int)heads, (__half*)k_cache,
                                                                          (__half*)v_cache, (int)past_len, scale, (__half*)out, partial, splits);
-    if (splits > 1) decode_merge_kernel<__half><<<(items + 3) / 4, 128, 0, ctx->stream>>>(partial, items, splits, (int)heads, (__half*)out);
+    if (splits > 1) launch_pdl(decode_merge_kernel<__half>, dim3((items + 3) / 4), dim3(128), 0, ctx->stream, partial, items, splits, (int)heads, (__half*)out);
   } else {
-    attention_decode_kernel<__nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16*)qkv, (int)B, (int)n_new, (int)heads,
+    launch_pdl(attention_decode_kernel<__nv_bfloat16>, dim3(grid), dim3(kThreads), 0, ctx->stream, (const __nv_bfloat16*)qkv, (int)B, (int)n_new, (int)heads,
                                                                                 (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (int)past_len,
                                                                                 scale, (__nv_bfloat16*)out, partial, splits);
     if (splits > 1)
-      decode_merge_kernel<__nv_bfloat16><<<(items + 3) / 4, 128, 0, ctx->stream>>>(partial, items, splits, (int)heads, (__nv_bfloat16*)out);
+      launch_pdl(decode_merge_kernel<__nv_bfloat16>, dim3((items + 3) / 4), dim3(128), 0, ctx->stream, partial, items, splits, (int)heads, (__nv_bfloat16*)out);
   }
   s = launched(ctx, "attention_decode");
   if (partial) {

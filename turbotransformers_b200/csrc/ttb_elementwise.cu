@@ -450,6 +450,8 @@ __global__ void __launch_bounds__(kRowsPerBlock * 32)
 layernorm_rows_generic_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
                               const TOut* __restrict__ beta, TOut* out, TOut* __restrict__ out_lo, float* __restrict__ out_f32, int64_t M,
                               int N, float eps) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int warps_total = gridDim.x * kRowsPerBlock;
   for (int64_t row = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); row < M; row += warps_total) {
@@ -568,7 +570,7 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   else if (aligned && N <= 1024) LN_CASE(4);
   else if (aligned && N <= 2048) LN_CASE(8);
   else
-    layernorm_rows_generic_kernel<TIn, TOut, ADD><<<grid_for(M, kRowsPerBlock, ctx->sm_count), kRowsPerBlock * 32, 0, ctx->stream>>>(
+    launch_pdl(layernorm_rows_generic_kernel<TIn, TOut, ADD>, dim3(grid_for(M, kRowsPerBlock, ctx->sm_count)), dim3(kRowsPerBlock * 32), 0, ctx->stream, 
         x, residual, bias, gamma, beta, out, out_lo, out_f32, M, (int)N, eps);
 #undef LN_CASE
   return launched(ctx, "layernorm");
@@ -586,6 +588,8 @@ template <int ACT> __device__ __forceinline__ float apply_act(float x) {
 template <typename T, int ACT, bool VEC>
 __global__ void __launch_bounds__(256)
 add_bias_act_kernel(T* __restrict__ out, const T* __restrict__ bias, int64_t M, int N) {
+  pdl_trigger();
+  pdl_wait();
   if (VEC) {
     const int64_t nvec = M * (int64_t)(N / 8);
     const int per_row = N / 8;
@@ -610,6 +614,8 @@ template <typename T, bool ADD_INPUT>
 __global__ void __launch_bounds__(256)
 add_bias_kernel(const T* __restrict__ in1, const T* __restrict__ in2, const T* __restrict__ bias, T* __restrict__ out,
                 int64_t M, int N) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t n = M * (int64_t)N;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float a = to_f(in1[i]) + to_f(bias[i % N]);
@@ -625,6 +631,8 @@ template <typename T, bool ADD>
 __global__ void __launch_bounds__(256)
 lookup_kernel(T* __restrict__ out, const T* __restrict__ table, const int64_t* __restrict__ ids, int64_t n_ids,
               int hidden, int64_t vocab, int* status) {
+  pdl_trigger();
+  pdl_wait();
   for (int64_t r = blockIdx.x; r < n_ids; r += gridDim.x) {
     int64_t id = ids[r];
     if (id < 0 || id >= vocab) {
@@ -656,6 +664,8 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
                     const T* __restrict__ token_type, const T* __restrict__ gamma, const T* __restrict__ beta,
                     int hidden, int64_t vocab, int64_t n_pos, int64_t n_types, float eps, T* __restrict__ out,
                     T* __restrict__ out_lo, float* __restrict__ out_f32, int* status) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int warps_total = gridDim.x * kRowsPerBlock;
   for (int64_t t = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); t < n_tokens; t += warps_total) {
@@ -778,6 +788,8 @@ embedding_ln16_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict
 // ------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void seq_pool_kernel(const T* __restrict__ in, int64_t B, int64_t L, int H, int type, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   for (int64_t b = blockIdx.x; b < B; b += gridDim.x) {
     for (int c = threadIdx.x; c < H; c += blockDim.x) {
       const T* base = in + b * L * H + c;
@@ -800,6 +812,8 @@ __global__ void seq_pool_kernel(const T* __restrict__ in, int64_t B, int64_t L, 
 template <typename T>
 __global__ void seq_pool_varlen_kernel(const T* __restrict__ in, const int32_t* __restrict__ cu, int64_t B, int H,
                                        int type, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   for (int64_t b = blockIdx.x; b < B; b += gridDim.x) {
     const int64_t lo = cu[b], hi = cu[b + 1];
     for (int c = threadIdx.x; c < H; c += blockDim.x) {
@@ -822,6 +836,8 @@ __global__ void seq_pool_varlen_kernel(const T* __restrict__ in, const int32_t* 
 __global__ void prepare_masks_kernel(int64_t B, int64_t L, const int64_t* __restrict__ mask_in,
                                      int64_t* __restrict__ mask_out, int64_t* __restrict__ type_out,
                                      int64_t* __restrict__ pos_out, float* __restrict__ ext_out) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t n = B * L;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t m = mask_in ? mask_in[i] : 1;
@@ -843,6 +859,8 @@ __global__ void __launch_bounds__(256)
 split_add_bias_transpose_kernel(const T* __restrict__ qkv, const T* __restrict__ bias, const int32_t* __restrict__ cu,
                                 int64_t B, int64_t L, int heads, int d, T* __restrict__ q, T* __restrict__ k,
                                 T* __restrict__ v) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t H = (int64_t)heads * d;
   const int64_t n = B * L * 3 * H;  // over the padded output index space
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -870,6 +888,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 transpose_for_score_kernel(const T* __restrict__ in, const int32_t* __restrict__ cu, int64_t B, int64_t L, int heads,
                            int d, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t H = (int64_t)heads * d;
   const int64_t n = B * L * H;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -893,6 +913,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 add_bias_transpose_kernel(const T* __restrict__ in, const T* __restrict__ bias, const int32_t* __restrict__ cu, int64_t B,
                           int64_t L, int heads, int d, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t H = (int64_t)heads * d;
   const int64_t n = B * L * H;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -920,6 +942,8 @@ template <typename T>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
 mask_softmax_kernel(T* __restrict__ scores, const float* __restrict__ mask, int64_t B, int heads, int64_t Lq,
                     int64_t Lk, float scale, int is_2d) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t rows = B * heads * Lq;
   const int warps_total = gridDim.x * kRowsPerBlock;
@@ -1286,8 +1310,8 @@ extern "C" int ttb_add_bias_act(ttb_ctx* ctx, int dtype, void* out, const void* 
   const bool vec = N % 8 == 0 && (reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(bias)) % 16 == 0;
   const int grid = grid_for(vec ? M * N / 8 : M * N, 256, ctx->sm_count);
 #define ACT_CASE(A)                                                                                    \
-  if (vec) add_bias_act_kernel<T, A, true><<<grid, 256, 0, ctx->stream>>>((T*)out, (const T*)bias, M, (int)N); \
-  else add_bias_act_kernel<T, A, false><<<grid, 256, 0, ctx->stream>>>((T*)out, (const T*)bias, M, (int)N)
+  if (vec) launch_pdl(add_bias_act_kernel<T, A, true>, dim3(grid), dim3(256), 0, ctx->stream, (T*)out, (const T*)bias, M, (int)N); \
+  else launch_pdl(add_bias_act_kernel<T, A, false>, dim3(grid), dim3(256), 0, ctx->stream, (T*)out, (const T*)bias, M, (int)N)
   TTB_DISPATCH_FLOAT(ctx, dtype, T, {
     if (act == TTB_ACT_GELU) { ACT_CASE(TTB_ACT_GELU); }
     else if (act == TTB_ACT_TANH) { ACT_CASE(TTB_ACT_TANH); }
@@ -1305,7 +1329,7 @@ extern "C" int ttb_add_bias(ttb_ctx* ctx, int dtype, void* out, const void* bias
   DeviceGuard g(ctx->device);
   const int grid = grid_for(M * N, 256, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (add_bias_kernel<T, false><<<grid, 256, 0, ctx->stream>>>((const T*)out, nullptr, (const T*)bias, (T*)out, M, (int)N)));
+                     (launch_pdl(add_bias_kernel<T, false>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)out, nullptr, (const T*)bias, (T*)out, M, (int)N)));
   return launched(ctx, "add_bias");
 }
 
@@ -1318,7 +1342,7 @@ extern "C" int ttb_add_input_bias(ttb_ctx* ctx, int dtype, const void* in1, cons
   DeviceGuard g(ctx->device);
   const int grid = grid_for(M * N, 256, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (add_bias_kernel<T, true><<<grid, 256, 0, ctx->stream>>>((const T*)in1, (const T*)in2, (const T*)bias, (T*)out, M, (int)N)));
+                     (launch_pdl(add_bias_kernel<T, true>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)in1, (const T*)in2, (const T*)bias, (T*)out, M, (int)N)));
   return launched(ctx, "add_input_bias");
 }
 
@@ -1332,8 +1356,8 @@ extern "C" int ttb_lookup_embedding(ttb_ctx* ctx, int dtype, void* out, const vo
   const int grid = (int)(n_ids < (int64_t)ctx->sm_count * 16 ? n_ids : (int64_t)ctx->sm_count * 16);
   const int block = hidden >= 256 ? 256 : 128;
   TTB_DISPATCH_FLOAT(ctx, dtype, T, {
-    if (add) lookup_kernel<T, true><<<grid, block, 0, ctx->stream>>>((T*)out, (const T*)table, ids, n_ids, (int)hidden, vocab, ctx->d_status);
-    else lookup_kernel<T, false><<<grid, block, 0, ctx->stream>>>((T*)out, (const T*)table, ids, n_ids, (int)hidden, vocab, ctx->d_status);
+    if (add) launch_pdl(lookup_kernel<T, true>, dim3(grid), dim3(block), 0, ctx->stream, (T*)out, (const T*)table, ids, n_ids, (int)hidden, vocab, ctx->d_status);
+    else launch_pdl(lookup_kernel<T, false>, dim3(grid), dim3(block), 0, ctx->stream, (T*)out, (const T*)table, ids, n_ids, (int)hidden, vocab, ctx->d_status);
   });
   return launched(ctx, "lookup_embedding");
 }
@@ -1382,7 +1406,7 @@ extern "C" int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* i
     return launched(ctx, "embedding_ln");
   }
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (embedding_ln_kernel<T><<<grid, kRowsPerBlock * 32, 0, ctx->stream>>>(
+                     (launch_pdl(embedding_ln_kernel<T>, dim3(grid), dim3(kRowsPerBlock * 32), 0, ctx->stream, 
                          ids, position_ids, token_type_ids, cu_seqlens, (int)B, (int)(seq_len > 0 ? seq_len : 1), n_tokens,
                          (const T*)word, (const T*)position, (const T*)token_type, (const T*)gamma, (const T*)beta,
                          (int)hidden, vocab, n_positions, n_types, eps, (T*)out, (T*)out_lo, out_f32, ctx->d_status)));
@@ -1398,7 +1422,7 @@ extern "C" int ttb_seq_pool(ttb_ctx* ctx, int dtype, const void* in, int64_t B, 
   TTB_REQUIRE(ctx, in && out, "seq_pool: null pointer");
   DeviceGuard g(ctx->device);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (seq_pool_kernel<T><<<(int)(B < 65535 ? B : 65535), 256, 0, ctx->stream>>>((const T*)in, B, L, (int)H, pool_type, (T*)out)));
+                     (launch_pdl(seq_pool_kernel<T>, dim3((int)(B < 65535 ? B : 65535)), dim3(256), 0, ctx->stream, (const T*)in, B, L, (int)H, pool_type, (T*)out)));
   return launched(ctx, "seq_pool");
 }
 
@@ -1411,7 +1435,7 @@ extern "C" int ttb_seq_pool_varlen(ttb_ctx* ctx, int dtype, const void* in, cons
   TTB_REQUIRE(ctx, in && out && cu_seqlens, "seq_pool_varlen: null pointer");
   DeviceGuard g(ctx->device);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (seq_pool_varlen_kernel<T><<<(int)(B < 65535 ? B : 65535), 256, 0, ctx->stream>>>((const T*)in, cu_seqlens, B, (int)H, pool_type, (T*)out)));
+                     (launch_pdl(seq_pool_varlen_kernel<T>, dim3((int)(B < 65535 ? B : 65535)), dim3(256), 0, ctx->stream, (const T*)in, cu_seqlens, B, (int)H, pool_type, (T*)out)));
   return launched(ctx, "seq_pool_varlen");
 }
 
@@ -1422,7 +1446,7 @@ extern "C" int ttb_prepare_bert_masks(ttb_ctx* ctx, int64_t B, int64_t L, const 
   TTB_REQUIRE(ctx, B >= 0 && L >= 0, "prepare_bert_masks: bad shape");
   if (B * L == 0) return TTB_OK;
   DeviceGuard g(ctx->device);
-  prepare_masks_kernel<<<grid_for(B * L, 256, ctx->sm_count), 256, 0, ctx->stream>>>(B, L, att_mask_in, att_mask_out, token_type_out,
+  launch_pdl(prepare_masks_kernel, dim3(grid_for(B * L, 256, ctx->sm_count)), dim3(256), 0, ctx->stream, B, L, att_mask_in, att_mask_out, token_type_out,
                                                                                       position_ids_out, extended_out);
   return launched(ctx, "prepare_bert_masks");
 }
@@ -1449,7 +1473,7 @@ extern "C" int ttb_split_add_bias_transpose_pad(ttb_ctx* ctx, int dtype, const v
   DeviceGuard g(ctx->device);
   const int grid = grid_for(B * maxL * 3 * heads * d, 256, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (split_add_bias_transpose_kernel<T><<<grid, 256, 0, ctx->stream>>>((const T*)qkv, (const T*)bias, cu_seqlens, B, maxL,
+                     (launch_pdl(split_add_bias_transpose_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)qkv, (const T*)bias, cu_seqlens, B, maxL,
                                                                                       (int)heads, (int)d, (T*)q, (T*)k, (T*)v)));
   return launched(ctx, "split_add_bias_transpose");
 }
@@ -1469,7 +1493,7 @@ extern "C" int ttb_transpose_for_score_pad(ttb_ctx* ctx, int dtype, const void* 
   DeviceGuard g(ctx->device);
   const int grid = grid_for(B * maxL * heads * d, 256, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (transpose_for_score_kernel<T><<<grid, 256, 0, ctx->stream>>>((const T*)in, cu_seqlens, B, maxL, (int)heads, (int)d, (T*)out)));
+                     (launch_pdl(transpose_for_score_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)in, cu_seqlens, B, maxL, (int)heads, (int)d, (T*)out)));
   return launched(ctx, "transpose_for_score");
 }
 
@@ -1489,7 +1513,7 @@ extern "C" int ttb_add_bias_transpose_for_score_pad(ttb_ctx* ctx, int dtype, con
   DeviceGuard g(ctx->device);
   const int grid = grid_for(B * maxL * heads * d, 256, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (add_bias_transpose_kernel<T><<<grid, 256, 0, ctx->stream>>>((const T*)in, (const T*)bias, cu_seqlens, B, maxL, (int)heads,
+                     (launch_pdl(add_bias_transpose_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)in, (const T*)bias, cu_seqlens, B, maxL, (int)heads,
                                                                                 (int)d, (T*)out)));
   return launched(ctx, "add_bias_transpose_for_score");
 }
@@ -1503,7 +1527,7 @@ extern "C" int ttb_mask_softmax(ttb_ctx* ctx, int dtype, void* scores, const flo
   DeviceGuard g(ctx->device);
   const int grid = grid_for(B * heads * Lq, kRowsPerBlock, ctx->sm_count);
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (mask_softmax_kernel<T><<<grid, kRowsPerBlock * 32, 0, ctx->stream>>>((T*)scores, mask, B, (int)heads, Lq, Lk, scale, mask_is_2d)));
+                     (launch_pdl(mask_softmax_kernel<T>, dim3(grid), dim3(kRowsPerBlock * 32), 0, ctx->stream, (T*)scores, mask, B, (int)heads, Lq, Lk, scale, mask_is_2d)));
   return launched(ctx, "mask_softmax");
 }
 

@@ -24,6 +24,8 @@ template <typename T, int BM, int BN, int TM, int TN, int BK>
 __global__ void __launch_bounds__(256, 2)
 gemm_simt_kernel(const T* __restrict__ A, int a_trans, const T* __restrict__ B, int b_trans, T* __restrict__ C, int M,
                  int N, int K, float alpha, float beta, int64_t strideA, int64_t strideB, int64_t strideC) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int kPad = BM == 32 ? 1 : 4;  // odd row pitch: the 32 k values a warp stages for one row land in 32 banks
   __shared__ float As[BK][BM + kPad];
   __shared__ float Bs[BK][BN + kPad];
@@ -148,6 +150,8 @@ __global__ void __launch_bounds__(256, LBM == 64 ? 3 : 2)
 gemm_simt_large_kernel(const T* __restrict__ A, int a_trans, const T* __restrict__ B, int b_trans, T* __restrict__ C, int M,
                        int N, int K, float alpha, float beta, int64_t strideA, int64_t strideB, int64_t strideC, int vec_a,
                        int vec_b, int vec_c, int splits, int k_chunk, float* __restrict__ partial) {
+  pdl_trigger();
+  pdl_wait();
   // splits > 1 (split-K, for problems with too few tiles to fill the GPU): blockIdx.z = batch * splits + s, this CTA sums
   // k in [s * k_chunk, (s + 1) * k_chunk) and writes its raw fp32 sums to partial[s][batch][M][N]; splitk_reduce_kernel adds
   // the slices in increasing s and applies alpha / beta.
@@ -290,6 +294,8 @@ gemm_simt_large_kernel(const T* __restrict__ A, int a_trans, const T* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ partial, int splits, int64_t total, float alpha, float beta, T* __restrict__ C) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (idx >= total) return;
   float s = 0.f;
@@ -335,13 +341,13 @@ int run(ttb_ctx* ctx, int dtype, const void* A, int a_trans, const void* B, int 
     if (s) return s;
     dim3 grid((unsigned)n128, (unsigned)((M + 63) / 64), (unsigned)(batch * splits));
     TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                       (gemm_simt_large_kernel<T, 64><<<grid, 256, 0, ctx->stream>>>((const T*)A, a_trans, (const T*)B, b_trans, (T*)C, (int)M, (int)N,
+                       (launch_pdl(gemm_simt_large_kernel<T, 64>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)A, a_trans, (const T*)B, b_trans, (T*)C, (int)M, (int)N,
                                                                                     (int)K, alpha, beta, M * K, K * N, M * N, vec_a, vec_b, 0, splits,
                                                                                     k_chunk, (float*)ws)));
     s = launched(ctx, what);
     if (!s) {
       TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                         (splitk_reduce_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>((const float*)ws, splits, total, alpha, beta,
+                         (launch_pdl(splitk_reduce_kernel<T>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, ctx->stream, (const float*)ws, splits, total, alpha, beta,
                                                                                                            (T*)C)));
       s = launched(ctx, what);
     }
@@ -356,7 +362,7 @@ int run(ttb_ctx* ctx, int dtype, const void* A, int a_trans, const void* B, int 
     dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)nb);
     if (small) {
       TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                         (gemm_simt_kernel<T, 32, 32, 2, 2, 64><<<grid, 256, 0, ctx->stream>>>((const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
+                         (launch_pdl(gemm_simt_kernel<T, 32, 32, 2, 2, 64>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
                                                                                           b_trans, (T*)C + b0 * M * N, (int)M, (int)N, (int)K,
                                                                                           alpha, beta, M * K, K * N, M * N)));
     } else if (large || medium) {
@@ -368,18 +374,18 @@ int run(ttb_ctx* ctx, int dtype, const void* A, int a_trans, const void* B, int 
       const int vec_c = f32 && al16(C) && N % 4 == 0;
       if (large) {
         TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                           (gemm_simt_large_kernel<T, 128><<<grid, 256, 0, ctx->stream>>>((const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
+                           (launch_pdl(gemm_simt_large_kernel<T, 128>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
                                                                                          b_trans, (T*)C + b0 * M * N, (int)M, (int)N, (int)K, alpha,
                                                                                          beta, M * K, K * N, M * N, vec_a, vec_b, vec_c, 1, (int)K, nullptr)));
       } else {
         TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                           (gemm_simt_large_kernel<T, 64><<<grid, 256, 0, ctx->stream>>>((const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
+                           (launch_pdl(gemm_simt_large_kernel<T, 64>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
                                                                                         b_trans, (T*)C + b0 * M * N, (int)M, (int)N, (int)K, alpha,
                                                                                         beta, M * K, K * N, M * N, vec_a, vec_b, vec_c, 1, (int)K, nullptr)));
       }
     } else {
       TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                         (gemm_simt_kernel<T, 64, 64, 4, 4, 16><<<grid, 256, 0, ctx->stream>>>((const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
+                         (launch_pdl(gemm_simt_kernel<T, 64, 64, 4, 4, 16>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)A + b0 * M * K, a_trans, (const T*)B + b0 * K * N,
                                                                                           b_trans, (T*)C + b0 * M * N, (int)M, (int)N, (int)K,
                                                                                           alpha, beta, M * K, K * N, M * N)));
     }

@@ -1386,6 +1386,8 @@ __device__ __forceinline__ float round_tf32(float x) {
   return __uint_as_float(u);
 }
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ hi, float* __restrict__ lo) {
+  pdl_trigger();
+  pdl_wait();
   // x may alias hi (in-place split of a weight): each element is read before it is written, by the same thread
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
     if (i + 4 <= n) {
@@ -1600,6 +1602,6 @@ extern "C" int ttb_split_tf32(ttb_ctx* ctx, const float* x, int64_t n, float* hi
   DeviceGuard g(ctx->device);
   const int64_t want = (n / 4 + 255) / 256 + 1;
   const int grid = (int)(want < (int64_t)ctx->sm_count * 16 ? want : (int64_t)ctx->sm_count * 16);
-  split_tf32_kernel<<<grid, 256, 0, ctx->stream>>>(x, n, hi, lo);
+  launch_pdl(split_tf32_kernel, dim3(grid), dim3(256), 0, ctx->stream, x, n, hi, lo);
   return launched(ctx, "split_tf32");
 }
