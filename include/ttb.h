@@ -331,6 +331,14 @@ int ttb_kv_cache_append(ttb_ctx* ctx, int dtype, const void* qkv, int64_t B, int
 int ttb_attention_decode(ttb_ctx* ctx, int dtype, const void* qkv, int64_t B, int64_t n_new, int64_t heads, int64_t d,
                          void* k_cache, void* v_cache, int64_t past_len, float scale, void* out);
 
+/* Cross attention of a decoder step, one query per sequence (the batch_gemm3 -> ApplyMaskAndSoftmax -> batch_gemm4 ->
+ * TransposeForScore sequence of multi_headed_attention.cpp:308-354 with a query length of 1).
+ *   q [B, heads*d] (bias already added), k and v [B, heads, Lk, d], mask fp32 [B, Lk] additive or NULL
+ *   probs [B, heads, 1, Lk] receives the probabilities, or NULL; out [B, heads*d]
+ * 1 <= Lk <= 1024; a head is a multiple of 16 bytes, at most 512. */
+int ttb_context_attention_step(ttb_ctx* ctx, int dtype, const void* q, const void* k, const void* v, const float* mask, int64_t B,
+                               int64_t heads, int64_t Lk, int64_t d, float scale, void* probs, void* out);
+
 /* BERTEmbedding::operator() (layers/bert_embedding.cpp:24-65) in one pass: three gathers + LayerNorm.
  * ids is [n_tokens]. token_type_ids may be NULL (all 0). position_ids may be NULL: the position of token t is
  * then t - cu_seqlens[b] for the sequence b that owns it (packed batches, B+1 prefix sums), or t % seq_len

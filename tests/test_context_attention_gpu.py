@@ -11,6 +11,7 @@ import torch
 import turbotransformers_b200 as tt
 from oracle import ref_driver, restate
 from tests.helpers import TORCH_DT, rounded
+from turbotransformers_b200 import _capi
 
 pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
@@ -148,3 +149,39 @@ def test_smart_batch_context_attention_with_query_and_key_length_lists(dt, flags
     with pytest.raises(Exception, match="batch size"):
         att(K, V, Q, q_lens, k_lens[:2], **kw)
     assert tt._cxx_module.device_status(0) == 0
+
+
+# one key, counts on both sides of a pass of the lane groups (64, 32 and 16 keys) and the longest; lanes per key of 8, 16 and 32
+# with and without idle ones
+@pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("B,heads,Lk,d", [(1, 1, 1, 64), (3, 4, 63, 64), (2, 3, 65, 40), (5, 2, 200, 128), (1, 2, 1024, 64), (2, 2, 33, 96)])
+@pytest.mark.parametrize("mask_kind", ["none", "padding", "all_masked", "all_lowest", "all_inf"])
+def test_context_attention_step_kernel(ctx, dt, B, heads, Lk, d, mask_kind):
+    g = torch.Generator(device="cuda").manual_seed(Lk + d)
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").to(TORCH_DT[dt]) for s in ((B, heads, d), (B, heads, Lk, d), (B, heads, Lk, d)))
+    mask = None
+    if mask_kind != "none":
+        mask = torch.zeros(B, Lk, device="cuda")
+        fill = {"padding": -1e18, "all_masked": -1e18, "all_lowest": torch.finfo(torch.float32).min, "all_inf": -float("inf")}[mask_kind]
+        mask[-1, (Lk // 2 if mask_kind == "padding" else 0):] = fill
+    probs, out = torch.empty(B, heads, 1, Lk, dtype=q.dtype, device="cuda"), torch.empty(B, heads * d, dtype=q.dtype, device="cuda")
+    scale = d ** -0.5
+    ctx.call("context_attention_step", _capi.dtype_code(q.dtype), q, k, v, mask, B, heads, Lk, d, scale, probs, out)
+    s = (q.double()[:, :, None] @ k.double().transpose(-1, -2))[:, :, 0] * scale
+    want = torch.softmax(s + (mask.double()[:, None] if mask is not None else 0.0), -1)
+    want_out = (want[:, :, None] @ v.double())[:, :, 0]
+    # fp32 arithmetic (scores of order one over at most 128 terms), then one rounding to the type
+    eps = {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt]
+    for got, ref in ((probs[:, :, 0], want), (out.view(B, heads, d), want_out)):
+        assert torch.equal(got.isnan(), ref.isnan())
+        bound = (eps + 2e-6) * ref.abs().nan_to_num() + 2e-6 + (2.0 ** -24 if dt == "f16" else 0.0)
+        assert bool(((got.double() - ref).abs().nan_to_num() <= bound).all())
+
+
+def test_context_attention_step_refuses_what_it_does_not_take(ctx):
+    t = torch.zeros(4096, device="cuda", dtype=torch.float16)
+    for Lk, d in ((0, 64), (1025, 64), (8, 12), (8, 264)):
+        with pytest.raises(_capi.TTBError):
+            ctx.call("context_attention_step", _capi.F16, t, t, t, None, 1, 1, Lk, d, 1.0, None, t)
+    with pytest.raises(_capi.TTBError):
+        ctx.call("context_attention_step", _capi.F16, t[1:], t, t, None, 1, 1, 8, 64, 1.0, None, t)

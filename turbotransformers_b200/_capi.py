@@ -50,6 +50,7 @@ SIGNATURES = {
     "ttb_arena_release": (i32, [p, p]),
     "ttb_bytes_allocated_total": (i32, [p, p]),
     "ttb_kv_cache_append": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64]),
+    "ttb_context_attention_step": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64, f32, p, p]),
     "ttb_attention_decode": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64, f32, p]),
     "ttb_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, f32, f32, p]),
     "ttb_batch_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, i64, f32, f32, p]),

@@ -683,15 +683,23 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
     q_in = &normed;
   }
   lin.Reshape(x.dtype(), {T, H}, kDLCUDA, dev, "context/gemm0/q_out1/Reshape");
-  q_.Forward(*q_in, T, TTB_EPI_NONE, nullptr, lin.raw_mut(), is_trans_weight, "context/gemm0");
-  q.Reshape(x.dtype(), {B, heads, Lq, d}, kDLCUDA, dev, "context/AddBiasTransposeForScore/q_out2/Reshape");
-  Check(ttb_add_bias_transpose_for_score_pad(c, dt, lin.raw(), q_.bias().raw(), cu_q.get(), B, Lq, heads, d, q.raw_mut()), c,
-        "context/AddBiasTransposeForScore");
+  // One query per sequence (a decoder step): the whole attention is one kernel, which reads the projected rows as they are,
+  // up to the 1024 keys whose scores it keeps on the chip (translation memories are a few hundred at most).
+  const bool memory_filled = memory_keys && !memory_keys->is_null() && !memory_values->is_null();
+  const int64_t step_keys = packed ? 0 : (memory_filled ? memory_keys->shape(2) : key_tensor.shape(1));
+  const int64_t head_bytes = d * (dt == TTB_F32 ? 4 : 2);
+  const bool step = Lq == 1 && B > 0 && step_keys > 0 && step_keys <= 1024 && head_bytes % 16 == 0 && head_bytes <= 512 &&
+                    (!memory_filled || ((reinterpret_cast<uintptr_t>(memory_keys->raw()) | reinterpret_cast<uintptr_t>(memory_values->raw())) & 15) == 0);
+  q_.Forward(*q_in, T, step ? TTB_EPI_BIAS : TTB_EPI_NONE, nullptr, lin.raw_mut(), is_trans_weight, "context/gemm0");
+  if (!step) {
+    q.Reshape(x.dtype(), {B, heads, Lq, d}, kDLCUDA, dev, "context/AddBiasTransposeForScore/q_out2/Reshape");
+    Check(ttb_add_bias_transpose_for_score_pad(c, dt, lin.raw(), q_.bias().raw(), cu_q.get(), B, Lq, heads, d, q.raw_mut()), c,
+          "context/AddBiasTransposeForScore");
+  }
 
   // 2) keys / values: from the cache when it is filled, otherwise projected (and filed when a cache entry was passed)
   Tensor k_local(nullptr), v_local(nullptr);
   Tensor *k = &k_local, *v = &v_local;
-  const bool memory_filled = memory_keys && !memory_keys->is_null() && !memory_values->is_null();
   if (memory_filled) {
     k = memory_keys;
     v = memory_values;
@@ -735,7 +743,8 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
   Tensor scores_local(nullptr), ctx_heads(nullptr), context(nullptr);
   Tensor* scores = att_score ? att_score : &scores_local;
   scores->Reshape(x.dtype(), {B, heads, Lq, Lk}, kDLCUDA, dev, "batch_gemm3/Reshape");
-  Check(ttb_batch_matmul(c, dt, q.raw(), 0, k->raw(), 1, B * heads, Lq, Lk, d, scale, 0.0f, scores->raw_mut()), c, "batch_gemm3");
+  if (!step)
+    Check(ttb_batch_matmul(c, dt, q.raw(), 0, k->raw(), 1, B * heads, Lq, Lk, d, scale, 0.0f, scores->raw_mut()), c, "batch_gemm3");
   const float* mask = nullptr;
   int is2d = 1;
   Tensor pad_mask(nullptr);
@@ -756,6 +765,13 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
     mask = attention_mask.data<float>();
     is2d = MaskIs2D(attention_mask) ? 1 : 0;
     if (!is2d) TT_ENFORCE_EQ(attention_mask.shape(-2), Lq, "a [B, Lq, Lk] attention mask must have one row per query");
+  }
+  if (step) {  // with one query per sequence both mask forms are [B, Lk]
+    context.Reshape(x.dtype(), {T, H}, kDLCUDA, dev, "batch_gemm4/Reshape");
+    Check(ttb_context_attention_step(c, dt, lin.raw(), k->raw(), v->raw(), mask, B, heads, Lk, d, scale, scores->raw_mut(), context.raw_mut()), c,
+          "context/step");
+    Finish(context, x, T, output, post_layernorm, post_add_input, is_trans_weight);
+    return;
   }
   Check(ttb_mask_softmax(c, dt, scores->raw_mut(), mask, B, heads, Lq, Lk, 1.0f, is2d), c, "ApplyMaskAndSoftmax");
   ctx_heads.Reshape(x.dtype(), {B, heads, Lq, d}, kDLCUDA, dev, "ApplyMaskAndSoftmax/Reshape");

@@ -223,6 +223,131 @@ decode_merge_kernel(const float* __restrict__ partial, int rows_heads, int split
   dst[32 + lane] = from_f<T>(o1 / L);
 }
 
+// ---- one query per sequence over the projected encoder memory ---------------------------------------------------------
+// The cross attention of a stepwise decoding pass: scores, additive mask, softmax, probabilities (which the caller returns)
+// and the weighted values in one launch instead of five (bias + transpose of the queries, batched product, mask + softmax,
+// batched product, transpose). Bound by latency: over 20 x 8 heads and 45 keys of 64, K and V are 1.8 MB, 0.3 us of memory
+// time; a launch measures 3.7 us, the five it replaces 17. One CTA per (sequence, head); G lanes share a key, 16 bytes of it
+// each; scores stay in shared memory in fp32.
+constexpr int kStepKeys = 1024;
+
+__device__ __forceinline__ void unpack_group(const uint4& raw, float (&f)[8], const __half* t) { unpack8(raw, f, t); }
+__device__ __forceinline__ void unpack_group(const uint4& raw, float (&f)[8], const __nv_bfloat16* t) { unpack8(raw, f, t); }
+__device__ __forceinline__ void unpack_group(const uint4& raw, float (&f)[4], const float*) {
+  f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
+}
+
+template <typename T, int G>
+__global__ void __launch_bounds__(kThreads)
+context_attention_step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ mask, int heads,
+                              int Lk, int d, float scale, T* __restrict__ probs, T* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int VE = 16 / (int)sizeof(T), NG = kThreads / G, U = 4, kWarps = kThreads / 32;
+  __shared__ float score[kStepKeys];
+  __shared__ float part[kWarps][32 * VE];
+  __shared__ float red[2][kWarps];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = tid / G, c = tid % G;
+  const long long item = blockIdx.x;  // sequence * heads + head
+  const bool active = c * VE < d;
+  const T* kp = k + item * Lk * d + c * VE;
+  const T* vp = v + item * Lk * d + c * VE;
+  const float* m = mask ? mask + item / heads * Lk : nullptr;
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  float qf[VE];
+  unpack_group(active ? *reinterpret_cast<const uint4*>(q + item * d + c * VE) : zero, qf, q);
+  for (int j0 = 0; j0 < Lk; j0 += NG * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = j0 + u * NG + g;
+      raw[u] = (active && j < Lk) ? *reinterpret_cast<const uint4*>(kp + (long long)j * d) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float kf[VE], dot = 0.f;
+      unpack_group(raw[u], kf, q);
+#pragma unroll
+      for (int e = 0; e < VE; ++e) dot = fmaf(qf[e], kf[e], dot);
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+      const int j = j0 + u * NG + g;
+      if (c == 0 && j < Lk) score[j] = dot * scale + (m ? m[j] : 0.f);
+    }
+  }
+  __syncthreads();
+  float mx = -INFINITY;
+  for (int j = tid; j < Lk; j += kThreads) mx = fmaxf(mx, score[j]);
+  mx = warp_max(mx);
+  if (lane == 0) red[0][warp] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) mx = fmaxf(mx, red[0][w]);
+  float sum = 0.f;
+  for (int j = tid; j < Lk; j += kThreads) {
+    const float e = expf(score[j] - mx);
+    score[j] = e;  // read and written by this thread alone until the next barrier
+    sum += e;
+  }
+  sum = warp_sum(sum);
+  if (lane == 0) red[1][warp] = sum;
+  __syncthreads();
+  sum = 0.f;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) sum += red[1][w];
+  const float inv = 1.0f / sum;
+  if (probs)
+    for (int j = tid; j < Lk; j += kThreads) probs[item * Lk + j] = from_f<T>(score[j] * inv);
+  float acc[VE];
+#pragma unroll
+  for (int e = 0; e < VE; ++e) acc[e] = 0.f;
+  for (int j0 = 0; j0 < Lk; j0 += NG * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = j0 + u * NG + g;
+      raw[u] = (active && j < Lk) ? *reinterpret_cast<const uint4*>(vp + (long long)j * d) : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = j0 + u * NG + g;
+      float vf[VE];
+      unpack_group(raw[u], vf, q);
+      const float p = j < Lk ? score[j] * inv : 0.f;
+#pragma unroll
+      for (int e = 0; e < VE; ++e) acc[e] = fmaf(p, vf[e], acc[e]);
+    }
+  }
+#pragma unroll
+  for (int o = G; o < 32; o <<= 1)
+#pragma unroll
+    for (int e = 0; e < VE; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+  if (lane < G)
+#pragma unroll
+    for (int e = 0; e < VE; ++e) part[warp][c * VE + e] = acc[e];
+  __syncthreads();
+  for (int i = tid; i < d; i += kThreads) {
+    float o = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) o += part[w][i];
+    out[item * d + i] = from_f<T>(o);
+  }
+}
+
+template <typename T>
+void launch_context_step(ttb_ctx* ctx, const void* q, const void* k, const void* v, const float* mask, int64_t B, int64_t heads, int64_t Lk, int64_t d,
+                         float scale, void* probs, void* out) {
+  const int lanes = (int)(d * sizeof(T) / 16);  // lanes that share a key
+  const dim3 grid((unsigned)(B * heads));
+#define STEP_CASE(G)                                                                                                                             \
+  launch_pdl(context_attention_step_kernel<T, G>, grid, dim3(kThreads), 0, ctx->stream, (const T*)q, (const T*)k, (const T*)v, mask, (int)heads, \
+             (int)Lk, (int)d, scale, (T*)probs, (T*)out)
+  if (lanes <= 8) STEP_CASE(8);
+  else if (lanes <= 16) STEP_CASE(16);
+  else STEP_CASE(32);
+#undef STEP_CASE
+}
+
 int check_decode(ttb_ctx* ctx, const char* what, int dtype, const void* qkv, int64_t B, int64_t n_new, int64_t heads, int64_t d,
                  const void* kc, const void* vc, int64_t past_len) {
   TTB_REQUIRE(ctx, dtype == TTB_F16 || dtype == TTB_BF16, "%s: dtype must be F16 or BF16", what);
@@ -294,4 +419,24 @@ extern "C" int ttb_attention_decode(ttb_ctx* ctx, int dtype, const void* qkv, in
     if (!s) s = f;
   }
   return s;
+}
+
+extern "C" int ttb_context_attention_step(ttb_ctx* ctx, int dtype, const void* q, const void* k, const void* v, const float* mask, int64_t B,
+                                          int64_t heads, int64_t Lk, int64_t d, float scale, void* probs, void* out) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, dtype == TTB_F32 || dtype == TTB_F16 || dtype == TTB_BF16, "context_attention_step: unknown dtype %d", dtype);
+  const int64_t row = d * (dtype == TTB_F32 ? 4 : 2);
+  TTB_REQUIRE(ctx, B >= 0 && heads > 0 && d > 0 && B * heads < (1ll << 31), "context_attention_step: bad shape");
+  TTB_REQUIRE(ctx, Lk > 0 && Lk <= kStepKeys && row % 16 == 0 && row <= 512,
+              "context_attention_step: 1 to %d keys and heads of a multiple of 16 bytes, at most 512 (Lk = %lld, d = %lld)", kStepKeys, (long long)Lk,
+              (long long)d);
+  if (B == 0) return TTB_OK;
+  TTB_REQUIRE(ctx, q && k && v && out, "context_attention_step: null pointer");
+  TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) == 0,
+              "context_attention_step: q, k and v must be 16-byte aligned");
+  DeviceGuard g(ctx->device);
+  if (dtype == TTB_F32) launch_context_step<float>(ctx, q, k, v, mask, B, heads, Lk, d, scale, probs, out);
+  else if (dtype == TTB_F16) launch_context_step<__half>(ctx, q, k, v, mask, B, heads, Lk, d, scale, probs, out);
+  else launch_context_step<__nv_bfloat16>(ctx, q, k, v, mask, B, heads, Lk, d, scale, probs, out);
+  return launched(ctx, "context_attention_step");
 }
