@@ -720,19 +720,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             // A row whose address is not a multiple of 4 (every other row of an odd 16-bit width) is shifted by half a word on
             // the way out, and its first and last elements go out alone: nothing beyond the row's own elements is written.
             __syncwarp();
-            const int n_cols = min(CH, p.N - col0);
-#pragma unroll 4
-            for (int r = 0; r < 32; ++r) {
-              if (row_base + r >= p.M) break;
+            const int n_cols = min(CH, p.N - col0), n_rows = min(32, p.M - row_base);
+            auto word = [&](int r) { return *reinterpret_cast<const uint32_t*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4); };
+            if (n_rows == 32 && n_cols == CH && EB == 2) {
+              // whole chunks: eight rows in flight, at most one word and one half-word store a row
+#pragma unroll
+              for (int r0 = 0; r0 < 32; r0 += 8) {
+                uint32_t w[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[i] = word(r0 + i);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                  uint16_t* dst = reinterpret_cast<uint16_t*>(out + (long long)(row_base + r0 + i) * p.ldo + col0);
+                  if ((reinterpret_cast<uintptr_t>(dst) & 2) == 0) {
+                    reinterpret_cast<uint32_t*>(dst)[lane] = w[i];
+                  } else {
+                    const uint32_t shifted = __funnelshift_r(w[i], __shfl_down_sync(0xffffffffu, w[i], 1), 16);  // elements 2 lane + 1, 2 lane + 2
+                    if (lane < 31) *reinterpret_cast<uint32_t*>(dst + 2 * lane + 1) = shifted;
+                    if (lane == 0 || lane == 31) dst[lane == 0 ? 0 : CH - 1] = (uint16_t)(lane == 0 ? w[i] : w[i] >> 16);
+                  }
+                }
+              }
+              continue;
+            }
+            for (int r = 0; r < n_rows; ++r) {
               OutT* dst = out + (long long)(row_base + r) * p.ldo + col0;
-              const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+              const uint32_t w = word(r);
               if (EB == 4) {
                 if (lane < n_cols) reinterpret_cast<uint32_t*>(dst)[lane] = w;
               } else if ((reinterpret_cast<uintptr_t>(dst) & 2) == 0) {
                 if (2 * lane + 1 < n_cols) reinterpret_cast<uint32_t*>(dst)[lane] = w;
                 else if (2 * lane < n_cols) reinterpret_cast<uint16_t*>(dst)[2 * lane] = (uint16_t)w;
               } else {
-                const uint32_t shifted = __funnelshift_r(w, __shfl_down_sync(0xffffffffu, w, 1), 16);  // elements 2 lane + 1, 2 lane + 2
+                const uint32_t shifted = __funnelshift_r(w, __shfl_down_sync(0xffffffffu, w, 1), 16);
                 if (lane < 31 && 2 * lane + 2 < n_cols) *reinterpret_cast<uint32_t*>(dst + 2 * lane + 1) = shifted;
                 else if (2 * lane + 1 < n_cols) reinterpret_cast<uint16_t*>(dst)[2 * lane + 1] = (uint16_t)shifted;
                 if (lane == 0) reinterpret_cast<uint16_t*>(dst)[0] = (uint16_t)w;
@@ -975,6 +995,8 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   const bool tma = BN >= 64 && aligned16 && p.ldo % EA == 0 && (p.N % EA == 0 || (p.epilogue == TTB_EPI_NONE && p.staged == STORE_TMA && !p.out_lo)) &&
                    (!p.residual || p.ldr % EA == 0);
   // Ragged or misaligned rows without bias, residual or second plane (a 50257-wide vocabulary): word stores.
+  // 8192 x 50257 x 768 in fp16 into a contiguous tensor: 845 us, against about 560 into padded rows and 585 for the pass that
+  // compacted them. What is left over the padded form are the partial 32-byte sectors at both ends of each 128 bytes.
   const bool words = BN >= 64 && !tma && p.epilogue == TTB_EPI_NONE && !p.out_lo;
   q.staged = tma ? STORE_TMA : (words ? STORE_WORDS : STORE_DIRECT);
   if (tma) {
