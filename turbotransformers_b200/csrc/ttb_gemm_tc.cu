@@ -50,11 +50,12 @@ constexpr int kPrefetchBlocks = 16;  // k-blocks of the first tile's weights tha
 // own 128 rows of A and its own half (BN/2 rows) of W, so a k-block costs 32 KB of L2->SM traffic per CTA instead of 48.
 // SK = split-K over a cluster (BN = 32 only): a shorter ring, plus room for the partial tiles of the other CTAs.
 constexpr int kLnMaxTiles = 4;  // kernels with the LayerNorm epilogue: N-tiles of 256 per row, N <= 1024
-template <int BN, bool TWO = false, bool SK = false> struct Cfg {
+// PA, PB = planes of A and W that one ring slot holds (see Planes).
+template <int BN, bool TWO = false, bool SK = false, int PA = 1, int PB = 1> struct Cfg {
   static constexpr int A_BYTES = BM * BK_BYTES;
   static constexpr int B_BYTES = (TWO ? BN / 2 : BN) * BK_BYTES;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = SK ? 4 : (TWO ? 6 : ((BN == 256) ? 4 : (BN == 128 ? 6 : 8)));
+  static constexpr int STAGE_BYTES = PA * A_BYTES + PB * B_BYTES;
+  static constexpr int STAGES = SK ? 4 : (192 * 1024 / STAGE_BYTES < 8 ? 192 * 1024 / STAGE_BYTES : 8);
   // Two MMA-issuing warps with an accumulator each (even and odd k-blocks) wherever a k-block's MMAs are short: see the issuer.
   static constexpr int ISSUERS = (!TWO && BN <= 128) ? 2 : 1;
   // Two TMA-issuing warps, one per operand, on the narrowest tiles: see the producer.
@@ -62,7 +63,7 @@ template <int BN, bool TWO = false, bool SK = false> struct Cfg {
   static constexpr int THREADS = kThreads + 32 * (ISSUERS - 1) + 32 * (PRODUCERS - 1);
   static constexpr int TMEM_COLS = 2 * ISSUERS * BN;
   static_assert(PRODUCERS == 1 || ISSUERS == 2, "warp numbers: 10 issues, 11 loads");
-  static_assert(STAGES % ISSUERS == 0 && TMEM_COLS >= 32 && TMEM_COLS <= 512, "ring slots divide evenly among the issuers; TMEM allocation");
+  static_assert(STAGES >= 2 && TMEM_COLS >= 32 && TMEM_COLS <= 512, "a slot for each issuer; TMEM allocation");
   // Epilogue staging: per epilogue warp one [32 rows x 128 B] swizzled tile that its TMA stores read (BN >= 64 only).
   static constexpr int STAGING_BYTES = (BN >= 64) ? 8 * 4096 : 0;
   static constexpr int REDUCE_BYTES = SK ? (kMaxSplit - 1) * BM * BN * 4 : 0;  // [slot][column][row] 32-bit words
@@ -74,6 +75,17 @@ template <int BN, bool TWO = false, bool SK = false> struct Cfg {
 // stores (16-byte-aligned rows of a multiple of 16 bytes); STORE_WORDS, through shared memory and word stores, 128 consecutive
 // bytes of one row per instruction whatever the row's alignment.
 enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
+
+// Products over two planes of an operand (bf16 hi + lo; fp32 as three tf32 products). On tiles of up to 128 columns, which are bound
+// by their loads, a ring slot holds both planes of a k-block and all its products are issued from there, so that no plane is
+// fetched twice: fp32 520 x 768 x 3072 51.2 -> 44.7 us, 128 x 768 x 3072 27 -> 17.9, bf16 3200 x 768 x 3072 45 -> 39. Tiles of 256
+// columns, bound by the MMAs, run the products as passes over K: with slots twice the size they have too few of them (bf16
+// 9000 x 2304 x 768 50.6 us in passes, 60.1 from shared slots).
+template <int BN, bool TWO, int KIND, typename OutT, int VAR> struct Planes {
+  static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR != 0)));
+  static constexpr int A = shared ? 2 : 1;
+  static constexpr int B = (shared && KIND == KIND_TF32) ? 2 : 1;
+};
 
 struct GemmParams {
   int M, N, K;             // K in elements, per pass
@@ -181,7 +193,9 @@ __global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
                const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1,
                const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmO2, const GemmParams p) {
-  using C = Cfg<BN, TWO, SK>;
+  using P = Planes<BN, TWO, KIND, OutT, VAR>;
+  using C = Cfg<BN, TWO, SK, P::A, P::B>;
+  constexpr bool FUSED = P::shared;  // all products of a k-block from one slot
   static_assert(!SK || (BN == 32 && !TWO), "split-K runs on single-CTA 128 x 32 tiles");
   static_assert(!LN || (BN == 256 && !SK && VAR == VAR_PLAIN && sizeof(OutT) == 2), "the LayerNorm epilogue: 16-bit 256-column tiles");
   constexpr int IN_BYTES = (KIND == KIND_I8) ? 1 : (KIND == KIND_TF32 ? 4 : 2);
@@ -253,7 +267,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
   const int num_m = (p.M + TILE_M - 1) / TILE_M, num_n = (p.N + BN - 1) / BN;
   const int num_tiles = num_m * num_n;
   const int num_kb = (p.K + BK_ELEMS - 1) / BK_ELEMS;   // k-blocks per pass
-  const int total_kb = num_kb * p.npass;
+  const int total_kb = FUSED ? num_kb : num_kb * p.npass;
   // this CTA's share of a tile's k-blocks: all of them, or (split-K) one contiguous range per cluster rank
   const int kb_begin = SK ? (int)(((long long)total_kb * rank) / group) : 0;
   const int kb_end = SK ? (int)(((long long)total_kb * (rank + 1)) / group) : total_kb;
@@ -267,6 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     int pass = kb_begin / num_kb, kk = kb_begin % num_kb;
     for (int kb = kb_begin; kb < min(kb_end, kb_begin + kPrefetchBlocks) && n_row < p.N; ++kb) {
       tma_prefetch_2d(((p.pass_b >> pass) & 1) ? &tmB1 : &tmB0, kk * BK_ELEMS, n_row);
+      if (FUSED && p.pass_b) tma_prefetch_2d(&tmB1, kk * BK_ELEMS, n_row);
       if (++kk == num_kb) { kk = 0; ++pass; }
     }
   }
@@ -289,16 +304,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
           const CUtensorMap* ma = ((p.pass_a >> pass) & 1) ? &tmA1 : &tmA0;
           const CUtensorMap* mb = ((p.pass_b >> pass) & 1) ? &tmB1 : &tmB0;
-          const uint32_t a_dst = tiles + stage * C::STAGE_BYTES;
+          const uint32_t a_dst = tiles + stage * C::STAGE_BYTES, b_dst = a_dst + (FUSED ? 2 : 1) * C::A_BYTES;
+          const bool a2 = FUSED && p.pass_a != 0, b2 = FUSED && p.pass_b != 0;  // second planes in the same slot
           if (TWO) {
             // CTA 0's barrier counts the bytes of both CTAs; only CTA 0 arms it.
             if (rank == 0) mbar_expect_tx(full_bar(stage), 2u * (uint32_t)C::STAGE_BYTES);
             tma_load_2d_pair(a_dst, ma, full_bar(stage), kk * BK_ELEMS, m_blk * TILE_M + (int)rank * BM);
-            tma_load_2d_pair(a_dst + C::A_BYTES, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN + (int)rank * (BN / 2));
+            tma_load_2d_pair(b_dst, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN + (int)rank * (BN / 2));
           } else {
-            mbar_expect_tx(full_bar(stage), (load_a ? (uint32_t)(p.a_rows * BK_BYTES) : 0u) + (load_b ? (uint32_t)C::B_BYTES : 0u));
+            mbar_expect_tx(full_bar(stage), (load_a ? (uint32_t)(p.a_rows * BK_BYTES * (a2 ? 2 : 1)) : 0u) + (load_b ? (uint32_t)(C::B_BYTES * (b2 ? 2 : 1)) : 0u));
             if (load_a) tma_load_2d(a_dst, ma, full_bar(stage), kk * BK_ELEMS, m_blk * BM);
-            if (load_b) tma_load_2d(a_dst + C::A_BYTES, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN);
+            if (load_b) tma_load_2d(b_dst, mb, full_bar(stage), kk * BK_ELEMS, n_blk * BN);
+            if (load_a && a2) tma_load_2d(a_dst + C::A_BYTES, &tmA1, full_bar(stage), kk * BK_ELEMS, m_blk * BM);
+            if (load_b && b2) tma_load_2d(b_dst + C::B_BYTES, &tmB1, full_bar(stage), kk * BK_ELEMS, n_blk * BN);
           }
           if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
           if (++kk == num_kb) { kk = 0; ++pass; }
@@ -344,11 +362,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         uint32_t accumulate = 0;
         for (int kb = kb_begin + issuer; kb < kb_end; kb += C::ISSUERS) {
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) { ok = false; break; }
-          const uint32_t b_lo = a_lo + (uint32_t)(C::A_BYTES >> 4);
+          const uint32_t b_lo = a_lo + (uint32_t)((FUSED ? 2 : 1) * C::A_BYTES >> 4);
+          for (int pass = 0; pass < (FUSED ? p.npass : 1); ++pass) {
+            const uint32_t a_at = a_lo + ((FUSED && ((p.pass_a >> pass) & 1)) ? (uint32_t)(C::A_BYTES >> 4) : 0u);
+            const uint32_t b_at = b_lo + ((FUSED && ((p.pass_b >> pass) & 1)) ? (uint32_t)(C::B_BYTES >> 4) : 0u);
 #pragma unroll
-          for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k) {
-            umma_ss<KIND, TWO>(d_tmem, a_lo + (uint32_t)(k * (UMMA_K_BYTES >> 4)), b_lo + (uint32_t)(k * (UMMA_K_BYTES >> 4)), IDESC, accumulate);
-            accumulate = 1;
+            for (int k = 0; k < BK_BYTES / UMMA_K_BYTES; ++k) {
+              umma_ss<KIND, TWO>(d_tmem, a_at + (uint32_t)(k * (UMMA_K_BYTES >> 4)), b_at + (uint32_t)(k * (UMMA_K_BYTES >> 4)), IDESC, accumulate);
+              accumulate = 1;
+            }
           }
           // the slot is free (in both CTAs when paired) once these MMAs have read it
           if (TWO) tc_commit_pair(empty_bar(stage));
@@ -970,7 +992,8 @@ struct Operands {
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR>
 int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
-  using C = Cfg<BN, TWO, SK>;
+  using P = Planes<BN, TWO, KIND, OutT, VAR>;
+  using C = Cfg<BN, TWO, SK, P::A, P::B>;
   constexpr int TILE_M = TWO ? 2 * BM : BM;
   constexpr int EA = (int)sizeof(OutT) == 4 ? 4 : 8;  // output elements per 16 bytes
   CUtensorMap tmA0, tmA1, tmB0, tmB1;
@@ -1179,7 +1202,8 @@ int splitk_cap() {
 // Clusters of `split` CTAs of the split-K kernel that can be resident on the device at once (cached per device and size).
 template <int KIND, typename OutT, int VAR>
 int max_resident_clusters(ttb_ctx* ctx, int split) {
-  using C = Cfg<32, false, true>;
+  using P = Planes<32, false, KIND, OutT, VAR>;
+  using C = Cfg<32, false, true, P::A, P::B>;
   static int cached[64][kMaxSplit + 1] = {};
   const int dev = ctx->device < 64 ? ctx->device : 63;
   if (ctx->device < 64 && cached[dev][split] != 0) return cached[dev][split] > 0 ? cached[dev][split] : 0;
@@ -1221,7 +1245,12 @@ int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
   const int64_t num_m = (p.M + BM - 1) / BM;
   auto tiles = [&](int bn) { return num_m * ((p.N + bn - 1) / bn); };
   const int64_t pair_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((p.N + 255) / 256);
-  const int64_t total_kb = (((int64_t)p.K * IN_BYTES + BK_BYTES - 1) / BK_BYTES) * p.npass;
+  // With both planes of a k-block in one slot the narrow tiles, which are bound by their loads, take 2 / 1.5 times a single
+  // product's k-block for three / two products; the 256-column ones take 3 / 2 times.
+  constexpr bool fused = Planes<32, false, KIND, OutT, VAR>::shared;
+  const int64_t num_kb = ((int64_t)p.K * IN_BYTES + BK_BYTES - 1) / BK_BYTES;
+  const int64_t wide = num_kb * p.npass, total_kb = fused ? num_kb : wide;
+  const int64_t narrow = (fused && p.npass > 1) ? num_kb * (p.npass + 1) / 2 : wide;
   const int64_t sms = ctx->sm_count;
   auto expect = [&](int64_t fixed, int64_t per_kb, int64_t epilogue, int64_t n, int64_t slots, int64_t kb) {
     return fixed + (n + slots - 1) / slots * std::max(per_kb * kb, epilogue);
@@ -1238,16 +1267,16 @@ int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
   auto consider = [&](int which, int64_t ns) {
     if (ns < best_ns) { best = which; best_ns = ns; }
   };
-  if (pair_mode() && pair_pays) consider(0, expect(7300, 310, 5400, pair_tiles, sms / 2, total_kb));
-  consider(256, expect(6300, 350, 6000, tiles(256), sms, total_kb));
-  consider(128, expect(3500, 235, 4300, tiles(128), sms, total_kb));
-  consider(64, expect(3800, 177, 3000, tiles(64), sms, total_kb));
-  consider(32, expect(3900, 155, 2000, tiles(32), sms, total_kb));
+  if (pair_mode() && pair_pays) consider(0, expect(7300, 310, 5400, pair_tiles, sms / 2, wide));
+  consider(256, expect(6300, 350, 6000, tiles(256), sms, wide));
+  consider(128, expect(3500, 235, 4300, tiles(128), sms, narrow));
+  consider(64, expect(3800, 177, 3000, tiles(64), sms, narrow));
+  consider(32, expect(3900, 155, 2000, tiles(32), sms, narrow));
   // Few 128 x 32 tiles and a mainloop of several k-blocks: the CTAs of a cluster may share each tile's K range, so that the
   // weights stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per
   // tile, 8.7 split four ways; 12 k-blocks are not worth the exchange.
   const int64_t t32 = tiles(32);
-  if (splitk_cap() > 1 && t32 * 2 <= sms && total_kb >= 24) {
+  if (splitk_cap() > 1 && t32 * 2 <= sms && wide >= 24) {
     int64_t s = sms / t32;
     if (s > splitk_cap()) s = splitk_cap();
     if (s > total_kb / 2) s = total_kb / 2;  // at least two k-blocks per CTA
@@ -1255,7 +1284,7 @@ int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
     // they pack into its GPCs
     while (s >= 2 && t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, (int)s)) --s;
     if (s >= 2) {
-      consider(1, expect(6900, 155, 2000, t32, t32, (total_kb + s - 1) / s));
+      consider(1, expect(6900, 155, 2000, t32, t32, (narrow + s - 1) / s));
       if (best == 1) {
         p.split_k = (int)s;
         return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
