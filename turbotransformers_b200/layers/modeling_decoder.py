@@ -17,9 +17,23 @@ import torch
 from .._cxx import cxx
 from .modules import MultiHeadedAttention, PositionwiseFeedForward
 from .return_type import ReturnType, convert_returns_as_type
-from .utils import create_empty_if_none, try_convert
+from .utils import AnyTensor, try_convert
 
 __all__ = ['TransformerDecoderLayer', 'TransformerDecoder']
+
+
+def _additive_masks(src_pad_mask: torch.Tensor, tgt_pad_mask: torch.Tensor, step: Optional[int], future: Optional[bool]):
+    """The masks that the attention layers add to their scores, from padding masks (true / 1 = padding)."""
+    src_mask = (src_pad_mask.float() * -1e18).contiguous()
+    if step is not None:
+        return src_mask, None
+    tgt_len = tgt_pad_mask.size(-1)
+    if not future:  # padding + future positions, [B, T, T]
+        future_mask = torch.ones([tgt_len, tgt_len], device=tgt_pad_mask.device, dtype=torch.float32).triu_(1)
+        dec_mask = torch.gt(tgt_pad_mask.float() + future_mask.view(1, tgt_len, tgt_len), 0).float()
+    else:           # padding only, [B, 1, T]
+        dec_mask = tgt_pad_mask.float()
+    return src_mask, (dec_mask * -1e18).contiguous()
 
 
 class TransformerDecoderLayer:
@@ -37,23 +51,19 @@ class TransformerDecoderLayer:
         (true / 1 = padding). Returns (output [B, T, H], context attention of head 0 [B, T, src_len], None)."""
         if with_align:
             raise ValueError("with_align must be False")
-        src_mask = src_pad_mask.float() * -1e18
-        dec_mask = None
-        if step is None:
-            tgt_len = tgt_pad_mask.size(-1)
-            if not future:  # padding + future positions, [B, T, T]
-                future_mask = torch.ones([tgt_len, tgt_len], device=tgt_pad_mask.device, dtype=torch.float32).triu_(1)
-                dec_mask = torch.gt(tgt_pad_mask.float() + future_mask.view(1, tgt_len, tgt_len), 0).float()
-            else:           # padding only, [B, 1, T]
-                dec_mask = tgt_pad_mask.float()
-            dec_mask = (dec_mask * -1e18).contiguous()
+        src_mask, dec_mask = _additive_masks(src_pad_mask, tgt_pad_mask, step, future)
+        out, attns = self._run(input_tensor, memory_bank, src_mask, dec_mask, layer_cache, return_type, output)
+        return out, convert_returns_as_type(attns, ReturnType.TORCH)[:, 0, :, :].contiguous(), None
+
+    def _run(self, input_tensor: AnyTensor, memory_bank: AnyTensor, src_mask: AnyTensor, dec_mask: Optional[AnyTensor], layer_cache: Optional[dict],
+             return_type: Optional[ReturnType], output: Optional[cxx.Tensor] = None):
+        """The block on additive masks; returns its output and the context attention of all heads as the runtime's tensor."""
         query, _ = self.self_attn(input_tensor, input_tensor, input_tensor, mask=dec_mask, layer_cache=layer_cache, attn_type="self",
                                   pre_layernorm=True, post_add_input=True, return_type=ReturnType.turbo_transformers)
-        mid, attns = self.context_attn(memory_bank, memory_bank, query, mask=src_mask.contiguous(), layer_cache=layer_cache,
+        mid, attns = self.context_attn(memory_bank, memory_bank, query, mask=src_mask, layer_cache=layer_cache,
                                        attn_type="context", pre_layernorm=True, post_add_input=True,
                                        return_type=ReturnType.turbo_transformers, output_attentions=True)
-        out = self.feed_forward(mid, return_type=return_type, is_trans_weight=self._ffn_trans, output=output)
-        return out, convert_returns_as_type(attns, ReturnType.TORCH)[:, 0, :, :].contiguous(), None
+        return self.feed_forward(mid, return_type=return_type, is_trans_weight=self._ffn_trans, output=output), attns
 
     _ffn_trans = True
 
@@ -104,9 +114,21 @@ class TransformerDecoder:
         src_pad_mask = ~(torch.arange(src_max_len, device=src_lens.device)[None, :] < src_lens[:, None]).unsqueeze(1)
         tgt_pad_mask = tgt_words.data.eq(self.embeddings.word_padding_idx).unsqueeze(1)  # [B, 1, T_tgt]
         attn = None
-        for i, layer in enumerate(self.transformer_layers):
-            layer_cache = self.state["cache"][f"layer_{i}"] if step is not None else None
-            output, attn, _ = layer(output, src_memory_bank, src_pad_mask, tgt_pad_mask, layer_cache=layer_cache, step=step)
+        # The masks are the same for every layer and only the last layer's attention is returned: masks and memory are converted
+        # once, and what travels between the layers stays the runtime's own tensor. Layers of a class of the caller's run as before.
+        own = all(type(layer).__call__ is TransformerDecoderLayer.__call__ for layer in self.transformer_layers)
+        if own and self.transformer_layers:
+            src_mask, dec_mask = _additive_masks(src_pad_mask, tgt_pad_mask, step, False)
+            memory, masks = try_convert(src_memory_bank), (try_convert(src_mask), None if dec_mask is None else try_convert(dec_mask))
+            last = len(self.transformer_layers) - 1
+            for i, layer in enumerate(self.transformer_layers):
+                layer_cache = self.state["cache"][f"layer_{i}"] if step is not None else None
+                output, attn = layer._run(output, memory, *masks, layer_cache, None if i == last else ReturnType.turbo_transformers)
+            attn = convert_returns_as_type(attn, ReturnType.TORCH)[:, 0, :, :]
+        else:
+            for i, layer in enumerate(self.transformer_layers):
+                layer_cache = self.state["cache"][f"layer_{i}"] if step is not None else None
+                output, attn, _ = layer(output, src_memory_bank, src_pad_mask, tgt_pad_mask, layer_cache=layer_cache, step=step)
         output = self.layer_norm(output)
         attns = {"std": attn.transpose(0, 1).contiguous()}
         if self._copy:

@@ -27,23 +27,30 @@ class MultiHeadedAttention(cxx.MultiHeadedAttention):
         output_attentions is set; otherwise it is a null tensor (the fused kernel never writes them)."""
         if isinstance(query_tensor, torch.Tensor):
             use_current_stream(query_tensor)
-        key_tensor, value_tensor, query_tensor = try_convert(key_tensor), try_convert(value_tensor), try_convert(query_tensor)
+        query, key, value = query_tensor, key_tensor, value_tensor
+        query_tensor = try_convert(query)
+        key_tensor = query_tensor if key is query else try_convert(key)
+        value_tensor = query_tensor if value is query else (key_tensor if value is key else try_convert(value))
         mask = try_convert(create_empty_if_none(mask))
         output, attn = create_empty_if_none(output), create_empty_if_none(attn)
-        cache = {k: (try_convert(v) if v is not None else _empty()) for k, v in (layer_cache or {}).items()}
         attn_type = attn_type or "self"
+        # self attention has no use for the memory entries of a layer's cache, nor context attention for the self entries
+        foreign = {"self": ("memory_keys", "memory_values"), "context": ("self_keys", "self_values")}.get(attn_type, ())
+        cache = {k: (try_convert(v) if v is not None else _empty()) for k, v in (layer_cache or {}).items() if k not in foreign}
         super().__call__(key_tensor, value_tensor, query_tensor, mask, attn_type, output,
                          attn if (output_attentions or attn_type == "context") else None, cache, pre_layernorm,
                          post_layernorm, post_add_input, is_trans_weight)
         if layer_cache is not None:
             # the caches go back to the caller's dict, as the reference does (modules.py:79-83): the projected encoder memory
-            # as torch tensors [B, heads, Lk, d]; the self-attention cache as the runtime's own tensor (its buffer is paged and
-            # reserved ahead, so it is handed back as it is and passed in again on the next step)
+            # as torch tensors [B, heads, Lk, d] (where the caller passed them filled they are only read: they stay as they are);
+            # the self-attention cache as the runtime's own tensor (its buffer is paged and reserved ahead, so it is handed back
+            # as it is and passed in again on the next step)
             for k, v in cache.items():
                 if v.is_null():
                     continue
                 if "memory" in k and attn_type == "context":
-                    layer_cache[k] = convert_returns_as_type(v, ReturnType.TORCH)
+                    if not isinstance(layer_cache[k], torch.Tensor):
+                        layer_cache[k] = convert_returns_as_type(v, ReturnType.TORCH)
                 elif "self" in k and attn_type == "self":
                     layer_cache[k] = v
         return convert_returns_as_type(output, return_type), attn
