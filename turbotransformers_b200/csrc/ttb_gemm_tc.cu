@@ -82,7 +82,7 @@ enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
 // columns, bound by the MMAs, run the products as passes over K: with slots twice the size they have too few of them (bf16
 // 9000 x 2304 x 768 50.6 us in passes, 60.1 from shared slots).
 template <int BN, bool TWO, int KIND, typename OutT, int VAR> struct Planes {
-  static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR != 0)));
+  static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR == 1)));
   static constexpr int A = shared ? 2 : 1;
   static constexpr int B = (shared && KIND == KIND_TF32) ? 2 : 1;
 };
@@ -185,8 +185,9 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 
 // ---- the kernel -----------------------------------------------------------------------------------
 // VAR selects an epilogue variant that costs registers, so that the plain kernels do not carry it:
-//   VAR_PLAIN, VAR_TWO_PLANES (16-bit output written as hi + lo planes), VAR_AFFINE (int8 with a per-tensor zero point)
-enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2 };
+//   VAR_PLAIN, VAR_TWO_PLANES (16-bit output written as hi + lo planes), VAR_AFFINE (int8 with a per-tensor zero point),
+//   VAR_WORDS (STORE_WORDS; carried by every kernel it cost packed fp16 batches 1 %: 4120 -> 4164 us, 4149 against 4159 without)
+enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3 };
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR, bool LN = false>
 __global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
@@ -738,7 +739,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               for (int g = 0; g < G16; ++g) lo_pack[(hh * G16 + g) % LO_N] = pack16<OutT>(&v[g * P16]);
             }
           }
-          if (p.staged == STORE_WORDS) {
+          if constexpr (VAR == VAR_WORDS) {
             // A row whose address is not a multiple of 4 (every other row of an odd 16-bit width) is shifted by half a word on
             // the way out, and its first and last elements go out alone: nothing beyond the row's own elements is written.
             __syncwarp();
@@ -1021,7 +1022,10 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   // 8192 x 50257 x 768 in fp16 into a contiguous tensor: 845 us, against about 560 into padded rows and 585 for the pass that
   // compacted them. What is left over the padded form are the partial 32-byte sectors at both ends of each 128 bytes.
   const bool words = BN >= 64 && !tma && p.epilogue == TTB_EPI_NONE && !p.out_lo;
-  q.staged = tma ? STORE_TMA : (words ? STORE_WORDS : STORE_DIRECT);
+  if constexpr (VAR == VAR_PLAIN && BN >= 64) {
+    if (words) return launch_tc<BN, KIND, OutT, TWO, SK, VAR_WORDS>(ctx, op, p);
+  }
+  q.staged = tma ? STORE_TMA : (VAR == VAR_WORDS ? STORE_WORDS : STORE_DIRECT);
   if (tma) {
     s = make_map(ctx, &tmO, out_kind<OutT>(), p.out, p.M, p.N, p.ldo, 32);
     if (s) return s;
