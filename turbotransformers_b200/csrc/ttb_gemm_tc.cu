@@ -30,6 +30,7 @@
 #include <unordered_map>
 
 #include "ttb_common.cuh"
+#include "ttb_ring.cuh"
 #include "ttb_sm100.cuh"
 
 using namespace ttb;
@@ -63,7 +64,8 @@ template <int BN, bool TWO = false, bool SK = false, int PA = 1, int PB = 1> str
   static constexpr int THREADS = kThreads + 32 * (ISSUERS - 1) + 32 * (PRODUCERS - 1);
   static constexpr int TMEM_COLS = 2 * ISSUERS * BN;
   static_assert(PRODUCERS == 1 || ISSUERS == 2, "warp numbers: 10 issues, 11 loads");
-  static_assert(STAGES >= 2 && TMEM_COLS >= 32 && TMEM_COLS <= 512, "a slot for each issuer; TMEM allocation");
+  static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512, "TMEM allocation");
+  static_assert(ISSUERS == 1 || STAGES >= ring::kMinStages, "two issuers tell a slot's uses apart by parity: see ttb_ring.cuh");
   // Epilogue staging: per epilogue warp one [32 rows x 128 B] swizzled tile that its TMA stores read (BN >= 64 only).
   static constexpr int STAGING_BYTES = (BN >= 64) ? 8 * 4096 : 0;
   static constexpr int REDUCE_BYTES = SK ? (kMaxSplit - 1) * BM * BN * 4 : 0;  // [slot][column][row] 32-bit words
@@ -362,6 +364,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
         const uint32_t d_tmem = tmem_base + (uint32_t)((acc * C::ISSUERS + issuer) * BN);
         uint32_t accumulate = 0;
         for (int kb = kb_begin + issuer; kb < kb_end; kb += C::ISSUERS) {
+          // a slot whose previous use was the other issuer's: see there
+          if (ring::wait_for_empty_first(C::STAGES, C::ISSUERS, kb_end - kb_begin, kb - kb_begin) &&
+              !mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
           if (!mbar_wait(full_bar(stage), phase, abort_flag)) { ok = false; break; }
           const uint32_t b_lo = a_lo + (uint32_t)((FUSED ? 2 : 1) * C::A_BYTES >> 4);
           for (int pass = 0; pass < (FUSED ? p.npass : 1); ++pass) {
