@@ -185,3 +185,24 @@ def test_context_attention_step_refuses_what_it_does_not_take(ctx):
             ctx.call("context_attention_step", _capi.F16, t, t, t, None, 1, 1, Lk, d, 1.0, None, t)
     with pytest.raises(_capi.TTBError):
         ctx.call("context_attention_step", _capi.F16, t[1:], t, t, None, 1, 1, 8, 64, 1.0, None, t)
+
+
+@pytest.mark.parametrize("given", ["memory_keys", "memory_values"])
+def test_a_half_filled_memory_cache_is_projected_and_replaced_as_a_pair(given):
+    H, heads, B, Lk = 256, 4, 2, 9
+    w = {k: rounded(v, "f16") for k, v in ref_driver.context_attention_weights(H, 15).items()}
+    r = np.random.default_rng(16)
+    mem, old, q = (on_dev(r.standard_normal(s).astype(np.float32), "f16") for s in ((B, Lk, H), (B, Lk, H), (B, 1, H)))
+    att = build(w, heads, "f16")
+    want, stale = ({"memory_keys": None, "memory_values": None} for _ in range(2))
+    want_out, _ = att(mem, mem, q, attn_type="context", layer_cache=want)
+    att(old, old, q, attn_type="context", layer_cache=stale)  # what an earlier sequence left
+    half = {"memory_keys": None, "memory_values": None, given: stale[given]}
+    out, _ = att(mem, mem, q, attn_type="context", layer_cache=half)
+    assert torch.equal(out, want_out)
+    for k in want:
+        assert torch.equal(half[k], want[k])
+    kept = dict(half)
+    again, _ = att(old, old, q, attn_type="context", layer_cache=half)  # filled: read, and left as they are
+    assert torch.equal(again, want_out) and all(half[k] is kept[k] for k in kept)
+    assert tt._cxx_module.device_status(0) == 0

@@ -37,19 +37,21 @@ class MultiHeadedAttention(cxx.MultiHeadedAttention):
         # self attention has no use for the memory entries of a layer's cache, nor context attention for the self entries
         foreign = {"self": ("memory_keys", "memory_values"), "context": ("self_keys", "self_values")}.get(attn_type, ())
         cache = {k: (try_convert(v) if v is not None else _empty()) for k, v in (layer_cache or {}).items() if k not in foreign}
+        # both memory entries filled: they are only read. Otherwise both are projected, whichever of them was given.
+        memory_read = all(k in cache and not cache[k].is_null() for k in ("memory_keys", "memory_values"))
         super().__call__(key_tensor, value_tensor, query_tensor, mask, attn_type, output,
                          attn if (output_attentions or attn_type == "context") else None, cache, pre_layernorm,
                          post_layernorm, post_add_input, is_trans_weight)
         if layer_cache is not None:
             # the caches go back to the caller's dict, as the reference does (modules.py:79-83): the projected encoder memory
-            # as torch tensors [B, heads, Lk, d] (where the caller passed them filled they are only read: they stay as they are);
+            # as torch tensors [B, heads, Lk, d] (torch tensors that were only read stay as they are);
             # the self-attention cache as the runtime's own tensor (its buffer is paged and reserved ahead, so it is handed back
             # as it is and passed in again on the next step)
             for k, v in cache.items():
                 if v.is_null():
                     continue
                 if "memory" in k and attn_type == "context":
-                    if not isinstance(layer_cache[k], torch.Tensor):
+                    if not (memory_read and isinstance(layer_cache[k], torch.Tensor)):
                         layer_cache[k] = convert_returns_as_type(v, ReturnType.TORCH)
                 elif "self" in k and attn_type == "self":
                     layer_cache[k] = v
