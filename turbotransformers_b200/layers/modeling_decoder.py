@@ -79,6 +79,15 @@ class TransformerDecoderLayer:
         return TransformerDecoderLayer(self_attn, context_attn, feed_forward)
 
 
+def _unmodified(layer) -> bool:
+    """Whether a layer and its parts run this module's own calls. A caller's class in the place of any of them, such as an
+    attention that wraps __call__, expects torch tensors for the layer's input, the memory and the masks."""
+    return (type(layer).__call__ is TransformerDecoderLayer.__call__ and type(layer)._run is TransformerDecoderLayer._run and
+            type(layer.self_attn).__call__ is MultiHeadedAttention.__call__ and
+            type(layer.context_attn).__call__ is MultiHeadedAttention.__call__ and
+            type(layer.feed_forward).__call__ is PositionwiseFeedForward.__call__)
+
+
 class TransformerDecoder:
     """The decoder stack: the embeddings and the final LayerNorm stay torch modules, as in the reference
     (modeling_decoder.py:230-329); tensors are time-major at this interface ([len, batch, ...]) like OpenNMT-py's."""
@@ -115,9 +124,8 @@ class TransformerDecoder:
         tgt_pad_mask = tgt_words.data.eq(self.embeddings.word_padding_idx).unsqueeze(1)  # [B, 1, T_tgt]
         attn = None
         # The masks are the same for every layer and only the last layer's attention is returned: masks and memory are converted
-        # once, and what travels between the layers stays the runtime's own tensor. Layers of a class of the caller's run as before.
-        own = all(type(layer).__call__ is TransformerDecoderLayer.__call__ for layer in self.transformer_layers)
-        if own and self.transformer_layers:
+        # once, and what travels between the layers stays the runtime's own tensor. Layers or parts of a caller's class get torch's.
+        if self.transformer_layers and all(_unmodified(layer) for layer in self.transformer_layers):
             src_mask, dec_mask = _additive_masks(src_pad_mask, tgt_pad_mask, step, False)
             memory, masks = try_convert(src_memory_bank), (try_convert(src_mask), None if dec_mask is None else try_convert(dec_mask))
             last = len(self.transformer_layers) - 1
