@@ -46,8 +46,8 @@ def make_layer(**parts):
     return layer
 
 
-def decode(layers):
-    dec = tt.TransformerDecoder(Embeddings(), layers, torch.nn.LayerNorm(H))
+def decode(layers, norm=None):
+    dec = tt.TransformerDecoder(Embeddings(), layers, norm or torch.nn.LayerNorm(H))
     dec.init_state(torch.zeros(S, B, 1), None, None)
     return dec(torch.zeros(T, B, 1, dtype=torch.int64), torch.ones(S, B, H), memory_lengths=torch.tensor([S, S - 1]))
 
@@ -68,3 +68,23 @@ def test_a_callers_own_parts_get_torch_tensors():
 def test_one_part_of_the_callers_is_enough(part, cls):
     assert modeling_decoder._unmodified(make_layer())
     assert not modeling_decoder._unmodified(make_layer(**{part: own(cls, [])}))
+
+
+def test_the_runtime_is_back_on_the_callers_stream_before_torch_reads_the_results(monkeypatch):
+    # Another thread may point the device's kernel stream elsewhere between two layers; pointing it back orders the caller's
+    # stream behind what was queued meanwhile.
+    log = []
+
+    def run(self, x, memory, src_mask, dec_mask, layer_cache, return_type, output=None):
+        log.append("layer")
+        return convert_returns_as_type(convert2tt_tensor(torch.ones(B, T, H)), return_type), convert2tt_tensor(torch.ones(B, HEADS, T, S))
+
+    class Norm(torch.nn.LayerNorm):
+        def forward(self, x):
+            log.append("torch")
+            return super().forward(x)
+
+    monkeypatch.setattr(tt.TransformerDecoderLayer, "_run", run)
+    monkeypatch.setattr(modeling_decoder, "use_current_stream", lambda t: log.append("stream"))
+    decode([make_layer(), make_layer()], Norm(H))
+    assert log == ["layer", "layer", "stream", "torch"]

@@ -17,7 +17,7 @@ import torch
 from .._cxx import cxx
 from .modules import MultiHeadedAttention, PositionwiseFeedForward
 from .return_type import ReturnType, convert_returns_as_type
-from .utils import AnyTensor, try_convert
+from .utils import AnyTensor, try_convert, use_current_stream
 
 __all__ = ['TransformerDecoderLayer', 'TransformerDecoder']
 
@@ -132,6 +132,9 @@ class TransformerDecoder:
             for i, layer in enumerate(self.transformer_layers):
                 layer_cache = self.state["cache"][f"layer_{i}"] if step is not None else None
                 output, attn = layer._run(output, memory, *masks, layer_cache, None if i == last else ReturnType.turbo_transformers)
+            # What torch reads next is ordered behind the last layer on the caller's stream, wherever another thread of the
+            # caller's may have pointed the runtime meanwhile.
+            use_current_stream(src_memory_bank)
             attn = convert_returns_as_type(attn, ReturnType.TORCH)[:, 0, :, :]
         else:
             for i, layer in enumerate(self.transformer_layers):
