@@ -151,11 +151,11 @@ def test_smart_batch_context_attention_with_query_and_key_length_lists(dt, flags
     assert tt._cxx_module.device_status(0) == 0
 
 
-# one key, counts on both sides of a pass of the lane groups (64 keys) and the longest; lanes per key of 8, 16 and 32 with and
-# without idle ones
+# one key, counts on both sides of a pass of the lane groups (64 keys; 32 and 16 of the shorter form) and the longest; lanes per
+# key of 8, 16 and 32 with and without idle ones
 @pytest.mark.parametrize("dt", ["f32", "f16", "bf16"])
 @pytest.mark.parametrize("B,heads,Lk,d", [(1, 1, 1, 64), (3, 4, 63, 64), (2, 3, 65, 40), (5, 2, 200, 128), (1, 2, 1024, 64), (2, 2, 33, 96),
-                                             (2, 2, 63, 128), (1, 3, 129, 128)])
+                                             (2, 2, 63, 128), (1, 3, 129, 128), (2, 1, 16, 128), (2, 2, 32, 64)])
 @pytest.mark.parametrize("mask_kind", ["none", "padding", "all_masked", "all_lowest", "all_inf"])
 def test_context_attention_step_kernel(ctx, dt, B, heads, Lk, d, mask_kind):
     g = torch.Generator(device="cuda").manual_seed(Lk + d)

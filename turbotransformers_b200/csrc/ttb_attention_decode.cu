@@ -228,9 +228,11 @@ decode_merge_kernel(const float* __restrict__ partial, int rows_heads, int split
 // and the weighted values in one launch instead of five (bias + transpose of the queries, batched product, mask + softmax,
 // batched product, transpose). Bound by latency: over 20 x 8 heads and 45 keys of 64, K and V are 1.8 MB, 0.3 us of memory
 // time; a launch measures 3.7 us, the five it replaces 17. One CTA per (sequence, head); G lanes share a key, 16 bytes of it
-// each; scores stay in shared memory in fp32. A pass over the keys is one round trip to memory and takes 64 of them whatever
-// their width, so that few heads of long rows do not wait for twice or four times as many:
-// 1 x 8 heads of 128 in fp32 and 1024 keys 45.0 -> 26.1 us (25.9 in five launches), 20 x 8 108.6 -> 49.2 (273).
+// each; scores stay in shared memory in fp32. A pass over the keys, U for each group of lanes, is one round trip to memory and
+// takes 64 of them whatever their width, so that few heads of long rows do not wait for twice or four times as many round trips:
+// 1 x 8 heads of 128 in fp32 and 1024 keys 45.0 -> 26.1 us (25.9 in five launches), 20 x 8 108.6 -> 49.2 (273). Where a pass of
+// U = 4 holds all keys it stays at that: keys that are not there cost their arithmetic (20 x 8 heads of 128, 16 keys 2.6 us, 3.8
+// in a pass of 64; left out by a branch, the 64 are no longer computed side by side and everything is half as slow again).
 constexpr int kStepKeys = 1024;
 
 __device__ __forceinline__ void unpack_group(const uint4& raw, float (&f)[8], const __half* t) { unpack8(raw, f, t); }
@@ -239,13 +241,13 @@ __device__ __forceinline__ void unpack_group(const uint4& raw, float (&f)[4], co
   f[0] = __uint_as_float(raw.x); f[1] = __uint_as_float(raw.y); f[2] = __uint_as_float(raw.z); f[3] = __uint_as_float(raw.w);
 }
 
-template <typename T, int G>
+template <typename T, int G, int U>
 __global__ void __launch_bounds__(kThreads)
 context_attention_step_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ mask, int heads,
                               int Lk, int d, float scale, T* __restrict__ probs, T* __restrict__ out) {
   pdl_trigger();
   pdl_wait();
-  constexpr int VE = 16 / (int)sizeof(T), NG = kThreads / G, U = 64 / NG, kWarps = kThreads / 32;
+  constexpr int VE = 16 / (int)sizeof(T), NG = kThreads / G, kWarps = kThreads / 32;
   __shared__ float score[kStepKeys];
   __shared__ float part[kWarps][32 * VE];
   __shared__ float red[2][kWarps];
@@ -342,12 +344,16 @@ void launch_context_step(ttb_ctx* ctx, const void* q, const void* k, const void*
   const int lanes = (int)(d * sizeof(T) / 16);  // lanes that share a key
   const dim3 grid((unsigned)(B * heads));
 #define STEP_CASE(G)                                                                                                                             \
-  launch_pdl(context_attention_step_kernel<T, G>, grid, dim3(kThreads), 0, ctx->stream, (const T*)q, (const T*)k, (const T*)v, mask, (int)heads, \
+  if (Lk <= kThreads / G * 4) STEP_LAUNCH(G, 4);                                                                                                 \
+  else STEP_LAUNCH(G, 64 * G / kThreads)
+#define STEP_LAUNCH(G, U)                                                                                                                        \
+  launch_pdl(context_attention_step_kernel<T, G, U>, grid, dim3(kThreads), 0, ctx->stream, (const T*)q, (const T*)k, (const T*)v, mask, (int)heads, \
              (int)Lk, (int)d, scale, (T*)probs, (T*)out)
-  if (lanes <= 8) STEP_CASE(8);
-  else if (lanes <= 16) STEP_CASE(16);
-  else STEP_CASE(32);
+  if (lanes <= 8) { STEP_LAUNCH(8, 4); }
+  else if (lanes <= 16) { STEP_CASE(16); }
+  else { STEP_CASE(32); }
 #undef STEP_CASE
+#undef STEP_LAUNCH
 }
 
 int check_decode(ttb_ctx* ctx, const char* what, int dtype, const void* qkv, int64_t B, int64_t n_new, int64_t heads, int64_t d,
