@@ -207,3 +207,17 @@ def test_a_half_filled_memory_cache_is_projected_and_replaced_as_a_pair(given):
     again, _ = att(old, old, q, attn_type="context", layer_cache=half)  # filled: read, and left as they are
     assert torch.equal(again, want_out) and all(half[k] is kept[k] for k in kept)
     assert tt._cxx_module.device_status(0) == 0
+
+
+def test_context_attention_without_a_query_bias_is_refused():
+    H, heads, B, Lk = 128, 2, 2, 5
+    w = ref_driver.context_attention_weights(H, 17)
+    mod = OnmtStyleAttention(w, heads).to(DEV).half()
+    packed = list(tt.MultiHeadedAttention.pack_parameter(mod))
+    packed[5] = tt._cxx_module.Tensor.create_empty()
+    att = tt.MultiHeadedAttention(*packed, heads)
+    x = torch.randn(B, Lk, H, device=DEV).half()
+    filled = {k: torch.randn(B, heads, Lk, H // heads, device=DEV).half() for k in ("memory_keys", "memory_values")}
+    for q in (x[:, :1].contiguous(), x):  # a step and a sequence, over a kept memory
+        with pytest.raises(Exception, match="context"):
+            att(x, x, q, attn_type="context", layer_cache=dict(filled))

@@ -650,9 +650,9 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
   // The reference's sequence (multi_headed_attention.cpp:45-167, 308-354) on this library's kernels: three separate
   // projections, AddBiasTransposeForScore into [B, heads, L, d], scores materialised, mask + softmax, weighted values,
   // transpose back, output projection. The encoder memory's keys / values are projected once per sequence when the caller
-  // passes layer_cache entries, so a decoding step costs one query projection and two small batched products.
+  // passes layer_cache entries, so a decoding step costs one query projection and one kernel for the rest up to the output projection.
   TT_ENFORCE(output, "The output tensor should not be nullptr.");
-  TT_ENFORCE(!q_.weight().is_null() && !k_.weight().is_null() && !v_.weight().is_null(),
+  TT_ENFORCE(!q_.weight().is_null() && !q_.bias().is_null() && !k_.weight().is_null() && !v_.weight().is_null(),
              "context attention needs the separate q, k, v weights and biases");
   const Tensor& x = query_tensor;
   const int dt = FloatType(x, "attention input");
