@@ -162,12 +162,14 @@ def test_linear_ragged_width_into_padded_rows_then_compacted(ctx, M, N, K):
 
 
 # Ragged and misaligned rows stored word by word: odd and even widths, a width just past a tile, rows that start on odd elements
-# (an odd pitch, an odd offset), fewer rows than a tile. Everything around the product keeps its value.
+# (an odd pitch, an odd offset), fewer rows than a tile, 32-column tiles and K split over a cluster. Everything around the
+# product keeps its value.
 @pytest.mark.parametrize("dt", ["f16", "bf16", "f32"])
-@pytest.mark.parametrize("M,N,ldo,off", [(1, 50257, 50257, 0), (130, 1001, 1001, 0), (131, 9001, 9003, 1), (300, 4130, 4131, 0),
-                                         (600, 2305, 2305, 0), (2100, 5003, 5003, 0)])
-def test_linear_ragged_rows_straight_into_the_output(ctx, dt, M, N, ldo, off):
-    K = 136
+@pytest.mark.parametrize("M,N,ldo,off,K", [(1, 50257, 50257, 0, 136), (130, 1001, 1001, 0, 136), (131, 9001, 9003, 1, 136),
+                                           (300, 4130, 4131, 0, 136), (600, 2305, 2305, 0, 136), (2100, 5003, 5003, 0, 136),
+                                           (40, 99, 99, 0, 136), (131, 95, 97, 1, 136), (200, 66, 66, 0, 136), (5, 33, 35, 3, 8),
+                                           (64, 257, 257, 0, 3072)])
+def test_linear_ragged_rows_straight_into_the_output(ctx, dt, M, N, ldo, off, K):
     g = torch.Generator(device="cuda").manual_seed(N + M)
     a, w = (torch.randn(*s, generator=g, device="cuda").to(TORCH_DT[dt]) for s in ((M, K), (N, K)))
     buf = torch.full((off + M * ldo + 8,), 7.0, dtype=TORCH_DT[dt], device="cuda")

@@ -904,6 +904,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               for (int j = 0; j < 8; ++j) o.v[j] = v[i * 8 + j];
               o.store(dstp + i * 8);
             }
+          } else if (BN == 32 && EB == 2 && col0 + 32 <= p.N) {
+            // a whole chunk of a row that is not 16-byte aligned: words, shifted by half a word where the row is
+            uint4 q4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q4[i] = pack16<OutT>(&v[(i * 8) % 32]);
+            const uint32_t w[16] = {q4[0].x, q4[0].y, q4[0].z, q4[0].w, q4[1].x, q4[1].y, q4[1].z, q4[1].w,
+                                    q4[2].x, q4[2].y, q4[2].z, q4[2].w, q4[3].x, q4[3].y, q4[3].z, q4[3].w};
+            if ((reinterpret_cast<uintptr_t>(dstp) & 2) == 0) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) reinterpret_cast<uint32_t*>(dstp)[j] = w[j];
+            } else {
+              uint16_t* d16 = reinterpret_cast<uint16_t*>(dstp);
+              d16[0] = (uint16_t)w[0];
+#pragma unroll
+              for (int j = 0; j < 15; ++j) *reinterpret_cast<uint32_t*>(d16 + 2 * j + 1) = __funnelshift_r(w[j], w[j + 1], 16);
+              d16[31] = (uint16_t)(w[15] >> 16);
+            }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
