@@ -362,6 +362,14 @@ int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* ids, const i
  * call waits for. */
 int ttb_build_cu_seqlens(ttb_ctx* ctx, const int64_t* host_seq_lens, int64_t B, int32_t* cu_seqlens_device);
 
+/* Which kernel a product [M, N] = [M, K] . [N, K]^T of the tensor-core Linear runs on (nothing is launched), for tests and
+ * measurements. dtype: of the operands (F16, BF16, F32, I8); products: 1, 2 (bf16 with a second activation plane), 3 (fp32);
+ * two_plane_out: bf16 output in two planes; whole: output rows that 16-byte stores can write.
+ * plan[5] receives the tile's columns, the CTAs of a pair (1 or 2), the CTAs that share a tile along K, the number of tiles, and
+ * how many of them run at a time. */
+int ttb_linear_plan(ttb_ctx* ctx, int dtype, int out_dtype, int products, int two_plane_out, int whole, int64_t M, int64_t N, int64_t K,
+                    int64_t* plan);
+
 /* Self-test of the bounded device-side waits that every tensor-core kernel's hang safety rests on (no reference
  * counterpart). Launches one small kernel in which a thread waits, for at most `limit_cycles` SM cycles (<= 1e8, a
  * twentieth of a second), on a barrier that nothing arrives at. The wait gives up by itself; the kernel then records

@@ -95,12 +95,13 @@ def test_linear_counts_of_k_blocks_between_the_two_issuing_warps(ctx, M, N, K):
     assert ctx.device_status() == _capi.OK
 
 
-# One shape each at which the tile rule turns to another kernel: 32- and 64-column tiles, split K, 128 columns in one wave and in
-# several, 256 columns, CTA pairs
-@pytest.mark.parametrize("M,N,K", [(90, 768, 768), (300, 2304, 768), (120, 768, 3072), (792, 2304, 768), (2050, 768, 3072), (6500, 768, 768),
-                                   (1100, 3072, 768), (3200, 768, 3072)])
+# One shape or two for each kernel that the rule chooses from: columns, CTAs of a pair, CTAs along K
+@pytest.mark.parametrize("M,N,K,plan", [(90, 768, 768, (32, 1, 1)), (300, 2304, 768, (64, 1, 1)), (120, 768, 3072, (32, 1, 4)), (129, 1024, 4096, (32, 1, 2)),
+                                        (792, 2304, 768, (128, 1, 1)), (6500, 768, 768, (128, 1, 1)), (2600, 3072, 768, (256, 1, 1)),
+                                        (3300, 2304, 768, (256, 1, 1)), (3200, 768, 3072, (256, 2, 1)), (4096, 3072, 768, (256, 2, 1))])
 @pytest.mark.parametrize("epi", ["bias", "bias_residual"])
-def test_linear_on_every_side_of_the_tile_rule(ctx, M, N, K, epi):
+def test_linear_on_every_side_of_the_tile_rule(ctx, M, N, K, plan, epi):
+    assert ctx.linear_plan(_capi.F16, _capi.F16, 1, M, N, K)[:3] == plan
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a = torch.randn(M, K, generator=g, device="cuda").half()
     w = (torch.randn(N, K, generator=g, device="cuda") * 0.05).half()

@@ -76,6 +76,7 @@ SIGNATURES = {
     "ttb_prepack_weight_int8": (i32, [p, i32, p, i32, i64, i64, p, p]),
     "ttb_linear": (i32, [p, i32, p, i64, p, p, p, i64, i64, i64, i64, i32, p, i64]),
     "ttb_linear_ex": (i32, [p, C.POINTER(LinearArgs)]),
+    "ttb_linear_plan": (i32, [p, i32, i32, i32, i32, i32, i64, i64, i64, C.POINTER(i64)]),
     "ttb_split_tf32": (i32, [p, p, i64, p, p]),
     "ttb_linear_layernorm": (i32, [p, i32, p, i64, p, p, p, i64, p, p, f32, i64, i64, i64, p, i64]),
     "ttb_prepack_weight_int8_affine": (i32, [p, i32, p, i32, i64, i64, p, p, p]),
@@ -163,6 +164,12 @@ class Context:
         a = LinearArgs(dtype, out_dtype, ptr(A), ptr(A2), lda or K, ptr(W), ptr(W2), ptr(bias), ptr(residual), ldr or N, M, N, K,
                        epilogue, ptr(out), ptr(out_lo), ldo or N)
         self.check(lib().ttb_linear_ex(self.h, C.byref(a)))
+
+    def linear_plan(self, dtype, out_dtype, products, M, N, K, two_plane_out=False, whole_rows=True):
+        """What ttb_linear_plan reports: (columns, CTAs of a pair, CTAs along K, tiles, tiles at a time)."""
+        plan = (i64 * 5)()
+        self.check(lib().ttb_linear_plan(self.h, dtype, out_dtype, products, int(two_plane_out), int(whole_rows), M, N, K, plan))
+        return tuple(plan)
 
     def set_stream(self, cuda_stream):
         """Queue what follows on this cudaStream_t (an int; 0 = the legacy default stream)."""

@@ -905,7 +905,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               o.store(dstp + i * 8);
             }
           } else if (BN == 32 && EB == 2 && col0 + 32 <= p.N) {
-            // a whole chunk of a row that is not 16-byte aligned: words, shifted by half a word where the row is
+            // A whole chunk of a row that is not 16-byte aligned: words, shifted by half a word where the row is. Element by
+            // element, 200 x 772 x 768 in fp16 takes 8.8 us, so 5.6; 300 x 130 x 1024 9.3, 5.9; 1024 x 65 x 768 8.7, 5.6.
             uint4 q4[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) q4[i] = pack16<OutT>(&v[(i * 8) % 32]);
@@ -1013,12 +1014,23 @@ struct Operands {
   const void* W2;  // second W plane or null
 };
 
+// Whether 16-byte stores can write the output's rows. The staged epilogue reads bias and residual one 16-byte group at a time, and
+// a TMA store clips a row at 16-byte granularity: with a ragged N it writes zeros into the columns up to the next multiple of 16
+// bytes. So a ragged N takes this route only without bias/residual and when the caller declared those columns scratch (p.staged on
+// entry).
+template <typename OutT> bool whole_rows(const GemmParams& p) {
+  constexpr int EA = (int)sizeof(OutT) == 4 ? 4 : 8;  // output elements per 16 bytes
+  const bool aligned16 = ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.out_lo) | reinterpret_cast<uintptr_t>(p.bias) |
+                           reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.col_sum)) & 15) == 0;
+  return aligned16 && p.ldo % EA == 0 && (p.N % EA == 0 || (p.epilogue == TTB_EPI_NONE && p.staged == STORE_TMA && !p.out_lo)) &&
+         (!p.residual || p.ldr % EA == 0);
+}
+
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR>
 int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   using P = Planes<BN, TWO, KIND, OutT, VAR>;
   using C = Cfg<BN, TWO, SK, P::A, P::B>;
   constexpr int TILE_M = TWO ? 2 * BM : BM;
-  constexpr int EA = (int)sizeof(OutT) == 4 ? 4 : 8;  // output elements per 16 bytes
   CUtensorMap tmA0, tmA1, tmB0, tmB1;
   // a few rows (decoding): a box of 32 or 64 rows, so that a slot is not filled up with zeros first
   const int a_rows = (TWO || p.M > 64) ? BM : (p.M > 32 ? 64 : 32);
@@ -1033,13 +1045,7 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   GemmParams q = p;
   q.a_rows = a_rows;
   CUtensorMap tmO = tmA0, tmO2 = tmA0;  // placeholders when the direct-store epilogue is used
-  const bool aligned16 = ((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.out_lo) | reinterpret_cast<uintptr_t>(p.bias) |
-                           reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.col_sum)) & 15) == 0;
-  // The staged epilogue reads bias and residual one 16-byte group at a time, and a TMA store clips a row at 16-byte
-  // granularity: with a ragged N it writes zeros into the columns up to the next multiple of 16 bytes. So a ragged N takes
-  // this route only without bias/residual and when the caller declared those columns scratch (p.staged on entry).
-  const bool tma = BN >= 64 && aligned16 && p.ldo % EA == 0 && (p.N % EA == 0 || (p.epilogue == TTB_EPI_NONE && p.staged == STORE_TMA && !p.out_lo)) &&
-                   (!p.residual || p.ldr % EA == 0);
+  const bool tma = BN >= 64 && whole_rows<OutT>(p);
   // Ragged or misaligned rows without bias, residual or second plane (a 50257-wide vocabulary): word stores.
   // 8192 x 50257 x 768 in fp16 into a contiguous tensor: 845 us, against about 560 into padded rows and 585 for the pass that
   // compacted them. What is left over the padded form are the partial 32-byte sectors at both ends of each 128 bytes.
@@ -1258,67 +1264,83 @@ int max_resident_clusters(ttb_ctx* ctx, int split) {
   return n;
 }
 
-template <int KIND, typename OutT, int VAR = VAR_PLAIN>
-int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
-  // The shape decides between tiles by what each is expected to take: waves of tiles over the chip, each wave its k-blocks or,
-  // where that takes longer, its epilogue, plus what a launch costs around them. The constants are nanoseconds fitted to
-  // graph-replayed runs of M = 128 .. 8192 by (N, K) = (2304, 768), (768, 768), (3072, 768), (768, 3072) in fp16, int8, bf16
-  // as two products and fp32 as three: a k-block is 128 bytes of every row whatever the type, and costs the same.
-  // Against the fixed thresholds that came before (the widest tile that still gives every SM one), us: fp16 2048 x 768 x 3072
-  // 21.8 -> 16.6 (128-column tiles in one wave instead of 64-column ones in two), 792 x 2304 x 768 8.9 -> 7.4, 6500 x 768 x 768
-  // 18.2 -> 15.7, 3200 x 768 x 3072 25.8 -> 22.8 (pairs), fp32 3000 x 768 x 3072 124 -> 75, 520 x 2304 x 768 31 -> 22.
+// Which kernel runs a product: the tile's columns, the CTAs that share one (2 = a pair on 256 x 256, split_k = CTAs along K).
+struct TilePlan {
+  int columns, split_k;
+  bool pair;
+  int64_t tiles, slots;  // tiles of the product, and how many run at a time
+};
+
+// What a kernel is expected to take, in nanoseconds: `fixed` for the launch, the fill of its ring and its last epilogue, and for
+// each wave of tiles over the chip its k-blocks or, where that takes longer, its epilogue. A k-block is 128 bytes of every row
+// whatever the type, and costs the same; with two or three products issued from one slot it costs per_kb[1] or [2].
+struct TileCost {
+  int fixed;
+  int per_kb[3];
+  int epilogue[3];  // 16-bit rows; fp32 rows or two planes; rows that leave in words
+};
+// Fitted to graph-replayed runs of every kernel on M = 1 .. 18424 by 18 pairs (N, K) from 128 x 128 to 4096 x 1024, 768 x 3072 and
+// a vocabulary, in fp16, int8, bf16 as two products (16-bit, two-plane and fp32 outputs) and fp32 as three: 1914 shapes. The kernel
+// chosen is on average 0.3 % slower than the best one; the widest tile that still gives every SM one would be 5 % slower.
+// (Constants fitted to single products of BERT-base widths alone took the narrow tiles' shared slots to be cheaper than they are:
+// bf16 4096 x 3072 x 768 37.7 us against 32.6 in pairs, fp32 4096 x 2304 x 768 63.3 against 54.8.)
+constexpr TileCost kCostPair = {8900, {265, 0, 0}, {1050, 3700, 8000}};
+constexpr TileCost kCost256 = {5150, {385, 0, 0}, {2950, 6750, 8300}};
+constexpr TileCost kCost128 = {2750, {255, 430, 520}, {2250, 3500, 4500}};
+constexpr TileCost kCost64 = {2150, {230, 345, 430}, {1850, 1900, 4400}};
+constexpr TileCost kCost32 = {2100, {200, 280, 405}, {1100, 1550, 1200}};
+constexpr int kCostSplit = 5650, kCostSplitCta = 280;  // instead of kCost32.fixed: a cluster launch and the exchange
+
+// words: rows that no 16-byte store can write (ragged or misaligned).
+template <int KIND, typename OutT, int VAR>
+TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, bool words) {
   constexpr int IN_BYTES = (KIND == KIND_I8) ? 1 : (KIND == KIND_TF32 ? 4 : 2);
-  const int64_t num_m = (p.M + BM - 1) / BM;
-  auto tiles = [&](int bn) { return num_m * ((p.N + bn - 1) / bn); };
-  const int64_t pair_tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * (int64_t)((p.N + 255) / 256);
-  // With both planes of a k-block in one slot the narrow tiles, which are bound by their loads, take 2 / 1.5 times a single
-  // product's k-block for three / two products; the 256-column ones take 3 / 2 times.
   constexpr bool fused = Planes<32, false, KIND, OutT, VAR>::shared;
-  const int64_t num_kb = ((int64_t)p.K * IN_BYTES + BK_BYTES - 1) / BK_BYTES;
-  const int64_t wide = num_kb * p.npass, total_kb = fused ? num_kb : wide;
-  const int64_t narrow = (fused && p.npass > 1) ? num_kb * (p.npass + 1) / 2 : wide;
-  const int64_t sms = ctx->sm_count;
-  auto expect = [&](int64_t fixed, int64_t per_kb, int64_t epilogue, int64_t n, int64_t slots, int64_t kb) {
-    return fixed + (n + slots - 1) / slots * std::max(per_kb * kb, epilogue);
-  };
+  const int64_t sms = ctx->sm_count, num_m = (M + BM - 1) / BM;
+  auto tiles = [&](int bn) { return num_m * ((N + bn - 1) / bn); };
+  const int64_t pair_tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + 255) / 256);
+  const int64_t num_kb = (K * IN_BYTES + BK_BYTES - 1) / BK_BYTES;
+  const int64_t wide_kb = num_kb * npass;                    // pairs and 256 columns: the products as passes over K
+  const int64_t narrow_kb = fused ? num_kb : wide_kb;
+  const int products = fused ? npass - 1 : 0;                // index of per_kb
+  const int store = words ? 2 : (sizeof(OutT) == 4 || VAR == VAR_TWO_PLANES ? 1 : 0);
   // Pairs lose where both the mainloop and the row of tiles are short (bias + residual epilogue: N = K = 768, M = 18424 25.7 us
   // single against 26.3 paired; N = K = 1024, M = 16384 37.1 against 35.8) and where a tile is bound by its epilogue (int8,
   // K = 768: 8000 x 3072 24.9 single, 27.5 paired).
-  const int64_t k_bytes = (int64_t)p.K * IN_BYTES * p.npass;
-  const bool pair_pays = k_bytes >= 4096 || (k_bytes >= 1536 && p.N >= 1536) || (k_bytes >= 2048 && p.N >= 1024);
-  p.split_k = 1;
-  if (pair_mode() == 2 && pair_tiles >= sms / 2) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
-  int best = 0;
+  const int64_t k_bytes = K * IN_BYTES * npass;
+  const bool pair_pays = k_bytes >= 4096 || (k_bytes >= 1536 && N >= 1536) || (k_bytes >= 2048 && N >= 1024);
+  const TilePlan pair{256, 1, true, pair_tiles, sms / 2};
+  if (pair_mode() == 2 && pair_tiles >= sms / 2) return pair;
+  TilePlan best{};
   int64_t best_ns = INT64_MAX;
-  auto consider = [&](int which, int64_t ns) {
-    if (ns < best_ns) { best = which; best_ns = ns; }
+  auto consider = [&](const TilePlan& plan, int64_t fixed, const TileCost& c, int n_products, int64_t kb) {
+    const int64_t waves = (plan.tiles + plan.slots - 1) / plan.slots;
+    const int64_t ns = fixed + waves * std::max<int64_t>(c.per_kb[n_products] * kb, c.epilogue[store]);
+    if (ns < best_ns) { best = plan; best_ns = ns; }
   };
-  if (pair_mode() && pair_pays) consider(0, expect(7300, 310, 5400, pair_tiles, sms / 2, wide));
-  consider(256, expect(6300, 350, 6000, tiles(256), sms, wide));
-  consider(128, expect(3500, 235, 4300, tiles(128), sms, narrow));
-  consider(64, expect(3800, 177, 3000, tiles(64), sms, narrow));
-  consider(32, expect(3900, 155, 2000, tiles(32), sms, narrow));
-  // Few 128 x 32 tiles and a mainloop of several k-blocks: the CTAs of a cluster may share each tile's K range, so that the
-  // weights stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per
-  // tile, 8.7 split four ways; 12 k-blocks are not worth the exchange.
+  if (pair_mode() && pair_pays) consider(pair, kCostPair.fixed, kCostPair, 0, wide_kb);
+  consider({256, 1, false, tiles(256), sms}, kCost256.fixed, kCost256, 0, wide_kb);
+  consider({128, 1, false, tiles(128), sms}, kCost128.fixed, kCost128, products, narrow_kb);
+  consider({64, 1, false, tiles(64), sms}, kCost64.fixed, kCost64, products, narrow_kb);
   const int64_t t32 = tiles(32);
-  if (splitk_cap() > 1 && t32 * 2 <= sms && wide >= 24) {
-    int64_t s = sms / t32;
-    if (s > splitk_cap()) s = splitk_cap();
-    if (s > total_kb / 2) s = total_kb / 2;  // at least two k-blocks per CTA
-    // all clusters must be resident at once (one wave): how many clusters of s CTAs the device holds depends on how
-    // they pack into its GPCs
-    while (s >= 2 && t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, (int)s)) --s;
-    if (s >= 2) {
-      consider(1, expect(6900, 155, 2000, t32, t32, (narrow + s - 1) / s));
-      if (best == 1) {
-        p.split_k = (int)s;
-        return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
-      }
-    }
+  consider({32, 1, false, t32, sms}, kCost32.fixed, kCost32, products, narrow_kb);
+  // Few 128 x 32 tiles: the CTAs of a cluster may share each tile's K range, two k-blocks or more each, so that the weights
+  // stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per tile, 8.7 split
+  // four ways. All clusters must be resident at once (one wave): how many the device holds depends on how they pack into its GPCs.
+  for (int s = splitk_cap(); s >= 2; --s) {
+    if (t32 * s > sms || s > narrow_kb / 2 || t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, s)) continue;
+    consider({32, s, false, t32, t32}, kCostSplit + kCostSplitCta * (s - 1), kCost32, products, (narrow_kb + s - 1) / s);
   }
-  switch (best) {
-    case 0: return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
+  return best;
+}
+
+template <int KIND, typename OutT, int VAR = VAR_PLAIN>
+int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
+  const TilePlan plan = choose_tile<KIND, OutT, VAR>(ctx, p.M, p.N, p.K, p.npass, !whole_rows<OutT>(p));
+  p.split_k = plan.split_k;
+  if (plan.pair) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
+  if (plan.split_k > 1) return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
+  switch (plan.columns) {
     case 256: return launch_tc<256, KIND, OutT, false, false, VAR>(ctx, op, p);
     case 128: return launch_tc<128, KIND, OutT, false, false, VAR>(ctx, op, p);
     case 64: return launch_tc<64, KIND, OutT, false, false, VAR>(ctx, op, p);
@@ -1517,6 +1539,30 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   if (odt == TTB_F32) return pick_tile<KIND_BF16, float>(ctx, op, p);
   if (a->out_lo) return pick_tile<KIND_BF16, __nv_bfloat16, VAR_TWO_PLANES>(ctx, op, p);
   return pick_tile<KIND_BF16, __nv_bfloat16>(ctx, op, p);
+}
+
+extern "C" int ttb_linear_plan(ttb_ctx* ctx, int dtype, int out_dtype, int products, int two_plane_out, int whole, int64_t M, int64_t N, int64_t K,
+                               int64_t* plan) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, M > 0 && N > 0 && K > 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31), "linear_plan: bad shape");
+  TTB_REQUIRE(ctx, plan != nullptr, "linear_plan: null pointer");
+  DeviceGuard g(ctx->device);
+  TilePlan t{};
+  const bool words = !whole;
+  if (dtype == TTB_F32 && out_dtype == TTB_F32 && products >= 1 && products <= 3) t = choose_tile<KIND_TF32, float, VAR_PLAIN>(ctx, M, N, K, products, words);
+  else if (dtype == TTB_I8 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_I8, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
+  else if (dtype == TTB_F16 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_F16, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
+  else if (dtype == TTB_BF16 && out_dtype == TTB_F32 && (products == 1 || products == 2)) t = choose_tile<KIND_BF16, float, VAR_PLAIN>(ctx, M, N, K, products, words);
+  else if (dtype == TTB_BF16 && out_dtype == TTB_BF16 && (products == 1 || products == 2))
+    t = two_plane_out ? choose_tile<KIND_BF16, __nv_bfloat16, VAR_TWO_PLANES>(ctx, M, N, K, products, words)
+                      : choose_tile<KIND_BF16, __nv_bfloat16, VAR_PLAIN>(ctx, M, N, K, products, words);
+  else return fail(ctx, TTB_ERR_INVALID, "linear_plan: no such product");
+  plan[0] = t.columns;
+  plan[1] = t.pair ? 2 : 1;
+  plan[2] = t.split_k;
+  plan[3] = t.tiles;
+  plan[4] = t.slots;
+  return TTB_OK;
 }
 
 extern "C" int ttb_linear(ttb_ctx* ctx, int dtype, const void* A, int64_t lda, const void* Wp, const void* bias,
