@@ -1283,7 +1283,7 @@ struct TileCost {
 // a vocabulary, in fp16, int8, bf16 as two products (16-bit, two-plane and fp32 outputs) and fp32 as three: 1914 shapes. The kernel
 // chosen is on average 0.3 % slower than the best one; the widest tile that still gives every SM one would be 5 % slower.
 // (Constants fitted to single products of BERT-base widths alone took the narrow tiles' shared slots to be cheaper than they are:
-// bf16 4096 x 3072 x 768 37.7 us against 32.6 in pairs, fp32 4096 x 2304 x 768 63.3 against 54.8.)
+// bf16 4096 x 3072 x 768 37.7 us, 33.3 in pairs; fp32 4096 x 2304 x 768 63.3, 56.1.)
 constexpr TileCost kCostPair = {8900, {265, 0, 0}, {1050, 3700, 8000}};
 constexpr TileCost kCost256 = {5150, {385, 0, 0}, {2950, 6750, 8300}};
 constexpr TileCost kCost128 = {2750, {255, 430, 520}, {2250, 3500, 4500}};
