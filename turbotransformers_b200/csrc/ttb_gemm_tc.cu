@@ -10,14 +10,14 @@
 //   warp 11     : second producer on tiles of up to 64 columns, which loads W while warp 0 loads A
 //   warps 2..9  : epilogue      - tcgen05.ld the accumulator (one row per thread), apply scale/bias/activation/
 //                 residual in fp32, convert, stage through a swizzled shared-memory tile and TMA-store it
-// Two accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the MMAs of tile i+1.
+// Two accumulators (of BN TMEM columns, twice as many with two issuers) let the epilogue of tile i overlap the MMAs of tile i+1.
 //
 // Operand kinds: fp16, bf16 (kind::f16), int8 (kind::i8, int32 accumulator) and fp32 read as tf32 (kind::tf32).
 // A launch may run up to three passes over K into the same accumulator, each pass reading the first or the second
 // of two A maps and of two W maps. That is how operands wider than the tensor core's formats are used at full accuracy:
 //   bf16 activations kept as hi + lo planes :  A_hi.W + A_lo.W                       (2 passes)
 //   fp32 as three tf32 products             :  A_hi.W_hi + A_lo.W_hi + A_hi.W_lo     (3 passes)
-// Small problems (M <= 128 with a long K) are split along K over the CTAs of a cluster: every CTA accumulates its K range
+// Products of few tiles with a long K are split along K over the CTAs of a cluster: every CTA accumulates its K range
 // in its own TMEM, the others hand their partial tile to the first CTA through distributed shared memory, and that CTA
 // adds them in rank order and runs the epilogue, so the result does not depend on timing.
 // Every mbarrier wait is bounded: on expiry the CTA raises a flag, all roles fall through to the common
@@ -1280,18 +1280,21 @@ struct TilePlan {
 struct TileCost {
   int fixed;
   int per_kb[3];
-  int epilogue[3];  // 16-bit rows; fp32 rows or two planes; rows that leave in words
+  int epilogue[2];  // 16-bit rows; fp32 rows or two planes
+  // Rows that no 16-byte store can write leave in words, one row after the other: `first` and `row` for each of them, up to the 32
+  // that a warp has (from shared memory, wider tiles) or for all that the tile has (from registers, 32 columns).
+  int first, row, most;
 };
 // Fitted to graph-replayed runs of every kernel on M = 1 .. 18424 by 18 pairs (N, K) from 128 x 128 to 4096 x 1024, 768 x 3072 and
 // a vocabulary, in fp16, int8, bf16 as two products (16-bit, two-plane and fp32 outputs) and fp32 as three: 1914 shapes. The kernel
 // chosen is on average 0.3 % slower than the best one; the widest tile that still gives every SM one would be 5 % slower.
 // (Constants fitted to single products of BERT-base widths alone took the narrow tiles' shared slots to be cheaper than they are:
 // bf16 4096 x 3072 x 768 37.7 us, 33.3 in pairs; fp32 4096 x 2304 x 768 63.3, 56.1.)
-constexpr TileCost kCostPair = {8900, {265, 0, 0}, {1050, 3700, 8000}};
-constexpr TileCost kCost256 = {5150, {385, 0, 0}, {2950, 6750, 8300}};
-constexpr TileCost kCost128 = {2750, {255, 430, 520}, {2250, 3500, 4500}};
-constexpr TileCost kCost64 = {2150, {230, 345, 430}, {1850, 1900, 4400}};
-constexpr TileCost kCost32 = {2100, {200, 280, 405}, {1100, 1550, 1200}};
+constexpr TileCost kCostPair = {8900, {265, 0, 0}, {1050, 3700}, 500, 230, 32};
+constexpr TileCost kCost256 = {5150, {385, 0, 0}, {2950, 6750}, 1000, 240, 32};
+constexpr TileCost kCost128 = {2750, {255, 430, 520}, {2250, 3500}, 1200, 110, 32};
+constexpr TileCost kCost64 = {2150, {230, 345, 430}, {1850, 1900}, 1200, 120, 32};
+constexpr TileCost kCost32 = {2100, {200, 280, 405}, {1100, 1550}, 500, 13, 128};
 constexpr int kCostSplit = 5650, kCostSplitCta = 280;  // instead of kCost32.fixed: a cluster launch and the exchange
 
 // words: rows that no 16-byte store can write (ragged or misaligned).
@@ -1306,7 +1309,12 @@ TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, b
   const int64_t wide_kb = num_kb * npass;                    // pairs and 256 columns: the products as passes over K
   const int64_t narrow_kb = fused ? num_kb : wide_kb;
   const int products = fused ? npass - 1 : 0;                // index of per_kb
-  const int store = words ? 2 : (sizeof(OutT) == 4 || VAR == VAR_TWO_PLANES ? 1 : 0);
+  const int store = (sizeof(OutT) == 4 || VAR == VAR_TWO_PLANES) ? 1 : 0;
+  auto epilogue = [&](const TileCost& c) -> int64_t {  // of an average tile: the last row of tiles may have few rows
+    if (!words) return c.epilogue[store];
+    const int64_t rest = M % BM, full = M / BM;
+    return (full * (c.first + c.row * c.most) + (rest ? c.first + c.row * std::min<int64_t>(rest, c.most) : 0)) / num_m;
+  };
   // Pairs lose where both the mainloop and the row of tiles are short (bias + residual epilogue: N = K = 768, M = 18424 25.7 us
   // single against 26.3 paired; N = K = 1024, M = 16384 37.1 against 35.8) and where a tile is bound by its epilogue (int8,
   // K = 768: 8000 x 3072 24.9 single, 27.5 paired).
@@ -1318,7 +1326,7 @@ TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, b
   int64_t best_ns = INT64_MAX;
   auto consider = [&](const TilePlan& plan, int64_t fixed, const TileCost& c, int n_products, int64_t kb) {
     const int64_t waves = (plan.tiles + plan.slots - 1) / plan.slots;
-    const int64_t ns = fixed + waves * std::max<int64_t>(c.per_kb[n_products] * kb, c.epilogue[store]);
+    const int64_t ns = fixed + waves * std::max<int64_t>(c.per_kb[n_products] * kb, epilogue(c));
     if (ns < best_ns) { best = plan; best_ns = ns; }
   };
   if (pair_mode() && pair_pays) consider(pair, kCostPair.fixed, kCostPair, 0, wide_kb);
