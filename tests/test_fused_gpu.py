@@ -188,6 +188,27 @@ def test_linear_ragged_rows_straight_into_the_output(ctx, dt, M, N, ldo, off, K)
     assert bool((rows[:, N:] == 7.0).all()) and bool((buf[:off] == 7.0).all()) and bool((out[M * ldo:] == 7.0).all())
 
 
+# The Linear layer without a bias: widths of whole 16-byte groups, ragged ones straight from the product, and ragged ones that are
+# computed into padded rows and compacted (few rows of a wide odd width), on both sides of each line between them
+@pytest.mark.parametrize("dt", ["f16", "bf16"])
+@pytest.mark.parametrize("M,N,K", [(40, 20000, 64), (16, 20001, 64), (17, 20001, 64), (1024, 16385, 64), (1025, 16385, 64), (195, 16385, 768),
+                                   (196, 16385, 768), (40, 16385, 776), (40, 16383, 64), (40, 20002, 64)])
+def test_linear_layer_without_a_bias_at_ragged_widths(dt, M, N, K):
+    import turbotransformers_b200 as tt
+    from turbotransformers_b200.layers.utils import convert2tt_tensor, use_current_stream
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x, w = (torch.randn(*s, generator=g, device="cuda").to(TORCH_DT[dt]) for s in ((M, K), (N, K)))
+    out = tt._cxx_module.Tensor.create_empty()
+    use_current_stream(x)
+    tt._cxx_module.Linear(convert2tt_tensor(w), tt._cxx_module.Tensor.create_empty(), True)(convert2tt_tensor(x), out)
+    got = torch.utils.dlpack.from_dlpack(out.to_dlpack())
+    want = x.double() @ w.double().T
+    assert tuple(got.shape) == (M, N) and got.is_contiguous()
+    # fp32 sums, one rounding to the type
+    assert float((got.double() - want).abs().max()) < (2.0 ** -11 if dt == "f16" else 2.0 ** -8) * float(want.abs().max()) + 1e-4 * math.sqrt(K)
+    assert tt._cxx_module.device_status(0) == 0
+
+
 def test_linear_weight_given_as_out_in(ctx):
     # is_trans_weight=True in the reference: the weight arrives as [N,K] and is only converted
     r = rng(5)

@@ -1067,10 +1067,15 @@ void Linear::operator()(const Tensor& input, Tensor* output) const {
   const int dt = core::ToTTBDtype(input.dtype());
   const int64_t N = dense_.out_dim(is_trans_), M = input.rows();
   output->Reshape(input.dtype(), WithLast(input, N), kDLCUDA, input.device_id(), "Linear/Reshape");
-  if (dt != TTB_F32 && N % 8 != 0 && !dense_.bias().is_null()) {
-    // Output rows that are not a multiple of 16 bytes, with a bias: the GEMM would add it and store element by element.
-    // Compute into a row-padded scratch, then compact. (Without a bias, such as a 50257-wide tied vocabulary, the GEMM stores
-    // ragged rows itself.)
+  // Output rows that are not a multiple of 16 bytes. With a bias the GEMM would add it and store element by element: compute into
+  // a row-padded scratch, then compact. Without one, such as a 50257-wide tied vocabulary, the GEMM stores ragged rows itself, in
+  // words; but where half of very many columns' rows are shifted by half a word (an odd width), and the product is too short to
+  // cover them, the padded form is still the faster one. us, padded / straight, 50257 columns in fp16: M = 200, K = 64 20.0 / 30.6,
+  // K = 256 22.6 / 31.8, K = 768 35.2 / 35.8; M = 32, K = 768 17.2 / 20.7; M = 300, K = 768 56.4 / 47.1; one row is 1.2 to 1.35 times
+  // faster straight at any K. (30522 columns: straight by up to 2.3 times throughout.)
+  const int64_t depth = dense_.in_dim(is_trans_) * (dt == TTB_BF16 && input.lo() && core::PreciseBF16() ? 2 : 1);
+  const bool shifted = N % 2 != 0 && N >= 16384 && M > 16 && M <= 1024 && depth <= 768 && M * depth <= 150000;
+  if (dt != TTB_F32 && N % 8 != 0 && (shifted || !dense_.bias().is_null())) {
     const int64_t Np = (N + 7) / 8 * 8;
     ttb_ctx* c = DeviceContext(input.device_id());
     Tensor padded(nullptr);
