@@ -164,3 +164,44 @@ def test_transformer_decoder_stack_fp32_matches_restatement():
     got = outs.transpose(0, 1).cpu().numpy()
     assert np.abs(got[keep] - want[keep]).max() < 2e-4
     assert np.abs(attns["std"].transpose(0, 1).cpu().numpy()[keep] - attn[keep]).max() < 1e-4
+
+
+class LayerOfACaller(tt.TransformerDecoderLayer):
+    """The framework's layer under a caller's class: the decoder runs it layer by layer on torch tensors."""
+
+    def __call__(self, *args, **kwargs):
+        out = super().__call__(*args, **kwargs)
+        self.calls = getattr(self, "calls", 0) + 1
+        return out
+
+
+@pytest.mark.parametrize("dt,steps", [("f16", 3), ("bf16", 3), ("f16", None), ("f32", None)])
+@pytest.mark.parametrize("B", [1, 3])
+@pytest.mark.parametrize("copy_attn", [False, True])
+def test_the_pass_over_runtime_tensors_equals_the_layer_by_layer_pass(dt, steps, B, copy_attn):
+    H, F, heads, Lt, Ls, n_layers, vocab = 256, 512, 4, 4, 9, 3, 50
+    torch.manual_seed(1)
+    lws = [round_weights(ref_driver.decoder_layer_weights(H, F, 80 + i), dt) for i in range(n_layers)]
+    modules = [OnmtStyleDecoderLayer(lw, heads).to(DEV).to(TORCH_DT[dt]) for lw in lws]
+    emb, ln = Embeddings(vocab, H).to(DEV).to(TORCH_DT[dt]), torch.nn.LayerNorm(H, eps=1e-6).to(DEV).to(TORCH_DT[dt])
+    memory_bank = torch.randn(Ls, B, H, device=DEV).to(TORCH_DT[dt])
+    lengths = torch.tensor([Ls, 5, 7][:B], device=DEV)
+    tgt = torch.randint(2, vocab, (Lt, B, 1), device=DEV)
+    tgt[3, B - 1, 0] = Embeddings.word_padding_idx
+    results = []
+    for cls in (tt.TransformerDecoderLayer, LayerOfACaller):
+        own = [tt.TransformerDecoderLayer.from_onmt(m) for m in modules]
+        layers = [cls(layer.self_attn, layer.context_attn, layer.feed_forward) for layer in own]
+        dec = tt.TransformerDecoder(emb, layers, ln, copy_attn)
+        dec.init_state(torch.zeros(Ls, B, 1), memory_bank, None)
+        if steps is None:
+            passes = [dec(tgt, memory_bank, memory_lengths=lengths)]
+        else:
+            passes = [dec(tgt[t:t + 1], memory_bank, step=t, memory_lengths=lengths) for t in range(steps)]
+        results.append(passes)
+        assert cls is tt.TransformerDecoderLayer or all(layer.calls == len(passes) for layer in layers)
+    for (out, attns), (want_out, want_attns) in zip(*results):
+        assert torch.equal(out, want_out) and set(attns) == set(want_attns) == ({"std", "copy"} if copy_attn else {"std"})
+        assert all(torch.equal(attns[k], want_attns[k]) for k in attns)
+        assert tuple(attns["std"].shape) == (out.shape[0], B, Ls)
+    assert tt._cxx_module.device_status(0) == 0

@@ -69,30 +69,72 @@ def test_linear_matches_unfused_reference(ctx, dt, M, N, K, epi):
     assert maxdiff(got, want) < tol
 
 
-# 128 x 32 tiles (one per block, then several), 128 x 64 and 128 x 128 tiles: one k-block, an odd count that leaves the ring of
-# slots in the middle between two tiles, a ragged last k-block, and split-K ranges of odd length (K = 1984: 31 k-blocks)
-@pytest.mark.parametrize("M,N", [(40, 96), (40, 9504), (1100, 700), (2500, 1200)])
-@pytest.mark.parametrize("K", [8, 64, 192, 584, 1984])
-def test_linear_counts_of_k_blocks_between_the_two_issuing_warps(ctx, M, N, K):
-    r = rng(M + N + K)
-    a = rounded(r.standard_normal((M, K)).astype(np.float32), "f16")
-    w = rounded(r.standard_normal((K, N)).astype(np.float32) * 0.05, "f16")
-    want = a @ w
-    Wp = prepack(ctx, w, "f16")
-    out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
-    ctx.call("linear", _capi.F16, dev(a, "f16"), K, Wp, None, None, 0, M, N, K, EPIS["none"], out, N)
+# Counts of k-blocks between the two issuing warps, in every form of the product: one, even and odd ones (which leave the ring of
+# slots in the middle from one tile of a CTA to the next), a ragged last one; tiles of 32, 64 and 128 columns, several a CTA, and
+# K split over a cluster.
+RING_FORMS = {"f16": (_capi.F16, _capi.F16, 1, False), "i8": (_capi.I8, _capi.F16, 1, False), "f32 x 3": (_capi.F32, _capi.F32, 3, False),
+              "bf16 x 2, two planes": (_capi.BF16, _capi.BF16, 2, True), "bf16 x 2, f32": (_capi.BF16, _capi.F32, 2, False)}
+RING_SHAPES = [(40, 96), (600, 320), (3300, 701), (2500, 1200), (1100, 3001), (70, 40001)]
+RING_BLOCKS = [1, 2, 3, 5, 7, 24, 31]
+
+
+def ring_k(form, blocks):
+    per_block, step = {"f16": (64, 8), "i8": (128, 16), "f32 x 3": (32, 4)}.get(form, (64, 8))
+    return per_block * blocks - (step if blocks > 1 else 0)
+
+
+@pytest.mark.parametrize("form", RING_FORMS)
+def test_the_shapes_below_reach_every_ring(ctx, form):
+    dt, odt, products, planes = RING_FORMS[form]
+    plans = [ctx.linear_plan(dt, odt, products, M, N, ring_k(form, blocks), planes, N % 8 == 0)
+             for M, N in RING_SHAPES for blocks in RING_BLOCKS if blocks % 2]
+    several = {columns for columns, pair, split, tiles, slots in plans if pair == 1 and split == 1 and tiles > slots}
+    assert {32, 64, 128} <= several
+    assert any(split > 1 for _, _, split, _, _ in plans)
+
+
+@pytest.mark.parametrize("form", RING_FORMS)
+@pytest.mark.parametrize("M,N", RING_SHAPES)
+@pytest.mark.parametrize("blocks", RING_BLOCKS)
+def test_linear_counts_of_k_blocks_between_the_two_issuing_warps(ctx, form, M, N, blocks):
+    dt, odt, products, planes = RING_FORMS[form]
+    K = ring_k(form, blocks)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    runs = []
+    if form == "i8":
+        a, w = (torch.randint(-127, 128, s, generator=g, device="cuda", dtype=torch.int8) for s in ((M, K), (N, K)))
+        row_scale, w_scale = torch.full((M,), 2.0 ** -16, device="cuda"), torch.ones(1, device="cuda")
+        want = (a.double() @ w.double().T) * 2.0 ** -16
+        for _ in range(2):
+            out = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+            ctx.call("linear_int8", _capi.F16, a, row_scale, w, w_scale, None, None, 0, M, N, K, EPIS["none"], out, N)
+            runs.append([out])
+        tol = (2.0 ** -11 + 2.0 ** -24) * float(want.abs().max()) + 2.0 ** -24  # exact sums, one rounding to fp32, one to fp16
+    else:
+        x, y = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") * 0.05
+        store = {_capi.F16: torch.float16, _capi.BF16: torch.bfloat16, _capi.F32: torch.float32}
+        if products == 3:  # tf32 planes
+            (A, A2), (W, W2) = ([torch.empty_like(t), torch.empty_like(t)] for t in (x, y))
+            ctx.call("split_tf32", x, x.numel(), A, A2)
+            ctx.call("split_tf32", y, y.numel(), W, W2)
+            want = x.double() @ y.double().T
+            # what the three products drop, and an accumulator that truncates: see the tests of ttb_linear_ex
+            tol = max(2e-5, 1.4e-8 * K) * max(1.0, float(want.abs().max()))
+        else:
+            A, W, A2, W2 = x.to(store[dt]), y.to(store[dt]), None, None
+            if products == 2:
+                A2 = (x - A.float()).to(store[dt])
+            want = (A.double() + (A2.double() if A2 is not None else 0.0)) @ W.double().T
+            rounding = {"f16": 2.0 ** -11, "bf16 x 2, two planes": 2.0 ** -16}.get(form, 0.0)
+            tol = rounding * float(want.abs().max()) + (1e-4 * math.sqrt(K) if form == "f16" else 3e-5 * max(1.0, float(want.abs().max())))
+        for _ in range(2):
+            out, lo = (torch.full((M, N), float("nan"), dtype=store[odt], device="cuda") for _ in range(2))
+            ctx.linear_ex(dt, odt, A, W, M, N, K, EPIS["none"], out, A2=A2, W2=W2, out_lo=lo if planes else None)
+            runs.append([out, lo] if planes else [out])
     assert ctx.device_status() == _capi.OK
-    # fp32 sums rounded once to fp16
-    assert maxdiff(host(out), want) < 2.0 ** -11 * float(np.abs(want).max()) + 1e-4 * math.sqrt(K)
-    aq, wq = r.integers(-127, 128, (M, 16 * ((K + 15) // 16))), r.integers(-127, 128, (N, 16 * ((K + 15) // 16)))
-    scale = np.full(M, 2.0 ** -16, np.float32)
-    outq = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
-    ctx.call("linear_int8", _capi.F16, dev(aq.astype(np.int8)), dev(scale), dev(wq.astype(np.int8)), dev(np.ones(1, np.float32)), None, None, 0,
-             M, N, aq.shape[1], EPIS["none"], outq, N)
-    # exact int32 sums (below 2^25: one fp32 rounding at most), then one rounding to fp16
-    wantq = (aq.astype(np.float64) @ wq.T.astype(np.float64)) * 2.0 ** -16
-    assert maxdiff(host(outq), wantq) < (2.0 ** -11 + 2.0 ** -24) * float(np.abs(wantq).max()) + 2.0 ** -24
-    assert ctx.device_status() == _capi.OK
+    got = sum(t.double() for t in runs[0])
+    assert float((got - want).abs().max()) < tol  # (a NaN fails, too)
+    assert all(torch.equal(t, u) for t, u in zip(*runs))
 
 
 # One shape or two for each kernel that the rule chooses from: columns, CTAs of a pair, CTAs along K
