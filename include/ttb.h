@@ -339,6 +339,56 @@ int ttb_attention_decode(ttb_ctx* ctx, int dtype, const void* qkv, int64_t B, in
 int ttb_context_attention_step(ttb_ctx* ctx, int dtype, const void* q, const void* k, const void* v, const float* mask, int64_t B,
                                int64_t heads, int64_t Lk, int64_t d, float scale, void* probs, void* out);
 
+/* A whole stack of transformer layers over few rows (at most TTB_CHAIN_MAX_ROWS) as one kernel. A request of a few tokens, or
+ * one decoding step of a batch, is a chain of some hundred small dependent products; as kernels of their own each costs a launch and a
+ * ramp that is longer than its work. Here the operations are a list, run in order by one resident grid (a cooperative launch)
+ * with a barrier over the grid between them; each sees everything the ones before it wrote. F16.
+ *   TTB_CHAIN_LINEAR     out[M,N] = act(A' . W[N,K]^T + bias) + residual, where A' = A, or LayerNorm(A) with gamma and beta when gamma is
+ *                        given (K <= 1024; the normalised rows also go to normed[M,K] if that is not NULL; N = 0 does nothing
+ *                        else; see ttb_chain_rows for the rows). act is TTB_CHAIN_ACT_*. A, gamma, beta, W, bias, normed start on 16 bytes; lda % 8 == 0.
+ *                        K <= 8192, with a divisor of at most 1024 that is a multiple of 64 and at least 256.
+ *   TTB_CHAIN_ATTENTION  softmax(scale * q . k + mask) . v for `rows` rows of `heads` heads of 64, q in the columns h*64 of q[rows, ldq],
+ *                        into out[rows, ldo]. What a row sees, by `keys`:
+ *     TTB_CHAIN_KEYS_ROWS    the rows of its own sequence of `length` rows, their k and v in the columns heads*64 + h*64 and
+ *                            2*heads*64 + h*64 of q (up to itself if causal). With k_cache, v_cache they are also filed as tokens
+ *                            0 .. length - 1 of a paged cache (ttb_attention_decode).
+ *     TTB_CHAIN_KEYS_CACHE   tokens 0 .. past - 1 of k_cache, v_cache and itself (one row per sequence), which is filed as token `past`.
+ *     TTB_CHAIN_KEYS_MEMORY  k, v [rows, heads, length, 64] (one row per sequence).
+ *                        mask: fp32, element (sequence, key) at mask[sequence * mask_pitch + key], or NULL. probs (MEMORY only, or NULL):
+ *                        [rows, length], the probabilities of head 0; needs scores, fp32 [rows, length] of scratch.
+ * `workspace` is TTB_CHAIN_WORKSPACE bytes of device memory, which no other call uses until this one has finished. */
+#define TTB_CHAIN_MAX_ROWS 64
+#define TTB_CHAIN_MAX_OPS 128
+#define TTB_CHAIN_WORKSPACE 256
+enum { TTB_CHAIN_LINEAR = 0, TTB_CHAIN_ATTENTION = 1 };
+enum { TTB_CHAIN_ACT_NONE = 0, TTB_CHAIN_ACT_GELU = 1, TTB_CHAIN_ACT_RELU = 2 };
+enum { TTB_CHAIN_KEYS_ROWS = 0, TTB_CHAIN_KEYS_CACHE = 1, TTB_CHAIN_KEYS_MEMORY = 2 };
+typedef struct ttb_chain_linear {
+  const void *A, *W, *bias, *residual, *gamma, *beta;
+  void *normed, *out;
+  int32_t M, N, K, lda, ldr, ldo, act;
+  float eps;
+} ttb_chain_linear;
+typedef struct ttb_chain_attention {
+  const void *q, *k, *v;
+  const float* mask;
+  void *k_cache, *v_cache, *out, *probs;
+  float* scores;
+  int32_t rows, heads, length, past, ldq, ldo, mask_pitch, keys, causal;
+  float scale;
+} ttb_chain_attention;
+typedef struct ttb_chain_op {
+  int32_t kind, reserved;
+  union {
+    ttb_chain_linear linear;
+    ttb_chain_attention attention;
+  } u;
+} ttb_chain_op;
+int ttb_chain_forward(ttb_ctx* ctx, int dtype, const ttb_chain_op* ops, int n_ops, void* workspace);
+/* The most rows that a chain takes whose products are `hidden` deep, normalised or not, and `inner` deep, not normalised: shared memory
+ * holds the normalised rows and a ring of weights. 0: none. */
+int64_t ttb_chain_rows(int64_t hidden, int64_t inner);
+
 /* BERTEmbedding::operator() (layers/bert_embedding.cpp:24-65) in one pass: three gathers + LayerNorm.
  * ids is [n_tokens]. token_type_ids may be NULL (all 0). position_ids may be NULL: the position of token t is
  * then t - cu_seqlens[b] for the sequence b that owns it (packed batches, B+1 prefix sums), or t % seq_len

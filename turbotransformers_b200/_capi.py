@@ -25,6 +25,28 @@ class LinearArgs(C.Structure):
                 ("ldo", i64)]
 
 
+class ChainLinear(C.Structure):
+    """ttb_chain_linear of include/ttb.h."""
+    _fields_ = [(n, p) for n in ("A", "W", "bias", "residual", "gamma", "beta", "normed", "out")] + \
+               [(n, C.c_int32) for n in ("M", "N", "K", "lda", "ldr", "ldo", "act")] + [("eps", f32)]
+
+
+class ChainAttention(C.Structure):
+    """ttb_chain_attention of include/ttb.h."""
+    _fields_ = [(n, p) for n in ("q", "k", "v", "mask", "k_cache", "v_cache", "out", "probs", "scores")] + \
+               [(n, C.c_int32) for n in ("rows", "heads", "length", "past", "ldq", "ldo", "mask_pitch", "keys", "causal")] + [("scale", f32)]
+
+
+class ChainOp(C.Structure):
+    """ttb_chain_op of include/ttb.h."""
+    class _U(C.Union):
+        _fields_ = [("linear", ChainLinear), ("attention", ChainAttention)]
+    _fields_ = [("kind", C.c_int32), ("reserved", C.c_int32), ("u", _U)]
+
+
+CHAIN_WORKSPACE = 256
+CHAIN_KEYS_ROWS, CHAIN_KEYS_CACHE, CHAIN_KEYS_MEMORY = 0, 1, 2
+
 # name -> (restype, argtypes); must list every function declared in include/ttb.h
 SIGNATURES = {
     "ttb_ctx_create": (i32, [i32, p, C.POINTER(p)]),
@@ -52,6 +74,8 @@ SIGNATURES = {
     "ttb_kv_cache_append": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64]),
     "ttb_context_attention_step": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64, f32, p, p]),
     "ttb_attention_decode": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64, f32, p]),
+    "ttb_chain_forward": (i32, [p, i32, C.POINTER(ChainOp), i32, p]),
+    "ttb_chain_rows": (i64, [i64, i64]),
     "ttb_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, f32, f32, p]),
     "ttb_batch_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, i64, f32, f32, p]),
     "ttb_split_add_bias_transpose": (i32, [p, i32, p, p, i64, i64, i64, i64, p, p, p]),
@@ -164,6 +188,18 @@ class Context:
         a = LinearArgs(dtype, out_dtype, ptr(A), ptr(A2), lda or K, ptr(W), ptr(W2), ptr(bias), ptr(residual), ldr or N, M, N, K,
                        epilogue, ptr(out), ptr(out_lo), ldo or N)
         self.check(lib().ttb_linear_ex(self.h, C.byref(a)))
+
+    def chain_forward(self, ops):
+        """ttb_chain_forward on operations given as ("linear" | "attention", {field: value}); tensors are passed as their pointers."""
+        import torch
+        block = (ChainOp * len(ops))()
+        for b, (kind, fields) in zip(block, ops):
+            b.kind = {"linear": 0, "attention": 1}[kind]
+            for name, value in fields.items():
+                setattr(getattr(b.u, kind), name, value.data_ptr() if hasattr(value, "data_ptr") else value)
+        workspace = torch.empty(CHAIN_WORKSPACE, dtype=torch.uint8, device=f"cuda:{self.device}")
+        self.check(lib().ttb_chain_forward(self.h, F16, block, len(ops), workspace.data_ptr()))
+        torch.cuda.synchronize(self.device)  # the workspace is in use until the kernel has finished
 
     def linear_plan(self, dtype, out_dtype, products, M, N, K, two_plane_out=False, whole_rows=True):
         """What ttb_linear_plan reports: (columns, CTAs of a pair, CTAs along K, tiles, tiles at a time)."""
