@@ -150,9 +150,10 @@ class Tensor {
   // Non-owning view of sub-tensor n along the first axis.
   Tensor operator[](int64_t n) const;
 
-  // Companion planes a layer may attach to a 16-bit activation it produced, for the next layer to use (they travel with
+  // Companion planes a layer may attach to an activation it produced, for the next layer to use (they travel with
   // the tensor through moves, and are dropped when it is reshaped or exported):
-  //   lo  : same shape and dtype, what rounding to the 16-bit type dropped (value = this + lo to 16 significant bits)
+  //   lo  : same shape and dtype, what rounding to the 16-bit type dropped (value = this + lo to 16 significant bits); of an fp32
+  //         activation what the tensor cores drop of it, as tf32
   //   f32 : same shape in fp32, the unrounded value (the residual stream of a bf16 model)
   const Tensor* lo() const;
   const Tensor* f32() const;

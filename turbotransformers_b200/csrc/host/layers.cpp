@@ -42,6 +42,14 @@ std::vector<int64_t> WithLast(const Tensor& t, int64_t last) {
 // for the residual stream, an fp32 copy; see core::Tensor::lo() / f32().
 bool PreciseMode(int dt) { return dt == TTB_BF16 && core::PreciseBF16(); }
 
+// fp32 models on the tensor cores: an activation travels with the plane that a product takes beside it (core::Tensor::lo(): what the
+// tensor cores drop of it), written by the kernel that makes the activation.
+bool Fp32Planes(int dt) { return dt == TTB_F32 && core::Fp32TensorCores(); }
+float* NewLo(Tensor* t) {
+  const auto shape = ShapeOf(*t);
+  return t->NewExtras().lo.Reshape<float>(shape, kDLCUDA, t->device_id(), "fp32/lo_plane");
+}
+
 // out = LN(in) with the companion planes attached to `out` (already reshaped to its 16-bit shape). `in` is fp32 when
 // in_f32, else of out's dtype.
 void LayerNormPlanes(ttb_ctx* c, bool in_f32, const void* in, Tensor* out, const Tensor& gamma, const Tensor& beta, int64_t M, int64_t N,
@@ -64,6 +72,14 @@ void LayerNormWithInt8(ttb_ctx* c, Tensor* t, const Tensor& gamma, const Tensor&
   int8_t* q = static_cast<int8_t*>(ex.q8.Reshape(core::kInt8, {M, N}, kDLCUDA, t->device_id(), "linear/int8_activations"));
   float* s = ex.q8_scale.Reshape<float>({M}, kDLCUDA, t->device_id(), "linear/int8_row_scales");
   Check(ttb_layernorm_quant_int8(c, dt, ptr, ptr, q, s, gamma.raw(), beta.raw(), M, N, eps), c, name);
+}
+
+// t = LN(t + input + bias) of an fp32 model, with the plane that the next product takes beside it.
+void AddBiasLayerNormF32(ttb_ctx* c, Tensor* t, const Tensor& input, const Tensor& bias, const Tensor& gamma, const Tensor& beta, int64_t M, int64_t N,
+                         const char* name) {
+  float* lo = Fp32Planes(TTB_F32) ? NewLo(t) : nullptr;
+  Check(ttb_add_bias_layernorm_f32(c, t->mutableData<float>(), lo, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
+        name);
 }
 
 // dst (16-bit, [M, N]) = src (fp32): the re-layout kernel with an already K-major source is a plain conversion.
@@ -182,18 +198,25 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
   if (!bias && epilogue == TTB_EPI_BIAS) epilogue = TTB_EPI_NONE;
   if (ldo == 0) ldo = N;
   TT_ENFORCE(ldo == N || (dt != TTB_F32 && !use_int8()), "%s: a padded output pitch is only supported on the 16-bit path", name);
-  TT_ENFORCE((!out_lo && !f32_out) || (dt == TTB_BF16 && !use_int8()), "%s: two-plane and fp32 outputs belong to the bf16 path", name);
+  TT_ENFORCE((!out_lo && !f32_out) || (dt == TTB_BF16 && !use_int8()) || (out_lo && Fp32Planes(dt) && K % 4 == 0),
+             "%s: two-plane and fp32 outputs belong to the bf16 path, a second fp32 plane to the tensor cores", name);
   if (dt == TTB_F32 && core::Fp32TensorCores() && K % 4 == 0 && M > 0) {
     // fp32 on the tensor cores: activations split into two tf32 planes, weights kept as two planes, three products
     // accumulated in one GEMM with the elementwise kernel that followed MatMul in the reference as its epilogue
     // (mat_mul.cpp:81-96 selects tensor-op math for the same product)
+    // (an activation that brings its second plane along is not split again: as fp32 it is its own first plane)
     Tensor planes(nullptr);
-    float* a = planes.Reshape<float>({2, M, K}, kDLCUDA, x.device_id(), "linear/tf32_activation_planes");
-    Check(ttb_split_tf32(c, x.data<float>(), M * K, a, a + M * K), c, name);
     const float* w = PackedTf32(is_trans);
     ttb_linear_args args{};
     args.dtype = TTB_F32; args.out_dtype = TTB_F32;
-    args.A = a; args.A2 = a + M * K; args.lda = K;
+    if (x.lo()) {
+      args.A = x.raw(); args.A2 = x.lo()->raw();
+    } else {
+      float* a = planes.Reshape<float>({2, M, K}, kDLCUDA, x.device_id(), "linear/tf32_activation_planes");
+      Check(ttb_split_tf32(c, x.data<float>(), M * K, a, a + M * K), c, name);
+      args.A = a; args.A2 = a + M * K;
+    }
+    args.lda = K; args.out_lo = out_lo;
     args.W = w; args.W2 = w + N * K;
     args.bias = bias; args.residual = residual; args.ldr = N;
     args.M = M; args.N = N; args.K = K; args.epilogue = epilogue;
@@ -300,6 +323,8 @@ void BERTEmbedding::operator()(const Tensor& input_ids, const Tensor& position_i
     core::TensorExtras& ex = output_tensor->NewExtras();
     lo = ex.lo.Reshape(word_embedings_.dtype(), {B, L, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({B, L, H}, kDLCUDA, dev, "precise/residual_stream");
+  } else if (Fp32Planes(dt)) {
+    lo = NewLo(output_tensor);
   }
   Check(ttb_embedding_ln_planes(c, dt, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
                                 token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), nullptr, B, L, B * L,
@@ -327,6 +352,8 @@ void BERTEmbedding::Packed(const Tensor& input_ids, const std::vector<int64_t>& 
     core::TensorExtras& ex = output_tensor->NewExtras();
     lo = ex.lo.Reshape(word_embedings_.dtype(), {1, T, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({1, T, H}, kDLCUDA, dev, "precise/residual_stream");
+  } else if (Fp32Planes(dt)) {
+    lo = NewLo(output_tensor);
   }
   const core::CuSeqlensHandle cu = core::CuSeqlens(dev, seq_lens);
   Check(ttb_embedding_ln_planes(c, dt, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
@@ -548,6 +575,25 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
             "attention_fwd");
     }
     if (att_score) *att_score = Tensor(nullptr);
+  } else if (Fp32Planes(dt) && !att_score && !cache_keys && d == 64 && B <= 65535 && (!causal_ || !attention_mask.is_null())) {
+    // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own
+    Tensor qkv(nullptr);
+    qkv.Reshape(x.dtype(), {T, 3 * H}, kDLCUDA, dev, "self/qkv_out1/Reshape");
+    qkv_.Forward(*gemm_in, T, TTB_EPI_BIAS, nullptr, qkv.raw_mut(), is_trans_weight, "self/gemm012_fused");
+    const core::CuSeqlensHandle cu_handle = seq_lens ? core::CuSeqlens(dev, *seq_lens) : core::UniformCuSeqlens(dev, B, maxL);
+    const float* mask = nullptr;
+    int64_t mbs = 0, mrs = 0;
+    if (!attention_mask.is_null()) {
+      TT_ENFORCE(attention_mask.on_gpu() && core::SameType(attention_mask.dtype(), core::kFloat32),
+                 "the attention mask must be an fp32 tensor on the GPU");
+      TT_ENFORCE_EQ(attention_mask.shape(-1), maxL, "attention mask width must equal the (padded) key length");
+      mask = attention_mask.data<float>();
+      if (MaskIs2D(attention_mask)) { mbs = maxL; mrs = 0; }
+      else { mrs = maxL; mbs = maxL * maxL; }
+    }
+    float* lo = NewLo(&context);
+    Check(ttb_attention_f32(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, context.mutableData<float>(), lo), c,
+          "attention_f32");
   } else {
     // The reference's own sequence (multi_headed_attention.cpp:168-232,320-354), scores materialised.
     TT_ENFORCE(!cache_keys, "layer_cache decoding is provided for 16-bit models with 64-wide heads");
@@ -629,9 +675,7 @@ void MultiHeadedAttention::Finish(const Tensor& context, const Tensor& x, int64_
     dense_.Forward(context, T, TTB_EPI_BIAS, nullptr, output->raw_mut(), is_trans_weight, "gemm5");
   } else if (dt == TTB_F32) {
     dense_.Forward(context, T, TTB_EPI_NONE, nullptr, output->raw_mut(), is_trans_weight, "gemm5");
-    Check(ttb_add_bias_layernorm(c, dt, output->raw_mut(), x.raw(), dense_.bias().raw(), layernorm_gamma_.raw(),
-                                 layernorm_beta_.raw(), T, H, 1e-12f),
-          c, "AddBiasLayerNorm");
+    AddBiasLayerNormF32(c, output, x, dense_.bias(), layernorm_gamma_, layernorm_beta_, T, H, "AddBiasLayerNorm");
   } else {
     if (dense_.int8_mode() == PackedLinear::kInt8PerRow) {
       dense_.Forward(context, T, TTB_EPI_BIAS_RESIDUAL, x.raw(), output->raw_mut(), is_trans_weight, "gemm5");
@@ -799,7 +843,8 @@ void BertIntermediate::operator()(const Tensor& input_tensor, Tensor* output_ten
   output_tensor->Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "BertIntermediate/Reshape");
   void* out = output_tensor->raw_mut();
   void* lo = nullptr;
-  if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came
+  if (Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0) lo = NewLo(output_tensor);
+  else if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came
     lo = output_tensor->NewExtras().lo.Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "precise/lo_plane");
   // int8 (per-row scheme): BertOutput's Linear takes this activation as int8, so it leaves with its int8 form attached
   Tensor* q8 = dense_.int8_mode() == PackedLinear::kInt8PerRow ? output_tensor : nullptr;
@@ -823,9 +868,7 @@ void BertOutput::operator()(const Tensor& hidden_states, const Tensor& input_ten
   output_tensor->Reshape(hidden_states.dtype(), WithLast(hidden_states, N), kDLCUDA, hidden_states.device_id(), "BertOutput/Reshape");
   if (dt == TTB_F32) {
     dense_.Forward(hidden_states, M, TTB_EPI_NONE, nullptr, output_tensor->raw_mut(), false, "BertOutput/MatMul");
-    Check(ttb_add_bias_layernorm(c, dt, output_tensor->raw_mut(), input_tensor.raw(), dense_.bias().raw(), layer_norm_weight_.raw(),
-                                 layer_norm_bias_.raw(), M, N, 1e-12f),
-          c, "BertOutput/AddBiasLayerNorm");
+    AddBiasLayerNormF32(c, output_tensor, input_tensor, dense_.bias(), layer_norm_weight_, layer_norm_bias_, M, N, "BertOutput/AddBiasLayerNorm");
   } else if (PreciseMode(dt) && input_tensor.f32() && !dense_.use_int8()) {
     Tensor sum(nullptr);
     float* s = sum.Reshape<float>({M, N}, kDLCUDA, hidden_states.device_id(), "BertOutput/fp32_sum");
@@ -854,7 +897,7 @@ void ProjectAddNorm(const PackedLinear& dense, const Tensor& act_in, const Tenso
   out->Reshape(act_in.dtype(), ShapeOf(residual), kDLCUDA, act_in.device_id(), name);
   if (dt == TTB_F32) {
     dense.Forward(act_in, M, TTB_EPI_NONE, nullptr, out->raw_mut(), is_trans, name);
-    Check(ttb_add_bias_layernorm(c, dt, out->raw_mut(), residual.raw(), dense.bias().raw(), gamma.raw(), beta.raw(), M, N, 1e-12f), c, name);
+    AddBiasLayerNormF32(c, out, residual, dense.bias(), gamma, beta, M, N, name);
   } else if (PreciseMode(dt) && residual.f32() && !dense.use_int8()) {
     Tensor sum(nullptr);
     float* s = sum.Reshape<float>({M, N}, kDLCUDA, act_in.device_id(), "fp32_sum");
@@ -1006,12 +1049,14 @@ void PositionwiseFeedForward::operator()(const Tensor& x, Tensor* output, bool i
 
 void FusedAddBiasGELU::operator()(Tensor* t) const {
   const int dt = FloatType(*t, "FusedAddBiasGELU input");
+  t->DropExtras();  // they belong to the value that is overwritten
   ttb_ctx* c = DeviceContext(t->device_id());
   Check(ttb_add_bias_act(c, dt, t->raw_mut(), bias_.raw(), t->rows(), t->shape(-1), TTB_ACT_GELU), c, "FusedAddBiasGELU");
 }
 
 void FusedAddBiasLayerNorm::operator()(const Tensor& input_tensor, Tensor* output_tensor) const {
   const int dt = FloatType(*output_tensor, "FusedAddBiasLayerNorm output");
+  output_tensor->DropExtras();  // they belong to the value that is overwritten
   SameTypeDevice(input_tensor, *output_tensor, "FusedAddBiasLayerNorm");
   ttb_ctx* c = DeviceContext(output_tensor->device_id());
   Check(ttb_add_bias_layernorm(c, dt, output_tensor->raw_mut(), input_tensor.raw(), bias_.raw(), norm_weight_.raw(), norm_bias_.raw(),

@@ -150,6 +150,17 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
+// What the tensor core drops of an fp32 value that it reads as tf32 (its last 13 bits), rounded to tf32: x as it is and this are the two
+// planes of an fp32 operand.
+__device__ __forceinline__ float tf32_rest(float x) {
+  uint32_t u;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x - __uint_as_float(__float_as_uint(x) & 0xffffe000u)));
+  return __uint_as_float(u);
+}
+// What is left of v after it has been stored as T and read by a product: the "lo" plane of a two-plane value.
+template <typename T> __device__ __forceinline__ float rest_of(float v) { return v - to_f(from_f<T>(v)); }
+template <> __device__ __forceinline__ float rest_of<float>(float v) { return tf32_rest(v); }
+
 // A group of 8 consecutive elements moved with 16-byte (or 2x16-byte for fp32) accesses.
 template <typename T> struct Vec8 {
   float v[8];

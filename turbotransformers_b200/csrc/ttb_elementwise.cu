@@ -109,7 +109,7 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
               if (out_lo) {
                 Vec8<TOut> l;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) l.v[j] = o.v[j] - to_f(from_f<TOut>(o.v[j]));
+                for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j]);
                 l.store(out_lo + row * N + col);
               }
             }
@@ -471,7 +471,7 @@ layernorm_rows_generic_kernel(const TIn* x, const TIn* __restrict__ residual, co
       const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
       out[row * N + c] = from_f<TOut>(y);
       if (out_f32) out_f32[row * N + c] = y;
-      if (out_lo) out_lo[row * N + c] = from_f<TOut>(y - to_f(from_f<TOut>(y)));
+      if (out_lo) out_lo[row * N + c] = from_f<TOut>(rest_of<TOut>(y));
     }
   }
 }
@@ -694,7 +694,7 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
       const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
       out[t * hidden + c] = from_f<T>(y);
       if (out_f32) out_f32[t * hidden + c] = y;
-      if (out_lo) out_lo[t * hidden + c] = from_f<T>(y - to_f(from_f<T>(y)));
+      if (out_lo) out_lo[t * hidden + c] = from_f<T>(rest_of<T>(y));
     }
   }
 }
@@ -1266,6 +1266,15 @@ extern "C" int ttb_add_bias_layernorm(ttb_ctx* ctx, int dtype, void* out, const 
                      return (launch_layernorm<T, T, true>(ctx, (const T*)out, (const T*)input, (const T*)bias, (const T*)gamma,
                                                           (const T*)beta, (T*)out, nullptr, nullptr, M, N, eps)));
   return TTB_OK;
+}
+
+extern "C" int ttb_add_bias_layernorm_f32(ttb_ctx* ctx, float* out, float* out_lo, const float* input, const float* bias, const float* gamma,
+                                          const float* beta, int64_t M, int64_t N, float eps) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, M >= 0 && N > 0, "add_bias_layernorm: bad shape M=%lld N=%lld", (long long)M, (long long)N);
+  TTB_REQUIRE(ctx, M == 0 || (out && input && bias && gamma && beta), "add_bias_layernorm: null pointer");
+  DeviceGuard g(ctx->device);
+  return launch_layernorm<float, float, true>(ctx, out, input, bias, gamma, beta, out, out_lo, nullptr, M, N, eps);
 }
 
 extern "C" int ttb_layernorm(ttb_ctx* ctx, int dtype, const void* in, void* out, const void* gamma, const void* beta,

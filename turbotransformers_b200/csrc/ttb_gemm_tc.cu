@@ -96,7 +96,7 @@ struct GemmParams {
   int pass_a, pass_b;      // bit p set: pass p reads the second A map / the second W map
   void* out;
   long long ldo;
-  void* out_lo;            // 16-bit outputs: plane that receives v - round(v) (same pitch as out), or null
+  void* out_lo;            // plane that receives what is left of v after it has been stored and read by a product (same pitch as out), or null
   const void* bias;        // OutT[N] or null
   const void* residual;    // OutT[M, ldr] or null
   long long ldr;
@@ -151,8 +151,6 @@ template <> __device__ __forceinline__ uint4 pack16<__nv_bfloat16>(const float* 
 template <> __device__ __forceinline__ uint4 pack16<float>(const float* f) {
   return make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
 }
-// What is left of v after rounding it to OutT (the "lo" plane of a two-plane 16-bit value).
-template <typename OutT> __device__ __forceinline__ float round_residue(float v) { return v - to_f(from_f<OutT>(v)); }
 
 // Instruction descriptor: accumulator format, operand formats, both operands K-major, N>>3, M>>4.
 template <int KIND, int BN, bool TWO = false> __host__ __device__ constexpr uint32_t make_idesc() {
@@ -187,7 +185,7 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 
 // ---- the kernel -----------------------------------------------------------------------------------
 // VAR selects an epilogue variant that costs registers, so that the plain kernels do not carry it:
-//   VAR_PLAIN, VAR_TWO_PLANES (16-bit output written as hi + lo planes), VAR_AFFINE (int8 with a per-tensor zero point),
+//   VAR_PLAIN, VAR_TWO_PLANES (output written with a second plane, what a product drops of the first), VAR_AFFINE (int8 with a per-tensor zero point),
 //   VAR_WORDS (STORE_WORDS; carried by every kernel it cost packed fp16 batches 1 %: 4120 -> 4164 us, 4149 against 4159 without)
 enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3 };
 
@@ -405,7 +403,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     constexpr int G16 = 32 * EB / 16;            // 16-byte groups per row of a 32-column half (4 or 8)
     constexpr int P16 = Per16<OutT>::value;      // elements per 16-byte group (8 or 4)
     constexpr int LO_N = (VAR == VAR_TWO_PLANES) ? 8 : 1;  // 16-byte groups of a chunk's second plane kept in registers
-    static_assert(VAR != VAR_TWO_PLANES || sizeof(OutT) == 2, "two-plane outputs are 16-bit");
     static_assert(VAR != VAR_AFFINE || KIND == KIND_I8, "the zero-point correction belongs to the int8 kind");
     const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are the ones this warp may read
     const int half = (warp - 2) >> 2;   // which half of the tile's column chunks this warp takes
@@ -742,7 +739,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               *reinterpret_cast<uint4*>(buf + lane * 128 + (((hh * G16 + g) ^ (lane & 7)) << 4)) = pack16<OutT>(&v[g * P16]);
             if (two_planes) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = round_residue<OutT>(v[j]);
+              for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j]);
 #pragma unroll
               for (int g = 0; g < G16; ++g) lo_pack[(hh * G16 + g) % LO_N] = pack16<OutT>(&v[g * P16]);
             }
@@ -897,7 +894,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           OutT* dstp = (plane == 0 ? out : static_cast<OutT*>(p.out_lo)) + (long long)row * p.ldo + col0;
           if (plane == 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = round_residue<OutT>(v[j]);
+            for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j]);
           }
           if (full) {
 #pragma unroll
@@ -1527,7 +1524,7 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   TTB_REQUIRE(ctx, dt == TTB_F16 || dt == TTB_BF16 || dt == TTB_F32, "linear_ex: operand dtype must be F16, BF16 or F32");
   TTB_REQUIRE(ctx, odt == dt || (odt == TTB_F32 && dt != TTB_F32), "linear_ex: the output is of the operand dtype, or F32 for 16-bit operands");
   TTB_REQUIRE(ctx, !a->W2 || (a->A2 && dt == TTB_F32), "linear_ex: a second weight plane belongs to the three-pass fp32 form (A, A2, W, W2)");
-  TTB_REQUIRE(ctx, !a->out_lo || odt == TTB_BF16, "linear_ex: the second output plane exists for BF16 outputs only");
+  TTB_REQUIRE(ctx, !a->out_lo || (odt == dt && dt != TTB_F16), "linear_ex: the second output plane exists for BF16 and F32 products only");
   const int pad_scratch = (a->epilogue & TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH) ? 1 : 0;
   const int epilogue = a->epilogue & ~TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH;
   const int k_align = dt == TTB_F32 ? 4 : 8;
@@ -1545,7 +1542,7 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   p.bias = a->bias; p.residual = a->residual; p.ldr = a->ldr;
   p.epilogue = epilogue; p.staged = pad_scratch ? STORE_TMA : STORE_DIRECT; p.split_k = 1; p.status = ctx->d_status;
   const Operands op{a->A, a->A2, a->lda, a->W, a->W2};
-  if (dt == TTB_F32) return pick_tile<KIND_TF32, float>(ctx, op, p);
+  if (dt == TTB_F32) return a->out_lo ? pick_tile<KIND_TF32, float, VAR_TWO_PLANES>(ctx, op, p) : pick_tile<KIND_TF32, float>(ctx, op, p);
   if (dt == TTB_F16) return odt == TTB_F32 ? pick_tile<KIND_F16, float>(ctx, op, p) : pick_tile<KIND_F16, __half>(ctx, op, p);
   if (odt == TTB_F32) return pick_tile<KIND_BF16, float>(ctx, op, p);
   if (a->out_lo) return pick_tile<KIND_BF16, __nv_bfloat16, VAR_TWO_PLANES>(ctx, op, p);
