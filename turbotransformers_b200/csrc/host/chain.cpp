@@ -1,0 +1,259 @@
+#include "chain.h"
+
+#include <algorithm>
+#include <cmath>
+#include <initializer_list>
+
+namespace turbo_transformers {
+namespace layers {
+
+using core::Check;
+using core::DeviceContext;
+using core::Tensor;
+
+namespace {
+
+constexpr int64_t kHead = 64;
+
+bool Aligned(std::initializer_list<const Tensor*> ts) {
+  uintptr_t x = 0;
+  for (const Tensor* t : ts) x |= reinterpret_cast<uintptr_t>(t->raw());
+  return (x & 15) == 0;
+}
+bool Half(const Tensor& t, const Tensor& like) {
+  return t.on_gpu() && core::SameType(t.dtype(), core::kFloat16) && t.device_id() == like.device_id();
+}
+bool Vector(const Tensor& t, int64_t n, const Tensor& like) { return Half(t, like) && t.numel() == n; }
+
+// A [K, N] product with a bias over rows like `x`.
+bool LinearFits(const PackedLinear& l, bool trans, int64_t K, int64_t N, const Tensor& x) {
+  return !l.use_int8() && Half(l.weight(), x) && l.weight().n_dim() == 2 && l.in_dim(trans) == K && l.out_dim(trans) == N && N % 8 == 0 && N <= 16384 &&
+         Vector(l.bias(), N, x) && Aligned({&l.bias()});
+}
+bool NormFits(const Tensor& gamma, const Tensor& beta, int64_t H, const Tensor& x) {
+  return Vector(gamma, H, x) && Vector(beta, H, x) && Aligned({&gamma, &beta});
+}
+// The rows up to which one kernel is the faster route: above, every CTA's normalising of all rows and its reading of all of the wide
+// activation outweigh the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 307 / 412, 16 340 / 434,
+// 24 421 / 436, 32 448 / 436, 64 672 / 484 (300 cached: 392 / 494, 479 / 527, 542 / 550 at 16, 24, 32); BERT-base, tokens: 1 286 / 432, 16 318 / 439,
+// 24 394 / 427, 32 409 / 437, 48 529 / 436; BERT-large 16 689 / 873, 32 888 / 868. Layers with context attention are more launches, and
+// Python, for the same products: six steps of six layers, 200 source tokens, 1 row 1443 / 3579, 32 2277 / 3659, 64 3401 / 3641.
+constexpr int64_t kMostRows = 24, kMostRowsContext = TTB_CHAIN_MAX_ROWS;
+bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
+  if (x.n_dim() != 3 || !x.on_gpu() || !core::SameType(x.dtype(), core::kFloat16)) return false;
+  const int64_t rows = x.numel() ? x.rows() : 0, H = x.shape(2);
+  // (narrower models keep the layer-by-layer pass, whose results are bit for bit those of its layers called one by one)
+  return rows > 0 && H == heads * kHead && H >= 512 && Aligned({&x}) && rows <= std::min(most, ttb_chain_rows(H, inner));
+}
+
+// The call's scratch memory, dealt out in pieces.
+struct Scratch {
+  Tensor buffer{nullptr};
+  size_t bytes = 0;
+  char* base = nullptr;
+  size_t Add(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  }
+  void Allocate(int dev) { base = reinterpret_cast<char*>(buffer.Reshape(core::kInt8, {(int64_t)bytes}, kDLCUDA, dev, "chain/scratch")); }
+};
+
+struct Ops {
+  std::vector<ttb_chain_op> list;
+  int M;
+  ttb_chain_linear* Linear(const void* A, int64_t K, const void* W, const void* bias, int64_t N, void* out, int act = TTB_CHAIN_ACT_NONE,
+                           const void* residual = nullptr) {
+    list.emplace_back();
+    ttb_chain_linear& o = list.back().u.linear;
+    list.back().kind = TTB_CHAIN_LINEAR;
+    o = ttb_chain_linear{};
+    o.A = A; o.W = W; o.bias = bias; o.residual = residual; o.out = out;
+    o.M = M; o.N = (int32_t)N; o.K = (int32_t)K; o.lda = (int32_t)K; o.ldr = (int32_t)N; o.ldo = (int32_t)N; o.act = act;
+    return &o;
+  }
+  void Norm(ttb_chain_linear* o, const Tensor& gamma, const Tensor& beta, float eps, void* normed = nullptr) {
+    o->gamma = gamma.raw(); o->beta = beta.raw(); o->eps = eps; o->normed = normed;
+  }
+  ttb_chain_attention* Attention(int keys, const void* q, int64_t ldq, int64_t heads, int64_t length, void* out) {
+    list.emplace_back();
+    ttb_chain_attention& o = list.back().u.attention;
+    list.back().kind = TTB_CHAIN_ATTENTION;
+    o = ttb_chain_attention{};
+    o.keys = keys; o.q = q; o.ldq = (int32_t)ldq; o.out = out; o.ldo = (int32_t)(heads * kHead); o.rows = M; o.heads = (int32_t)heads;
+    o.length = (int32_t)length; o.scale = 1.0f / std::sqrt((float)kHead);
+    return &o;
+  }
+};
+
+}  // namespace
+
+bool Chain::Encoder(const std::vector<EncoderBlock>& blocks, const Tensor& x, const Tensor& mask, Tensor* out) {
+  if (blocks.empty() || x.is_null() || 5 * blocks.size() + 1 > TTB_CHAIN_MAX_OPS) return false;
+  const int64_t heads = blocks[0].attention->num_attention_heads_;
+  const int64_t F = blocks[0].intermediate->dense_.out_dim(false);
+  if (!RowsFit(x, heads, F, kMostRows)) return false;
+  const int64_t B = x.shape(0), L = x.shape(1), H = x.shape(2), M = B * L;
+  const float* mask_ptr = nullptr;
+  if (!mask.is_null()) {  // one row of L keys per sequence; everything else is the general path's business
+    if (!mask.on_gpu() || mask.device_id() != x.device_id() || !core::SameType(mask.dtype(), core::kFloat32) || mask.n_dim() < 2 || mask.n_dim() > 4 ||
+        mask.shape(-1) != L || mask.numel() != B * L || mask.shape(0) != B)
+      return false;
+    mask_ptr = mask.data<float>();
+  }
+  for (const EncoderBlock& b : blocks) {
+    const MultiHeadedAttention& a = *b.attention;
+    if (a.num_attention_heads_ != heads || a.causal_ || a.qkv_.weight().is_null() || !LinearFits(a.qkv_, false, H, 3 * H, x) ||
+        !LinearFits(a.dense_, false, H, H, x) || !NormFits(a.layernorm_gamma_, a.layernorm_beta_, H, x) ||
+        !LinearFits(b.intermediate->dense_, false, H, F, x) || !LinearFits(b.output->dense_, false, F, H, x) ||
+        !NormFits(b.output->layer_norm_weight_, b.output->layer_norm_bias_, H, x))
+      return false;
+  }
+  const int dev = x.device_id();
+  ttb_ctx* c = DeviceContext(dev);
+  Scratch s;
+  const size_t workspace = s.Add(TTB_CHAIN_WORKSPACE), qkv = s.Add(M * 3 * H * 2), context = s.Add(M * H * 2), sum = s.Add(M * H * 2),
+               normed = s.Add(M * H * 2), inter = s.Add(M * F * 2);
+  s.Allocate(dev);
+  out->Reshape(x.dtype(), {B, L, H}, kDLCUDA, dev, "chain/out");
+  Ops ops;
+  ops.M = (int)M;
+  ops.list.reserve(5 * blocks.size() + 1);
+  const EncoderBlock* before = nullptr;
+  for (const EncoderBlock& b : blocks) {
+    const MultiHeadedAttention& a = *b.attention;
+    // the layer norm of the block before, whose result is this block's residual
+    ttb_chain_linear* o = ops.Linear(before ? s.base + sum : x.raw(), H, a.qkv_.Packed(false), a.qkv_.bias().raw(), 3 * H, s.base + qkv);
+    if (before) ops.Norm(o, before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, s.base + normed);
+    ttb_chain_attention* at = ops.Attention(TTB_CHAIN_KEYS_ROWS, s.base + qkv, 3 * H, heads, L, s.base + context);
+    at->mask = mask_ptr;
+    at->mask_pitch = (int32_t)L;
+    ops.Linear(s.base + context, H, a.dense_.Packed(false), a.dense_.bias().raw(), H, s.base + sum, TTB_CHAIN_ACT_NONE, before ? s.base + normed : x.raw());
+    o = ops.Linear(s.base + sum, H, b.intermediate->dense_.Packed(false), b.intermediate->dense_.bias().raw(), F, s.base + inter, TTB_CHAIN_ACT_GELU);
+    ops.Norm(o, a.layernorm_gamma_, a.layernorm_beta_, 1e-12f, s.base + normed);
+    ops.Linear(s.base + inter, F, b.output->dense_.Packed(false), b.output->dense_.bias().raw(), H, s.base + sum, TTB_CHAIN_ACT_NONE, s.base + normed);
+    before = &b;
+  }
+  ops.Norm(ops.Linear(s.base + sum, H, nullptr, nullptr, 0, nullptr), before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, out->raw_mut());
+  Check(ttb_chain_forward(c, TTB_F16, ops.list.data(), (int)ops.list.size(), s.base + workspace), c, "encoder chain");
+  return true;
+}
+
+bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bool trans_a, bool trans_f, const LayerNorm* final, const class Linear* head,
+                    const Tensor* memory, const Tensor* memory_mask, Tensor* hidden, Tensor* logits, Tensor* attn) {
+  const bool context = !blocks.empty() && blocks[0].context;
+  if (blocks.empty() || x.is_null() || (context ? 8 : 5) * blocks.size() + 1 > TTB_CHAIN_MAX_OPS) return false;
+  const int64_t heads = blocks[0].attention->num_attention_heads_;
+  const int64_t F = blocks[0].ffn->dense1_.out_dim(trans_f);
+  if (!RowsFit(x, heads, F, context ? kMostRowsContext : kMostRows)) return false;
+  const int64_t B = x.shape(0), L = x.shape(1), H = x.shape(2), M = B * L;
+  const bool cached = blocks[0].self_keys != nullptr;
+  const int64_t past = cached && !blocks[0].self_keys->is_null() ? blocks[0].self_keys->shape(0) : 0;
+  if ((past > 0 || context) && L != 1) return false;
+  if (past > (1 << 24)) return false;
+  int64_t Lk = 0;
+  if (context) {
+    const Tensor* k = blocks[0].memory_keys;
+    if (!k || !memory_mask || !attn) return false;
+    Lk = !k->is_null() && k->n_dim() == 4 ? k->shape(2) : (memory && memory->n_dim() == 3 ? memory->shape(1) : 0);
+    if (Lk < 1 || !memory_mask->on_gpu() || memory_mask->device_id() != x.device_id() || !core::SameType(memory_mask->dtype(), core::kFloat32) ||
+        memory_mask->shape(-1) != Lk || memory_mask->numel() != B * Lk)
+      return false;
+  }
+  for (const DecoderBlock& b : blocks) {
+    const MultiHeadedAttention& a = *b.attention;
+    const PositionwiseFeedForward& f = *b.ffn;
+    if (a.num_attention_heads_ != heads || a.qkv_.weight().is_null() || !LinearFits(a.qkv_, trans_a, H, 3 * H, x) || !LinearFits(a.dense_, trans_a, H, H, x) ||
+        !NormFits(a.layernorm_gamma_, a.layernorm_beta_, H, x) || a.causal_ != blocks[0].attention->causal_ || !LinearFits(f.dense1_, trans_f, H, F, x) ||
+        !LinearFits(f.dense2_, trans_f, F, H, x) || !NormFits(f.layer_norm_weight_, f.layer_norm_bias_, H, x) || (b.context != nullptr) != context)
+      return false;
+    if ((b.self_keys != nullptr) != cached || (b.self_values != nullptr) != cached) return false;
+    if (cached) {  // every block has cached the same tokens of this batch
+      for (const Tensor* t : {b.self_keys, b.self_values}) {
+        if (t->is_null() ? past != 0 : (past == 0 || t->n_dim() != 3 || t->shape(0) != past || t->shape(1) != B || t->shape(2) != H || !Half(*t, x) || !Aligned({t})))
+          return false;
+      }
+    }
+    if (context) {
+      const MultiHeadedAttention& m = *b.context;
+      if (m.num_attention_heads_ != heads || m.q_.weight().is_null() || m.k_.weight().is_null() || m.v_.weight().is_null() || !LinearFits(m.q_, trans_a, H, H, x) ||
+          !LinearFits(m.dense_, trans_a, H, H, x) || !NormFits(m.layernorm_gamma_, m.layernorm_beta_, H, x) || !b.memory_keys || !b.memory_values)
+        return false;
+      const bool filled = !b.memory_keys->is_null() && !b.memory_values->is_null();
+      if (filled) {
+        for (const Tensor* t : {b.memory_keys, b.memory_values})
+          if (!Half(*t, x) || !Aligned({t}) || t->n_dim() != 4 || t->shape(0) != B || t->shape(1) != heads || t->shape(2) != Lk || t->shape(3) != kHead) return false;
+      } else if (!memory || memory->n_dim() != 3 || memory->shape(0) != B || memory->shape(1) != Lk || memory->shape(2) != H || !Half(*memory, x) ||
+                 m.k_.use_int8() || m.v_.use_int8() || !Half(m.k_.weight(), x) || !Half(m.v_.weight(), x) || m.k_.in_dim(trans_a) != H || m.v_.in_dim(trans_a) != H ||
+                 m.k_.out_dim(trans_a) != H || m.v_.out_dim(trans_a) != H || m.k_.bias().is_null() || m.v_.bias().is_null()) {
+        return false;
+      }
+    }
+  }
+  if (final && !NormFits(final->gamma_, final->beta_, H, x)) return false;
+  int64_t V = 0;
+  if (head) {
+    const PackedLinear& l = head->dense_;
+    if (!final || !logits || l.use_int8() || !Half(l.weight(), x) || l.in_dim(head->is_trans_) != H || !l.bias().is_null()) return false;
+    V = l.out_dim(head->is_trans_);
+    if (V < 1 || V > (1 << 24)) return false;
+  }
+  const int dev = x.device_id();
+  ttb_ctx* c = DeviceContext(dev);
+  for (const DecoderBlock& b : blocks)
+    if (context && (b.memory_keys->is_null() || b.memory_values->is_null())) b.context->ProjectMemory(*memory, *memory, b.memory_keys, b.memory_values, trans_a);
+  Scratch s;
+  const size_t workspace = s.Add(TTB_CHAIN_WORKSPACE), qkv = s.Add(M * 3 * H * 2), ctx = s.Add(M * H * 2), stream = s.Add(M * H * 2), inter = s.Add(M * F * 2),
+               scores = s.Add(context ? M * Lk * 4 : 0);
+  s.Allocate(dev);
+  hidden->Reshape(x.dtype(), {B, L, H}, kDLCUDA, dev, "chain/hidden");
+  if (head) logits->Reshape(x.dtype(), {B, L, V}, kDLCUDA, dev, "chain/logits");
+  if (context) attn->Reshape(x.dtype(), {B, 1, Lk}, kDLCUDA, dev, "chain/attention");
+  Ops ops;
+  ops.M = (int)M;
+  ops.list.reserve(8 * blocks.size() + 1);
+  const void* in = x.raw();  // the residual stream: the caller's tensor until the first block has added to it
+  for (const DecoderBlock& b : blocks) {
+    const MultiHeadedAttention& a = *b.attention;
+    const PositionwiseFeedForward& f = *b.ffn;
+    const bool last = &b == &blocks.back();
+    ops.Norm(ops.Linear(in, H, a.qkv_.Packed(trans_a), a.qkv_.bias().raw(), 3 * H, s.base + qkv), a.layernorm_gamma_, a.layernorm_beta_, a.pre_ln_eps_);
+    ttb_chain_attention* at = ops.Attention(past > 0 ? TTB_CHAIN_KEYS_CACHE : TTB_CHAIN_KEYS_ROWS, s.base + qkv, 3 * H, heads, L, s.base + ctx);
+    at->past = (int32_t)past;
+    at->causal = a.causal_ ? 1 : 0;
+    if (cached) {
+      EnsureCacheRows(b.self_keys, x.dtype(), past, L, B, H, dev);
+      EnsureCacheRows(b.self_values, x.dtype(), past, L, B, H, dev);
+      at->k_cache = b.self_keys->raw_mut();
+      at->v_cache = b.self_values->raw_mut();
+    }
+    ops.Linear(s.base + ctx, H, a.dense_.Packed(trans_a), a.dense_.bias().raw(), H, s.base + stream, TTB_CHAIN_ACT_NONE, in);
+    in = s.base + stream;
+    if (context) {
+      const MultiHeadedAttention& m = *b.context;
+      ops.Norm(ops.Linear(in, H, m.q_.Packed(trans_a), m.q_.bias().raw(), H, s.base + qkv), m.layernorm_gamma_, m.layernorm_beta_, m.pre_ln_eps_);
+      at = ops.Attention(TTB_CHAIN_KEYS_MEMORY, s.base + qkv, H, heads, Lk, s.base + ctx);
+      at->k = b.memory_keys->raw();
+      at->v = b.memory_values->raw();
+      at->mask = memory_mask->data<float>();
+      at->mask_pitch = (int32_t)Lk;
+      if (last) {
+        at->probs = attn->raw_mut();
+        at->scores = reinterpret_cast<float*>(s.base + scores);
+      }
+      ops.Linear(s.base + ctx, H, m.dense_.Packed(trans_a), m.dense_.bias().raw(), H, s.base + stream, TTB_CHAIN_ACT_NONE, in);
+    }
+    const int act = f.act_ == TTB_ACT_GELU ? TTB_CHAIN_ACT_GELU : TTB_CHAIN_ACT_RELU;
+    ops.Norm(ops.Linear(in, H, f.dense1_.Packed(trans_f), f.dense1_.bias().raw(), F, s.base + inter, act), f.layer_norm_weight_, f.layer_norm_bias_, f.eps_);
+    ops.Linear(s.base + inter, F, f.dense2_.Packed(trans_f), f.dense2_.bias().raw(), H, last && !final ? hidden->raw_mut() : s.base + stream, TTB_CHAIN_ACT_NONE, in);
+  }
+  if (final) {
+    ttb_chain_linear* o = ops.Linear(in, H, head ? head->dense_.Packed(head->is_trans_) : nullptr, nullptr, V, head ? logits->raw_mut() : nullptr);
+    ops.Norm(o, final->gamma_, final->beta_, final->eps_, hidden->raw_mut());
+  }
+  Check(ttb_chain_forward(c, TTB_F16, ops.list.data(), (int)ops.list.size(), s.base + workspace), c, "decoder chain");
+  return true;
+}
+
+}  // namespace layers
+}  // namespace turbo_transformers

@@ -431,7 +431,6 @@ void MultiHeadedAttention::operator()(const Tensor& key_tensor, const Tensor& va
       cache_v);
 }
 
-namespace {
 // Makes a cache hold past + n_new tokens, keeping the first `past`. The tensor's shape is the logical [T, B, H]; its buffer is
 // paged ([pages, B, 16, H], see ttb_attention_decode) and reserved ahead (a Tensor keeps its buffer across Reshape calls while
 // it is large enough), so most steps only change the logical shape; when the reserve runs out the pages move to a buffer
@@ -453,7 +452,6 @@ void EnsureCacheRows(Tensor* t, DLDataType dtype, int64_t past, int64_t n_new, i
   }
   t->Reshape(dtype, want, kDLCUDA, dev, "layer_cache");
 }
-}  // namespace
 
 void MultiHeadedAttentionSmartBatch::operator()(const Tensor& key_tensor, const Tensor& value_tensor, const Tensor& query_tensor,
                                                 const Tensor& attention_mask, const std::string& attn_type, Tensor* output,
@@ -686,6 +684,42 @@ void MultiHeadedAttention::Finish(const Tensor& context, const Tensor& x, int64_
   }
 }
 
+void MultiHeadedAttention::ProjectMemory(const Tensor& key_tensor, const Tensor& value_tensor, Tensor* k, Tensor* v, bool is_trans_weight,
+                                         const std::vector<int64_t>* k_lens) const {
+  TT_ENFORCE(!k_.weight().is_null() && !v_.weight().is_null(), "context attention needs the separate q, k, v weights and biases");
+  const int dt = FloatType(key_tensor, "attention memory");
+  const int dev = key_tensor.device_id();
+  ttb_ctx* c = DeviceContext(dev);
+  const DLDataType type = key_tensor.dtype();
+  const int64_t H = k_.out_dim(is_trans_weight), heads = num_attention_heads_, d = H / heads;
+  const int64_t B = k_lens ? (int64_t)k_lens->size() : key_tensor.shape(0);
+  if (k_lens) {
+    const int64_t sum_k = std::accumulate(k_lens->begin(), k_lens->end(), (int64_t)0);
+    TT_ENFORCE(key_tensor.shape(0) == 1 && key_tensor.shape(1) == sum_k, "The key_tensor shape 1 should be the sum of seq_len_list.");
+    TT_ENFORCE(value_tensor.shape(0) == 1 && value_tensor.shape(1) == sum_k, "The value_tensor shape 1 should be the sum of seq_len_list.");
+    TT_ENFORCE(key_tensor.shape(2) == H && value_tensor.shape(2) == H, "key_tensor and value_tensor must be [1, sum_key_len, hidden]");
+  } else {
+    TT_ENFORCE(key_tensor.shape(1) == value_tensor.shape(1) && key_tensor.shape(2) == H && value_tensor.shape(2) == H && value_tensor.shape(0) == B,
+               "key_tensor and value_tensor must both be [batch, key_len, hidden]");
+  }
+  SameTypeDevice(key_tensor, k_.weight(), "attention");
+  SameTypeDevice(value_tensor, v_.weight(), "attention");
+  const core::CuSeqlensHandle cu_k = k_lens ? core::CuSeqlens(dev, *k_lens) : core::CuSeqlensHandle();
+  const int64_t Lk = k_lens ? *std::max_element(k_lens->begin(), k_lens->end()) : key_tensor.shape(1);  // padded key length
+  const int64_t Tk = key_tensor.rows();
+  Tensor k_lin(nullptr), v_lin(nullptr);
+  k_lin.Reshape(type, {Tk, H}, kDLCUDA, dev, "context/gemm2/k_out1/Reshape");
+  v_lin.Reshape(type, {Tk, H}, kDLCUDA, dev, "context/gemm1/v_out1/Reshape");
+  k_.Forward(key_tensor, Tk, TTB_EPI_NONE, nullptr, k_lin.raw_mut(), is_trans_weight, "context/gemm1");
+  v_.Forward(value_tensor, Tk, TTB_EPI_NONE, nullptr, v_lin.raw_mut(), is_trans_weight, "context/gemm2");
+  k->Reshape(type, {B, heads, Lk, d}, kDLCUDA, dev, "context/keys/AddBiasTransposeForScore/Reshape");
+  v->Reshape(type, {B, heads, Lk, d}, kDLCUDA, dev, "context/values/AddBiasTransposeForScore/Reshape");
+  Check(ttb_add_bias_transpose_for_score_pad(c, dt, k_lin.raw(), k_.bias().raw(), cu_k.get(), B, Lk, heads, d, k->raw_mut()), c,
+        "context/keys/AddBiasTransposeForScore");
+  Check(ttb_add_bias_transpose_for_score_pad(c, dt, v_lin.raw(), v_.bias().raw(), cu_k.get(), B, Lk, heads, d, v->raw_mut()), c,
+        "context/values/AddBiasTransposeForScore");
+}
+
 void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& value_tensor, const Tensor& query_tensor,
                                       const Tensor& attention_mask, Tensor* output, Tensor* att_score, Tensor* memory_keys,
                                       Tensor* memory_values, bool pre_layernorm, bool post_layernorm, bool post_add_input,
@@ -711,7 +745,6 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
   const int64_t T = x.rows();
   // prefix sums of the packed rows (null handles = equal lengths, rows b * L + l)
   const core::CuSeqlensHandle cu_q = packed ? core::CuSeqlens(dev, *q_lens) : core::CuSeqlensHandle();
-  const core::CuSeqlensHandle cu_k = packed ? core::CuSeqlens(dev, *k_lens) : core::CuSeqlensHandle();
   TT_ENFORCE_EQ(d * heads, H, "hidden size %lld is not divisible by %lld heads", (long long)H, (long long)heads);
   TT_ENFORCE_EQ(q_.out_dim(is_trans_weight), H, "q weight does not map hidden -> hidden");
   if (pre_layernorm || post_layernorm) TT_ENFORCE(!layernorm_gamma_.is_null(), "this attention layer was built without layer norm weights");
@@ -753,33 +786,9 @@ void MultiHeadedAttention::RunContext(const Tensor& key_tensor, const Tensor& va
                    core::SameType(v->dtype(), x.dtype()),
                "layer_cache memory_values does not match memory_keys");
   } else {
-    if (packed) {
-      const int64_t sum_k = std::accumulate(k_lens->begin(), k_lens->end(), (int64_t)0);
-      TT_ENFORCE(key_tensor.shape(0) == 1 && key_tensor.shape(1) == sum_k, "The key_tensor shape 1 should be the sum of seq_len_list.");
-      TT_ENFORCE(value_tensor.shape(0) == 1 && value_tensor.shape(1) == sum_k, "The value_tensor shape 1 should be the sum of seq_len_list.");
-      TT_ENFORCE(key_tensor.shape(2) == H && value_tensor.shape(2) == H, "key_tensor and value_tensor must be [1, sum_key_len, hidden]");
-    } else {
-      TT_ENFORCE_EQ(key_tensor.shape(0), B, "key_tensor and query_tensor disagree on the batch size");
-      TT_ENFORCE(key_tensor.shape(1) == value_tensor.shape(1) && key_tensor.shape(2) == H && value_tensor.shape(2) == H &&
-                     value_tensor.shape(0) == B,
-                 "key_tensor and value_tensor must both be [batch, key_len, hidden]");
-    }
-    SameTypeDevice(key_tensor, k_.weight(), "attention");
-    SameTypeDevice(value_tensor, v_.weight(), "attention");
-    const int64_t Lk = packed ? *std::max_element(k_lens->begin(), k_lens->end()) : key_tensor.shape(1);  // padded key length
-    const int64_t Tk = key_tensor.rows();
     if (memory_keys) { k = memory_keys; v = memory_values; }
-    Tensor k_lin(nullptr), v_lin(nullptr);
-    k_lin.Reshape(x.dtype(), {Tk, H}, kDLCUDA, dev, "context/gemm2/k_out1/Reshape");
-    v_lin.Reshape(x.dtype(), {Tk, H}, kDLCUDA, dev, "context/gemm1/v_out1/Reshape");
-    k_.Forward(key_tensor, Tk, TTB_EPI_NONE, nullptr, k_lin.raw_mut(), is_trans_weight, "context/gemm1");
-    v_.Forward(value_tensor, Tk, TTB_EPI_NONE, nullptr, v_lin.raw_mut(), is_trans_weight, "context/gemm2");
-    k->Reshape(x.dtype(), {B, heads, Lk, d}, kDLCUDA, dev, "context/keys/AddBiasTransposeForScore/Reshape");
-    v->Reshape(x.dtype(), {B, heads, Lk, d}, kDLCUDA, dev, "context/values/AddBiasTransposeForScore/Reshape");
-    Check(ttb_add_bias_transpose_for_score_pad(c, dt, k_lin.raw(), k_.bias().raw(), cu_k.get(), B, Lk, heads, d, k->raw_mut()), c,
-          "context/keys/AddBiasTransposeForScore");
-    Check(ttb_add_bias_transpose_for_score_pad(c, dt, v_lin.raw(), v_.bias().raw(), cu_k.get(), B, Lk, heads, d, v->raw_mut()), c,
-          "context/values/AddBiasTransposeForScore");
+    if (!packed) TT_ENFORCE_EQ(key_tensor.shape(0), B, "key_tensor and query_tensor disagree on the batch size");
+    ProjectMemory(key_tensor, value_tensor, k, v, is_trans_weight, k_lens);
   }
   const int64_t Lk = k->shape(2);
 

@@ -98,6 +98,7 @@ class BERTEmbedding {
 };
 
 class MultiHeadedAttention {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   MultiHeadedAttention(core::Tensor k_weight, core::Tensor k_bias, core::Tensor v_weight, core::Tensor v_bias,
                        core::Tensor q_weight, core::Tensor q_bias, core::Tensor dense_weight, core::Tensor dense_bias,
@@ -122,6 +123,10 @@ class MultiHeadedAttention {
   void Run(const core::Tensor& query_tensor, const core::Tensor& attention_mask, const std::vector<int64_t>* seq_lens,
            core::Tensor* output, core::Tensor* att_score, bool pre_layernorm, bool post_layernorm, bool post_add_input,
            bool is_trans_weight, core::Tensor* cache_keys = nullptr, core::Tensor* cache_values = nullptr) const;
+
+  // The encoder memory's keys and values of context attention, projected into [B, heads, Lk, d].
+  void ProjectMemory(const core::Tensor& key_tensor, const core::Tensor& value_tensor, core::Tensor* keys, core::Tensor* values,
+                     bool is_trans_weight, const std::vector<int64_t>* k_lens = nullptr) const;
 
   // `att_score` is a per-call choice: a 16-bit model given nullptr skips the [B,heads,L,L] score tensor (the largest HBM
   // round trip of the reference path) and runs the fused attention kernel; given a tensor it materialises the scores into
@@ -154,6 +159,9 @@ class MultiHeadedAttention {
   float pre_ln_eps_ = 1e-6f;
 };
 
+// Makes a paged self-attention cache hold past + n_new tokens, keeping the first `past`.
+void EnsureCacheRows(core::Tensor* t, DLDataType dtype, int64_t past, int64_t n_new, int64_t B, int64_t H, int dev);
+
 class MultiHeadedAttentionSmartBatch : public MultiHeadedAttention {
  public:
   using MultiHeadedAttention::MultiHeadedAttention;
@@ -178,6 +186,7 @@ class BertAttention : public MultiHeadedAttention {
 };
 
 class BertIntermediate {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   BertIntermediate(core::Tensor dense_weight, core::Tensor dense_bias) : dense_(std::move(dense_weight), std::move(dense_bias)) {
     EnforceShapeAndType();
@@ -191,6 +200,7 @@ class BertIntermediate {
 };
 
 class BertOutput {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   BertOutput(core::Tensor dense_weight, core::Tensor dense_bias, core::Tensor layer_norm_weight, core::Tensor layer_norm_bias)
       : dense_(std::move(dense_weight), std::move(dense_bias)), layer_norm_weight_(std::move(layer_norm_weight)),
@@ -238,6 +248,7 @@ class PrepareBertMasks {
 // Pre-LN feed-forward block: out = x + W2 act(W1 LN(x) + b1) + b2 (positionwise_ffn.cpp:31-75).
 // The reference's activation is ReLU; "gelu" selects the tanh-form GELU for GPT-2 style blocks.
 class PositionwiseFeedForward {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   PositionwiseFeedForward(core::Tensor dense_weight_1, core::Tensor dense_bias_1, core::Tensor dense_weight_2,
                           core::Tensor dense_bias_2, core::Tensor layer_norm_weight, core::Tensor layer_norm_bias)
@@ -310,6 +321,7 @@ class FusedAddBiasLayerNorm {
 
 // Stand-alone LayerNorm (kernels::LayerNorm, layer_norm.cpp:32-91) for pre-LN models' final norm.
 class LayerNorm {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   LayerNorm(core::Tensor gamma, core::Tensor beta, float eps) : gamma_(std::move(gamma)), beta_(std::move(beta)), eps_(eps) {}
   void operator()(const core::Tensor& input, core::Tensor* output) const;
@@ -334,6 +346,7 @@ class TokenPositionEmbedding {
 
 // out = x . W (+ bias): kernels::MatMul as a layer, used for the tied-embedding logits of decoder models.
 class Linear {
+  friend class Chain;  // runs whole stacks of layers as one kernel
  public:
   Linear(core::Tensor weight, core::Tensor bias, bool is_trans_weight)
       : dense_(std::move(weight), std::move(bias)), is_trans_(is_trans_weight) {}

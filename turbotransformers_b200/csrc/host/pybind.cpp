@@ -9,6 +9,7 @@
 #include <cstring>
 
 #include "bert_model.h"
+#include "chain.h"
 #include "layers.h"
 #include "npz.h"
 
@@ -222,6 +223,39 @@ PYBIND11_MODULE(turbo_transformers_cxx, m) {
   py::class_<layers::BertPooler>(m, "BertPooler")
       .def(py::init([](Tensor& w, Tensor& b) { return new layers::BertPooler(std::move(w), std::move(b)); }))
       .def("__call__", &layers::BertPooler::operator());
+
+  // ---- stacks of layers over few rows as one kernel; false: not taken, nothing done
+  m.def("encoder_chain", [](const py::list& blocks, const Tensor& x, const Tensor& mask, Tensor* out) {
+    std::vector<layers::Chain::EncoderBlock> list;
+    for (const py::handle& h : blocks) {
+      const py::tuple t = py::reinterpret_borrow<py::tuple>(h);
+      list.push_back({t[0].cast<const layers::BertAttention*>(), t[1].cast<const layers::BertIntermediate*>(), t[2].cast<const layers::BertOutput*>()});
+    }
+    return layers::Chain::Encoder(list, x, mask, out);
+  });
+  // blocks: (self attention, context attention or None, feed-forward); caches: None, or per block (self_keys, self_values[,
+  // memory_keys, memory_values])
+  m.def("decoder_chain", [](const py::list& blocks, const py::object& caches, const Tensor& x, bool trans_attention, bool trans_ffn,
+                            const layers::LayerNorm* final, const layers::Linear* head, const Tensor* memory, const Tensor* memory_mask, Tensor* hidden,
+                            Tensor* logits, Tensor* attn) {
+    std::vector<layers::Chain::DecoderBlock> list;
+    for (size_t i = 0; i < blocks.size(); ++i) {
+      const py::tuple t = py::reinterpret_borrow<py::tuple>(blocks[i]);
+      layers::Chain::DecoderBlock b{t[0].cast<const layers::MultiHeadedAttention*>(), t[1].cast<const layers::MultiHeadedAttention*>(),
+                                    t[2].cast<const layers::PositionwiseFeedForward*>(), nullptr, nullptr, nullptr, nullptr};
+      if (!caches.is_none()) {
+        const py::tuple k = py::reinterpret_borrow<py::tuple>(py::reinterpret_borrow<py::list>(caches)[i]);
+        b.self_keys = k[0].cast<Tensor*>();
+        b.self_values = k[1].cast<Tensor*>();
+        if (k.size() > 2) {
+          b.memory_keys = k[2].cast<Tensor*>();
+          b.memory_values = k[3].cast<Tensor*>();
+        }
+      }
+      list.push_back(b);
+    }
+    return layers::Chain::Decoder(list, x, trans_attention, trans_ffn, final, head, memory, memory_mask, hidden, logits, attn);
+  });
 
   // ---- the Python-free model of the C++ API (example/cpp/bert_model.cpp of the reference), reachable from Python for tests
   m.def("npz_load", [](const std::string& filename) {

@@ -9,7 +9,7 @@
 //     shared-memory ring (cp.async.bulk) until the ring is full: about a layer ahead of the arithmetic. Norm weights and biases
 //     travel the same way, and cached keys and values are brought to L2.
 //   * The products run on mma.sync m16n8k16 with the eight columns of a unit as its n: 128-row tcgen05 tiles would be empty but for a few
-//     rows, and the round trip through tensor memory is longer than the whole product. The sixteen warps split the rows (16 each)
+//     rows, and the round trip through tensor memory is longer than the whole product. The warps split the rows (16 each)
 //     and K; the order of k inside a 32-wide chunk is permuted alike for both operands so that each thread loads 16 bytes at a time: A straight
 //     from global memory into fragments (no warp reads what another does), W from the ring without bank conflicts (row pitch 64
 //     bytes past a multiple of 128). Partial sums meet in shared memory.
@@ -25,7 +25,7 @@ using namespace ttb;
 
 namespace {
 
-constexpr int kWarps = 16;                      // (a warp more, for the loads alone, would cost each thread a quarter of its registers)
+constexpr int kWarps = 8;                       // the operations are bound by what every warp has to do anyway: fewer warps, with more registers
 constexpr int kThreads = kWarps * 32;
 constexpr int kGroup = 4;                       // most units of eight columns that a CTA computes at a time
 constexpr int kRowPad = 64;                     // bytes between the rows of a ring slot, for the banks
@@ -68,7 +68,7 @@ struct Feed {
 // The units of a product that belong to this CTA, and whether it takes part in the operation at all: CTA r also writes normalised row r.
 struct Share {
   int lo, hi;
-  bool writes, part, params;
+  bool writes, part, params;  // params: norm weights or a bias come with it
   __device__ __forceinline__ Share() {}
   __device__ __forceinline__ explicit Share(const ttb_chain_linear& o) {
     const uint32_t units = ((uint32_t)o.N + 7) >> 3;  // N <= 2^24: the products stay below 2^32 on any GPU
@@ -81,10 +81,10 @@ struct Share {
 };
 
 struct Shared {
+  ttb_chain_op ops[TTB_CHAIN_MAX_OPS];   // (read from the kernel's parameters, every operation's first use would miss the constant cache)
+  Share share[TTB_CHAIN_MAX_OPS];
   float red[kWarps * kGroup * 128];      // partial sums of a group of units, or attention states
   uint8_t params[kParamSlots][kParamBytes];
-  uint32_t op[2][32];                    // the operation, and the next
-  Share share[2];
   uint64_t full[kMaxSlots], pfull[kParamSlots];
   Feed feed;
   volatile int abort_flag;
@@ -137,12 +137,6 @@ __device__ __forceinline__ float gelu16(float x) {  // the form of the tensor-co
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(0.7978845608028654f * (x + 0.044715f * x * x * x)));
   return 0.5f * x * (1.0f + y);
-}
-// For polling: without the acquire, which would empty the L1 cache at every attempt.
-__device__ __forceinline__ int ld_relaxed_gpu(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -207,9 +201,9 @@ __device__ __noinline__ void feed(const ChainParams& prm, Shared& sm, uint32_t r
   Feed f = sm.feed;
   __syncwarp();
   for (; f.op < prm.n_ops; ++f.op) {
-    if (prm.ops[f.op].kind != TTB_CHAIN_LINEAR) continue;
-    const ttb_chain_linear& o = prm.ops[f.op].u.linear;
-    const Share s(o);
+    if (sm.ops[f.op].kind != TTB_CHAIN_LINEAR) continue;
+    const ttb_chain_linear& o = sm.ops[f.op].u.linear;
+    const Share s = sm.share[f.op];
     if (!f.begun) {
       if (s.params) {
         if (f.p_issued - p_consumed >= kParamSlots) break;
@@ -230,11 +224,24 @@ __device__ __noinline__ void feed(const ChainParams& prm, Shared& sm, uint32_t r
       f.first = s.lo;
       f.unit = f.k = f.batch = 0;
     }
-    if (!feed_units(o, prm.ops[f.op].reserved & 0xffff, prm.ops[f.op].reserved >> 16, s.hi, prm, sm, ring, kpb, consumed, f)) break;
+    if (!feed_units(o, sm.ops[f.op].reserved & 0xffff, sm.ops[f.op].reserved >> 16, s.hi, prm, sm, ring, kpb, consumed, f)) break;
     f.begun = 0;
   }
   if (lane == 0) sm.feed = f;
   __syncwarp();
+}
+
+// Waits for the norm weights, bias and weights with which the CTA's share of an operation begins. One warp does it for all of them, ahead of
+// a barrier of the CTA and mostly in the shadow of the grid's.
+__device__ __forceinline__ bool wait_ahead(const ttb_chain_op& op, const Share& s, int slots, Shared& sm, Cursor w, const Cursor& p) {
+  if (op.kind != TTB_CHAIN_LINEAR || !s.part) return true;
+  bool ok = !s.params || wait(sm100::smem_u32(&sm.pfull[p.slot]), p.parity, &sm.abort_flag);
+  const int n = min(op.reserved >> 16, s.hi - s.lo) * div_small(op.u.linear.K, op.reserved & 0xffff);
+  for (int i = 0; ok && i < n; ++i) {
+    ok = wait(sm100::smem_u32(&sm.full[w.slot]), w.parity, &sm.abort_flag);
+    w.next(slots);
+  }
+  return ok;
 }
 
 // Brings the keys and values that an earlier launch has written, and that this CTA reads two operations later, to L2.
@@ -262,12 +269,12 @@ struct Read {
   int slots = 0, params = 0;
 };
 
-// The layout of a product: MT tiles of 16 rows, and the 16 warps are MT tiles x KW shares of K. A chunk is 32 of K: thread t of a quad
+// The layout of a product: MT tiles of 16 rows, and the warps are MT tiles x KW shares of K. A chunk is 32 of K: thread t of a quad
 // holds 8 of them, in 16 bytes, for its rows g and g + 8. Chunk c of a ring slot's part of K belongs to share c % KW, CPK of them
 // to a warp at most.
 template <int MT> struct Layout {
   static constexpr int KW = kWarps / MT, CPK = kPart / 32 / KW;
-  static constexpr int kBatch = 8 / CPK;  // parts of K whose fragments (64 registers) are held at a time
+  static constexpr int kBatch = CPK <= 8 ? 16 / CPK : 1;  // parts of K whose fragments (up to 128 registers) are held at a time
   static constexpr int kItems = (MT * 16 * kGroup * 4 + kThreads - 1) / kThreads;  // pairs of output columns per thread and group
 };
 
@@ -337,62 +344,125 @@ __device__ __forceinline__ void epilogue(const ttb_chain_linear& o, const Shared
   }
 }
 
+// Two fp32 numbers that one instruction works on.
+struct Two {
+  unsigned long long v;
+  __device__ __forceinline__ Two() {}
+  __device__ __forceinline__ Two(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+  __device__ __forceinline__ float2 get() const {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+  }
+};
+__device__ __forceinline__ Two operator+(Two a, Two b) {
+  Two r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Two operator*(Two a, Two b) {
+  Two r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
+  Two r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ void unpack2(const uint4& q, Two (&f)[4]) {
+  const __half2* h = reinterpret_cast<const __half2*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = __half22float2(h[i]);
+    f[i] = Two(v.x, v.y);
+  }
+}
+
 // Layer norm of the operation's rows into shared memory, a warp per row (64 bytes past a multiple of 128 between rows, as in the ring).
+// Where a warp has several rows it takes two at a time, so that one's reductions wait while the other's are under way.
 template <int MT>
-__device__ __forceinline__ bool normalise(const ttb_chain_linear& o, const Share& s, Shared& sm, uint32_t a_smem, const Read& read) {
-  constexpr int kEach = MT;  // rows of a warp
+__device__ __forceinline__ void normalise(const ttb_chain_linear& o, const Share& s, Shared& sm, uint32_t a_smem, const Read& read) {
+  constexpr int kEach = MT * 16 / kWarps, kIters = kPart / 256;  // rows of a warp, 16-byte pieces of a row per lane
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, K = o.K, M = o.M;
-  uint4 x[kEach][kPart / 256];
+  uint4 x[kEach][kIters];
   const __half* src = static_cast<const __half*>(o.A) + (long long)warp * o.lda + lane * 8;
 #pragma unroll
   for (int r = 0; r < kEach; ++r)
 #pragma unroll
-    for (int i = 0; i < kPart / 256; ++i) {
+    for (int i = 0; i < kIters; ++i) {
       x[r][i] = make_uint4(0, 0, 0, 0);
       if (warp + r * kWarps < M && i * 256 + lane * 8 < K) x[r][i] = *reinterpret_cast<const uint4*>(src + (long long)r * kWarps * o.lda + i * 256);
     }
-  const bool ok = wait(sm100::smem_u32(&sm.pfull[read.p.slot]), read.p.parity, &sm.abort_flag);
   const uint32_t gamma = sm100::smem_u32(sm.params[read.p.slot]) + lane * 16;
   const float inv_k = __fdividef(1.f, (float)K), eps = o.eps;
 #pragma unroll
-  for (int r = 0; r < kEach; ++r) {
-    const int row = warp + r * kWarps;
-    if (row >= M) break;
-    float sum = 0.f, sq = 0.f;
+  for (int r = 0; r < kEach; r += 2) {
+    if (warp + r * kWarps >= M) break;
+    Two f[2][kIters][4];
+    float mean[2], rstd[2];
 #pragma unroll
-    for (int i = 0; i < kPart / 256; ++i)
-      if (i * 256 + lane * 8 < K) {
-        float f[8];
-        unpack(x[r][i], f);
-        sum += ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+    for (int h = 0; h < 2; ++h) {
+      Two sum(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < kIters; ++i) {  // (lanes beyond the row hold zeros)
+        unpack2(x[r + h][i], f[h][i]);
+        sum = sum + ((f[h][i][0] + f[h][i][1]) + (f[h][i][2] + f[h][i][3]));
       }
-    const float mean = warp_sum(sum) * inv_k;
+      mean[h] = sum.get().x + sum.get().y;
+    }
 #pragma unroll
-    for (int i = 0; i < kPart / 256; ++i)
+    for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) mean[h] += __shfl_xor_sync(0xffffffffu, mean[h], d);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mean[h] *= inv_k;
+      const Two minus(-mean[h], -mean[h]);
+      Two sq(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < kIters; ++i)
+        if (i * 256 + lane * 8 < K)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            f[h][i][e] = f[h][i][e] + minus;
+            sq = fma2(f[h][i][e], f[h][i][e], sq);
+          }
+      rstd[h] = sq.get().x + sq.get().y;
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) rstd[h] += __shfl_xor_sync(0xffffffffu, rstd[h], d);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) rstd[h] = rsqrtf(rstd[h] * inv_k + eps);
+#pragma unroll
+    for (int i = 0; i < kIters; ++i)
       if (i * 256 + lane * 8 < K) {
-        float f[8];
-        unpack(x[r][i], f);
+        Two ga[4], be[4];
+        unpack2(lds128(gamma + i * 512), ga);
+        unpack2(lds128(gamma + kPart * 2 + i * 512), be);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sq = fmaf(f[e] - mean, f[e] - mean, sq);
-      }
-    const float rstd = rsqrtf(warp_sum(sq) * inv_k + eps);
+        for (int h = 0; h < 2; ++h) {
+          const int row = warp + (r + h) * kWarps;
+          const Two scale(rstd[h], rstd[h]);
+          float y[8];
 #pragma unroll
-    for (int i = 0; i < kPart / 256; ++i)
-      if (i * 256 + lane * 8 < K) {
-        float ga[8], be[8], f[8];
-        unpack(lds128(gamma + i * 512), ga);
-        unpack(lds128(gamma + kPart * 2 + i * 512), be);
-        unpack(x[r][i], f);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = fmaf((f[e] - mean) * rstd, ga[e], be[e]);
-        const uint4 y = pack(f);
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_smem + row * (K * 2 + kRowPad) + i * 512 + lane * 16), "r"(y.x), "r"(y.y), "r"(y.z),
-                     "r"(y.w)
-                     : "memory");
-        if (s.writes && (int)blockIdx.x == row) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = y;
+          for (int e = 0; e < 4; ++e) {
+            const float2 v = fma2(f[h][i][e] * scale, ga[e], be[e]).get();
+            y[2 * e] = v.x;
+            y[2 * e + 1] = v.y;
+          }
+          const uint4 q = pack(y);
+          if (row < M) {
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_smem + row * (K * 2 + kRowPad) + i * 512 + lane * 16), "r"(q.x), "r"(q.y), "r"(q.z),
+                         "r"(q.w)
+                         : "memory");
+            if (s.writes && (int)blockIdx.x == row) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = q;
+          }
+        }
       }
   }
-  return ok;
 }
 
 // Product of the rows that normalise() has left in shared memory; K is one part.
@@ -402,7 +472,8 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
   constexpr int KW = Layout<MT>::KW, CPK = Layout<MT>::CPK;
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int mt = warp % MT, share = warp / MT, chunks = ks / 32;
-  bool ok = normalise<MT>(o, s, sm, a_smem, read);
+  normalise<MT>(o, s, sm, a_smem, read);
+  bool ok = true;
   const uint32_t lane_at = g * (ks * 2 + kRowPad) + share * 64 + t * 16;
   const uint32_t w_lane = ring + lane_at, a_lane = a_smem + mt * 16 * (ks * 2 + kRowPad) + lane_at, a_eight = 8 * (ks * 2 + kRowPad);
   const bool low = mt * 16 < o.M, high = mt * 16 + 8 < o.M;  // rows of the tile's halves (rows that are not there leave sums that nobody reads)
@@ -417,7 +488,7 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[u][e] = 0.f;
       if (u < nu) {
-        ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
+        if (u0 != s.lo) ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
         at[u] = w_lane + read.w.slot * prm.slot_bytes;
         read.w.next(prm.slots);
         ++read.slots;
@@ -455,7 +526,7 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
         Feed f = sm.feed;
         __syncwarp();
         if (f.op == op) {
-          feed_units(prm.ops[op].u.linear, ks, group, s.hi, prm, sm, ring, Layout<MT>::kBatch, read.slots, f);
+          feed_units(o, ks, group, s.hi, prm, sm, ring, Layout<MT>::kBatch, read.slots, f);
           if (lane == 0) sm.feed = f;
           __syncwarp();
         }
@@ -484,7 +555,7 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
     const int nu = min(group, s.hi - u0);
     __half2 res[Layout<MT>::kItems];
     for (int kb = 0; kb < parts; kb += kBatch) {
-      uint4 a0[8], a1[8];
+      uint4 a0[kBatch * CPK], a1[kBatch * CPK];
 #pragma unroll
       for (int kl = 0; kl < kBatch; ++kl) {
         const __half* p0 = a_lane + (kb + kl) * ks;
@@ -504,7 +575,7 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
 #pragma unroll
         for (int kl = 0; kl < kBatch; ++kl)
           if (kb + kl < parts) {
-            ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
+            if (u0 != s.lo) ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
             const uint32_t at = w_lane + read.w.slot * prm.slot_bytes;
 #pragma unroll
             for (int i = 0; i < CPK; ++i)
@@ -528,7 +599,6 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
         dst[32] = v1;
       }
     }
-    if (u0 == s.lo && o.bias) ok = wait(sm100::smem_u32(&sm.pfull[read.p.slot]), read.p.parity, &sm.abort_flag) && ok;
     __syncthreads();
     epilogue<MT>(o, sm, sm.params[read.p.slot] + kPart * 4 + (u0 - s.lo) * 16, u0, nu, res);
     if (u0 + group < s.hi) {
@@ -536,7 +606,7 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
         Feed f = sm.feed;
         __syncwarp();
         if (f.op == op) {
-          feed_units(prm.ops[op].u.linear, ks, group, s.hi, prm, sm, ring, kBatch, read.slots, f);
+          feed_units(o, ks, group, s.hi, prm, sm, ring, kBatch, read.slots, f);
           if (lane == 0) sm.feed = f;
           __syncwarp();
         }
@@ -554,8 +624,8 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
 // ---------------------------------------------------------------------------------------------
 // attention
 // ---------------------------------------------------------------------------------------------
-// (row, head) pairs go round the CTAs; a CTA's 16 warps are shared out among as many of its pairs as they serve at once, each taking
-// every W-th page of 16 keys: four keys a load, a page of keys and one of values in flight per warp.
+// (row, head) pairs go round the CTAs; a CTA's warps are shared out among as many of its pairs as they serve at once, each taking
+// every W-th page of 16 keys: four keys a load, two pages of keys and two of values in flight per warp.
 __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& sm) {
   constexpr int kState = kHeadDim + 2;
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, sub = lane & 7, kg = lane >> 3;
@@ -603,40 +673,52 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
       unpack(*reinterpret_cast<const uint4*>(qrow + sub * 8), q);
 #pragma unroll
       for (int e = 0; e < 8; ++e) q[e] *= o.scale * kLog2e;
+      // the new token's key and value are filed by the warp with the fewest keys (pairs of the same row write its other heads)
+      const bool files = wi == W - 1 && lane < 16 && o.k_cache && keys != TTB_CHAIN_KEYS_MEMORY;
+      uint4 newest = make_uint4(0, 0, 0, 0), *file_to = nullptr;
+      if (files) {
+        const int sequences = keys == TTB_CHAIN_KEYS_CACHE ? o.rows : div_small(o.rows, o.length);
+        newest = *reinterpret_cast<const uint4*>(qrow + (lane < 8 ? H : 2 * H) + sub * 8);
+        file_to = reinterpret_cast<uint4*>(static_cast<__half*>(lane < 8 ? o.k_cache : o.v_cache) + cache_row(place_in, seq, sequences, H) + h * kHeadDim + sub * 8);
+      }
       const int fresh = keys == TTB_CHAIN_KEYS_CACHE ? n - 1 : -1;  // the key that is not in the cache yet
       const __half *kp = k0 + wi * page + (long long)kg * pitch + sub * 8, *vp = v0 + wi * page + (long long)kg * pitch + sub * 8;
-      auto load = [&](uint4 (&dst)[4], const __half* from, const __half* newest, int j0) {
+      auto load = [&](uint4 (&dst)[8], const __half* from, const __half* own, int j0) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = j0 + u * 4 + kg;
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + (u >> 2) * 16 * W + (u & 3) * 4 + kg;
           dst[u] = make_uint4(0, 0, 0, 0);
-          if (j < n) dst[u] = *reinterpret_cast<const uint4*>(j == fresh ? newest + sub * 8 : from + u * 4 * pitch);
+          if (j < n) dst[u] = *reinterpret_cast<const uint4*>(j == fresh ? own + sub * 8 : from + (u >> 2) * W * page + (u & 3) * 4 * pitch);
         }
       };
-      uint4 kr[4], vr[4];
+      uint4 kr[8], vr[8];
       load(kr, kp, qrow + H, wi * 16);
       load(vr, vp, qrow + 2 * H, wi * 16);
-      for (int j0 = wi * 16; j0 < n; j0 += 16 * W) {
-        float sc[4], top = m;
+      for (int j0 = wi * 16; j0 < n; j0 += 32 * W) {
+        float sc[8], top = m;
+        const int pages = j0 + 16 * W < n ? 8 : 4;  // the second page may not be there
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          float f[8], dot[2];
-          unpack(kr[u], f);
-          dot[0] = q[0] * f[0];
-          dot[1] = q[1] * f[1];
+        for (int u = 0; u < 8; ++u)
+          if (u < pages) {
+            float f[8], dot[2];
+            unpack(kr[u], f);
+            dot[0] = q[0] * f[0];
+            dot[1] = q[1] * f[1];
 #pragma unroll
-          for (int e = 2; e < 8; ++e) dot[e & 1] = fmaf(q[e], f[e], dot[e & 1]);
-          sc[u] = dot[0] + dot[1];
-        }
-        kp += W * page;
-        load(kr, kp, qrow + H, j0 + 16 * W);  // the next page's keys travel while this page is finished
+            for (int e = 2; e < 8; ++e) dot[e & 1] = fmaf(q[e], f[e], dot[e & 1]);
+            sc[u] = dot[0] + dot[1];
+          } else {
+            sc[u] = 0.f;
+          }
+        kp += 2 * W * page;
+        load(kr, kp, qrow + H, j0 + 32 * W);  // the next pages' keys travel while these are finished
 #pragma unroll
         for (int o2 = 1; o2 < 8; o2 <<= 1)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o2);
+          for (int u = 0; u < 8; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o2);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = j0 + u * 4 + kg;
+        for (int u = 0; u < 8; ++u) {
+          const int j = j0 + (u >> 2) * 16 * W + (u & 3) * 4 + kg;
           if (j < n) {
             if (mask) sc[u] += mask[j] * kLog2e;
             if (scores && sub == 0) scores[j] = sc[u];
@@ -651,24 +733,19 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] *= keep;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float pr = ex2f(sc[u] - base);
-          float f[8];
-          unpack(vr[u], f);
-          l += pr;
+        for (int u = 0; u < 8; ++u)
+          if (u < pages) {
+            const float pr = ex2f(sc[u] - base);
+            float f[8];
+            unpack(vr[u], f);
+            l += pr;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) acc[e] = fmaf(pr, f[e], acc[e]);
-        }
-        vp += W * page;
-        load(vr, vp, qrow + 2 * H, j0 + 16 * W);
+            for (int e = 0; e < 8; ++e) acc[e] = fmaf(pr, f[e], acc[e]);
+          }
+        vp += 2 * W * page;
+        load(vr, vp, qrow + 2 * H, j0 + 32 * W);
       }
-      // the new token's key and value are filed (pairs of the same row write its other heads)
-      if (wi == 0 && lane < 16 && o.k_cache && keys != TTB_CHAIN_KEYS_MEMORY) {
-        const int sequences = keys == TTB_CHAIN_KEYS_CACHE ? o.rows : div_small(o.rows, o.length);
-        const __half* src = qrow + (lane < 8 ? H : 2 * H) + sub * 8;
-        __half* dst = static_cast<__half*>(lane < 8 ? o.k_cache : o.v_cache) + cache_row(place_in, seq, sequences, H) + h * kHeadDim + sub * 8;
-        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-      }
+      if (files) *file_to = newest;
     }
     // the four groups of a warp, then the warps
 #pragma unroll
@@ -731,20 +808,28 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
     sm.abort_flag = 0;
     sm100::mbar_init_fence();
   }
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(prm.ops);
-  if (warp == 1) {
-    if (lane < kOpWords) sm.op[0][lane] = words[lane];
-    if (lane == 0 && prm.ops[0].kind == TTB_CHAIN_LINEAR) sm.share[0] = Share(prm.ops[0].u.linear);
+  {
+    const uint32_t* from = reinterpret_cast<const uint32_t*>(prm.ops);
+    asm volatile("" : "+l"(from));  // as memory: a constant load with an address for each thread would go one thread after the other
+    uint32_t* to = reinterpret_cast<uint32_t*>(sm.ops);
+    for (int i = tid; i < prm.n_ops * kOpWords; i += kThreads) to[i] = from[i];
   }
   __syncthreads();
+  for (int i = tid; i < prm.n_ops; i += kThreads)
+    if (sm.ops[i].kind == TTB_CHAIN_LINEAR) sm.share[i] = Share(sm.ops[i].u.linear);
+  __syncthreads();
   Read read;
-  if (warp == kWarps - 1) feed(prm, sm, ring, Layout<MT>::kBatch, 0, 0);
-  for (int i = 0;;) {
-    const ttb_chain_op& op = *reinterpret_cast<const ttb_chain_op*>(sm.op[i & 1]);
+  if (warp == kWarps - 1) {
+    feed(prm, sm, ring, Layout<MT>::kBatch, 0, 0);
+    wait_ahead(sm.ops[0], sm.share[0], prm.slots, sm, read.w, read.p);
+  }
+  __syncthreads();
+  for (int i = 0; !sm.abort_flag;) {
+    const ttb_chain_op& op = sm.ops[i];
     bool ok = true;
     if (op.kind == TTB_CHAIN_ATTENTION) {
       attention(op.u.attention, sm);
-    } else if (const Share s = sm.share[i & 1]; s.part) {
+    } else if (const Share s = sm.share[i]; s.part) {
       if (op.u.linear.gamma) ok = linear_norm<MT>(op.u.linear, s, op.reserved & 0xffff, op.reserved >> 16, i, prm, sm, rows, ring, read);
       else ok = linear_plain<MT>(op.u.linear, s, op.reserved & 0xffff, op.reserved >> 16, i, prm, sm, ring, read);
     }
@@ -756,24 +841,22 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(prm.counter) : "memory");
       const int target = (int)gridDim.x * i;
       const long long t0 = clock64();
-      while (ld_relaxed_gpu(prm.counter) < target) {
+      // (polling without the acquire and fencing once behind it takes 1000 cycles longer: a fence makes a trip of its own)
+      while (sm100::ld_acquire_gpu(prm.counter) < target) {
         if (sm.abort_flag) break;
         if (clock64() - t0 > sm100::kWaitCycles) {
           sm.abort_flag = 1;
           atomicExch(prm.status, (int)TTB_ERR_DEVICE_WAIT);
         }
       }
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    } else if (warp == 1) {
-      if (lane < kOpWords) sm.op[i & 1][lane] = words[i * kOpWords + lane];
-      if (lane == 0 && prm.ops[i].kind == TTB_CHAIN_LINEAR) sm.share[i & 1] = Share(prm.ops[i].u.linear);
     } else if (warp == kWarps - 1) {
       feed(prm, sm, ring, Layout<MT>::kBatch, read.slots, read.params);
-    } else if (warp >= 4 && i + 1 < prm.n_ops && prm.ops[i + 1].kind == TTB_CHAIN_ATTENTION) {
-      prefetch_keys(prm.ops[i + 1].u.attention, tid - 4 * 32, (kWarps - 5) * 32);
+    } else if (warp == kWarps - 2) {
+      if (!wait_ahead(sm.ops[i], sm.share[i], prm.slots, sm, read.w, read.p) && lane == 0) atomicExch(prm.status, (int)TTB_ERR_DEVICE_WAIT);
+    } else if (warp >= 1 && i + 1 < prm.n_ops && sm.ops[i + 1].kind == TTB_CHAIN_ATTENTION) {
+      prefetch_keys(sm.ops[i + 1].u.attention, tid - 32, (kWarps - 3) * 32);
     }
     __syncthreads();
-    if (sm.abort_flag) break;
   }
   if (warp == kWarps - 1) {  // every copy lands before the CTA's shared memory goes, also where a wait has run out
     const Feed f = sm.feed;

@@ -15,7 +15,7 @@ from typing import Optional, Sequence
 import torch
 
 from .._cxx import cxx
-from .modules import MultiHeadedAttention, PositionwiseFeedForward
+from .modules import MultiHeadedAttention, PositionwiseFeedForward, _empty
 from .return_type import ReturnType, convert_returns_as_type
 from .utils import AnyTensor, try_convert, use_current_stream
 
@@ -117,15 +117,20 @@ class TransformerDecoder:
         emb = self.embeddings(tgt, step=step)
         assert emb.dim() == 3  # len x batch x embedding_dim
         output = emb.transpose(0, 1).contiguous()
-        src_memory_bank = memory_bank.transpose(0, 1).contiguous()
         src_lens = kwargs["memory_lengths"]
         src_max_len = self.state["src"].shape[0]
-        src_pad_mask = ~(torch.arange(src_max_len, device=src_lens.device)[None, :] < src_lens[:, None]).unsqueeze(1)
+        src_pad_mask = (torch.arange(src_max_len, device=src_lens.device)[None, :] >= src_lens[:, None]).unsqueeze(1)
+        unmodified = bool(self.transformer_layers) and all(_unmodified(layer) for layer in self.transformer_layers)
+        if unmodified and step is not None:
+            stepped = self._chain(output, memory_bank, src_pad_mask)
+            if stepped is not None:
+                return self._finish(*stepped)
+        src_memory_bank = memory_bank.transpose(0, 1).contiguous()
         tgt_pad_mask = tgt_words.data.eq(self.embeddings.word_padding_idx).unsqueeze(1)  # [B, 1, T_tgt]
         attn = None
         # The masks are the same for every layer and only the last layer's attention is returned: masks and memory are converted
         # once, and what travels between the layers stays the runtime's own tensor. Layers or parts of a caller's class get torch's.
-        if self.transformer_layers and all(_unmodified(layer) for layer in self.transformer_layers):
+        if unmodified:
             src_mask, dec_mask = _additive_masks(src_pad_mask, tgt_pad_mask, step, False)
             memory, masks = try_convert(src_memory_bank), (try_convert(src_mask), None if dec_mask is None else try_convert(dec_mask))
             last = len(self.transformer_layers) - 1
@@ -140,6 +145,37 @@ class TransformerDecoder:
             for i, layer in enumerate(self.transformer_layers):
                 layer_cache = self.state["cache"][f"layer_{i}"] if step is not None else None
                 output, attn, _ = layer(output, src_memory_bank, src_pad_mask, tgt_pad_mask, layer_cache=layer_cache, step=step)
+        return self._finish(output, attn)
+
+    def _chain(self, x: torch.Tensor, memory_bank: torch.Tensor, src_pad_mask: torch.Tensor):
+        """One decoding step of a small batch through all layers in one kernel: (output, attention of head 0), or None where the
+        call is not such a step and nothing has been done."""
+        if x.dtype != torch.float16 or x.size(1) != 1 or x.size(0) > 64 or len({l._ffn_trans for l in self.transformer_layers}) != 1:
+            return None
+        parts = [(l.self_attn, l.context_attn, l.feed_forward) for l in self.transformer_layers]
+        caches = [self.state["cache"][f"layer_{i}"] for i in range(len(parts))]
+        names = ("self_keys", "self_values", "memory_keys", "memory_values")
+        if not all(set(c) == set(names) for c in caches) or not all(
+                type(s) is MultiHeadedAttention and type(c) is MultiHeadedAttention and type(f) is PositionwiseFeedForward for s, c, f in parts):
+            return None
+        use_current_stream(x)
+        held = [tuple(_empty() if c[k] is None else try_convert(c[k]) for k in names) for c in caches]
+        # a memory entry is only read where both of a layer are filled; otherwise both are projected, whichever was given
+        projected = [h[2].is_null() or h[3].is_null() for h in held]
+        memory = memory_bank.transpose(0, 1).contiguous() if any(projected) else None
+        src_mask = (src_pad_mask.float() * -1e18).contiguous()
+        out, attn = _empty(), _empty()
+        if not cxx.decoder_chain(parts, held, try_convert(x), False, self.transformer_layers[0]._ffn_trans, None, None, try_convert(memory),
+                                 try_convert(src_mask), out, None, attn):
+            return None
+        use_current_stream(x)  # torch reads the results on the caller's stream, wherever another thread has pointed the runtime meanwhile
+        for c, h, fresh in zip(caches, held, projected):
+            c["self_keys"], c["self_values"] = h[0], h[1]
+            if fresh:
+                c["memory_keys"], c["memory_values"] = (convert_returns_as_type(t, ReturnType.TORCH) for t in h[2:])
+        return convert_returns_as_type(out, ReturnType.TORCH), convert_returns_as_type(attn, ReturnType.TORCH)
+
+    def _finish(self, output: torch.Tensor, attn: torch.Tensor):
         output = self.layer_norm(output)
         attns = {"std": attn.transpose(0, 1).contiguous()}
         if self._copy:

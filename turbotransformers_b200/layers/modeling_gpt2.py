@@ -62,6 +62,13 @@ class GPT2Model:
             B, L = ids.shape(0), ids.shape(1)
             m = torch.triu(torch.full((L, L), -10000.0, dtype=torch.float32, device="cuda"), 1)
             mask = convert2tt_tensor(m.unsqueeze(0).repeat(B, 1, 1).contiguous())
+        logits, padded_logits = None, return_logits and not contiguous_logits and return_type in (None, ReturnType.TORCH)
+        if self._chain(x, past, hidden := _empty(), logits_t := _empty() if return_logits and not padded_logits else None):
+            if padded_logits:
+                logits = self._padded_logits(hidden)
+            elif return_logits:
+                logits = convert_returns_as_type(logits_t, return_type)
+            return convert_returns_as_type(hidden, return_type), logits
         for i, (attn, ffn) in enumerate(self.blocks):
             a, y = _empty(), _empty()
             # no score tensor is asked for (None): 16-bit models run the fused attention kernel; pre-LN, + input
@@ -70,16 +77,28 @@ class GPT2Model:
             x = y
         h = _empty()
         self.final_norm(x, h)
-        logits = None
-        if return_logits and not contiguous_logits and return_type in (None, ReturnType.TORCH):
-            padded = _empty()
-            self.lm_head.padded(h, padded)
-            logits = convert_returns_as_type(padded, ReturnType.TORCH)[..., :self.lm_head.width()]
+        if padded_logits:
+            logits = self._padded_logits(h)
         elif return_logits:
             logits = _empty()
             self.lm_head(h, logits)
             logits = convert_returns_as_type(logits, return_type)
         return convert_returns_as_type(h, return_type), logits
+
+    def _padded_logits(self, h):
+        padded = _empty()
+        self.lm_head.padded(h, padded)
+        return convert_returns_as_type(padded, ReturnType.TORCH)[..., :self.lm_head.width()]
+
+    def _chain(self, x, past, hidden, logits) -> bool:
+        """All blocks, the final norm and (unless logits is None) the logits in one kernel, for the few rows of a decoding step or a
+        short prompt; False: not such a call, nothing done. A caller's class in the place of a layer is called as such."""
+        if not (all(type(a) is cxx.MultiHeadedAttention and type(f) is cxx.PositionwiseFeedForward for a, f in self.blocks) and
+                type(self.final_norm) is cxx.LayerNorm and type(self.lm_head) is cxx.Linear):
+            return False
+        caches = None if past is None else [(c["self_keys"], c["self_values"]) for c in past]
+        return cxx.decoder_chain([(a, None, f) for a, f in self.blocks], caches, x, False, False, self.final_norm,
+                                 None if logits is None else self.lm_head, None, None, hidden, logits, None)
 
     @staticmethod
     def from_torch(model, device: Optional[torch.device] = None, backend: Optional[str] = None):
