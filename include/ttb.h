@@ -168,6 +168,10 @@ int ttb_add_bias_act(ttb_ctx* ctx, int dtype, void* out, const void* bias, int64
  * [0,vocab) is clamped and TTB_ERR_BAD_INDEX is recorded in the device status word. ---- */
 int ttb_lookup_embedding(ttb_ctx* ctx, int dtype, void* out, const void* table, const int64_t* ids,
                          int64_t n_ids, int64_t hidden, int64_t vocab, int add);
+/* Two of them in one pass: out[b*seq_len + i, :] = token[ids[b*seq_len + i], :] + position[i, :] (positions beyond the table are the caller's
+ * business). */
+int ttb_token_position_embedding(ttb_ctx* ctx, int dtype, void* out, const void* token, const void* position, const int64_t* ids, int64_t B,
+                                 int64_t seq_len, int64_t hidden, int64_t vocab);
 /* ---- A10: kernels::AddBias / AddInputBias (utils.cpp:103-169). ---- */
 int ttb_add_bias(ttb_ctx* ctx, int dtype, void* out, const void* bias, int64_t M, int64_t N);
 int ttb_add_input_bias(ttb_ctx* ctx, int dtype, const void* in1, const void* in2, const void* bias, int64_t M,

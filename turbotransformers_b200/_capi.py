@@ -75,6 +75,7 @@ SIGNATURES = {
     "ttb_context_attention_step": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64, f32, p, p]),
     "ttb_attention_decode": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64, f32, p]),
     "ttb_chain_forward": (i32, [p, i32, C.POINTER(ChainOp), i32, p]),
+    "ttb_token_position_embedding": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64]),
     "ttb_chain_rows": (i64, [i64, i64]),
     "ttb_attention_f32": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p]),
     "ttb_add_bias_layernorm_f32": (i32, [p, p, p, p, p, p, p, i64, i64, f32]),

@@ -1096,17 +1096,12 @@ void TokenPositionEmbedding::operator()(const Tensor& input_ids, Tensor* output,
   const int64_t B = input_ids.shape(0), L = input_ids.shape(1), H = token_.shape(1);
   const int dev = input_ids.device_id();
   ttb_ctx* c = DeviceContext(dev);
-  Tensor pos(nullptr);
-  int64_t* pos_ids = pos.Reshape<int64_t>({B, L}, kDLCUDA, dev, "TokenPositionEmbedding/positions");
-  Check(ttb_prepare_bert_masks(c, B, L, nullptr, nullptr, nullptr, pos_ids, nullptr), c, "TokenPositionEmbedding/positions");
-  output->Reshape(token_.dtype(), {B, L, H}, kDLCUDA, dev, "TokenPositionEmbedding/Reshape");
-  Check(ttb_lookup_embedding(c, dt, output->raw_mut(), token_.raw(), input_ids.data<int64_t>(), B * L, H, token_.shape(0), 0), c,
-        "TokenPositionEmbedding/token");
   TT_ENFORCE(position_offset >= 0 && position_offset + L <= position_.shape(0), "positions %lld..%lld exceed the %lld the model has",
              (long long)position_offset, (long long)(position_offset + L - 1), (long long)position_.shape(0));
+  output->Reshape(token_.dtype(), {B, L, H}, kDLCUDA, dev, "TokenPositionEmbedding/Reshape");
   const char* table = static_cast<const char*>(position_.raw()) + (size_t)position_offset * (size_t)H * (dt == TTB_F32 ? 4 : 2);
-  Check(ttb_lookup_embedding(c, dt, output->raw_mut(), table, pos_ids, B * L, H, position_.shape(0) - position_offset, 1), c,
-        "TokenPositionEmbedding/position");
+  Check(ttb_token_position_embedding(c, dt, output->raw_mut(), token_.raw(), table, input_ids.data<int64_t>(), B, L, H, token_.shape(0)), c,
+        "TokenPositionEmbedding");
   if (PreciseMode(dt)) {
     // start the fp32 residual stream of a bf16 model from the embedding sum (its one rounding is 2^-9 of a value of the
     // embeddings' size, far below what the blocks add)
