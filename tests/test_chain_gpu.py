@@ -161,3 +161,19 @@ def test_refusals(ctx):
         ctx.chain_forward([("linear", good)] * 129)
     with pytest.raises(_capi.TTBError):
         ctx.chain_forward([("attention", dict(q=x, out=out, rows=4, heads=1, length=3, ldq=192, ldo=64, keys=_capi.CHAIN_KEYS_ROWS))])
+
+
+def test_rows_that_a_chain_takes(ctx):
+    rows = _capi.lib().ttb_chain_rows
+    assert [rows(512, 2048), rows(768, 3072), rows(1024, 4096), rows(768, 100), rows(100, 512), rows(2048, 8192)] == [64, 64, 32, 0, 0, 0]
+    for hidden, inner in ((768, 3072), (1024, 4096)):  # the kernel agrees
+        for M in (rows(hidden, inner), rows(hidden, inner) + 1):
+            x, h, w1, w2 = half(M, hidden, seed=1), half(M, inner, seed=2), half(8, hidden, seed=3), half(8, inner, seed=4)
+            out, g = torch.zeros(M, 8, device=DEV).half(), half(hidden, seed=5)
+            ops = [("linear", dict(A=x, W=w1, out=out, M=M, N=8, K=hidden, lda=hidden, ldo=8, gamma=g, beta=g)),
+                   ("linear", dict(A=h, W=w2, out=out, M=M, N=8, K=inner, lda=inner, ldo=8))]
+            if M > rows(hidden, inner):
+                with pytest.raises(_capi.TTBError):
+                    ctx.chain_forward(ops)
+            else:
+                ctx.chain_forward(ops)

@@ -34,10 +34,10 @@ bool NormFits(const Tensor& gamma, const Tensor& beta, int64_t H, const Tensor& 
   return Vector(gamma, H, x) && Vector(beta, H, x) && Aligned({&gamma, &beta});
 }
 // The rows up to which one kernel is the faster route: above, every CTA's normalising of all rows and its reading of all of the wide
-// activation outweigh the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 307 / 412, 16 340 / 434,
-// 24 421 / 436, 32 448 / 436, 64 672 / 484 (300 cached: 392 / 494, 479 / 527, 542 / 550 at 16, 24, 32); BERT-base, tokens: 1 286 / 432, 16 318 / 439,
-// 24 394 / 427, 32 409 / 437, 48 529 / 436; BERT-large 16 689 / 873, 32 888 / 868. Layers with context attention are more launches, and
-// Python, for the same products: six steps of six layers, 200 source tokens, 1 row 1443 / 3579, 32 2277 / 3659, 64 3401 / 3641.
+// activation outweigh the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 286 / 414, 16 334 / 435,
+// 24 397 / 436, 32 443 / 436, 64 639 / 484 (300 cached: 370 / 492, 446 / 526, 526 / 549 at 16, 24, 32); BERT-base, tokens: 1 261 / 395, 16 307 / 399,
+// 24 368 / 399, 32 398 / 400, 48 509 / 406; BERT-large 16 669 / 873, 32 875 / 874. Layers with context attention are more launches, and
+// Python, for the same products: six steps of six layers, 200 source tokens, 1 row 1356 / 3292, 32 2233 / 3466, 64 3230 / 3415.
 constexpr int64_t kMostRows = 24, kMostRowsContext = TTB_CHAIN_MAX_ROWS;
 bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
   if (x.n_dim() != 3 || !x.on_gpu() || !core::SameType(x.dtype(), core::kFloat16)) return false;

@@ -15,6 +15,10 @@
 //     bytes past a multiple of 128). Partial sums meet in shared memory.
 //   * A layer norm in front of a product: every CTA normalises all rows itself into shared memory, which is cheaper than a barrier.
 //   * Attention: the warps of a CTA share a (row, head), or several; eight lanes a key, online softmax, merged through shared memory.
+//   * Code. Every operation runs through its instructions once, so that fetching them counts: loops over what differs from call to call are
+//     not unrolled and waits and copies are functions (167 -> 67 KB for 16 rows: 306 -> 286 us a step of the above, 349 -> 320 of 8 rows
+//     with 300 cached tokens).
+// Now 286 us a step (layer by layer 414 on the same box): 61 operations of 4.7 us, of which the barrier is about 1.2, the rows' trip from L2 0.5.
 #include <algorithm>
 #include <initializer_list>
 
@@ -149,6 +153,7 @@ __device__ __forceinline__ long long cache_row(int j, int b, int B, int H) { ret
 // A bounded wait (each attempt suspends the thread for up to 20 us, 2^17 of them are some seconds) without a call: what is live around a
 // call would be spilled, and a spill costs a trip to L2 here, since the barrier's acquire empties the L1 cache.
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
   for (int tries = 0; tries < (1 << 17); ++tries) {
     if (sm100::mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
@@ -168,6 +173,7 @@ __device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ bool feed_units(const ttb_chain_linear& o, int ks, int group, int hi, const ChainParams& prm, Shared& sm, uint32_t ring, int kpb,
                                            int consumed, Feed& f) {
   const int lane = threadIdx.x & 31, parts = div_small(o.K, ks);
+#pragma unroll 1
   while (f.first < hi) {  // groups of units; in a group all units of one batch of parts of K, then of the next
     if (f.issued - consumed >= prm.slots) return false;
     const uint32_t bar = sm100::smem_u32(&sm.full[f.w.slot]);
@@ -200,6 +206,7 @@ __device__ __noinline__ void feed(const ChainParams& prm, Shared& sm, uint32_t r
   const int lane = threadIdx.x & 31;
   Feed f = sm.feed;
   __syncwarp();
+#pragma unroll 1
   for (; f.op < prm.n_ops; ++f.op) {
     if (sm.ops[f.op].kind != TTB_CHAIN_LINEAR) continue;
     const ttb_chain_linear& o = sm.ops[f.op].u.linear;
@@ -231,17 +238,23 @@ __device__ __noinline__ void feed(const ChainParams& prm, Shared& sm, uint32_t r
   __syncwarp();
 }
 
-// Waits for the norm weights, bias and weights with which the CTA's share of an operation begins. One warp does it for all of them, ahead of
-// a barrier of the CTA and mostly in the shadow of the grid's.
-__device__ __forceinline__ bool wait_ahead(const ttb_chain_op& op, const Share& s, int slots, Shared& sm, Cursor w, const Cursor& p) {
-  if (op.kind != TTB_CHAIN_LINEAR || !s.part) return true;
-  bool ok = !s.params || wait(sm100::smem_u32(&sm.pfull[p.slot]), p.parity, &sm.abort_flag);
-  const int n = min(op.reserved >> 16, s.hi - s.lo) * div_small(op.u.linear.K, op.reserved & 0xffff);
+// Waits for the next n slots of the ring.
+__device__ __noinline__ bool wait_slots(int n, int slots, Shared& sm, Cursor w) {
+  bool ok = true;
+#pragma unroll 1
   for (int i = 0; ok && i < n; ++i) {
     ok = wait(sm100::smem_u32(&sm.full[w.slot]), w.parity, &sm.abort_flag);
     w.next(slots);
   }
   return ok;
+}
+
+// Waits for the norm weights, bias and weights with which the CTA's share of an operation begins. One warp does it for all of them, ahead of
+// a barrier of the CTA and mostly in the shadow of the grid's.
+__device__ __forceinline__ bool wait_ahead(const ttb_chain_op& op, const Share& s, int slots, Shared& sm, Cursor w, const Cursor& p) {
+  if (op.kind != TTB_CHAIN_LINEAR || !s.part) return true;
+  const bool ok = !s.params || wait(sm100::smem_u32(&sm.pfull[p.slot]), p.parity, &sm.abort_flag);
+  return ok && wait_slots(min(op.reserved >> 16, s.hi - s.lo) * div_small(op.u.linear.K, op.reserved & 0xffff), slots, sm, w);
 }
 
 // Brings the keys and values that an earlier launch has written, and that this CTA reads two operations later, to L2.
@@ -250,8 +263,10 @@ __device__ __forceinline__ void prefetch_keys(const ttb_chain_attention& o, int 
   const int H = o.heads * kHeadDim;
   const bool cached = o.keys == TTB_CHAIN_KEYS_CACHE;
   const int n = cached ? o.past : o.length;
+#pragma unroll 1
   for (int unit = blockIdx.x; unit < o.rows * o.heads; unit += gridDim.x) {
     const int row = div_small(unit, o.heads), h = unit - row * o.heads;
+#pragma unroll 1
     for (int j = thread; j < n; j += threads) {
       const long long at = cached ? cache_row(j, row, o.rows, H) + h * kHeadDim : ((long long)unit * o.length + j) * kHeadDim;
       prefetch_l2(static_cast<const __half*>(cached ? o.k_cache : o.k) + at);
@@ -380,87 +395,61 @@ __device__ __forceinline__ void unpack2(const uint4& q, Two (&f)[4]) {
 }
 
 // Layer norm of the operation's rows into shared memory, a warp per row (64 bytes past a multiple of 128 between rows, as in the ring).
-// Where a warp has several rows it takes two at a time, so that one's reductions wait while the other's are under way.
-template <int MT>
+// The next row of a warp is on its way while one is normalised.
 __device__ __forceinline__ void normalise(const ttb_chain_linear& o, const Share& s, Shared& sm, uint32_t a_smem, const Read& read) {
-  constexpr int kEach = MT * 16 / kWarps, kIters = kPart / 256;  // rows of a warp, 16-byte pieces of a row per lane
+  constexpr int kIters = kPart / 256;  // 16-byte pieces of a row per lane
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, K = o.K, M = o.M;
-  uint4 x[kEach][kIters];
   const __half* src = static_cast<const __half*>(o.A) + (long long)warp * o.lda + lane * 8;
-#pragma unroll
-  for (int r = 0; r < kEach; ++r)
-#pragma unroll
-    for (int i = 0; i < kIters; ++i) {
-      x[r][i] = make_uint4(0, 0, 0, 0);
-      if (warp + r * kWarps < M && i * 256 + lane * 8 < K) x[r][i] = *reinterpret_cast<const uint4*>(src + (long long)r * kWarps * o.lda + i * 256);
-    }
   const uint32_t gamma = sm100::smem_u32(sm.params[read.p.slot]) + lane * 16;
   const float inv_k = __fdividef(1.f, (float)K), eps = o.eps;
+  uint4 next[kIters];
 #pragma unroll
-  for (int r = 0; r < kEach; r += 2) {
-    if (warp + r * kWarps >= M) break;
-    Two f[2][kIters][4];
-    float mean[2], rstd[2];
+  for (int i = 0; i < kIters; ++i) {
+    next[i] = make_uint4(0, 0, 0, 0);
+    if (warp < M && i * 256 + lane * 8 < K) next[i] = *reinterpret_cast<const uint4*>(src + i * 256);
+  }
+#pragma unroll 1
+  for (int row = warp; row < M; row += kWarps) {
+    Two f[kIters][4], sum(0.f, 0.f), sq(0.f, 0.f);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      Two sum(0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < kIters; ++i) {  // (lanes beyond the row hold zeros)
-        unpack2(x[r + h][i], f[h][i]);
-        sum = sum + ((f[h][i][0] + f[h][i][1]) + (f[h][i][2] + f[h][i][3]));
-      }
-      mean[h] = sum.get().x + sum.get().y;
+    for (int i = 0; i < kIters; ++i) {  // (lanes beyond the row hold zeros)
+      unpack2(next[i], f[i]);
+      sum = sum + ((f[i][0] + f[i][1]) + (f[i][2] + f[i][3]));
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) mean[h] += __shfl_xor_sync(0xffffffffu, mean[h], d);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      mean[h] *= inv_k;
-      const Two minus(-mean[h], -mean[h]);
-      Two sq(0.f, 0.f);
+    src += (long long)kWarps * o.lda;
+    if (row + kWarps < M)
 #pragma unroll
       for (int i = 0; i < kIters; ++i)
-        if (i * 256 + lane * 8 < K)
+        if (i * 256 + lane * 8 < K) next[i] = *reinterpret_cast<const uint4*>(src + i * 256);
+    const float mean = warp_sum(sum.get().x + sum.get().y) * inv_k;
+    const Two minus(-mean, -mean);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            f[h][i][e] = f[h][i][e] + minus;
-            sq = fma2(f[h][i][e], f[h][i][e], sq);
-          }
-      rstd[h] = sq.get().x + sq.get().y;
-    }
+    for (int i = 0; i < kIters; ++i)
+      if (i * 256 + lane * 8 < K)
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) rstd[h] += __shfl_xor_sync(0xffffffffu, rstd[h], d);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) rstd[h] = rsqrtf(rstd[h] * inv_k + eps);
+        for (int e = 0; e < 4; ++e) {
+          f[i][e] = f[i][e] + minus;
+          sq = fma2(f[i][e], f[i][e], sq);
+        }
+    const float rstd = rsqrtf(warp_sum(sq.get().x + sq.get().y) * inv_k + eps);
+    const Two scale(rstd, rstd);
+    const uint32_t to = a_smem + row * (K * 2 + kRowPad) + lane * 16;
 #pragma unroll
     for (int i = 0; i < kIters; ++i)
       if (i * 256 + lane * 8 < K) {
         Two ga[4], be[4];
         unpack2(lds128(gamma + i * 512), ga);
         unpack2(lds128(gamma + kPart * 2 + i * 512), be);
+        float y[8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = warp + (r + h) * kWarps;
-          const Two scale(rstd[h], rstd[h]);
-          float y[8];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 v = fma2(f[h][i][e] * scale, ga[e], be[e]).get();
-            y[2 * e] = v.x;
-            y[2 * e + 1] = v.y;
-          }
-          const uint4 q = pack(y);
-          if (row < M) {
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a_smem + row * (K * 2 + kRowPad) + i * 512 + lane * 16), "r"(q.x), "r"(q.y), "r"(q.z),
-                         "r"(q.w)
-                         : "memory");
-            if (s.writes && (int)blockIdx.x == row) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = q;
-          }
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = fma2(f[i][e] * scale, ga[e], be[e]).get();
+          y[2 * e] = v.x;
+          y[2 * e + 1] = v.y;
         }
+        const uint4 q = pack(y);
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + i * 512), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+        if (s.writes && (int)blockIdx.x == row) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = q;
       }
   }
 }
@@ -472,14 +461,16 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
   constexpr int KW = Layout<MT>::KW, CPK = Layout<MT>::CPK;
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int mt = warp % MT, share = warp / MT, chunks = ks / 32;
-  normalise<MT>(o, s, sm, a_smem, read);
+  normalise(o, s, sm, a_smem, read);
   bool ok = true;
   const uint32_t lane_at = g * (ks * 2 + kRowPad) + share * 64 + t * 16;
   const uint32_t w_lane = ring + lane_at, a_lane = a_smem + mt * 16 * (ks * 2 + kRowPad) + lane_at, a_eight = 8 * (ks * 2 + kRowPad);
   const bool low = mt * 16 < o.M, high = mt * 16 + 8 < o.M;  // rows of the tile's halves (rows that are not there leave sums that nobody reads)
   __syncthreads();
+#pragma unroll 1
   for (int u0 = s.lo; u0 < s.hi; u0 += group) {
     const int nu = min(group, s.hi - u0);
+    if (u0 != s.lo) ok = wait_slots(nu, prm.slots, sm, read.w) && ok;
     uint32_t at[kGroup];
     float acc[kGroup][4];
 #pragma unroll
@@ -488,7 +479,6 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[u][e] = 0.f;
       if (u < nu) {
-        if (u0 != s.lo) ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
         at[u] = w_lane + read.w.slot * prm.slot_bytes;
         read.w.next(prm.slots);
         ++read.slots;
@@ -522,15 +512,7 @@ __device__ __forceinline__ bool linear_norm(const ttb_chain_linear& o, const Sha
     fetch_residual<MT>(o, u0, nu, res);
     epilogue<MT>(o, sm, sm.params[read.p.slot] + kPart * 4 + (u0 - s.lo) * 16, u0, nu, res);
     if (u0 + group < s.hi) {
-      if (warp == kWarps - 1) {  // the ring behind a wide product, such as a vocabulary, is filled as it goes
-        Feed f = sm.feed;
-        __syncwarp();
-        if (f.op == op) {
-          feed_units(o, ks, group, s.hi, prm, sm, ring, Layout<MT>::kBatch, read.slots, f);
-          if (lane == 0) sm.feed = f;
-          __syncwarp();
-        }
-      }
+      if (warp == kWarps - 1) feed(prm, sm, ring, Layout<MT>::kBatch, read.slots, read.params);  // behind a wide product, such as a vocabulary
       __syncthreads();  // the next group's partial sums take the same place
     }
   }
@@ -551,9 +533,12 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
   const __half* a_lane = static_cast<const __half*>(o.A) + (long long)r0 * o.lda + share * 32 + t * 8;
   const uint32_t w_lane = ring + g * (ks * 2 + kRowPad) + share * 64 + t * 16;
   bool ok = true;
+#pragma unroll 1
   for (int u0 = s.lo; u0 < s.hi; u0 += group) {
     const int nu = min(group, s.hi - u0);
+    if (u0 != s.lo) ok = wait_slots(nu * parts, prm.slots, sm, read.w) && ok;
     __half2 res[Layout<MT>::kItems];
+#pragma unroll 1
     for (int kb = 0; kb < parts; kb += kBatch) {
       uint4 a0[kBatch * CPK], a1[kBatch * CPK];
 #pragma unroll
@@ -570,12 +555,12 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
         }
       }
       if (kb == 0) fetch_residual<MT>(o, u0, nu, res);  // what the epilogue adds is on its way before the products
+#pragma unroll 1
       for (int u = 0; u < nu; ++u) {
         float acc[2][4] = {};  // two chains of sums
 #pragma unroll
         for (int kl = 0; kl < kBatch; ++kl)
           if (kb + kl < parts) {
-            if (u0 != s.lo) ok = wait(sm100::smem_u32(&sm.full[read.w.slot]), read.w.parity, &sm.abort_flag) && ok;
             const uint32_t at = w_lane + read.w.slot * prm.slot_bytes;
 #pragma unroll
             for (int i = 0; i < CPK; ++i)
@@ -602,15 +587,7 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
     __syncthreads();
     epilogue<MT>(o, sm, sm.params[read.p.slot] + kPart * 4 + (u0 - s.lo) * 16, u0, nu, res);
     if (u0 + group < s.hi) {
-      if (warp == kWarps - 1) {
-        Feed f = sm.feed;
-        __syncwarp();
-        if (f.op == op) {
-          feed_units(o, ks, group, s.hi, prm, sm, ring, kBatch, read.slots, f);
-          if (lane == 0) sm.feed = f;
-          __syncwarp();
-        }
-      }
+      if (warp == kWarps - 1) feed(prm, sm, ring, kBatch, read.slots, read.params);
       __syncthreads();
     }
   }
@@ -625,7 +602,7 @@ __device__ __forceinline__ bool linear_plain(const ttb_chain_linear& o, const Sh
 // attention
 // ---------------------------------------------------------------------------------------------
 // (row, head) pairs go round the CTAs; a CTA's warps are shared out among as many of its pairs as they serve at once, each taking
-// every W-th page of 16 keys: four keys a load, two pages of keys and two of values in flight per warp.
+// every W-th page of 16 keys: four keys a load, the next page on its way while one is worked on.
 __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& sm) {
   constexpr int kState = kHeadDim + 2;
   const int tid = thread(), warp = tid >> 5, lane = tid & 31, sub = lane & 7, kg = lane >> 3;
@@ -634,6 +611,7 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
   if (total <= (int)blockIdx.x) return;
   const int W = max(1, div_small(kWarps, mine)), S = div_small(kWarps, W);  // warps a pair, pairs at once
   const int place = div_small(warp, W), wi = warp - place * W;
+#pragma unroll 1
   for (int first = 0; first < mine; first += S) {
     const bool active = place < S && first + place < mine;
     const int unit = active ? (first + place) * (int)gridDim.x + (int)blockIdx.x : 0;
@@ -683,23 +661,26 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
       }
       const int fresh = keys == TTB_CHAIN_KEYS_CACHE ? n - 1 : -1;  // the key that is not in the cache yet
       const __half *kp = k0 + wi * page + (long long)kg * pitch + sub * 8, *vp = v0 + wi * page + (long long)kg * pitch + sub * 8;
-      auto load = [&](uint4 (&dst)[8], const __half* from, const __half* own, int j0) {
+      uint4 kr[4], vr[4], kn[4], vn[4];
+#pragma unroll 1
+      for (int j0 = (wi - W) * 16; j0 < n; j0 += 16 * W) {
+        // the next page is on its way while this one (there is none at first) is worked on
+        const int j1 = j0 + 16 * W + kg;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int j = j0 + (u >> 2) * 16 * W + (u & 3) * 4 + kg;
-          dst[u] = make_uint4(0, 0, 0, 0);
-          if (j < n) dst[u] = *reinterpret_cast<const uint4*>(j == fresh ? own + sub * 8 : from + (u >> 2) * W * page + (u & 3) * 4 * pitch);
+        for (int u = 0; u < 4; ++u) {
+          kn[u] = vn[u] = make_uint4(0, 0, 0, 0);
+          const int j = j1 + u * 4;
+          if (j < n) {
+            kn[u] = *reinterpret_cast<const uint4*>(j == fresh ? qrow + H + sub * 8 : kp + u * 4 * pitch);
+            vn[u] = *reinterpret_cast<const uint4*>(j == fresh ? qrow + 2 * H + sub * 8 : vp + u * 4 * pitch);
+          }
         }
-      };
-      uint4 kr[8], vr[8];
-      load(kr, kp, qrow + H, wi * 16);
-      load(vr, vp, qrow + 2 * H, wi * 16);
-      for (int j0 = wi * 16; j0 < n; j0 += 32 * W) {
-        float sc[8], top = m;
-        const int pages = j0 + 16 * W < n ? 8 : 4;  // the second page may not be there
+        kp += W * page;
+        vp += W * page;
+        if (j0 >= 0) {
+          float sc[4], top = m;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (u < pages) {
+          for (int u = 0; u < 4; ++u) {
             float f[8], dot[2];
             unpack(kr[u], f);
             dot[0] = q[0] * f[0];
@@ -707,34 +688,29 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
 #pragma unroll
             for (int e = 2; e < 8; ++e) dot[e & 1] = fmaf(q[e], f[e], dot[e & 1]);
             sc[u] = dot[0] + dot[1];
-          } else {
-            sc[u] = 0.f;
           }
-        kp += 2 * W * page;
-        load(kr, kp, qrow + H, j0 + 32 * W);  // the next pages' keys travel while these are finished
 #pragma unroll
-        for (int o2 = 1; o2 < 8; o2 <<= 1)
+          for (int d = 1; d < 8; d <<= 1)
 #pragma unroll
-          for (int u = 0; u < 8; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], o2);
+            for (int u = 0; u < 4; ++u) sc[u] += __shfl_xor_sync(0xffffffffu, sc[u], d);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int j = j0 + (u >> 2) * 16 * W + (u & 3) * 4 + kg;
-          if (j < n) {
-            if (mask) sc[u] += mask[j] * kLog2e;
-            if (scores && sub == 0) scores[j] = sc[u];
-          } else {
-            sc[u] = -INFINITY;
+          for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * 4 + kg;
+            if (j < n) {
+              if (mask) sc[u] += mask[j] * kLog2e;
+              if (scores && sub == 0) scores[j] = sc[u];
+            } else {
+              sc[u] = -INFINITY;
+            }
+            top = fmaxf(top, sc[u]);
           }
-          top = fmaxf(top, sc[u]);
-        }
-        const float base = top == -INFINITY ? 0.f : top, keep = ex2f(m - base);
-        m = top;
-        l *= keep;
+          const float base = top == -INFINITY ? 0.f : top, keep = ex2f(m - base);
+          m = top;
+          l *= keep;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] *= keep;
+          for (int e = 0; e < 8; ++e) acc[e] *= keep;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-          if (u < pages) {
+          for (int u = 0; u < 4; ++u) {
             const float pr = ex2f(sc[u] - base);
             float f[8];
             unpack(vr[u], f);
@@ -742,8 +718,12 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
 #pragma unroll
             for (int e = 0; e < 8; ++e) acc[e] = fmaf(pr, f[e], acc[e]);
           }
-        vp += 2 * W * page;
-        load(vr, vp, qrow + 2 * H, j0 + 32 * W);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          kr[u] = kn[u];
+          vr[u] = vn[u];
+        }
       }
       if (files) *file_to = newest;
     }
@@ -785,6 +765,7 @@ __device__ __forceinline__ void attention(const ttb_chain_attention& o, Shared& 
         *reinterpret_cast<__half2*>(static_cast<__half*>(o.out) + (long long)row * o.ldo + h * kHeadDim + lane * 2) = __floats2half2_rn(v.x * inv, v.y * inv);
       }
       if (scores)
+#pragma unroll 1
         for (int j = wi * 32 + lane; j < n; j += W * 32)
           static_cast<__half*>(o.probs)[(long long)row * o.length + j] = __float2half_rn(ex2f(scores[j] - base) * inv);
     }
@@ -812,9 +793,11 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
     const uint32_t* from = reinterpret_cast<const uint32_t*>(prm.ops);
     asm volatile("" : "+l"(from));  // as memory: a constant load with an address for each thread would go one thread after the other
     uint32_t* to = reinterpret_cast<uint32_t*>(sm.ops);
+#pragma unroll 1
     for (int i = tid; i < prm.n_ops * kOpWords; i += kThreads) to[i] = from[i];
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < prm.n_ops; i += kThreads)
     if (sm.ops[i].kind == TTB_CHAIN_LINEAR) sm.share[i] = Share(sm.ops[i].u.linear);
   __syncthreads();
@@ -824,6 +807,7 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
     wait_ahead(sm.ops[0], sm.share[0], prm.slots, sm, read.w, read.p);
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = 0; !sm.abort_flag;) {
     const ttb_chain_op& op = sm.ops[i];
     bool ok = true;
@@ -860,8 +844,10 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
   }
   if (warp == kWarps - 1) {  // every copy lands before the CTA's shared memory goes, also where a wait has run out
     const Feed f = sm.feed;
+#pragma unroll 1
     for (int s = 0; s < prm.slots; ++s)
       if (s < f.issued) drain(sm100::smem_u32(&sm.full[s]), s < f.w.slot ? f.w.parity : f.w.parity ^ 1);
+#pragma unroll 1
     for (int s = 0; s < kParamSlots; ++s)
       if (s < f.p_issued) drain(sm100::smem_u32(&sm.pfull[s]), s < f.p.slot ? f.p.parity : f.p.parity ^ 1);
   }
