@@ -67,7 +67,7 @@ def test_product_of_rows_as_they_are(ctx, M, N, K):
     assert torch.equal(lo, rest(out))
 
 
-@pytest.mark.parametrize("M,N", [(1, 768), (37, 1024), (3000, 768), (5, 770)])
+@pytest.mark.parametrize("M,N", [(1, 768), (37, 1024), (1184, 768), (1185, 768), (3000, 768), (5, 770)])
 def test_layer_norm(ctx, M, N):
     g = torch.Generator(device=DEV).manual_seed(N)
     x, y = torch.randn(M, N, generator=g, device=DEV), torch.randn(M, N, generator=g, device=DEV)

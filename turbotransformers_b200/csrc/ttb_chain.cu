@@ -18,7 +18,7 @@
 //   * Code. Every operation runs through its instructions once, so that fetching them counts: loops over what differs from call to call are
 //     not unrolled and waits and copies are functions (167 -> 67 KB for 16 rows: 306 -> 286 us a step of the above, 349 -> 320 of 8 rows
 //     with 300 cached tokens).
-// Now 286 us a step (layer by layer 414 on the same box): 61 operations of 4.7 us, of which the barrier is about 1.2, the rows' trip from L2 0.5.
+// Now 286 us a step (layer by layer 414 on the same GPU): 61 operations of 4.7 us, of which the barrier is about 1.2, the rows' trip from L2 0.5.
 #include <algorithm>
 #include <initializer_list>
 
