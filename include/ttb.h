@@ -47,6 +47,9 @@ typedef enum {
  * [N, round_up(N, 8)) of every output row scratch (the fast store path overwrites them with zeros). Without it
  * such an output takes a slower element-wise store that leaves those columns untouched. */
 #define TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH 0x100
+/* May be OR-ed into ttb_linear_ex's `epilogue` for an F32 product with out_lo: out and out_lo receive the two planes that ttb_split_tf32 makes
+ * of the result, in place of the result, so that the product that reads them sees every value to 2^-23. */
+#define TTB_EPI_FLAG_TF32_PLANES 0x200
 
 /* ---- context: replaces core::CUDADeviceContext (turbo_transformers/core/cuda_device_context.cpp:23-60),
  * one per device (and per host thread, if callers want concurrency) instead of one global singleton. ---- */
@@ -150,9 +153,12 @@ int ttb_mask_softmax(ttb_ctx* ctx, int dtype, void* scores, const float* mask, i
  * `eps` is honoured (the reference GPU kernel ignored it, gpu_layer_norm_kernel.cu:48,98). ---- */
 int ttb_add_bias_layernorm(ttb_ctx* ctx, int dtype, void* out, const void* input, const void* bias,
                            const void* gamma, const void* beta, int64_t M, int64_t N, float eps);
-/* The same for fp32, leaving beside out the plane out_lo (may be NULL) that ttb_linear_ex takes as A2. */
+/* The same for fp32, leaving beside out the plane out_lo (may be NULL) that ttb_linear_ex takes as A2 where out itself is A; or, in
+ * hi and lo (both or neither), the planes that ttb_split_tf32 makes of out, which hold it to one bit more. */
 int ttb_add_bias_layernorm_f32(ttb_ctx* ctx, float* out, float* out_lo, const float* input, const float* bias, const float* gamma,
                                const float* beta, int64_t M, int64_t N, float eps);
+int ttb_add_bias_layernorm_f32_planes(ttb_ctx* ctx, float* out, float* hi, float* lo, const float* input, const float* bias, const float* gamma,
+                                      const float* beta, int64_t M, int64_t N, float eps);
 /* ---- A7: kernels::LayerNorm (layer_norm.cpp:32-91): in place. `in` may equal `out`. ---- */
 int ttb_layernorm(ttb_ctx* ctx, int dtype, const void* in, void* out, const void* gamma, const void* beta,
                   int64_t M, int64_t N, float eps);
@@ -213,13 +219,13 @@ int ttb_linear(ttb_ctx* ctx, int dtype, const void* A, int64_t lda, const void* 
  *   dtype F16 / BF16, A2 != NULL           out = epilogue(A . W^T + A2 . W^T): activations kept as a rounded value plus what
  *                                          the rounding dropped (see out_lo), so a bf16 model's GEMMs see 16 significant bits
  *   dtype F32 (A, A2, W, W2 all given)     out = epilogue(A . W^T + A2 . W^T + A . W2^T) on tf32 tensor cores: A/A2 and W/W2
- *                                          are the hi/lo planes ttb_split_tf32 makes; or A is fp32 as it is, of which the tensor
- *                                          cores take the first 19 bits, and A2 what they drop (out_lo). The sum has fp32-level accuracy. This is
+ *                                          are the hi/lo planes ttb_split_tf32 makes (values to 2^-23); or A is fp32 as it is, of which
+ *                                          the tensor cores take the first 19 bits, and A2 what they drop (out_lo; values to 2^-22). This is
  *                                          the tensor-core route of kernels::MatMul for fp32 models (mat_mul.cpp:81-96, where
  *                                          the reference selects CUBLAS_GEMM_DEFAULT_TENSOR_OP)
  * out_dtype is dtype, or F32 for 16-bit operands (an fp32 residual stream); bias and residual are of out_dtype. out_lo
  * (BF16 and F32 products, may be NULL) receives, with out's pitch, what a product that reads out drops of every value v: v - round(v), or
- * for F32 the last 13 bits of v, as tf32. W and W2 are
+ * for F32 the last 13 bits of v, as tf32 (see TTB_EPI_FLAG_TF32_PLANES for both planes of a rounding). W and W2 are
  * K-major [N, K] (ttb_prepack_weight). K % 8 == 0 (16-bit) or K % 4 == 0 (F32); lda likewise. */
 typedef struct ttb_linear_args {
   int dtype, out_dtype;
@@ -328,9 +334,12 @@ int ttb_attention_fwd(ttb_ctx* ctx, int dtype, const void* qkv, int64_t total_to
 
 /* Self-attention of fp32 models over packed tokens (the same five kernels in one, in fp32 throughout): qkv fp32 [T, 3*heads*64] with the bias
  * added, cu_seqlens, mask and out as for ttb_attention_fwd. out_lo [T, heads*64] receives the plane that ttb_linear_ex takes as A2
- * beside out (what the tensor cores drop of it), or NULL. d == 64, 16-byte aligned buffers. */
+ * beside out (what the tensor cores drop of it), or NULL; ttb_attention_f32_planes leaves the two planes that ttb_split_tf32 makes of the
+ * output in its place. d == 64, 16-byte aligned buffers. */
 int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
                       const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo);
+int ttb_attention_f32_planes(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
+                             const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* hi, float* lo);
 
 /* Decoder step with a key/value cache: replaces the per-step Concat of the whole cache and the padded attention sequence
  * of `layer_cache` self-attention (multi_headed_attention.cpp:207-231, 320-354; Concat: kernels/utils.cpp:32-97).
@@ -414,7 +423,8 @@ int ttb_embedding_ln(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64_t*
                      const void* gamma, const void* beta, int64_t hidden, int64_t vocab, int64_t n_positions,
                      int64_t n_types, float eps, void* out);
 
-/* ttb_embedding_ln with the two extra outputs of ttb_layernorm_planes (either may be NULL). */
+/* ttb_embedding_ln with the two extra outputs of ttb_layernorm_planes (either may be NULL). F32: out_f32 and out_lo given together receive
+ * the two planes that ttb_split_tf32 makes of out; out_lo alone what the tensor cores drop of it. */
 int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64_t* position_ids,
                             const int64_t* token_type_ids, const int32_t* cu_seqlens, int64_t B, int64_t seq_len,
                             int64_t n_tokens, const void* word, const void* position, const void* token_type,

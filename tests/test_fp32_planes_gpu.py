@@ -77,3 +77,80 @@ def test_layer_norm(ctx, M, N):
     ctx.call("add_bias_layernorm_f32", out, lo, y, bias, gamma, beta, M, N, 1e-12)
     assert err(out, want) < 1e-6
     assert torch.equal(lo, rest(out))
+
+
+def split(ctx, x):
+    hi, lo = torch.zeros_like(x), torch.zeros_like(x)
+    ctx.call("split_tf32", x, x.numel(), hi, lo)
+    return torch.stack([hi, lo])
+
+
+@pytest.mark.parametrize("M,N", [(1, 768), (128, 3072), (200, 100), (1100, 3072), (3000, 3072), (130, 770), (77, 2316)])
+def test_planes_of_a_product(ctx, M, N):
+    """Every tile of the product (few rows, split along K, wide, pairs, ragged) leaves, in place of its output, what splitting that output gives."""
+    K = 768 if M != 130 else 64
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x, w, bias = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV) * K ** -0.5, torch.randn(N, generator=g, device=DEV)
+    a, b = split(ctx, x), split(ctx, w)
+    hi, lo, plain, rest_of_plain = (torch.full((M, N), 7.0, device=DEV) for _ in range(4))
+    product = lambda epilogue, out, **kw: ctx.linear_ex(_capi.F32, _capi.F32, a[0], b[0], M, N, K, epilogue, out, A2=a[1], W2=b[1], bias=bias, **kw)
+    product(_capi.EPI_BIAS_GELU | _capi.EPI_FLAG_TF32_PLANES, hi, out_lo=lo)
+    product(_capi.EPI_BIAS_GELU, plain, out_lo=rest_of_plain)  # the same tile, and with it the same sums
+    assert torch.equal(torch.stack([hi, lo]), split(ctx, plain))
+    with pytest.raises(_capi.TTBError):
+        product(_capi.EPI_BIAS_GELU | _capi.EPI_FLAG_TF32_PLANES, plain)
+
+
+def test_planes_of_layer_norm_attention_and_embedding(ctx):
+    g = torch.Generator(device=DEV).manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device=DEV)
+    for M, N in ((1, 768), (37, 1024), (1184, 768), (1185, 768), (5, 770)):
+        out, hi, lo = rand(M, N), torch.zeros(M, N, device=DEV), torch.zeros(M, N, device=DEV)
+        ctx.call("add_bias_layernorm_f32_planes", out, hi, lo, rand(M, N), rand(N), rand(N), rand(N), M, N, 1e-12)
+        assert torch.equal(torch.stack([hi, lo]), split(ctx, out))
+    for lens in ([1], [7, 64, 33, 120], [65] * 30):
+        T, H = sum(lens), 768
+        cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+        qkv, out, hi, lo = rand(T, 3 * H), *(torch.zeros(T, H, device=DEV) for _ in range(3))
+        ctx.call("attention_f32", qkv, cu, len(lens), max(lens), 12, 64, None, 0, 0, 0, 0.125, out, None)
+        ctx.call("attention_f32_planes", qkv, cu, len(lens), max(lens), 12, 64, None, 0, 0, 0, 0.125, hi, lo)
+        assert torch.equal(torch.stack([hi, lo]), split(ctx, out))
+    ids, out, planes = torch.randint(0, 100, (3, 7), generator=g, device=DEV), torch.zeros(21, 768, device=DEV), torch.zeros(2, 21, 768, device=DEV)
+    ctx.call("embedding_ln_planes", _capi.F32, ids, None, None, None, 3, 7, 21, rand(100, 768), rand(16, 768), rand(2, 768), rand(768), rand(768), 768, 100, 16, 2,
+             1e-12, out, planes[1], planes[0])
+    assert torch.equal(planes, split(ctx, out))
+
+
+@pytest.mark.parametrize("B,L", [(1, 17), (3, 64), (9, 200)])
+def test_planes_hold_an_activation_to_the_last_bit_that_splitting_it_would(B, L):
+    """A layer gives the same bits for an activation that brings its planes along and for the same values without them."""
+    import turbotransformers_b200 as tt
+    from turbotransformers_b200 import synthetic
+    from turbotransformers_b200._cxx import cxx
+    hf = synthetic.make_hf_bert("bert-base", num_layers=1).to(DEV).encoder.layer[0]
+    attention, inter, out = tt.BertAttention.from_torch(hf.attention), tt.BertIntermediate.from_torch(hf.intermediate), tt.BertOutput.from_torch(hf.output)
+    turbo = tt.ReturnType.turbo_transformers
+    bare = lambda t: torch.from_numpy(cxx.tensor2nparrayf(t)).to(DEV)
+    x = torch.randn(B, L, 768, generator=torch.Generator(device=DEV).manual_seed(B), device=DEV)
+    a = attention(x, return_type=turbo)[0]
+    i = inter(a, return_type=turbo)
+    assert torch.equal(bare(i), inter(bare(a)))
+    y = out(i, a, return_type=turbo)
+    assert torch.equal(bare(y), out(bare(i), bare(a)))
+    assert torch.equal(attention(y)[0], attention(bare(y))[0])
+    # a NaN or an infinity, from the largest values on, is not lost on the way
+    for bad in (float("nan"), float("inf"), 3.4e38):
+        z = bare(y).clone()
+        z.view(-1, 768)[0, 5] = bad
+        assert not torch.isfinite(out(inter(z, return_type=turbo), z).view(-1, 768)[0]).any()
+        w = attention(z)[0].view(B, L, 768)
+        assert not torch.isfinite(out(inter(w, return_type=turbo), w)[0, 0]).any() and torch.isfinite(w[1:]).all()
+    # between the two products of a layer the activation is its planes
+    planes = cxx.Tensor.create_empty()
+    inter.for_output(a, planes)
+    assert err(out(planes, a), bare(y)) < 2e-6  # (the tile of the first product, and with it the order of its sums, may be another)
+    cxx.set_fp32_tensor_cores(False)
+    try:  # and stays what it is when the switch is thrown in between
+        assert err(out(planes, a), bare(y)) < 1e-4
+    finally:
+        cxx.set_fp32_tensor_cores(True)

@@ -14,6 +14,7 @@ F32, F16, BF16, I8 = 0, 1, 2, 3
 ACT_GELU, ACT_TANH, ACT_RELU = 0, 1, 2
 POOL_FIRST, POOL_LAST, POOL_MEAN, POOL_MAX = 0, 1, 2, 3
 EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESIDUAL, EPI_BIAS_TANH = 0, 1, 2, 3, 4
+EPI_FLAG_TF32_PLANES = 0x200
 ERR_INVALID, ERR_CUDA, ERR_UNSUPPORTED, ERR_OOM, ERR_DEVICE_WAIT, ERR_BAD_INDEX = 1, 2, 3, 4, 5, 6
 
 p, i32, i64, f32, sz = C.c_void_p, C.c_int, C.c_int64, C.c_float, C.c_size_t
@@ -78,7 +79,9 @@ SIGNATURES = {
     "ttb_token_position_embedding": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64]),
     "ttb_chain_rows": (i64, [i64, i64]),
     "ttb_attention_f32": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p]),
+    "ttb_attention_f32_planes": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p]),
     "ttb_add_bias_layernorm_f32": (i32, [p, p, p, p, p, p, p, i64, i64, f32]),
+    "ttb_add_bias_layernorm_f32_planes": (i32, [p, p, p, p, p, p, p, p, i64, i64, f32]),
     "ttb_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, f32, f32, p]),
     "ttb_batch_matmul": (i32, [p, i32, p, i32, p, i32, i64, i64, i64, i64, f32, f32, p]),
     "ttb_split_add_bias_transpose": (i32, [p, i32, p, p, i64, i64, i64, i64, p, p, p]),

@@ -155,7 +155,7 @@ struct BertModel::Impl {
     (*embedding_)(ids, pos, seq_type, &hidden);
     for (const auto& layer : layers_) {
       layer->attention(hidden, ext_mask, &att_out);
-      layer->intermediate(att_out, &inter);
+      layer->intermediate.ForOutput(att_out, &inter);
       layer->output(inter, att_out, &hidden);
     }
     std::vector<float> out;
@@ -185,7 +185,7 @@ struct BertModel::Impl {
     embedding_->Packed(ids, lens, &hidden);
     for (const auto& layer : layers_) {
       layer->attention.Run(hidden, no_mask, &lens, &att_out, nullptr, false, true, false, false);
-      layer->intermediate(att_out, &inter);
+      layer->intermediate.ForOutput(att_out, &inter);
       layer->output(inter, att_out, &hidden);
     }
     std::vector<float> out;

@@ -152,11 +152,13 @@ class Tensor {
 
   // Companion planes a layer may attach to an activation it produced, for the next layer to use (they travel with
   // the tensor through moves, and are dropped when it is reshaped or exported):
-  //   lo  : same shape and dtype, what rounding to the 16-bit type dropped (value = this + lo to 16 significant bits); of an fp32
-  //         activation what the tensor cores drop of it, as tf32
+  //   lo  : same shape and dtype, what rounding to the 16-bit type dropped (value = this + lo to 16 significant bits); of an fp32 tensor
+  //         that travels between two of the runtime's own products only, or with hi, what rounding to tf32 dropped
   //   f32 : same shape in fp32, the unrounded value (the residual stream of a bf16 model)
+  //   hi  : of an fp32 activation, the value rounded to tf32 (the tensor itself is the unrounded value, hi + lo what a product reads)
   const Tensor* lo() const;
   const Tensor* f32() const;
+  const Tensor* hi() const;
   const Tensor* q8() const;
   const Tensor* q8_scale() const;
   TensorExtras& NewExtras();
@@ -175,6 +177,7 @@ class Tensor {
 struct TensorExtras {
   Tensor lo{nullptr};
   Tensor f32{nullptr};
+  Tensor hi{nullptr};
   // int8 models: the per-row symmetric int8 form of this activation and its row scales, written by the layer norm that
   // produced it so that the next int8 Linear does not quantise it again
   Tensor q8{nullptr};
@@ -182,6 +185,7 @@ struct TensorExtras {
 };
 inline const Tensor* Tensor::lo() const { return extras_ && !extras_->lo.is_null() ? &extras_->lo : nullptr; }
 inline const Tensor* Tensor::f32() const { return extras_ && !extras_->f32.is_null() ? &extras_->f32 : nullptr; }
+inline const Tensor* Tensor::hi() const { return extras_ && !extras_->hi.is_null() ? &extras_->hi : nullptr; }
 inline const Tensor* Tensor::q8() const { return extras_ && !extras_->q8.is_null() ? &extras_->q8 : nullptr; }
 inline const Tensor* Tensor::q8_scale() const { return extras_ && !extras_->q8_scale.is_null() ? &extras_->q8_scale : nullptr; }
 inline TensorExtras& Tensor::NewExtras() {

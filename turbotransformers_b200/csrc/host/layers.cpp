@@ -42,12 +42,16 @@ std::vector<int64_t> WithLast(const Tensor& t, int64_t last) {
 // for the residual stream, an fp32 copy; see core::Tensor::lo() / f32().
 bool PreciseMode(int dt) { return dt == TTB_BF16 && core::PreciseBF16(); }
 
-// fp32 models on the tensor cores: an activation travels with the plane that a product takes beside it (core::Tensor::lo(): what the
-// tensor cores drop of it), written by the kernel that makes the activation.
+// fp32 models on the tensor cores: an activation travels with the two planes that a product takes (core::Tensor::hi(), lo()), written by the
+// kernel that makes the activation; where nothing but a product reads it, it is the first plane itself and lo() the second. Both are
+// the planes of a rounding. With the activation as it is for the first, which the tensor cores truncate, the second would have 13 bits for 11
+// and always the activation's sign, so that what the accumulator cuts off a product no longer averages out: whole models 4 % less accurate.
 bool Fp32Planes(int dt) { return dt == TTB_F32 && core::Fp32TensorCores(); }
-float* NewLo(Tensor* t) {
-  const auto shape = ShapeOf(*t);
-  return t->NewExtras().lo.Reshape<float>(shape, kDLCUDA, t->device_id(), "fp32/lo_plane");
+float* NewLo(Tensor* t) { return t->NewExtras().lo.Reshape<float>(ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/lo_plane"); }
+void NewPlanes(Tensor* t, float** hi, float** lo) {
+  core::TensorExtras& ex = t->NewExtras();
+  *hi = ex.hi.Reshape<float>(ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/hi_plane");
+  *lo = ex.lo.Reshape<float>(ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/lo_plane");
 }
 
 // out = LN(in) with the companion planes attached to `out` (already reshaped to its 16-bit shape). `in` is fp32 when
@@ -74,11 +78,13 @@ void LayerNormWithInt8(ttb_ctx* c, Tensor* t, const Tensor& gamma, const Tensor&
   Check(ttb_layernorm_quant_int8(c, dt, ptr, ptr, q, s, gamma.raw(), beta.raw(), M, N, eps), c, name);
 }
 
-// t = LN(t + input + bias) of an fp32 model, with the plane that the next product takes beside it.
+// t = LN(t + input + bias) of an fp32 model, with the planes that the next product takes.
 void AddBiasLayerNormF32(ttb_ctx* c, Tensor* t, const Tensor& input, const Tensor& bias, const Tensor& gamma, const Tensor& beta, int64_t M, int64_t N,
                          const char* name) {
-  float* lo = Fp32Planes(TTB_F32) ? NewLo(t) : nullptr;
-  Check(ttb_add_bias_layernorm_f32(c, t->mutableData<float>(), lo, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
+  float* out = t->mutableData<float>();
+  float *hi = nullptr, *lo = nullptr;
+  if (Fp32Planes(TTB_F32)) NewPlanes(t, &hi, &lo);
+  Check(ttb_add_bias_layernorm_f32_planes(c, out, hi, lo, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
         name);
 }
 
@@ -199,18 +205,18 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
   if (ldo == 0) ldo = N;
   TT_ENFORCE(ldo == N || (dt != TTB_F32 && !use_int8()), "%s: a padded output pitch is only supported on the 16-bit path", name);
   TT_ENFORCE((!out_lo && !f32_out) || (dt == TTB_BF16 && !use_int8()) || (out_lo && Fp32Planes(dt) && K % 4 == 0),
-             "%s: two-plane and fp32 outputs belong to the bf16 path, a second fp32 plane to the tensor cores", name);
-  if (dt == TTB_F32 && core::Fp32TensorCores() && K % 4 == 0 && M > 0) {
+             "%s: two-plane and fp32 outputs belong to the bf16 path, fp32 planes to the tensor cores", name);
+  if (dt == TTB_F32 && (core::Fp32TensorCores() || (x.lo() && !x.hi())) && K % 4 == 0 && M > 0) {
     // fp32 on the tensor cores: activations split into two tf32 planes, weights kept as two planes, three products
     // accumulated in one GEMM with the elementwise kernel that followed MatMul in the reference as its epilogue
     // (mat_mul.cpp:81-96 selects tensor-op math for the same product)
-    // (an activation that brings its second plane along is not split again: as fp32 it is its own first plane)
+    // (an activation that brings its planes along is not split again)
     Tensor planes(nullptr);
     const float* w = PackedTf32(is_trans);
     ttb_linear_args args{};
     args.dtype = TTB_F32; args.out_dtype = TTB_F32;
     if (x.lo()) {
-      args.A = x.raw(); args.A2 = x.lo()->raw();
+      args.A = x.hi() ? x.hi()->raw() : x.raw(); args.A2 = x.lo()->raw();
     } else {
       float* a = planes.Reshape<float>({2, M, K}, kDLCUDA, x.device_id(), "linear/tf32_activation_planes");
       Check(ttb_split_tf32(c, x.data<float>(), M * K, a, a + M * K), c, name);
@@ -219,7 +225,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     args.lda = K; args.out_lo = out_lo;
     args.W = w; args.W2 = w + N * K;
     args.bias = bias; args.residual = residual; args.ldr = N;
-    args.M = M; args.N = N; args.K = K; args.epilogue = epilogue;
+    args.M = M; args.N = N; args.K = K; args.epilogue = out_lo ? epilogue | TTB_EPI_FLAG_TF32_PLANES : epilogue;
     args.out = out; args.ldo = N;
     Check(ttb_linear_ex(c, &args), c, name);
     return;
@@ -324,7 +330,9 @@ void BERTEmbedding::operator()(const Tensor& input_ids, const Tensor& position_i
     lo = ex.lo.Reshape(word_embedings_.dtype(), {B, L, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({B, L, H}, kDLCUDA, dev, "precise/residual_stream");
   } else if (Fp32Planes(dt)) {
-    lo = NewLo(output_tensor);
+    float* rest;
+    NewPlanes(output_tensor, &f32, &rest);
+    lo = rest;
   }
   Check(ttb_embedding_ln_planes(c, dt, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
                                 token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), nullptr, B, L, B * L,
@@ -353,7 +361,9 @@ void BERTEmbedding::Packed(const Tensor& input_ids, const std::vector<int64_t>& 
     lo = ex.lo.Reshape(word_embedings_.dtype(), {1, T, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({1, T, H}, kDLCUDA, dev, "precise/residual_stream");
   } else if (Fp32Planes(dt)) {
-    lo = NewLo(output_tensor);
+    float* rest;
+    NewPlanes(output_tensor, &f32, &rest);
+    lo = rest;
   }
   const core::CuSeqlensHandle cu = core::CuSeqlens(dev, seq_lens);
   Check(ttb_embedding_ln_planes(c, dt, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
@@ -589,9 +599,9 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
       if (MaskIs2D(attention_mask)) { mbs = maxL; mrs = 0; }
       else { mrs = maxL; mbs = maxL * maxL; }
     }
+    float* hi = context.mutableData<float>();
     float* lo = NewLo(&context);
-    Check(ttb_attention_f32(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, context.mutableData<float>(), lo), c,
-          "attention_f32");
+    Check(ttb_attention_f32_planes(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, hi, lo), c, "attention_f32");
   } else {
     // The reference's own sequence (multi_headed_attention.cpp:168-232,320-354), scores materialised.
     TT_ENFORCE(!cache_keys, "layer_cache decoding is provided for 16-bit models with 64-wide heads");
@@ -844,7 +854,7 @@ void BertIntermediate::EnforceShapeAndType() const {
   TT_ENFORCE_EQ(dense_.weight().shape(1), dense_.bias().shape(0), "weight and bias shape mismatch");
 }
 
-void BertIntermediate::operator()(const Tensor& input_tensor, Tensor* output_tensor) const {
+void BertIntermediate::Run(const Tensor& input_tensor, Tensor* output_tensor, bool for_output) const {
   TT_ENFORCE(output_tensor, "The output tensor should not be nullptr.");
   FloatType(input_tensor, "BertIntermediate input");
   const int dt = core::ToTTBDtype(input_tensor.dtype());
@@ -852,7 +862,7 @@ void BertIntermediate::operator()(const Tensor& input_tensor, Tensor* output_ten
   output_tensor->Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "BertIntermediate/Reshape");
   void* out = output_tensor->raw_mut();
   void* lo = nullptr;
-  if (Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0) lo = NewLo(output_tensor);
+  if (for_output && Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0 && dense_.out_dim(false) % 4 == 0) lo = NewLo(output_tensor);
   else if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came
     lo = output_tensor->NewExtras().lo.Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "precise/lo_plane");
   // int8 (per-row scheme): BertOutput's Linear takes this activation as int8, so it leaves with its int8 form attached

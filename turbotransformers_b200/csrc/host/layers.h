@@ -192,10 +192,13 @@ class BertIntermediate {
     EnforceShapeAndType();
   }
   void EnforceShapeAndType() const;
-  void operator()(const core::Tensor& input_tensor, core::Tensor* output_tensor) const;
+  void operator()(const core::Tensor& input_tensor, core::Tensor* output_tensor) const { Run(input_tensor, output_tensor, false); }
+  // For a BertOutput and nothing else: an fp32 model's activation may leave as the two planes that the next product takes, in its place.
+  void ForOutput(const core::Tensor& input_tensor, core::Tensor* output_tensor) const { Run(input_tensor, output_tensor, true); }
   void QuantizeInt8(int mode = PackedLinear::kInt8PerRow) { dense_.set_int8_mode(mode); }
 
  private:
+  void Run(const core::Tensor& input_tensor, core::Tensor* output_tensor, bool for_output) const;
   PackedLinear dense_;
 };
 

@@ -206,6 +206,7 @@ PYBIND11_MODULE(turbo_transformers_cxx, m) {
   py::class_<layers::BertIntermediate>(m, "BertIntermediate")
       .def(py::init([](Tensor& w, Tensor& b) { return new layers::BertIntermediate(std::move(w), std::move(b)); }))
       .def("__call__", &layers::BertIntermediate::operator())
+      .def("for_output", &layers::BertIntermediate::ForOutput)
       .def("quantize_int8", &layers::BertIntermediate::QuantizeInt8, py::arg("mode") = 1);
 
   py::class_<layers::BertOutput>(m, "BertOutput")

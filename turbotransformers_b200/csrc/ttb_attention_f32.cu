@@ -6,7 +6,7 @@
 // arithmetic, were the time. A CTA has 8 R query rows of one (sequence, head) and goes over the keys in tiles of 64 with an online
 // softmax; a thread computes R x 4 scores, then R x 4 outputs, from 16-byte reads of shared memory (rows of 68 floats: the lanes of a read
 // hit different banks). BERT-base fp32, us a pass, with the second planes below: 8 requests of 10 to 120 tokens 2571 -> 1784, 1 x 128 1187 -> 1166 (its
-// Linears are what is left). The output may leave with the plane that the next product takes beside it.
+// Linears are what is left). The output may leave as the two planes that the next product takes.
 #include "ttb_common.cuh"
 
 using namespace ttb;
@@ -21,7 +21,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 template <int R> constexpr int kSmem = (2 * 8 * R + 2 * kKeys) * kPitch * 4;
 
-template <int R>
+// ROUNDED: the output leaves as its two planes, in place of it. (As a choice at run time it cost 15 registers and 1.2 us of 18 at 527 rows.)
+template <int R, bool ROUNDED>
 __global__ void __launch_bounds__(kThreads)
 attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ cu, int heads, const float* __restrict__ mask, long long mask_batch,
                      long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo) {
@@ -148,24 +149,23 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
     const float inv = 1.0f / sum;
     const float4 y = make_float4(acc[r][0] * inv, acc[r][1] * inv, acc[r][2] * inv, acc[r][3] * inv);
     const long long at = (long long)(begin + i) * H + h * D + kg * 4;
-    *reinterpret_cast<float4*>(out + at) = y;
-    if (out_lo) *reinterpret_cast<float4*>(out_lo + at) = make_float4(tf32_rest(y.x), tf32_rest(y.y), tf32_rest(y.z), tf32_rest(y.w));
+    *reinterpret_cast<float4*>(out + at) = ROUNDED ? make_float4(tf32_hi(y.x), tf32_hi(y.y), tf32_hi(y.z), tf32_hi(y.w)) : y;
+    if (ROUNDED || out_lo) *reinterpret_cast<float4*>(out_lo + at) = make_float4(tf32_lo(y.x, ROUNDED), tf32_lo(y.y, ROUNDED), tf32_lo(y.z, ROUNDED), tf32_lo(y.w, ROUNDED));
   }
 }
 
-template <int R>
+template <int R, bool ROUNDED>
 cudaError_t launch_f32(ttb_ctx* ctx, dim3 grid, const float* qkv, const int32_t* cu, int heads, const float* mask, int64_t mbs, int64_t mrs, int causal, float scale,
                        float* out, float* out_lo) {
-  cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<R>);
+  cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<R, ROUNDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<R>);
   if (e != cudaSuccess) return e;
-  return launch_pdl(attention_f32_kernel<R>, grid, dim3(kThreads), (size_t)kSmem<R>, ctx->stream, qkv, cu, heads, mask, (long long)mbs, (long long)mrs, causal, scale, out,
+  return launch_pdl(attention_f32_kernel<R, ROUNDED>, grid, dim3(kThreads), (size_t)kSmem<R>, ctx->stream, qkv, cu, heads, mask, (long long)mbs, (long long)mrs, causal, scale, out,
                     out_lo);
 }
 
-}  // namespace
-
-extern "C" int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
-                                 int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
+template <bool ROUNDED>
+int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
+                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, d == D && heads > 0 && heads <= 65535 && B >= 0 && B <= 65535 && max_seqlen >= 0 && max_seqlen < (1 << 30), "attention_f32: bad shape");
   if (B == 0 || max_seqlen == 0) return TTB_OK;
@@ -176,10 +176,23 @@ extern "C" int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* 
   // 32 rows a CTA read a tile of keys half as often as 16; with few (sequence, head, rows) the chip has room for twice the CTAs
   const int64_t ctas = B * heads * ((max_seqlen + 31) / 32);
   if (ctas >= 2 * ctx->sm_count)
-    TTB_CUDA(ctx, launch_f32<4>(ctx, dim3((unsigned)((max_seqlen + 31) / 32), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo));
+    TTB_CUDA(ctx, (launch_f32<4, ROUNDED>(ctx, dim3((unsigned)((max_seqlen + 31) / 32), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
+                                causal, scale, out, out_lo)));
   else
-    TTB_CUDA(ctx, launch_f32<2>(ctx, dim3((unsigned)((max_seqlen + 15) / 16), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo));
+    TTB_CUDA(ctx, (launch_f32<2, ROUNDED>(ctx, dim3((unsigned)((max_seqlen + 15) / 16), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
+                                causal, scale, out, out_lo)));
   return launched(ctx, "attention_f32");
+}
+
+}  // namespace
+
+extern "C" int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
+                                 int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
+  return attention_f32<false>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, out, out_lo);
+}
+
+extern "C" int ttb_attention_f32_planes(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
+                                        const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* hi, float* lo) {
+  if (ctx && B > 0 && max_seqlen > 0) TTB_REQUIRE(ctx, lo, "attention_f32_planes: null pointer");
+  return attention_f32<true>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, hi, lo);
 }

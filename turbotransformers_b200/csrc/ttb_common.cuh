@@ -150,16 +150,23 @@ template <> __device__ __forceinline__ float from_f<float>(float v) { return v; 
 template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-// What the tensor core drops of an fp32 value that it reads as tf32 (its last 13 bits), rounded to tf32: x as it is and this are the two
-// planes of an fp32 operand.
-__device__ __forceinline__ float tf32_rest(float x) {
+__device__ __forceinline__ float round_tf32(float x) {
   uint32_t u;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x - __uint_as_float(__float_as_uint(x) & 0xffffe000u)));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
   return __uint_as_float(u);
 }
-// What is left of v after it has been stored as T and read by a product: the "lo" plane of a two-plane value.
-template <typename T> __device__ __forceinline__ float rest_of(float v) { return v - to_f(from_f<T>(v)); }
-template <> __device__ __forceinline__ float rest_of<float>(float v) { return tf32_rest(v); }
+// The two planes of an fp32 operand: x rounded to tf32, and what the rounding dropped, rounded likewise. Together 2^-23 off at most:
+// the remainder of a rounding has 12 bits, of which tf32 keeps 11. Where x itself serves as the first plane (rounded: false) the tensor
+// core drops its last 13 bits, and the second plane is those, rounded: 2^-22 off at most.
+// The first rounding is two integer instructions, with round_tf32's result but for some NaNs, of which the second plane takes care: a conversion
+// runs at a quarter of their rate, and with three for a value FFN1's epilogue took 34.5 us at 527 rows, 30.5 with one.
+__device__ __forceinline__ float tf32_hi(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+__device__ __forceinline__ float tf32_lo(float x, bool rounded) {
+  return round_tf32(x - (rounded ? tf32_hi(x) : __uint_as_float(__float_as_uint(x) & 0xffffe000u)));
+}
+// What is left of v after it has been stored as T: the second plane of a 16-bit value; of fp32, as tf32_lo.
+template <typename T> __device__ __forceinline__ float rest_of(float v, bool) { return v - to_f(from_f<T>(v)); }
+template <> __device__ __forceinline__ float rest_of<float>(float v, bool rounded) { return tf32_lo(v, rounded); }
 
 // A group of 8 consecutive elements moved with 16-byte (or 2x16-byte for fp32) accesses.
 template <typename T> struct Vec8 {

@@ -28,7 +28,8 @@ inline int grid_for(int64_t work, int per_block, int sm_count) {
 constexpr int kLnWarps = 8;
 constexpr int kLnRows = 2;
 
-template <typename TIn, typename TOut, int ITERS, bool ADD, bool EXTRA, int WARPS, int ROWS>
+// EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo.
+template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
                       const TOut* __restrict__ beta, TOut* out, TOut* __restrict__ out_lo, float* __restrict__ out_f32, int64_t M, int N,
@@ -100,16 +101,16 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
             for (int j = 0; j < 8; ++j) o.v[j] = b.v[j] + g.v[j] * rstd[r] * (v[r][it][j] - mean[r]);
             o.store(out + row * N + col);
             if (EXTRA) {
-              if (out_f32) {
+              if (EXTRA == 2 || out_f32) {
                 Vec8<float> f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) f.v[j] = o.v[j];
+                for (int j = 0; j < 8; ++j) f.v[j] = EXTRA == 2 ? tf32_hi(o.v[j]) : o.v[j];
                 f.store(out_f32 + row * N + col);
               }
-              if (out_lo) {
+              if (EXTRA == 2 || out_lo) {
                 Vec8<TOut> l;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j]);
+                for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j], EXTRA == 2);
                 l.store(out_lo + row * N + col);
               }
             }
@@ -470,8 +471,8 @@ layernorm_rows_generic_kernel(const TIn* x, const TIn* __restrict__ residual, co
     for (int c = lane; c < N; c += 32) {
       const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
       out[row * N + c] = from_f<TOut>(y);
-      if (out_f32) out_f32[row * N + c] = y;
-      if (out_lo) out_lo[row * N + c] = from_f<TOut>(rest_of<TOut>(y));
+      if (out_f32) out_f32[row * N + c] = std::is_same<TOut, float>::value && out_lo ? tf32_hi(y) : y;
+      if (out_lo) out_lo[row * N + c] = from_f<TOut>(rest_of<TOut>(y, out_f32 != nullptr));
     }
   }
 }
@@ -484,23 +485,31 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   const int grid = grid_for(pair_warps, kLnWarps, ctx->sm_count);
   const int block = kLnWarps * 32;
   const bool extra = out_lo != nullptr || out_f32 != nullptr;
+  constexpr int kPlanes = std::is_same<TOut, float>::value ? 2 : 1;  // fp32 with both extras: its planes
+  const bool planes = kPlanes == 2 && out_lo && out_f32;
   // Sixteen rows a CTA leave most SMs without one while the rest move 200 KB each (128 fp32 rows: 8 CTAs): up to eight rows an SM,
   // CTAs of two rows. The rows' arithmetic is the same. BERT-base fp32, 24 layer norms a pass: 1 x 128 1171 -> 1068 us, 527 rows 1814 -> 1727.
   const bool few = M <= 8 * (int64_t)ctx->sm_count;
   const int few_grid = (int)((M + 1) / 2);
 #define LN_CASE(IT)                                                                                                              \
   do {                                                                                                                           \
-    if (few && extra)                                                                                                            \
-      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, true, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
+    if (few && planes)                                                                                                           \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+    else if (planes)                                                                                                             \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+    else if (few && extra)                                                                                                       \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (few)                                                                                                                \
-      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, false, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (extra)                                                                                                              \
-      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, true, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else                                                                                                                         \
-      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, false, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
   } while (0)
   const bool aligned = (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo) |
@@ -732,11 +741,21 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
     float sq = 0.f;
     for (int c = lane; c < hidden; c += 32) { float d = val(c) - mean; sq += d * d; }
     const float rstd = rsqrtf(warp_sum(sq) / (float)hidden + eps);
+    if (std::is_same<T, float>::value && out_f32 && out_lo) {  // (a loop of its own: stores under conditions keep the loads from going ahead)
+#pragma unroll 4
+      for (int c = lane; c < hidden; c += 32) {
+        const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
+        out[t * hidden + c] = from_f<T>(y);
+        out_f32[t * hidden + c] = tf32_hi(y);
+        out_lo[t * hidden + c] = from_f<T>(tf32_lo(y, true));
+      }
+      continue;
+    }
     for (int c = lane; c < hidden; c += 32) {
       const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
       out[t * hidden + c] = from_f<T>(y);
       if (out_f32) out_f32[t * hidden + c] = y;
-      if (out_lo) out_lo[t * hidden + c] = from_f<T>(rest_of<T>(y));
+      if (out_lo) out_lo[t * hidden + c] = from_f<T>(rest_of<T>(y, false));
     }
   }
 }
@@ -1310,13 +1329,24 @@ extern "C" int ttb_add_bias_layernorm(ttb_ctx* ctx, int dtype, void* out, const 
   return TTB_OK;
 }
 
-extern "C" int ttb_add_bias_layernorm_f32(ttb_ctx* ctx, float* out, float* out_lo, const float* input, const float* bias, const float* gamma,
-                                          const float* beta, int64_t M, int64_t N, float eps) {
+namespace {
+int add_bias_layernorm_f32(ttb_ctx* ctx, float* out, float* out_hi, float* out_lo, const float* input, const float* bias, const float* gamma,
+                           const float* beta, int64_t M, int64_t N, float eps) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, M >= 0 && N > 0, "add_bias_layernorm: bad shape M=%lld N=%lld", (long long)M, (long long)N);
   TTB_REQUIRE(ctx, M == 0 || (out && input && bias && gamma && beta), "add_bias_layernorm: null pointer");
   DeviceGuard g(ctx->device);
-  return launch_layernorm<float, float, true>(ctx, out, input, bias, gamma, beta, out, out_lo, nullptr, M, N, eps);
+  return launch_layernorm<float, float, true>(ctx, out, input, bias, gamma, beta, out, out_lo, out_hi, M, N, eps);
+}
+}  // namespace
+extern "C" int ttb_add_bias_layernorm_f32(ttb_ctx* ctx, float* out, float* out_lo, const float* input, const float* bias, const float* gamma,
+                                          const float* beta, int64_t M, int64_t N, float eps) {
+  return add_bias_layernorm_f32(ctx, out, nullptr, out_lo, input, bias, gamma, beta, M, N, eps);
+}
+extern "C" int ttb_add_bias_layernorm_f32_planes(ttb_ctx* ctx, float* out, float* hi, float* lo, const float* input, const float* bias, const float* gamma,
+                                                 const float* beta, int64_t M, int64_t N, float eps) {
+  if (ctx && M > 0) TTB_REQUIRE(ctx, !hi == !lo, "add_bias_layernorm_f32_planes: one plane without the other");
+  return add_bias_layernorm_f32(ctx, out, hi, lo, input, bias, gamma, beta, M, N, eps);
 }
 
 extern "C" int ttb_layernorm(ttb_ctx* ctx, int dtype, const void* in, void* out, const void* gamma, const void* beta,

@@ -185,9 +185,10 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 
 // ---- the kernel -----------------------------------------------------------------------------------
 // VAR selects an epilogue variant that costs registers, so that the plain kernels do not carry it:
-//   VAR_PLAIN, VAR_TWO_PLANES (output written with a second plane, what a product drops of the first), VAR_AFFINE (int8 with a per-tensor zero point),
+//   VAR_PLAIN, VAR_TWO_PLANES (output written with a second plane, what a product drops of the first), VAR_TF32_PLANES (fp32 output rounded to tf32, and
+//   what that dropped; as a choice at run time of the one before, 3 us of 30 at 527 x 3072 x 768), VAR_AFFINE (int8 with a per-tensor zero point),
 //   VAR_WORDS (STORE_WORDS; carried by every kernel it cost packed fp16 batches 1 %: 4120 -> 4164 us, 4149 against 4159 without)
-enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3 };
+enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3, VAR_TF32_PLANES = 4 };
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR, bool LN = false>
 __global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
@@ -402,7 +403,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     constexpr int HALVES = CH / 32;              // 32-column TMEM loads per chunk
     constexpr int G16 = 32 * EB / 16;            // 16-byte groups per row of a 32-column half (4 or 8)
     constexpr int P16 = Per16<OutT>::value;      // elements per 16-byte group (8 or 4)
-    constexpr int LO_N = (VAR == VAR_TWO_PLANES) ? 8 : 1;  // 16-byte groups of a chunk's second plane kept in registers
+    constexpr int LO_N = (VAR == VAR_TWO_PLANES || VAR == VAR_TF32_PLANES) ? 8 : 1;  // 16-byte groups of a chunk's second plane kept in registers
     static_assert(VAR != VAR_AFFINE || KIND == KIND_I8, "the zero-point correction belongs to the int8 kind");
     const int quad = warp & 3;          // TMEM lanes [32*quad, 32*quad+32) are the ones this warp may read
     const int half = (warp - 2) >> 2;   // which half of the tile's column chunks this warp takes
@@ -413,7 +414,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     constexpr bool affine = (VAR == VAR_AFFINE);
     const float act_scale = affine ? p.act_qparams[0] : 1.0f;
     const int zero_point = affine ? (int)p.act_qparams[1] : 0;
-    constexpr bool two_planes = (VAR == VAR_TWO_PLANES);
+    constexpr bool rounded = (VAR == VAR_TF32_PLANES), two_planes = (VAR == VAR_TWO_PLANES) || rounded;
+    static_assert(!rounded || EB == 4, "planes as tf32 are fp32 words");
     const bool vec_ok = (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                         ((reinterpret_cast<uintptr_t>(p.out_lo) & 15) == 0) &&
                         (!bias || (reinterpret_cast<uintptr_t>(bias) & 15) == 0) &&
@@ -735,11 +737,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
               for (int j = 0; j < 32; ++j) row_max = fmaxf(row_max, fabsf(v[j]));
             }
 #pragma unroll
-            for (int g = 0; g < G16; ++g)
-              *reinterpret_cast<uint4*>(buf + lane * 128 + (((hh * G16 + g) ^ (lane & 7)) << 4)) = pack16<OutT>(&v[g * P16]);
+            for (int g = 0; g < G16; ++g) {
+              float first[P16];
+#pragma unroll
+              for (int j = 0; j < P16; ++j) first[j] = rounded ? tf32_hi(v[g * P16 + j]) : v[g * P16 + j];
+              *reinterpret_cast<uint4*>(buf + lane * 128 + (((hh * G16 + g) ^ (lane & 7)) << 4)) = pack16<OutT>(first);
+            }
             if (two_planes) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j]);
+              for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j], rounded);
 #pragma unroll
               for (int g = 0; g < G16; ++g) lo_pack[(hh * G16 + g) % LO_N] = pack16<OutT>(&v[g * P16]);
             }
@@ -894,14 +900,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           OutT* dstp = (plane == 0 ? out : static_cast<OutT*>(p.out_lo)) + (long long)row * p.ldo + col0;
           if (plane == 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j]);
+            for (int j = 0; j < 32; ++j) v[j] = rest_of<OutT>(v[j], rounded);
           }
+          auto value = [&](float x) { return rounded && plane == 0 ? tf32_hi(x) : x; };
           if (full) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               Vec8<OutT> o;
 #pragma unroll
-              for (int j = 0; j < 8; ++j) o.v[j] = v[i * 8 + j];
+              for (int j = 0; j < 8; ++j) o.v[j] = value(v[i * 8 + j]);
               o.store(dstp + i * 8);
             }
           } else if (BN == 32 && EB == 2 && col0 + 32 <= p.N) {
@@ -925,7 +932,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (col0 + j < p.N) dstp[j] = from_f<OutT>(v[j]);
+              if (col0 + j < p.N) dstp[j] = from_f<OutT>(value(v[j]));
           }
         }
       }
@@ -1485,13 +1492,8 @@ __global__ void __launch_bounds__(256) int8_row_sum_kernel(const int8_t* __restr
   if (lane == 0) col_sum[n] = acc;
 }
 
-// fp32 -> two tf32-representable planes: hi = x rounded to 10 mantissa bits, lo = (x - hi) rounded likewise. hi + lo carries
-// 21 of x's 24 significant bits, which is what three tf32 products recover.
-__device__ __forceinline__ float round_tf32(float x) {
-  uint32_t u;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-  return __uint_as_float(u);
-}
+// fp32 -> two tf32-representable planes: hi = x rounded to 10 mantissa bits, lo = (x - hi) rounded likewise. hi + lo
+// is x to 2^-23, which is what three tf32 products recover.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ hi, float* __restrict__ lo) {
   pdl_trigger();
   pdl_wait();
@@ -1526,7 +1528,9 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   TTB_REQUIRE(ctx, !a->W2 || (a->A2 && dt == TTB_F32), "linear_ex: a second weight plane belongs to the three-pass fp32 form (A, A2, W, W2)");
   TTB_REQUIRE(ctx, !a->out_lo || (odt == dt && dt != TTB_F16), "linear_ex: the second output plane exists for BF16 and F32 products only");
   const int pad_scratch = (a->epilogue & TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH) ? 1 : 0;
-  const int epilogue = a->epilogue & ~TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH;
+  const bool planes = (a->epilogue & TTB_EPI_FLAG_TF32_PLANES) != 0;
+  TTB_REQUIRE(ctx, !planes || (dt == TTB_F32 && a->out_lo), "linear_ex: planes as tf32 belong to an F32 product with out_lo");
+  const int epilogue = a->epilogue & ~(TTB_EPI_FLAG_ROW_PADDING_IS_SCRATCH | TTB_EPI_FLAG_TF32_PLANES);
   const int k_align = dt == TTB_F32 ? 4 : 8;
   int s = check_linear(ctx, "linear", a->A, a->W, a->bias, a->residual, a->M, a->N, a->K, epilogue, a->out, a->ldo, k_align);
   if (s || a->M == 0) return s;
@@ -1542,6 +1546,7 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   p.bias = a->bias; p.residual = a->residual; p.ldr = a->ldr;
   p.epilogue = epilogue; p.staged = pad_scratch ? STORE_TMA : STORE_DIRECT; p.split_k = 1; p.status = ctx->d_status;
   const Operands op{a->A, a->A2, a->lda, a->W, a->W2};
+  if (planes) return pick_tile<KIND_TF32, float, VAR_TF32_PLANES>(ctx, op, p);
   if (dt == TTB_F32) return a->out_lo ? pick_tile<KIND_TF32, float, VAR_TWO_PLANES>(ctx, op, p) : pick_tile<KIND_TF32, float>(ctx, op, p);
   if (dt == TTB_F16) return odt == TTB_F32 ? pick_tile<KIND_F16, float>(ctx, op, p) : pick_tile<KIND_F16, __half>(ctx, op, p);
   if (odt == TTB_F32) return pick_tile<KIND_BF16, float>(ctx, op, p);

@@ -99,6 +99,15 @@ class BertOutput(cxx.BertOutput):
                             ('dense.weight', 'dense.bias', 'LayerNorm.weight', 'LayerNorm.bias')))
 
 
+def feed_forward(intermediate, output, x, return_type):
+    """output(intermediate(x), x). What passes between the two stays between them where both are this module's own classes."""
+    if type(intermediate) is not BertIntermediate or type(output) is not BertOutput:
+        return output(intermediate(x, return_type=ReturnType.turbo_transformers), x, return_type=return_type)
+    inner = cxx.Tensor.create_empty()
+    intermediate.for_output(x, inner)
+    return output(inner, x, return_type=return_type)
+
+
 def pack_qkv(attention):
     """(qkv_weight [H,3H], qkv_bias [3H]) from a HuggingFace BertAttention, q|k|v column blocks."""
     p = {k: v.detach() for k, v in attention.named_parameters()}
@@ -154,8 +163,7 @@ class BertLayer:
         self_attention_outputs = self.attention(hidden_states, attention_mask, head_mask, output_attentions=output_attentions,
                                                 return_type=ReturnType.turbo_transformers)
         attention_output = self_attention_outputs[0]
-        intermediate_output = self.intermediate(attention_output, return_type=ReturnType.turbo_transformers)
-        layer_output = self.output(intermediate_output, attention_output, return_type=return_type)
+        layer_output = feed_forward(self.intermediate, self.output, attention_output, return_type)
         return (layer_output, ) + self_attention_outputs[1:]
 
     @staticmethod

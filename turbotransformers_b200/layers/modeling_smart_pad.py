@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from .._cxx import cxx
-from .modeling_bert import (BertEmbeddings, BertIntermediate, BertOutput, BertPooler, PoolingMap, PoolingType, _npz, _require_cuda,
+from .modeling_bert import (BertEmbeddings, BertIntermediate, BertOutput, BertPooler, PoolingMap, PoolingType, _npz, _require_cuda, feed_forward,
                             _t, pack_qkv)
 from .return_type import ReturnType, convert_returns_as_type
 from .utils import AnyTensor, convert2tt_tensor, create_empty_if_none, try_convert, use_current_stream
@@ -102,8 +102,7 @@ class BertLayerSmartBatch:
         att_out, att_probs = self.attention(hidden_states, hidden_states, hidden_states, query_seq_len_list, [], mask=attention_mask,
                                             layer_cache=None, attn_type="self", post_layernorm=True,
                                             return_type=ReturnType.turbo_transformers, output_attentions=output_attentions)
-        intermediate_output = self.intermediate(att_out, return_type=ReturnType.turbo_transformers)
-        layer_output = self.output(intermediate_output, att_out, return_type=return_type)
+        layer_output = feed_forward(self.intermediate, self.output, att_out, return_type)
         return (layer_output, att_probs) if output_attentions else (layer_output, )
 
     @staticmethod
