@@ -61,6 +61,8 @@ int ttb_ctx_destroy(ttb_ctx* ctx);
  * at the same time use one context each. */
 int ttb_ctx_set_stream(ttb_ctx* ctx, void* cuda_stream);
 void* ttb_ctx_stream(ttb_ctx* ctx);
+/* The SMs of the context's GPU that the process sees (0 for a null context). */
+int ttb_ctx_sm_count(ttb_ctx* ctx);
 int ttb_ctx_device(ttb_ctx* ctx);
 int ttb_ctx_sync(ttb_ctx* ctx);
 /* Text of the last failure seen on this context ("" if none). Valid until the next call on the context. */

@@ -54,6 +54,7 @@ SIGNATURES = {
     "ttb_ctx_destroy": (i32, [p]),
     "ttb_ctx_set_stream": (i32, [p, p]),
     "ttb_ctx_stream": (p, [p]),
+    "ttb_ctx_sm_count": (i32, [p]),
     "ttb_ctx_device": (i32, [p]),
     "ttb_ctx_sync": (i32, [p]),
     "ttb_last_error": (C.c_char_p, [p]),

@@ -1,5 +1,7 @@
 #include "chain.h"
 
+#include "../ttb_chain_rules.cuh"
+
 #include <algorithm>
 #include <cmath>
 #include <initializer_list>
@@ -27,7 +29,8 @@ bool Vector(const Tensor& t, int64_t n, const Tensor& like) { return Half(t, lik
 
 // A [K, N] product with a bias over rows like `x`.
 bool LinearFits(const PackedLinear& l, bool trans, int64_t K, int64_t N, const Tensor& x) {
-  return !l.use_int8() && Half(l.weight(), x) && l.weight().n_dim() == 2 && l.in_dim(trans) == K && l.out_dim(trans) == N && N % 8 == 0 && N <= 16384 &&
+  return !l.use_int8() && Half(l.weight(), x) && l.weight().n_dim() == 2 && l.in_dim(trans) == K && l.out_dim(trans) == N && N % 8 == 0 &&
+         N <= ttb::chain::bias_columns(ttb_ctx_sm_count(DeviceContext(x.device_id()))) &&
          Vector(l.bias(), N, x) && Aligned({&l.bias()});
 }
 bool NormFits(const Tensor& gamma, const Tensor& beta, int64_t H, const Tensor& x) {
@@ -43,7 +46,8 @@ bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
   if (x.n_dim() != 3 || !x.on_gpu() || !core::SameType(x.dtype(), core::kFloat16)) return false;
   const int64_t rows = x.numel() ? x.rows() : 0, H = x.shape(2);
   // (narrower models keep the layer-by-layer pass, whose results are bit for bit those of its layers called one by one)
-  return rows > 0 && H == heads * kHead && H >= 512 && Aligned({&x}) && rows <= std::min(most, ttb_chain_rows(H, inner));
+  return rows > 0 && H == heads * kHead && H >= 512 && Aligned({&x}) && rows <= std::min(most, ttb_chain_rows(H, inner)) &&
+         ttb::chain::rows_have_writers(rows, ttb_ctx_sm_count(DeviceContext(x.device_id())));
 }
 
 // The call's scratch memory, dealt out in pieces.

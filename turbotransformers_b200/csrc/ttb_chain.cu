@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <initializer_list>
 
+#include "ttb_chain_rules.cuh"
 #include "ttb_common.cuh"
 #include "ttb_sm100.cuh"
 
@@ -36,7 +37,7 @@ constexpr int kRowPad = 64;                     // bytes between the rows of a r
 constexpr int kPart = 1024;                     // most of K in a slot
 constexpr int kMaxSlots = 24;
 constexpr int kParamSlots = 4;
-constexpr int kBiasUnits = 16;                  // most units a CTA may have where there is a bias
+using chain::kBiasUnits;
 constexpr int kParamBytes = 2 * kPart * 2 + kBiasUnits * 16;
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kHeadDim = 64;
@@ -75,9 +76,9 @@ struct Share {
   bool writes, part, params;  // params: norm weights or a bias come with it
   __device__ __forceinline__ Share() {}
   __device__ __forceinline__ explicit Share(const ttb_chain_linear& o) {
-    const uint32_t units = ((uint32_t)o.N + 7) >> 3;  // N <= 2^24: the products stay below 2^32 on any GPU
-    lo = (int)(units * blockIdx.x / gridDim.x);
-    hi = (int)(units * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t units = ((uint32_t)o.N + 7) >> 3;
+    lo = (int)chain::first_unit(units, blockIdx.x, gridDim.x);
+    hi = (int)chain::first_unit(units, blockIdx.x + 1, gridDim.x);
     writes = o.gamma && o.normed && (int)blockIdx.x < o.M;
     part = hi > lo || writes;
     params = part && (o.gamma || (o.bias && hi > lo));
@@ -449,7 +450,7 @@ __device__ __forceinline__ void normalise(const ttb_chain_linear& o, const Share
         }
         const uint4 q = pack(y);
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(to + i * 512), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
-        if (s.writes && (int)blockIdx.x == row) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = q;
+        if (s.writes && chain::writes_row(row, (int)blockIdx.x)) *reinterpret_cast<uint4*>(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8) = q;
       }
   }
 }
@@ -920,8 +921,9 @@ extern "C" int ttb_chain_forward(ttb_ctx* ctx, int dtype, const ttb_chain_op* op
                   (reinterpret_cast<uintptr_t>(o.out) & 1) == 0, "chain_forward: operation %d: misaligned operand", i);
       TTB_REQUIRE(ctx, !o.gamma || (o.beta && ks == o.K), "chain_forward: operation %d: a layer norm takes at most %d columns and both of its weights", i, kPart);
       TTB_REQUIRE(ctx, o.N > 0 || (o.gamma && o.normed), "chain_forward: operation %d does nothing", i);
+      TTB_REQUIRE(ctx, !o.normed || chain::rows_have_writers(o.M, ctx->sm_count), "chain_forward: operation %d: more rows than SMs", i);
       TTB_REQUIRE(ctx, (!o.bias && !o.residual) || o.N % 8 == 0, "chain_forward: operation %d: a bias or residual needs a width that is a multiple of 8", i);
-      TTB_REQUIRE(ctx, !o.bias || o.N / 8 <= (int64_t)(kBiasUnits - 1) * ctx->sm_count, "chain_forward: operation %d: too wide for a bias", i);
+      TTB_REQUIRE(ctx, !o.bias || o.N <= chain::bias_columns(ctx->sm_count), "chain_forward: operation %d: too wide for a bias", i);
       TTB_REQUIRE(ctx, o.act >= 0 && o.act <= TTB_CHAIN_ACT_RELU, "chain_forward: operation %d: unknown activation", i);
       prm.ops[i].reserved = ks;
       rows = std::max(rows, (int)o.M);

@@ -88,6 +88,8 @@ extern "C" int ttb_ctx_set_stream(ttb_ctx* c, void* s) {
   return TTB_OK;
 }
 
+extern "C" int ttb_ctx_sm_count(ttb_ctx* c) { return c ? c->sm_count : 0; }
+
 extern "C" void* ttb_ctx_stream(ttb_ctx* c) { return c ? (void*)c->stream : nullptr; }
 extern "C" int ttb_ctx_device(ttb_ctx* c) { return c ? c->device : -1; }
 
