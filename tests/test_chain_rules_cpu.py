@@ -1,6 +1,7 @@
 """CPU: the rules by which the chain kernel deals out its work (ttb_chain_rules.cuh), compiled for the host, on grids of every size."""
 import ctypes
 import os
+import re
 import subprocess
 
 import pytest
@@ -41,3 +42,12 @@ def test_a_bias_that_is_accepted_has_room_in_every_cta(rules, ctas):
     units = rules.bias_columns(ctas) // 8
     assert max(rules.first_unit(units, c + 1, ctas) - rules.first_unit(units, c, ctas) for c in range(ctas)) <= rules.bias_units()
     assert units >= 15 * ctas
+
+
+def test_the_result_of_every_bounded_wait_is_used():
+    """A wait that runs out has to reach the status word: none may stand as a statement of its own."""
+    source = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "ttb_chain.cu")).read())
+    calls = re.findall(r"([^\n]*)\b(?:wait|wait_slots|wait_ahead)\(", source)
+    assert len(calls) >= 7
+    for before in calls:
+        assert re.search(r"(return|=|!|&&|\|\||bool)\s*$", before) or "bool" in before, before

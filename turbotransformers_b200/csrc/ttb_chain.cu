@@ -153,7 +153,7 @@ __device__ __forceinline__ long long cache_row(int j, int b, int B, int H) { ret
 // ---------------------------------------------------------------------------------------------
 // A bounded wait (each attempt suspends the thread for up to 20 us, 2^17 of them are some seconds) without a call: what is live around a
 // call would be spilled, and a spill costs a trip to L2 here, since the barrier's acquire empties the L1 cache.
-__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+[[nodiscard]] __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
 #pragma unroll 1
   for (int tries = 0; tries < (1 << 17); ++tries) {
     if (sm100::mbar_try_wait(bar, parity)) return true;
@@ -240,7 +240,7 @@ __device__ __noinline__ void feed(const ChainParams& prm, Shared& sm, uint32_t r
 }
 
 // Waits for the next n slots of the ring.
-__device__ __noinline__ bool wait_slots(int n, int slots, Shared& sm, Cursor w) {
+[[nodiscard]] __device__ __noinline__ bool wait_slots(int n, int slots, Shared& sm, Cursor w) {
   bool ok = true;
 #pragma unroll 1
   for (int i = 0; ok && i < n; ++i) {
@@ -252,7 +252,7 @@ __device__ __noinline__ bool wait_slots(int n, int slots, Shared& sm, Cursor w) 
 
 // Waits for the norm weights, bias and weights with which the CTA's share of an operation begins. One warp does it for all of them, ahead of
 // a barrier of the CTA and mostly in the shadow of the grid's.
-__device__ __forceinline__ bool wait_ahead(const ttb_chain_op& op, const Share& s, int slots, Shared& sm, Cursor w, const Cursor& p) {
+[[nodiscard]] __device__ __forceinline__ bool wait_ahead(const ttb_chain_op& op, const Share& s, int slots, Shared& sm, Cursor w, const Cursor& p) {
   if (op.kind != TTB_CHAIN_LINEAR || !s.part) return true;
   const bool ok = !s.params || wait(sm100::smem_u32(&sm.pfull[p.slot]), p.parity, &sm.abort_flag);
   return ok && wait_slots(min(op.reserved >> 16, s.hi - s.lo) * div_small(op.u.linear.K, op.reserved & 0xffff), slots, sm, w);
@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
   Read read;
   if (warp == kWarps - 1) {
     feed(prm, sm, ring, Layout<MT>::kBatch, 0, 0);
-    wait_ahead(sm.ops[0], sm.share[0], prm.slots, sm, read.w, read.p);
+    if (!wait_ahead(sm.ops[0], sm.share[0], prm.slots, sm, read.w, read.p) && lane == 0) atomicExch(prm.status, (int)TTB_ERR_DEVICE_WAIT);
   }
   __syncthreads();
 #pragma unroll 1
