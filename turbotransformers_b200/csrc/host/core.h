@@ -129,12 +129,19 @@ class Tensor {
   bool on_gpu() const { return !is_null() && view_.device.device_type == kDLCUDA; }
 
   const void* raw() const { return is_null() ? nullptr : static_cast<const char*>(view_.data) + view_.byte_offset; }
-  void* raw_mut() { return const_cast<void*>(raw()); }
+  // A pointer to write through: the companion planes (below) belong to the value that is overwritten, and are dropped.
+  void* raw_mut() {
+    DropExtras();
+    return const_cast<void*>(raw());
+  }
   template <typename T> const T* data() const {
     TT_ENFORCE(!is_null() && SameType(view_.dtype, DataTypeTrait<T>::value()), "data type mismatch");
     return static_cast<const T*>(raw());
   }
-  template <typename T> T* mutableData() { return const_cast<T*>(data<T>()); }
+  template <typename T> T* mutableData() {
+    DropExtras();
+    return const_cast<T*>(data<T>());
+  }
 
   // Makes this tensor hold `shape` of `dtype` on the device, keeping its storage when it owns enough
   // bytes on the same device (tensor.h:317-338 of the reference), else allocating by `name`.
@@ -151,7 +158,7 @@ class Tensor {
   Tensor operator[](int64_t n) const;
 
   // Companion planes a layer may attach to an activation it produced, for the next layer to use (they travel with
-  // the tensor through moves, and are dropped when it is reshaped or exported):
+  // the tensor through moves, and are dropped when it is reshaped, exported or asked for a pointer to write through):
   //   lo  : same shape and dtype, what rounding to the 16-bit type dropped (value = this + lo to 16 significant bits); of an fp32 tensor
   //         that travels between two of the runtime's own products only, or with hi, what rounding to tf32 dropped
   //   f32 : same shape in fp32, the unrounded value (the residual stream of a bf16 model)

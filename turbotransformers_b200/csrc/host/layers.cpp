@@ -1068,14 +1068,12 @@ void PositionwiseFeedForward::operator()(const Tensor& x, Tensor* output, bool i
 
 void FusedAddBiasGELU::operator()(Tensor* t) const {
   const int dt = FloatType(*t, "FusedAddBiasGELU input");
-  t->DropExtras();  // they belong to the value that is overwritten
   ttb_ctx* c = DeviceContext(t->device_id());
   Check(ttb_add_bias_act(c, dt, t->raw_mut(), bias_.raw(), t->rows(), t->shape(-1), TTB_ACT_GELU), c, "FusedAddBiasGELU");
 }
 
 void FusedAddBiasLayerNorm::operator()(const Tensor& input_tensor, Tensor* output_tensor) const {
   const int dt = FloatType(*output_tensor, "FusedAddBiasLayerNorm output");
-  output_tensor->DropExtras();  // they belong to the value that is overwritten
   SameTypeDevice(input_tensor, *output_tensor, "FusedAddBiasLayerNorm");
   ttb_ctx* c = DeviceContext(output_tensor->device_id());
   Check(ttb_add_bias_layernorm(c, dt, output_tensor->raw_mut(), input_tensor.raw(), bias_.raw(), norm_weight_.raw(), norm_bias_.raw(),
