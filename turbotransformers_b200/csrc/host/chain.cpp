@@ -27,27 +27,29 @@ bool Half(const Tensor& t, const Tensor& like) {
 }
 bool Vector(const Tensor& t, int64_t n, const Tensor& like) { return Half(t, like) && t.numel() == n; }
 
+int64_t Ctas(const Tensor& x) { return ttb_ctx_sm_count(DeviceContext(x.device_id())); }
 // A [K, N] product with a bias over rows like `x`.
 bool LinearFits(const PackedLinear& l, bool trans, int64_t K, int64_t N, const Tensor& x) {
   return !l.use_int8() && Half(l.weight(), x) && l.weight().n_dim() == 2 && l.in_dim(trans) == K && l.out_dim(trans) == N && N % 8 == 0 &&
-         N <= ttb::chain::bias_columns(ttb_ctx_sm_count(DeviceContext(x.device_id()))) &&
+         N <= ttb::chain::bias_columns(Ctas(x)) &&
          Vector(l.bias(), N, x) && Aligned({&l.bias()});
 }
 bool NormFits(const Tensor& gamma, const Tensor& beta, int64_t H, const Tensor& x) {
   return Vector(gamma, H, x) && Vector(beta, H, x) && Aligned({&gamma, &beta});
 }
+// (How many keys those rows may have: history_fits and memory_fits of ttb_chain_rules.cuh.)
 // The rows up to which one kernel is the faster route: above, every CTA's normalising of all rows and its reading of all of the wide
 // activation outweigh the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 286 / 414, 16 334 / 435,
 // 24 397 / 436, 32 443 / 436, 64 639 / 484 (300 cached: 370 / 492, 446 / 526, 526 / 549 at 16, 24, 32); BERT-base, tokens: 1 261 / 395, 16 307 / 399,
 // 24 368 / 399, 32 398 / 400, 48 509 / 406; BERT-large 16 669 / 873, 32 875 / 874. Layers with context attention are more launches, and
-// Python, for the same products: six steps of six layers, 200 source tokens, 1 row 1356 / 3292, 32 2233 / 3466, 64 3230 / 3415.
+// Python, for the same products: a step of six layers, 200 source tokens, 1 row 223 / 508, 32 316 / 537, 64 436 / 532.
 constexpr int64_t kMostRows = 24, kMostRowsContext = TTB_CHAIN_MAX_ROWS;
 bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
   if (x.n_dim() != 3 || !x.on_gpu() || !core::SameType(x.dtype(), core::kFloat16)) return false;
   const int64_t rows = x.numel() ? x.rows() : 0, H = x.shape(2);
   // (narrower models keep the layer-by-layer pass, whose results are bit for bit those of its layers called one by one)
   return rows > 0 && H == heads * kHead && H >= 512 && Aligned({&x}) && rows <= std::min(most, ttb_chain_rows(H, inner)) &&
-         ttb::chain::rows_have_writers(rows, ttb_ctx_sm_count(DeviceContext(x.device_id())));
+         ttb::chain::rows_have_writers(rows, Ctas(x));
 }
 
 // The call's scratch memory, dealt out in pieces.
@@ -154,7 +156,7 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
   const bool cached = blocks[0].self_keys != nullptr;
   const int64_t past = cached && !blocks[0].self_keys->is_null() ? blocks[0].self_keys->shape(0) : 0;
   if ((past > 0 || context) && L != 1) return false;
-  if (past > (1 << 24)) return false;
+  if (!context && past > 0 && !ttb::chain::history_fits(M, heads, Ctas(x), past)) return false;
   int64_t Lk = 0;
   if (context) {
     const Tensor* k = blocks[0].memory_keys;
@@ -163,6 +165,7 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
     if (Lk < 1 || !memory_mask->on_gpu() || memory_mask->device_id() != x.device_id() || !core::SameType(memory_mask->dtype(), core::kFloat32) ||
         memory_mask->shape(-1) != Lk || memory_mask->numel() != B * Lk)
       return false;
+    if (!ttb::chain::memory_fits(M, heads, Ctas(x), Lk, past) || past > (1 << 24)) return false;
   }
   for (const DecoderBlock& b : blocks) {
     const MultiHeadedAttention& a = *b.attention;

@@ -30,7 +30,7 @@ using namespace ttb;
 
 namespace {
 
-constexpr int kWarps = 8;                       // the operations are bound by what every warp has to do anyway: fewer warps, with more registers
+using chain::kWarps;                            // the operations are bound by what every warp has to do anyway: fewer warps, with more registers
 constexpr int kThreads = kWarps * 32;
 constexpr int kGroup = 4;                       // most units of eight columns that a CTA computes at a time
 constexpr int kRowPad = 64;                     // bytes between the rows of a ring slot, for the banks

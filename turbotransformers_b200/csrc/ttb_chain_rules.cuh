@@ -26,5 +26,31 @@ TTB_CHAIN_FN bool rows_have_writers(int64_t rows, int64_t ctas) { return rows <=
 // The widest product with a bias that a grid takes, in columns (dealt out unevenly, a CTA may have a unit more than another).
 TTB_CHAIN_FN int64_t bias_columns(int64_t ctas) { return (kBiasUnits - 1) * 8 * ctas; }
 
+// ---- attention: up to how many keys the chain is the faster route ------------------------------------------------------------
+// A (row, head) is one CTA's: where a CTA has `pairs` of them, its eight warps are shared out among them, kWarps / pairs each. Layer by layer
+// a long history is split over up to sixteen CTAs a head, so that the chain, which wins by the launches it saves, loses again where a
+// warp walks far. Both sides were measured up to 4000 keys (fp16, a step of the whole model, us, chain / layer by layer).
+constexpr int kWarps = 8;  // of a CTA
+
+TTB_CHAIN_FN int64_t pairs_of_cta(int64_t rows, int64_t heads, int64_t ctas) { return (rows * heads + ctas - 1) / ctas; }
+
+// Tokens in a decoder-only model's cache. Eight warps a pair: GPT-2 small 1 row, 2500 tokens 500 / 507, 3000 552 / 513; 8 rows, 3000 592 / 656, 4000
+// 696 / 704; 8 heads of 64, 18 rows, 3000 659 / 674. Four: 8 heads, 20 rows, 1000 501 / 510, 1300 552 / 538; 12 heads, 18 rows, 1300 626 / 647,
+// 1600 693 / 684; 16 heads (24 layers), 12 rows, 1600 1274 / 1362, 2000 1487 / 1452. Two: 16 heads, 20 rows, 300 1005 / 1090, 700 1271 / 1247.
+TTB_CHAIN_FN bool history_fits(int64_t rows, int64_t heads, int64_t ctas, int64_t tokens) {
+  const int64_t pairs = pairs_of_cta(rows, heads, ctas);
+  if (pairs <= 1) return tokens <= (rows < 8 ? 2400 + 140 * rows : 3500);
+  if (pairs == 2) return tokens <= 550 + 80 * heads;
+  return pairs <= 4 && tokens <= 640;
+}
+
+// Keys of an encoder memory (and tokens in the cache, as many again to walk). Layer by layer the host is the limit, about 550 us for six layers,
+// and beyond the 1024 keys of its one-kernel cross attention (ttb_context_attention_step) that pass takes 1200 us and more. 8 heads: 64
+// rows, 600 keys 551 / 555, 700 600 / 550; 48 rows, 700 539 / 572, 1000 615 / 608; 36 rows, 1000 481 / 566; 64 rows, 1300 and more far ahead. 16 heads:
+// 32 rows, 1000 643 / 666.
+TTB_CHAIN_FN bool memory_fits(int64_t rows, int64_t heads, int64_t ctas, int64_t keys, int64_t tokens) {
+  return keys > 1024 || pairs_of_cta(rows, heads, ctas) * (keys + tokens) <= 300 * heads;
+}
+
 }  // namespace chain
 }  // namespace ttb
