@@ -306,3 +306,36 @@ def test_a_long_history_goes_layer_by_layer():
         (got, _), n = launches(lambda: model(ids[:, t:t + 1].contiguous(), past=past))
         assert (n <= 3) if t <= 1190 else (n >= 12), t
     assert err(got, exact(ids).last_hidden_state[:, -1:]) < TOL
+
+
+# ---- calls that the route does not take ------------------------------------------------------------------------------------
+@pytest.mark.parametrize("H,F,B,S", [(1024, 4096, 33, 20), (512, 2048, 65, 9), (512, 2048, 64, 700)])
+def test_a_step_outside_the_rule_costs_no_list_of_operations(monkeypatch, H, F, B, S):
+    """The rule is asked before parts and caches of every layer are gathered and converted (65 us a step of six layers)."""
+    dec = tt.TransformerDecoder.from_onmt(weights(Stack(H, F, 2), 3), DEV)
+    memory, lengths = torch.randn(S, B, H, device=DEV).half(), torch.full((B, ), S, device=DEV)
+    dec.init_state(torch.zeros(S, B, 1), memory, None)
+    monkeypatch.setattr(cxx, "decoder_chain", lambda *a: pytest.fail("gathered"))
+    for t in range(2):
+        out, n = launches(lambda: dec(ids_of(300, 1, B, 1), memory, step=t, memory_lengths=lengths))
+        assert n >= 20 and torch.isfinite(out[0]).all()
+
+
+def test_a_call_of_more_rows_costs_no_list_of_operations(monkeypatch):
+    monkeypatch.setattr(cxx, "decoder_chain", lambda *a: pytest.fail("gathered"))
+    monkeypatch.setattr(cxx, "encoder_chain", lambda *a: pytest.fail("gathered"))
+    hf, model, exact = bert(768, 3072, 2)
+    assert torch.isfinite(model(ids_of(500, 1, 25))[0]).all()
+    model, exact = gpt2(768, 2)
+    assert torch.isfinite(model(ids_of(1003, 1, 25))[0]).all()
+
+
+def test_a_long_history_goes_layer_by_layer():
+    model, exact = gpt2(512, 2, positions=1400)
+    ids = ids_of(1003, 20, 1201, seed=4)
+    past = model.new_cache()
+    model(ids[:, :1180].contiguous(), return_logits=False, past=past)
+    for t in range(1180, 1201):  # twenty rows of eight heads are two to a CTA: up to 1190 tokens in the cache
+        (got, _), n = launches(lambda: model(ids[:, t:t + 1].contiguous(), past=past))
+        assert (n <= 3) if t <= 1190 else (n >= 12), t
+    assert err(got, exact(ids).last_hidden_state[:, -1:]) < TOL

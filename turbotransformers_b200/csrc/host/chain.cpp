@@ -94,11 +94,23 @@ struct Ops {
 
 }  // namespace
 
+bool Chain::EncoderTakes(const BertAttention& attention, const BertIntermediate& intermediate, const Tensor& x) {
+  return !x.is_null() && RowsFit(x, attention.num_attention_heads_, intermediate.dense_.out_dim(false), kMostRows);
+}
+
+bool Chain::DecoderTakes(const MultiHeadedAttention& attention, const PositionwiseFeedForward& ffn, bool trans_f, const Tensor& x, int64_t past, int64_t memory_keys) {
+  const bool context = memory_keys > 0;
+  const int64_t heads = attention.num_attention_heads_;
+  if (x.is_null() || !RowsFit(x, heads, ffn.dense1_.out_dim(trans_f), context ? kMostRowsContext : kMostRows)) return false;
+  if (((past > 0 || context) && x.shape(1) != 1) || past > (1 << 24)) return false;
+  if (context) return ttb::chain::memory_fits(x.rows(), heads, Ctas(x), memory_keys, past);
+  return past == 0 || ttb::chain::history_fits(x.rows(), heads, Ctas(x), past);
+}
+
 bool Chain::Encoder(const std::vector<EncoderBlock>& blocks, const Tensor& x, const Tensor& mask, Tensor* out) {
-  if (blocks.empty() || x.is_null() || 5 * blocks.size() + 1 > TTB_CHAIN_MAX_OPS) return false;
+  if (blocks.empty() || 5 * blocks.size() + 1 > TTB_CHAIN_MAX_OPS || !EncoderTakes(*blocks[0].attention, *blocks[0].intermediate, x)) return false;
   const int64_t heads = blocks[0].attention->num_attention_heads_;
   const int64_t F = blocks[0].intermediate->dense_.out_dim(false);
-  if (!RowsFit(x, heads, F, kMostRows)) return false;
   const int64_t B = x.shape(0), L = x.shape(1), H = x.shape(2), M = B * L;
   const float* mask_ptr = nullptr;
   if (!mask.is_null()) {  // one row of L keys per sequence; everything else is the general path's business
@@ -148,15 +160,12 @@ bool Chain::Encoder(const std::vector<EncoderBlock>& blocks, const Tensor& x, co
 bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bool trans_a, bool trans_f, const LayerNorm* final, const class Linear* head,
                     const Tensor* memory, const Tensor* memory_mask, Tensor* hidden, Tensor* logits, Tensor* attn) {
   const bool context = !blocks.empty() && blocks[0].context;
-  if (blocks.empty() || x.is_null() || (context ? 8 : 5) * blocks.size() + 1 > TTB_CHAIN_MAX_OPS) return false;
+  if (blocks.empty() || x.n_dim() != 3 || (context ? 8 : 5) * blocks.size() + 1 > TTB_CHAIN_MAX_OPS) return false;
   const int64_t heads = blocks[0].attention->num_attention_heads_;
   const int64_t F = blocks[0].ffn->dense1_.out_dim(trans_f);
-  if (!RowsFit(x, heads, F, context ? kMostRowsContext : kMostRows)) return false;
   const int64_t B = x.shape(0), L = x.shape(1), H = x.shape(2), M = B * L;
   const bool cached = blocks[0].self_keys != nullptr;
   const int64_t past = cached && !blocks[0].self_keys->is_null() ? blocks[0].self_keys->shape(0) : 0;
-  if ((past > 0 || context) && L != 1) return false;
-  if (!context && past > 0 && !ttb::chain::history_fits(M, heads, Ctas(x), past)) return false;
   int64_t Lk = 0;
   if (context) {
     const Tensor* k = blocks[0].memory_keys;
@@ -165,8 +174,8 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
     if (Lk < 1 || !memory_mask->on_gpu() || memory_mask->device_id() != x.device_id() || !core::SameType(memory_mask->dtype(), core::kFloat32) ||
         memory_mask->shape(-1) != Lk || memory_mask->numel() != B * Lk)
       return false;
-    if (!ttb::chain::memory_fits(M, heads, Ctas(x), Lk, past) || past > (1 << 24)) return false;
   }
+  if (!DecoderTakes(*blocks[0].attention, *blocks[0].ffn, trans_f, x, past, Lk)) return false;
   for (const DecoderBlock& b : blocks) {
     const MultiHeadedAttention& a = *b.attention;
     const PositionwiseFeedForward& f = *b.ffn;

@@ -226,6 +226,8 @@ PYBIND11_MODULE(turbo_transformers_cxx, m) {
       .def("__call__", &layers::BertPooler::operator());
 
   // ---- stacks of layers over few rows as one kernel; false: not taken, nothing done
+  m.def("encoder_chain_takes", &layers::Chain::EncoderTakes);
+  m.def("decoder_chain_takes", &layers::Chain::DecoderTakes);
   m.def("encoder_chain", [](const py::list& blocks, const Tensor& x, const Tensor& mask, Tensor* out) {
     std::vector<layers::Chain::EncoderBlock> list;
     for (const py::handle& h : blocks) {

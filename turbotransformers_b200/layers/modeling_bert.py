@@ -194,7 +194,9 @@ class BertEncoder:
         all_hidden_states, all_attentions = (), ()
         hidden_states = try_convert(hidden_states)
         attention_mask = try_convert(attention_mask)
-        if not output_attentions and not output_hidden_states and all(map(_unmodified, self.layer)):
+        first = self.layer[0] if self.layer else None
+        if (not output_attentions and not output_hidden_states and _unmodified(first) and
+                cxx.encoder_chain_takes(first.attention, first.intermediate, hidden_states) and all(map(_unmodified, self.layer))):
             # few tokens: all layers in one kernel
             out = cxx.Tensor.create_empty()
             if cxx.encoder_chain([(l.attention, l.intermediate, l.output) for l in self.layer], hidden_states, create_empty_if_none(attention_mask), out):

@@ -150,7 +150,14 @@ class TransformerDecoder:
     def _chain(self, x: torch.Tensor, memory_bank: torch.Tensor, src_pad_mask: torch.Tensor):
         """One decoding step of a small batch through all layers in one kernel: (output, attention of head 0), or None where the
         call is not such a step and nothing has been done."""
-        if x.dtype != torch.float16 or x.size(1) != 1 or x.size(0) > 64 or len({l._ffn_trans for l in self.transformer_layers}) != 1:
+        if x.dtype != torch.float16 or x.size(1) != 1 or len({l._ffn_trans for l in self.transformer_layers}) != 1:
+            return None
+        first, keys = self.transformer_layers[0], self.state["cache"]["layer_0"].get("self_keys")
+        use_current_stream(x)
+        x = try_convert(x)
+        past = 0 if keys is None or not isinstance(keys, cxx.Tensor) or keys.is_null() else keys.shape(0)
+        if not (isinstance(first.self_attn, cxx.MultiHeadedAttention) and isinstance(first.feed_forward, cxx.PositionwiseFeedForward) and
+                cxx.decoder_chain_takes(first.self_attn, first.feed_forward, first._ffn_trans, x, past, src_pad_mask.size(-1))):
             return None
         parts = [(l.self_attn, l.context_attn, l.feed_forward) for l in self.transformer_layers]
         caches = [self.state["cache"][f"layer_{i}"] for i in range(len(parts))]
@@ -158,17 +165,16 @@ class TransformerDecoder:
         if not all(set(c) == set(names) for c in caches) or not all(
                 type(s) is MultiHeadedAttention and type(c) is MultiHeadedAttention and type(f) is PositionwiseFeedForward for s, c, f in parts):
             return None
-        use_current_stream(x)
         held = [tuple(_empty() if c[k] is None else try_convert(c[k]) for k in names) for c in caches]
         # a memory entry is only read where both of a layer are filled; otherwise both are projected, whichever was given
         projected = [h[2].is_null() or h[3].is_null() for h in held]
         memory = memory_bank.transpose(0, 1).contiguous() if any(projected) else None
         src_mask = (src_pad_mask.float() * -1e18).contiguous()
         out, attn = _empty(), _empty()
-        if not cxx.decoder_chain(parts, held, try_convert(x), False, self.transformer_layers[0]._ffn_trans, None, None, try_convert(memory),
+        if not cxx.decoder_chain(parts, held, x, False, first._ffn_trans, None, None, try_convert(memory),
                                  try_convert(src_mask), out, None, attn):
             return None
-        use_current_stream(x)  # torch reads the results on the caller's stream, wherever another thread has pointed the runtime meanwhile
+        use_current_stream(src_mask)  # torch reads the results on the caller's stream, wherever another thread has pointed the runtime meanwhile
         for c, h, fresh in zip(caches, held, projected):
             c["self_keys"], c["self_values"] = h[0], h[1]
             if fresh:
