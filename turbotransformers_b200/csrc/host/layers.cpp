@@ -584,7 +584,8 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
     }
     if (att_score) *att_score = Tensor(nullptr);
   } else if (Fp32Planes(dt) && !att_score && !cache_keys && d == 64 && B <= 65535 && (!causal_ || !attention_mask.is_null())) {
-    // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own
+    // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own (a causal layer's
+    // mask tensor says what its rows see, as it does in the sequence below; the kernel's own causal form is the C call's)
     Tensor qkv(nullptr);
     qkv.Reshape(x.dtype(), {T, 3 * H}, kDLCUDA, dev, "self/qkv_out1/Reshape");
     qkv_.Forward(*gemm_in, T, TTB_EPI_BIAS, nullptr, qkv.raw_mut(), is_trans_weight, "self/gemm012_fused");

@@ -130,7 +130,8 @@ class MultiHeadedAttention {
 
   // `att_score` is a per-call choice: a 16-bit model given nullptr skips the [B,heads,L,L] score tensor (the largest HBM
   // round trip of the reference path) and runs the fused attention kernel; given a tensor it materialises the scores into
-  // it as the reference does. fp32 models always materialise (into a temporary when att_score is nullptr).
+  // it as the reference does. fp32 models given nullptr run a fused kernel of their own (64-wide heads; a causal layer needs its mask
+  // tensor there); other head sizes materialise into a temporary.
   void set_pre_layernorm_eps(float eps) { pre_ln_eps_ = eps; }  // the reference hard-codes 1e-6
   void set_causal(bool on) { causal_ = on; }                    // decoder-style self-attention without a mask tensor
   void QuantizeInt8() { qkv_.set_int8(true); dense_.set_int8(true); }

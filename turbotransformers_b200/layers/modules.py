@@ -23,8 +23,8 @@ class MultiHeadedAttention(cxx.MultiHeadedAttention):
                  post_layernorm: bool = False, post_add_input: bool = False, is_trans_weight: bool = False,
                  return_type: Optional[ReturnType] = None, output: Optional[cxx.Tensor] = None, attn: Optional[cxx.Tensor] = None,
                  output_attentions: bool = False):
-        """Returns (output, attn). `attn` holds the attention probabilities only for fp32 models or when
-        output_attentions is set; otherwise it is a null tensor (the fused kernel never writes them)."""
+        """Returns (output, attn). `attn` holds the attention probabilities when output_attentions is set or for
+        context attention; otherwise it is a null tensor (the fused kernels never write them)."""
         if isinstance(query_tensor, torch.Tensor):
             use_current_stream(query_tensor)
         query, key, value = query_tensor, key_tensor, value_tensor
