@@ -6,8 +6,8 @@
 // arithmetic, were the time. A CTA has 8 R query rows of one (sequence, head) and goes over the keys in tiles of 64 with an online
 // softmax; a thread computes R x 4 scores, then R x 4 outputs, from 16-byte reads of shared memory (rows of 68 floats: the lanes of a read
 // hit different banks). BERT-base fp32, us a pass, with the planes below, against
-// those five: 8 requests of 10 to 120 tokens 2591 -> 1800, 16 of 8 to 512 13283 -> 5900, 1 x 128 1187 -> 1084, 8 x 512 8826 -> 6150, 32 x 512 32363 ->
-// 23400 (with the layer norms of few rows; its Linears are what is left); one layer's attention over 1 x 4096 tokens 2693 -> 1705. The output may leave as the two planes that the next product takes.
+// those five: 8 requests of 10 to 120 tokens 2591 -> 1730, 16 of 8 to 512 13283 -> 5670, 1 x 128 1187 -> 1084, 8 x 512 8826 -> 6050, 32 x 512 32363 ->
+// 22300 (with the layer norms of few rows; its Linears are what is left); one layer's attention over 1 x 4096 tokens 2693 -> 1705. The output may leave as the two planes that the next product takes.
 #include "ttb_common.cuh"
 
 using namespace ttb;

@@ -28,7 +28,9 @@ inline int grid_for(int64_t work, int per_block, int sm_count) {
 constexpr int kLnWarps = 8;
 constexpr int kLnRows = 2;
 
-// EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo.
+// EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
+// same with the lanes trading places before they store (more than a CTA of two rows an SM: bound by the stores, which write 512 bytes in a row then,
+// not every other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1735 us; with 128 rows the exchange is latency, 1084 -> 1099).
 template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
@@ -99,18 +101,35 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
             Vec8<TOut> o;
 #pragma unroll
             for (int j = 0; j < 8; ++j) o.v[j] = b.v[j] + g.v[j] * rstd[r] * (v[r][it][j] - mean[r]);
+            if (EXTRA == 3 && (it + 1) * 256 <= N) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                float w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float first = __shfl_sync(0xffffffffu, o.v[j], h * 16 + (lane >> 1)), second = __shfl_sync(0xffffffffu, o.v[4 + j], h * 16 + (lane >> 1));
+                  w[j] = (lane & 1) ? second : first;
+                }
+                const int64_t at = row * N + it * 256 + h * 128 + lane * 4;
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = make_float4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<float4*>(out_f32 + at) = make_float4(tf32_hi(w[0]), tf32_hi(w[1]), tf32_hi(w[2]), tf32_hi(w[3]));
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(out_lo) + at) =
+                    make_float4(tf32_lo(w[0], true), tf32_lo(w[1], true), tf32_lo(w[2], true), tf32_lo(w[3], true));
+              }
+              continue;
+            }
             o.store(out + row * N + col);
             if (EXTRA) {
-              if (EXTRA == 2 || out_f32) {
+              if (EXTRA >= 2 || out_f32) {
                 Vec8<float> f;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) f.v[j] = EXTRA == 2 ? tf32_hi(o.v[j]) : o.v[j];
+                for (int j = 0; j < 8; ++j) f.v[j] = EXTRA >= 2 ? tf32_hi(o.v[j]) : o.v[j];
                 f.store(out_f32 + row * N + col);
               }
-              if (EXTRA == 2 || out_lo) {
+              if (EXTRA >= 2 || out_lo) {
                 Vec8<TOut> l;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j], EXTRA == 2);
+                for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j], EXTRA >= 2);
                 l.store(out_lo + row * N + col);
               }
             }
@@ -485,19 +504,23 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   const int grid = grid_for(pair_warps, kLnWarps, ctx->sm_count);
   const int block = kLnWarps * 32;
   const bool extra = out_lo != nullptr || out_f32 != nullptr;
-  constexpr int kPlanes = std::is_same<TOut, float>::value ? 2 : 1;  // fp32 with both extras: its planes
-  const bool planes = kPlanes == 2 && out_lo && out_f32;
+  constexpr bool kFloat = std::is_same<TOut, float>::value;  // fp32 with both extras: its planes
+  constexpr int kPlanes = kFloat ? 2 : 1, kPlanesTraded = kFloat ? 3 : 1;
+  const bool planes = kFloat && out_lo && out_f32, traded = planes && M > 2 * (int64_t)ctx->sm_count;
   // Sixteen rows a CTA leave most SMs without one while the rest move 200 KB each (128 fp32 rows: 8 CTAs): up to eight rows an SM,
   // CTAs of two rows. The rows' arithmetic is the same. BERT-base fp32, 24 layer norms a pass: 1 x 128 1171 -> 1068 us, 527 rows 1814 -> 1727.
   const bool few = M <= 8 * (int64_t)ctx->sm_count;
   const int few_grid = (int)((M + 1) / 2);
 #define LN_CASE(IT)                                                                                                              \
   do {                                                                                                                           \
-    if (few && planes)                                                                                                           \
+    if (few && traded)                                                                                                           \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+    else if (few && planes)                                                                                                      \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (planes)                                                                                                             \
-      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
+      launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
                  out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (few && extra)                                                                                                       \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
