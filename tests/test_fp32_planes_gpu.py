@@ -104,7 +104,7 @@ def test_planes_of_a_product(ctx, M, N):
 def test_planes_of_layer_norm_attention_and_embedding(ctx):
     g = torch.Generator(device=DEV).manual_seed(1)
     rand = lambda *shape: torch.randn(*shape, generator=g, device=DEV)
-    for M, N in ((1, 768), (37, 1024), (296, 768), (297, 768), (1184, 768), (1185, 768), (5, 770), (600, 776), (600, 2048), (1500, 264), (900, 248)):
+    for M, N in ((1, 768), (37, 1024), (148, 768), (149, 768), (297, 768), (1184, 768), (1185, 768), (5, 770), (600, 776), (600, 2048), (1500, 264), (900, 248)):
         out, hi, lo = rand(M, N), torch.zeros(M, N, device=DEV), torch.zeros(M, N, device=DEV)
         ctx.call("add_bias_layernorm_f32_planes", out, hi, lo, rand(M, N), rand(N), rand(N), rand(N), M, N, 1e-12)
         assert torch.equal(torch.stack([hi, lo]), split(ctx, out))

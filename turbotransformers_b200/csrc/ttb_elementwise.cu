@@ -29,8 +29,8 @@ constexpr int kLnWarps = 8;
 constexpr int kLnRows = 2;
 
 // EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
-// same with the lanes trading places before they store (more than a CTA of two rows an SM: bound by the stores, which write 512 bytes in a row then,
-// not every other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1735 us; with 128 rows the exchange is latency, 1084 -> 1099).
+// same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
+// other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099).
 template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
@@ -506,7 +506,7 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   const bool extra = out_lo != nullptr || out_f32 != nullptr;
   constexpr bool kFloat = std::is_same<TOut, float>::value;  // fp32 with both extras: its planes
   constexpr int kPlanes = kFloat ? 2 : 1, kPlanesTraded = kFloat ? 3 : 1;
-  const bool planes = kFloat && out_lo && out_f32, traded = planes && M > 2 * (int64_t)ctx->sm_count;
+  const bool planes = kFloat && out_lo && out_f32, traded = planes && M > (int64_t)ctx->sm_count;
   // Sixteen rows a CTA leave most SMs without one while the rest move 200 KB each (128 fp32 rows: 8 CTAs): up to eight rows an SM,
   // CTAs of two rows. The rows' arithmetic is the same. BERT-base fp32, 24 layer norms a pass: 1 x 128 1171 -> 1068 us, 527 rows 1814 -> 1727.
   const bool few = M <= 8 * (int64_t)ctx->sm_count;
