@@ -411,6 +411,13 @@ typedef struct ttb_chain_op {
   } u;
 } ttb_chain_op;
 int ttb_chain_forward(ttb_ctx* ctx, int dtype, const ttb_chain_op* ops, int n_ops, void* workspace);
+/* The same without barriers. `flow` is device memory, on 16 bytes, through which the operations hand their results on: every operand that one
+ * of them writes and another reads (other than the keys and values of TTB_CHAIN_KEYS_CACHE and _MEMORY, which none may write for another) lies in it,
+ * each result in a place of its own behind those of the operations before (normed before out), of whole 32-bit words. The call sets it to
+ * TTB_CHAIN_UNWRITTEN, which no pair of results that a rounding to fp16 has made can be, and an operation reads a word of it again until it is
+ * another one; the reads are bounded, like every wait (TTB_ERR_DEVICE_WAIT). */
+#define TTB_CHAIN_UNWRITTEN 0xffffffffu
+int ttb_chain_forward_flow(ttb_ctx* ctx, int dtype, const ttb_chain_op* ops, int n_ops, void* flow, int64_t flow_bytes);
 /* The most rows that a chain takes whose products are `hidden` deep, normalised or not, and `inner` deep, not normalised: shared memory
  * holds the normalised rows and a ring of weights. 0: none. */
 int64_t ttb_chain_rows(int64_t hidden, int64_t inner);

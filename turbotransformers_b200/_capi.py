@@ -77,6 +77,7 @@ SIGNATURES = {
     "ttb_context_attention_step": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64, f32, p, p]),
     "ttb_attention_decode": (i32, [p, i32, p, i64, i64, i64, i64, p, p, i64, f32, p]),
     "ttb_chain_forward": (i32, [p, i32, C.POINTER(ChainOp), i32, p]),
+    "ttb_chain_forward_flow": (i32, [p, i32, C.POINTER(ChainOp), i32, p, i64]),
     "ttb_token_position_embedding": (i32, [p, i32, p, p, p, p, i64, i64, i64, i64]),
     "ttb_chain_rows": (i64, [i64, i64]),
     "ttb_attention_f32": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p]),
@@ -196,17 +197,27 @@ class Context:
                        epilogue, ptr(out), ptr(out_lo), ldo or N)
         self.check(lib().ttb_linear_ex(self.h, C.byref(a)))
 
-    def chain_forward(self, ops):
-        """ttb_chain_forward on operations given as ("linear" | "attention", {field: value}); tensors are passed as their pointers."""
-        import torch
+    @staticmethod
+    def _chain_block(ops):
         block = (ChainOp * len(ops))()
         for b, (kind, fields) in zip(block, ops):
             b.kind = {"linear": 0, "attention": 1}[kind]
             for name, value in fields.items():
                 setattr(getattr(b.u, kind), name, value.data_ptr() if hasattr(value, "data_ptr") else value)
+        return block
+
+    def chain_forward(self, ops):
+        """ttb_chain_forward on operations given as ("linear" | "attention", {field: value}); tensors are passed as their pointers."""
+        import torch
+        block = self._chain_block(ops)
         workspace = torch.empty(CHAIN_WORKSPACE, dtype=torch.uint8, device=f"cuda:{self.device}")
         self.check(lib().ttb_chain_forward(self.h, F16, block, len(ops), workspace.data_ptr()))
         torch.cuda.synchronize(self.device)  # the workspace is in use until the kernel has finished
+
+    def chain_forward_flow(self, ops, flow):
+        """ttb_chain_forward_flow, operations as in chain_forward; flow: the tensor that their results lie in."""
+        block = self._chain_block(ops)
+        self.check(lib().ttb_chain_forward_flow(self.h, F16, block, len(ops), flow.data_ptr(), flow.numel() * flow.element_size()))
 
     def linear_plan(self, dtype, out_dtype, products, M, N, K, two_plane_out=False, whole_rows=True):
         """What ttb_linear_plan reports: (columns, CTAs of a pair, CTAs along K, tiles, tiles at a time)."""

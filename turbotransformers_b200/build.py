@@ -85,7 +85,7 @@ def build_cxx_module(force=False, verbose=False):
     if not srcs:
         return None
     out = cxx_module_path()
-    deps = srcs + glob.glob(os.path.join(host, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    deps = srcs + glob.glob(os.path.join(host, "*.h")) + glob.glob(os.path.join(ROOT, "include", "*.h")) + glob.glob(os.path.join(CSRC, "*_rules.cuh"))
     if not force and not _newer(out, deps):
         return out
     import pybind11

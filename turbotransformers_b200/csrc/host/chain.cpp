@@ -38,12 +38,15 @@ bool NormFits(const Tensor& gamma, const Tensor& beta, int64_t H, const Tensor& 
   return Vector(gamma, H, x) && Vector(beta, H, x) && Aligned({&gamma, &beta});
 }
 // (How many keys those rows may have: history_fits and memory_fits of ttb_chain_rules.cuh.)
-// The rows up to which one kernel is the faster route: above, every CTA's normalising of all rows and its reading of all of the wide
-// activation outweigh the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 286 / 414, 16 334 / 435,
-// 24 397 / 436, 32 443 / 436, 64 639 / 484 (300 cached: 370 / 492, 446 / 526, 526 / 549 at 16, 24, 32); BERT-base, tokens: 1 261 / 395, 16 307 / 399,
-// 24 368 / 399, 32 398 / 400, 48 509 / 406; BERT-large 16 669 / 873, 32 875 / 874. Layers with context attention are more launches, and
-// Python, for the same products: a step of six layers, 200 source tokens, 1 row 223 / 508, 32 316 / 537, 64 436 / 532.
-constexpr int64_t kMostRows = 24, kMostRowsContext = TTB_CHAIN_MAX_ROWS;
+// The rows up to which one kernel is the faster route: above 32 the rows are eight tiles for the kernel, and every CTA's reading of all of them outweighs
+// the launches saved. us, one kernel / layer by layer. GPT-2 small, a step with 30 cached tokens: 1 row 171 / 398, 16 234 / 414, 24 303 / 420,
+// 32 339 / 417, 40 539 / 422, 64 601 / 448; BERT-base, tokens: 1 161 / 426, 16 218 / 425, 24 288 / 421, 32 310 / 425, 33 490 / 423; BERT-large 16 474 / 875,
+// 24 676 / 878, 32 764 / 874. Layers with context attention are more launches, and Python, for the same products: a step of six layers, 45
+// source tokens, 1 row 215 / 592, 32 234 / 623, 64 381 / 621.
+// From 25 rows on, stacks of four layers and more: 12 layers 303 / 395, four 108 / 143. What shorter ones would gain is a few launches, and their
+// layer-by-layer pass gives bit for bit the results of its layers called one by one.
+constexpr int64_t kMostRows = 24, kMostRowsDeep = 32, kDeep = 4, kMostRowsContext = TTB_CHAIN_MAX_ROWS;
+int64_t MostRows(int64_t layers) { return layers >= kDeep ? kMostRowsDeep : kMostRows; }
 bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
   if (x.n_dim() != 3 || !x.on_gpu() || !core::SameType(x.dtype(), core::kFloat16)) return false;
   const int64_t rows = x.numel() ? x.rows() : 0, H = x.shape(2);
@@ -52,17 +55,22 @@ bool RowsFit(const Tensor& x, int64_t heads, int64_t inner, int64_t most) {
          ttb::chain::rows_have_writers(rows, Ctas(x));
 }
 
-// The call's scratch memory, dealt out in pieces.
-struct Scratch {
+// The call's scratch memory: what operations hand on to others, every result in a place of its own in the order in which they write them.
+struct Flow {
   Tensor buffer{nullptr};
-  size_t bytes = 0;
+  int64_t bytes = 0, at = 0;
   char* base = nullptr;
-  size_t Add(size_t n) {
-    const size_t at = bytes;
-    bytes += (n + 255) / 256 * 256;
-    return at;
+  static int64_t Size(int64_t rows, int64_t columns) { return (rows * columns * 2 + 255) / 256 * 256; }
+  void Allocate(int64_t n, int dev) {
+    bytes = n;
+    base = reinterpret_cast<char*>(buffer.Reshape(core::kInt8, {n}, kDLCUDA, dev, "chain/flow"));
   }
-  void Allocate(int dev) { base = reinterpret_cast<char*>(buffer.Reshape(core::kInt8, {(int64_t)bytes}, kDLCUDA, dev, "chain/scratch")); }
+  void* Next(int64_t rows, int64_t columns) {
+    TT_ENFORCE(at + Size(rows, columns) <= bytes, "chain: the flow is too short");
+    void* p = base + at;
+    at += Size(rows, columns);
+    return p;
+  }
 };
 
 struct Ops {
@@ -94,21 +102,22 @@ struct Ops {
 
 }  // namespace
 
-bool Chain::EncoderTakes(const BertAttention& attention, const BertIntermediate& intermediate, const Tensor& x) {
-  return !x.is_null() && RowsFit(x, attention.num_attention_heads_, intermediate.dense_.out_dim(false), kMostRows);
+bool Chain::EncoderTakes(const BertAttention& attention, const BertIntermediate& intermediate, const Tensor& x, int64_t layers) {
+  return !x.is_null() && RowsFit(x, attention.num_attention_heads_, intermediate.dense_.out_dim(false), MostRows(layers));
 }
 
-bool Chain::DecoderTakes(const MultiHeadedAttention& attention, const PositionwiseFeedForward& ffn, bool trans_f, const Tensor& x, int64_t past, int64_t memory_keys) {
+bool Chain::DecoderTakes(const MultiHeadedAttention& attention, const PositionwiseFeedForward& ffn, bool trans_f, const Tensor& x, int64_t past, int64_t memory_keys,
+                         int64_t layers) {
   const bool context = memory_keys > 0;
   const int64_t heads = attention.num_attention_heads_;
-  if (x.is_null() || !RowsFit(x, heads, ffn.dense1_.out_dim(trans_f), context ? kMostRowsContext : kMostRows)) return false;
+  if (x.is_null() || !RowsFit(x, heads, ffn.dense1_.out_dim(trans_f), context ? kMostRowsContext : MostRows(layers))) return false;
   if (((past > 0 || context) && x.shape(1) != 1) || past > (1 << 24)) return false;
   if (context) return ttb::chain::memory_fits(x.rows(), heads, Ctas(x), memory_keys, past);
   return past == 0 || ttb::chain::history_fits(x.rows(), heads, Ctas(x), past);
 }
 
 bool Chain::Encoder(const std::vector<EncoderBlock>& blocks, const Tensor& x, const Tensor& mask, Tensor* out) {
-  if (blocks.empty() || 5 * blocks.size() + 1 > TTB_CHAIN_MAX_OPS || !EncoderTakes(*blocks[0].attention, *blocks[0].intermediate, x)) return false;
+  if (blocks.empty() || 5 * blocks.size() + 1 > TTB_CHAIN_MAX_OPS || !EncoderTakes(*blocks[0].attention, *blocks[0].intermediate, x, (int64_t)blocks.size())) return false;
   const int64_t heads = blocks[0].attention->num_attention_heads_;
   const int64_t F = blocks[0].intermediate->dense_.out_dim(false);
   const int64_t B = x.shape(0), L = x.shape(1), H = x.shape(2), M = B * L;
@@ -129,31 +138,40 @@ bool Chain::Encoder(const std::vector<EncoderBlock>& blocks, const Tensor& x, co
   }
   const int dev = x.device_id();
   ttb_ctx* c = DeviceContext(dev);
-  Scratch s;
-  const size_t workspace = s.Add(TTB_CHAIN_WORKSPACE), qkv = s.Add(M * 3 * H * 2), context = s.Add(M * H * 2), sum = s.Add(M * H * 2),
-               normed = s.Add(M * H * 2), inter = s.Add(M * F * 2);
-  s.Allocate(dev);
+  Flow f;
+  f.Allocate((int64_t)blocks.size() * (Flow::Size(M, 3 * H) + 5 * Flow::Size(M, H) + Flow::Size(M, F)), dev);
   out->Reshape(x.dtype(), {B, L, H}, kDLCUDA, dev, "chain/out");
   Ops ops;
   ops.M = (int)M;
   ops.list.reserve(5 * blocks.size() + 1);
   const EncoderBlock* before = nullptr;
+  const void *in = x.raw(), *residual = x.raw();  // what the block before has added up, and the layer norm of that: this block's residual
   for (const EncoderBlock& b : blocks) {
     const MultiHeadedAttention& a = *b.attention;
-    // the layer norm of the block before, whose result is this block's residual
-    ttb_chain_linear* o = ops.Linear(before ? s.base + sum : x.raw(), H, a.qkv_.Packed(false), a.qkv_.bias().raw(), 3 * H, s.base + qkv);
-    if (before) ops.Norm(o, before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, s.base + normed);
-    ttb_chain_attention* at = ops.Attention(TTB_CHAIN_KEYS_ROWS, s.base + qkv, 3 * H, heads, L, s.base + context);
+    void* normed = before ? f.Next(M, H) : nullptr;
+    void* qkv = f.Next(M, 3 * H);
+    ttb_chain_linear* o = ops.Linear(in, H, a.qkv_.Packed(false), a.qkv_.bias().raw(), 3 * H, qkv);
+    if (before) {
+      ops.Norm(o, before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, normed);
+      residual = normed;
+    }
+    void* context = f.Next(M, H);
+    ttb_chain_attention* at = ops.Attention(TTB_CHAIN_KEYS_ROWS, qkv, 3 * H, heads, L, context);
     at->mask = mask_ptr;
     at->mask_pitch = (int32_t)L;
-    ops.Linear(s.base + context, H, a.dense_.Packed(false), a.dense_.bias().raw(), H, s.base + sum, TTB_CHAIN_ACT_NONE, before ? s.base + normed : x.raw());
-    o = ops.Linear(s.base + sum, H, b.intermediate->dense_.Packed(false), b.intermediate->dense_.bias().raw(), F, s.base + inter, TTB_CHAIN_ACT_GELU);
-    ops.Norm(o, a.layernorm_gamma_, a.layernorm_beta_, 1e-12f, s.base + normed);
-    ops.Linear(s.base + inter, F, b.output->dense_.Packed(false), b.output->dense_.bias().raw(), H, s.base + sum, TTB_CHAIN_ACT_NONE, s.base + normed);
+    void* sum = f.Next(M, H);
+    ops.Linear(context, H, a.dense_.Packed(false), a.dense_.bias().raw(), H, sum, TTB_CHAIN_ACT_NONE, residual);
+    normed = f.Next(M, H);
+    void* inter = f.Next(M, F);
+    o = ops.Linear(sum, H, b.intermediate->dense_.Packed(false), b.intermediate->dense_.bias().raw(), F, inter, TTB_CHAIN_ACT_GELU);
+    ops.Norm(o, a.layernorm_gamma_, a.layernorm_beta_, 1e-12f, normed);
+    void* next = f.Next(M, H);
+    ops.Linear(inter, F, b.output->dense_.Packed(false), b.output->dense_.bias().raw(), H, next, TTB_CHAIN_ACT_NONE, normed);
+    in = next;
     before = &b;
   }
-  ops.Norm(ops.Linear(s.base + sum, H, nullptr, nullptr, 0, nullptr), before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, out->raw_mut());
-  Check(ttb_chain_forward(c, TTB_F16, ops.list.data(), (int)ops.list.size(), s.base + workspace), c, "encoder chain");
+  ops.Norm(ops.Linear(in, H, nullptr, nullptr, 0, nullptr), before->output->layer_norm_weight_, before->output->layer_norm_bias_, 1e-12f, out->raw_mut());
+  Check(ttb_chain_forward_flow(c, TTB_F16, ops.list.data(), (int)ops.list.size(), f.base, f.at), c, "encoder chain");
   return true;
 }
 
@@ -175,7 +193,7 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
         memory_mask->shape(-1) != Lk || memory_mask->numel() != B * Lk)
       return false;
   }
-  if (!DecoderTakes(*blocks[0].attention, *blocks[0].ffn, trans_f, x, past, Lk)) return false;
+  if (!DecoderTakes(*blocks[0].attention, *blocks[0].ffn, trans_f, x, past, Lk, (int64_t)blocks.size())) return false;
   for (const DecoderBlock& b : blocks) {
     const MultiHeadedAttention& a = *b.attention;
     const PositionwiseFeedForward& f = *b.ffn;
@@ -218,23 +236,31 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
   ttb_ctx* c = DeviceContext(dev);
   for (const DecoderBlock& b : blocks)
     if (context && (b.memory_keys->is_null() || b.memory_values->is_null())) b.context->ProjectMemory(*memory, *memory, b.memory_keys, b.memory_values, trans_a);
-  Scratch s;
-  const size_t workspace = s.Add(TTB_CHAIN_WORKSPACE), qkv = s.Add(M * 3 * H * 2), ctx = s.Add(M * H * 2), stream = s.Add(M * H * 2), inter = s.Add(M * F * 2),
-               scores = s.Add(context ? M * Lk * 4 : 0);
-  s.Allocate(dev);
+  Flow f;
+  f.Allocate((int64_t)blocks.size() * (Flow::Size(M, 3 * H) + (context ? 6 : 3) * Flow::Size(M, H) + Flow::Size(M, F)), dev);
+  Tensor scores(nullptr);
   hidden->Reshape(x.dtype(), {B, L, H}, kDLCUDA, dev, "chain/hidden");
   if (head) logits->Reshape(x.dtype(), {B, L, V}, kDLCUDA, dev, "chain/logits");
-  if (context) attn->Reshape(x.dtype(), {B, 1, Lk}, kDLCUDA, dev, "chain/attention");
+  if (context) {
+    attn->Reshape(x.dtype(), {B, 1, Lk}, kDLCUDA, dev, "chain/attention");
+    scores.Reshape<float>({M, Lk}, kDLCUDA, dev, "chain/scores");
+  }
   Ops ops;
   ops.M = (int)M;
   ops.list.reserve(8 * blocks.size() + 1);
   const void* in = x.raw();  // the residual stream: the caller's tensor until the first block has added to it
+  auto add = [&](const void* A, int64_t K, const PackedLinear& l, bool trans) {
+    void* sum = f.Next(M, H);
+    ops.Linear(A, K, l.Packed(trans), l.bias().raw(), H, sum, TTB_CHAIN_ACT_NONE, in);
+    in = sum;
+  };
   for (const DecoderBlock& b : blocks) {
     const MultiHeadedAttention& a = *b.attention;
-    const PositionwiseFeedForward& f = *b.ffn;
+    const PositionwiseFeedForward& ffn = *b.ffn;
     const bool last = &b == &blocks.back();
-    ops.Norm(ops.Linear(in, H, a.qkv_.Packed(trans_a), a.qkv_.bias().raw(), 3 * H, s.base + qkv), a.layernorm_gamma_, a.layernorm_beta_, a.pre_ln_eps_);
-    ttb_chain_attention* at = ops.Attention(past > 0 ? TTB_CHAIN_KEYS_CACHE : TTB_CHAIN_KEYS_ROWS, s.base + qkv, 3 * H, heads, L, s.base + ctx);
+    void *qkv = f.Next(M, 3 * H), *ctx = f.Next(M, H);
+    ops.Norm(ops.Linear(in, H, a.qkv_.Packed(trans_a), a.qkv_.bias().raw(), 3 * H, qkv), a.layernorm_gamma_, a.layernorm_beta_, a.pre_ln_eps_);
+    ttb_chain_attention* at = ops.Attention(past > 0 ? TTB_CHAIN_KEYS_CACHE : TTB_CHAIN_KEYS_ROWS, qkv, 3 * H, heads, L, ctx);
     at->past = (int32_t)past;
     at->causal = a.causal_ ? 1 : 0;
     if (cached) {
@@ -243,31 +269,34 @@ bool Chain::Decoder(const std::vector<DecoderBlock>& blocks, const Tensor& x, bo
       at->k_cache = b.self_keys->raw_mut();
       at->v_cache = b.self_values->raw_mut();
     }
-    ops.Linear(s.base + ctx, H, a.dense_.Packed(trans_a), a.dense_.bias().raw(), H, s.base + stream, TTB_CHAIN_ACT_NONE, in);
-    in = s.base + stream;
+    add(ctx, H, a.dense_, trans_a);
     if (context) {
       const MultiHeadedAttention& m = *b.context;
-      ops.Norm(ops.Linear(in, H, m.q_.Packed(trans_a), m.q_.bias().raw(), H, s.base + qkv), m.layernorm_gamma_, m.layernorm_beta_, m.pre_ln_eps_);
-      at = ops.Attention(TTB_CHAIN_KEYS_MEMORY, s.base + qkv, H, heads, Lk, s.base + ctx);
+      void* q = f.Next(M, H);
+      ctx = f.Next(M, H);
+      ops.Norm(ops.Linear(in, H, m.q_.Packed(trans_a), m.q_.bias().raw(), H, q), m.layernorm_gamma_, m.layernorm_beta_, m.pre_ln_eps_);
+      at = ops.Attention(TTB_CHAIN_KEYS_MEMORY, q, H, heads, Lk, ctx);
       at->k = b.memory_keys->raw();
       at->v = b.memory_values->raw();
       at->mask = memory_mask->data<float>();
       at->mask_pitch = (int32_t)Lk;
       if (last) {
         at->probs = attn->raw_mut();
-        at->scores = reinterpret_cast<float*>(s.base + scores);
+        at->scores = scores.mutableData<float>();
       }
-      ops.Linear(s.base + ctx, H, m.dense_.Packed(trans_a), m.dense_.bias().raw(), H, s.base + stream, TTB_CHAIN_ACT_NONE, in);
+      add(ctx, H, m.dense_, trans_a);
     }
-    const int act = f.act_ == TTB_ACT_GELU ? TTB_CHAIN_ACT_GELU : TTB_CHAIN_ACT_RELU;
-    ops.Norm(ops.Linear(in, H, f.dense1_.Packed(trans_f), f.dense1_.bias().raw(), F, s.base + inter, act), f.layer_norm_weight_, f.layer_norm_bias_, f.eps_);
-    ops.Linear(s.base + inter, F, f.dense2_.Packed(trans_f), f.dense2_.bias().raw(), H, last && !final ? hidden->raw_mut() : s.base + stream, TTB_CHAIN_ACT_NONE, in);
+    const int act = ffn.act_ == TTB_ACT_GELU ? TTB_CHAIN_ACT_GELU : TTB_CHAIN_ACT_RELU;
+    void* inter = f.Next(M, F);
+    ops.Norm(ops.Linear(in, H, ffn.dense1_.Packed(trans_f), ffn.dense1_.bias().raw(), F, inter, act), ffn.layer_norm_weight_, ffn.layer_norm_bias_, ffn.eps_);
+    if (last && !final) ops.Linear(inter, F, ffn.dense2_.Packed(trans_f), ffn.dense2_.bias().raw(), H, hidden->raw_mut(), TTB_CHAIN_ACT_NONE, in);
+    else add(inter, F, ffn.dense2_, trans_f);
   }
   if (final) {
     ttb_chain_linear* o = ops.Linear(in, H, head ? head->dense_.Packed(head->is_trans_) : nullptr, nullptr, V, head ? logits->raw_mut() : nullptr);
     ops.Norm(o, final->gamma_, final->beta_, final->eps_, hidden->raw_mut());
   }
-  Check(ttb_chain_forward(c, TTB_F16, ops.list.data(), (int)ops.list.size(), s.base + workspace), c, "decoder chain");
+  Check(ttb_chain_forward_flow(c, TTB_F16, ops.list.data(), (int)ops.list.size(), f.base, f.at), c, "decoder chain");
   return true;
 }
 

@@ -1,4 +1,4 @@
-// Stacks of layers over few rows as one kernel (ttb_chain_forward): which calls take that route, and their list of operations.
+// Stacks of layers over few rows as one kernel (ttb_chain_forward_flow): which calls take that route, and their list of operations.
 #pragma once
 #include <utility>
 #include <vector>
@@ -25,11 +25,11 @@ class Chain {
     const BertIntermediate* intermediate;
     const BertOutput* output;
   };
-  // Whether a call on x could take the route, by what costs nothing to look at: type, width, rows and keys (`past` cached tokens; memory_keys
-  // of context attention, 0 without). The two calls below check the rest.
-  static bool EncoderTakes(const BertAttention& attention, const BertIntermediate& intermediate, const core::Tensor& x);
+  // Whether a call on x could take the route, by what costs nothing to look at: type, width, rows, layers and keys (`past` cached tokens;
+  // memory_keys of context attention, 0 without). The two calls below check the rest.
+  static bool EncoderTakes(const BertAttention& attention, const BertIntermediate& intermediate, const core::Tensor& x, int64_t layers);
   static bool DecoderTakes(const MultiHeadedAttention& attention, const PositionwiseFeedForward& ffn, bool is_trans_weight_ffn, const core::Tensor& x, int64_t past,
-                           int64_t memory_keys);
+                           int64_t memory_keys, int64_t layers);
   // Post-LN encoder layers: x [B, L, H] -> out. mask: null tensor, or additive fp32 with one row per sequence.
   static bool Encoder(const std::vector<EncoderBlock>& blocks, const core::Tensor& x, const core::Tensor& mask, core::Tensor* out);
   // Pre-LN decoder blocks: x [B, L, H] -> hidden. Without cached tokens any L (causal where the attention says so), with them L = 1. final

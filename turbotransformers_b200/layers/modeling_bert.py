@@ -196,7 +196,7 @@ class BertEncoder:
         attention_mask = try_convert(attention_mask)
         first = self.layer[0] if self.layer else None
         if (not output_attentions and not output_hidden_states and _unmodified(first) and
-                cxx.encoder_chain_takes(first.attention, first.intermediate, hidden_states) and all(map(_unmodified, self.layer))):
+                cxx.encoder_chain_takes(first.attention, first.intermediate, hidden_states, len(self.layer)) and all(map(_unmodified, self.layer))):
             # few tokens: all layers in one kernel
             out = cxx.Tensor.create_empty()
             if cxx.encoder_chain([(l.attention, l.intermediate, l.output) for l in self.layer], hidden_states, create_empty_if_none(attention_mask), out):

@@ -157,7 +157,8 @@ class TransformerDecoder:
         x = try_convert(x)
         past = 0 if keys is None or not isinstance(keys, cxx.Tensor) or keys.is_null() else keys.shape(0)
         if not (isinstance(first.self_attn, cxx.MultiHeadedAttention) and isinstance(first.feed_forward, cxx.PositionwiseFeedForward) and
-                cxx.decoder_chain_takes(first.self_attn, first.feed_forward, first._ffn_trans, x, past, src_pad_mask.size(-1))):
+                cxx.decoder_chain_takes(first.self_attn, first.feed_forward, first._ffn_trans, x, past, src_pad_mask.size(-1),
+                                        len(self.transformer_layers))):
             return None
         parts = [(l.self_attn, l.context_attn, l.feed_forward) for l in self.transformer_layers]
         caches = [self.state["cache"][f"layer_{i}"] for i in range(len(parts))]

@@ -95,7 +95,7 @@ class GPT2Model:
         short prompt; False: not such a call, nothing done. A caller's class in the place of a layer is called as such."""
         first = self.blocks[0] if self.blocks else (None, None)
         if not (type(first[0]) is cxx.MultiHeadedAttention and type(first[1]) is cxx.PositionwiseFeedForward and
-                cxx.decoder_chain_takes(first[0], first[1], False, x, 0 if past is None else self.cached_length(past), 0)):
+                cxx.decoder_chain_takes(first[0], first[1], False, x, 0 if past is None else self.cached_length(past), 0, len(self.blocks))):
             return False
         if not (all(type(a) is cxx.MultiHeadedAttention and type(f) is cxx.PositionwiseFeedForward for a, f in self.blocks) and
                 type(self.final_norm) is cxx.LayerNorm and type(self.lm_head) is cxx.Linear):
