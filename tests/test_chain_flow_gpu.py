@@ -58,7 +58,7 @@ def weights_of(M, H, F, seed, past=37):
                  k=half(past // 16 + 1, M, 16, H, seed=seed + i + 60), v=half(past // 16 + 1, M, 16, H, seed=seed + i + 70)) for i in range(2)]
 
 
-@pytest.mark.parametrize("H,F,V", [(512, 2048, 1003), (768, 3072, 50257), (1024, 4096, 8), (320, 640, 24)])
+@pytest.mark.parametrize("H,F,V", [(512, 2048, 1003), (768, 3072, 50257), (1024, 4096, 8), (320, 640, 24), (960, 6720, 40)])
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 24, 25, 32, 33, 64])
 def test_the_same_bits_as_with_barriers(ctx, M, H, F, V):
     if M > _capi.lib().ttb_chain_rows(H, F):

@@ -58,7 +58,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 struct ChainParams {
   ttb_chain_op ops[TTB_CHAIN_MAX_OPS];  // `reserved` holds what kGroupMask and the constants beside it say
   int n_ops;
-  int ring_bytes, a_bytes;  // shared memory of the weights' ring and of the normalised rows
+  int ring_bytes, a_bytes, sums_bytes;  // shared memory of the weights' ring, of the normalised rows and of partial sums
   int* counter;  // arrivals at the grid's barrier
   int* status;
 };
@@ -177,10 +177,12 @@ __device__ __forceinline__ void look(uint32_t& top, const uint4& v) { top = max(
   return false;
 }
 // Waits for sixteen bytes of the warp's: while there is nothing, many rows are too much to ask for again and again.
-__device__ __forceinline__ void wait_piece(const void* p, int& tries, Shared& sm) {
+[[nodiscard]] __device__ __forceinline__ bool wait_ahead(const void* p, Shared& sm) {
   uint4 v;
+  int tries = 0;
   do v = load16(p);
   while (again(max(max(v.x, v.y), max(v.z, v.w)) == kUnwritten, tries, sm));
+  return tries < kMostTries;
 }
 // The same for a word of one thread. Out of line: a row of an operation before the last is nearly always there.
 __device__ __noinline__ uint32_t wait_word(const void* p, Shared& sm, int phase) {
@@ -214,7 +216,7 @@ __device__ __forceinline__ void sync_warps() { asm volatile("bar.sync 1, %0;" ::
 }
 
 // Waits until fewer than `most` of the `issued` things are in use, or `all` that there were are done with. Bounded by the waits of the warps that use them, which raise the flag.
-[[nodiscard]] __device__ __forceinline__ bool wait_room(const int& done, int issued, int most, Shared& sm, int all = -1) {
+[[nodiscard]] __device__ __forceinline__ bool wait_slots(const int& done, int issued, int most, Shared& sm, int all = -1) {
   const uint32_t at = sm100::smem_u32(&done);
 #pragma unroll 1
   for (int tries = 0; tries < (1 << 27); ++tries) {
@@ -287,8 +289,8 @@ __device__ __forceinline__ int feed(const ChainParams& prm, Shared& sm, uint32_t
       const int nu = min(group, hi - first);
       const int before = at.end;
       at.take(nu * unit_bytes(K), prm.ring_bytes);
-      if (!wait_room(sm.groups_done, groups, kBars, sm) || !wait_room(sm.bytes_done, at.end, prm.ring_bytes + 1, sm, before) ||
-          (first == lo && !wait_room(sm.params_done, params, kParamSlots, sm)))
+      if (!wait_slots(sm.groups_done, groups, kBars, sm) || !wait_slots(sm.bytes_done, at.end, prm.ring_bytes + 1, sm, before) ||
+          (first == lo && !wait_slots(sm.params_done, params, kParamSlots, sm)))
         return groups;
       const uint32_t bar = sm100::smem_u32(&sm.full[groups % kBars]);
       const int rows = min(nu * 8, N - first * 8);
@@ -346,11 +348,11 @@ template <int RT, int CPW> struct Layout {
   static constexpr int RG = RT <= 4 ? 1 : RT / 2, TW = RT / RG, KW = kWarps / RG;
   static constexpr int kStep = 32 * KW * CPW;                               // of K, that all warps work on at a time
   // steps of K whose rows (up to 64 registers) are held at a time
-  static constexpr int kMost = (RT == 8 ? 12 : 16) / (CPW * TW), kHeld = kMost >= 4 ? (CPW > 3 ? 3 : 4) : kMost > 1 ? kMost : 1;
+  static constexpr int kMost = (RT == 8 && CPW == 2 ? 12 : 16) / (CPW * TW), kHeld = kMost >= 4 ? (CPW > 3 ? 3 : 4) : kMost > 1 ? kMost : 1;
   static constexpr int kItems = (kGroup * RT + kWarps - 1) / kWarps;        // (unit, tile) pairs that a warp finishes
   static constexpr int kRed = kGroup * RT * KW * 64;                        // sums: [unit][tile][share][column][row]
   // Two places for the sums, so that a warp need not wait for those that still read the ones before; with many tiles, one, and a barrier.
-  static constexpr int kPlaces = RT <= 2 ? 2 : 1;
+  static constexpr int kPlaces = RT <= 3 ? 2 : 1;
   static_assert(RG * TW == RT && kHeld >= 1 && kRed >= kWarps * (kHeadDim + 2));
 };
 
@@ -398,7 +400,7 @@ __device__ __forceinline__ bool normalise(const ttb_chain_linear& o, bool flows,
   const uint32_t gamma = params + lane * 16;
   const float inv_k = __fdividef(1.f, (float)K), eps = o.eps;
   int tries = 0;
-  bool there[kIters];
+  bool there_yet = true, there[kIters];
 #pragma unroll
   for (int i = 0; i < kIters; ++i) there[i] = i * 256 + lane * 8 < K;
   Two ga[kIters][4], be[kIters][4];
@@ -413,7 +415,7 @@ __device__ __forceinline__ bool normalise(const ttb_chain_linear& o, bool flows,
     const __half* src = static_cast<const __half*>(o.A) + (long long)row0 * o.lda + lane * 8;
     uint4 x[R][kIters];
     uint32_t top;
-    if (flows && M > 2 && row0 == warp) wait_piece(src, tries, sm);
+    if (flows && M > 2 && row0 == warp) there_yet = wait_ahead(src, sm);
     do {
       top = 0;
 #pragma unroll
@@ -496,7 +498,7 @@ __device__ __forceinline__ bool normalise(const ttb_chain_linear& o, bool flows,
           for (int i = 0; i < kIters; ++i)
             if (there[i]) store16(static_cast<__half*>(o.normed) + (long long)row * K + i * 256 + lane * 8, x[r][i]);
   }
-  return tries < kMostTries;
+  return there_yet && tries < kMostTries;
 }
 
 // Steps of K one behind the other, as far as there are any: a step that is not there is jumped over together with those behind it.
@@ -920,7 +922,7 @@ __global__ void __launch_bounds__(kBlock, 1) chain_kernel(const __grid_constant_
   Shared& sm = *reinterpret_cast<Shared*>(smem);
   Place at;
   at.red = reinterpret_cast<float*>(smem + kSharedBytes);
-  at.rows = sm100::smem_u32(smem) + kSharedBytes + L::kPlaces * L::kRed * 4;
+  at.rows = sm100::smem_u32(smem) + kSharedBytes + prm.sums_bytes;
   at.ring = at.rows + prm.a_bytes;
   at.ring_bytes = prm.ring_bytes;
   const int tid = threadIdx.x;
@@ -993,7 +995,8 @@ __global__ void __launch_bounds__(kBlock, 1) chain_kernel(const __grid_constant_
 // Which kernel runs a chain: tiles of eight rows and chunks of K a warp.
 int row_tiles(int rows) { return rows <= 8 ? 1 : rows <= 16 ? 2 : rows <= 24 ? 3 : rows <= 32 ? 4 : 8; }
 int share_of(int tiles) { return tiles <= 4 ? kWarps : 2 * kWarps / tiles; }  // Layout::KW
-int sums_of(int tiles) { return (tiles <= 2 ? 2 : 1) * kGroup * tiles * share_of(tiles) * 64 * 4; }  // Layout::kPlaces * kRed words
+// Layout::kPlaces * kRed words; as many as `group` units need where there is one place.
+int sums_of(int tiles, int group) { return (tiles <= 3 ? 2 * kGroup : std::max(group, 2)) * tiles * share_of(tiles) * 64 * 4; }
 
 // Whether a chain takes a product so deep: the depth is a whole number of parts of 256 to 1024 columns, in 64s.
 bool depth_fits(int64_t K) {
@@ -1006,16 +1009,20 @@ bool depth_fits(int64_t K) {
 // How a chain of products so deep runs: the chunks of K that a warp works on at a time (Layout::CPW), and whether every product is a whole number of them for
 // all warps (EXACT); chunks = 0: the ring does not hold a unit of the deepest. The rest of the shared memory is the ring.
 struct Plan {
-  int tiles = 0, chunks = 0, ring_bytes = 0, a_bytes = 0;
+  int tiles = 0, chunks = 0, group = 0, ring_bytes = 0, a_bytes = 0;
   bool exact = false;
 };
-Plan plan_of(int tiles, const std::vector<int64_t>& depths, int normed_k) {
+Plan plan_of_tiles(int tiles, const std::vector<int64_t>& depths, int normed_k) {
   Plan p;
   p.tiles = tiles;
   p.a_bytes = normed_k ? tiles * 8 * (normed_k * 2 + kRowPad) : 0;
-  p.ring_bytes = kSmemLimit - kSharedBytes - sums_of(tiles) - p.a_bytes;
-  for (int64_t K : depths)
-    if (unit_bytes((int)K) > p.ring_bytes) return p;
+  int64_t deepest = 0;
+  for (int64_t K : depths) deepest = std::max(deepest, K);
+  for (p.group = kGroup; p.group > 0; p.group -= 2) {  // sums of fewer units at a time, where the ring would have no room for a unit otherwise
+    p.ring_bytes = kSmemLimit - kSharedBytes - sums_of(tiles, p.group) - p.a_bytes;
+    if (unit_bytes((int)deepest) <= p.ring_bytes) break;
+  }
+  if (p.group <= 0) return p;
   for (int chunks = 4; chunks >= 2 && !p.exact; --chunks) {
     p.chunks = chunks;
     p.exact = tiles > 4 || normed_k <= 256 * chunks;  // (rows are normalised in pieces of 256)
@@ -1024,9 +1031,17 @@ Plan plan_of(int tiles, const std::vector<int64_t>& depths, int normed_k) {
   if (!p.exact) p.chunks = 4;
   return p;
 }
+// The kernel for so many rows, or one for more that leaves the ring more room.
+Plan plan_of(int rows, const std::vector<int64_t>& depths, int normed_k) {
+  const int tiles = row_tiles(rows);
+  Plan p = plan_of_tiles(tiles, depths, normed_k);
+  if (!p.chunks && tiles < 4) p = plan_of_tiles(4, depths, normed_k);
+  if (!p.chunks && tiles < 8) p = plan_of_tiles(8, depths, normed_k);
+  return p;
+}
 
 template <int RT, int CPW, bool EXACT> cudaError_t launch(ttb_ctx* ctx, const ChainParams& prm) {
-  const int smem = kSharedBytes + Layout<RT, CPW>::kPlaces * Layout<RT, CPW>::kRed * 4 + prm.a_bytes + prm.ring_bytes;
+  const int smem = kSharedBytes + prm.sums_bytes + prm.a_bytes + prm.ring_bytes;
   cudaError_t e = cudaFuncSetAttribute(chain_kernel<RT, CPW, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -1049,9 +1064,9 @@ template <int RT> cudaError_t launch(ttb_ctx* ctx, const Plan& plan, const Chain
 }  // namespace
 
 extern "C" int64_t ttb_chain_rows(int64_t hidden, int64_t inner) {
-  if (hidden > kNormed || !depth_fits(hidden) || !depth_fits(inner)) return 0;
+  if (hidden > kNormed || (hidden != 0 && !depth_fits(hidden)) || !depth_fits(inner)) return 0;
   for (int rows : {64, 32, 24, 16, 8})
-    if (plan_of(row_tiles(rows), {hidden, inner}, (int)hidden).chunks) return rows;
+    if (plan_of(rows, {hidden, inner}, (int)hidden).chunks) return rows;
   return 0;
 }
 static_assert(TTB_CHAIN_MAX_ROWS == 64, "the most rows of the widest kernel");
@@ -1135,13 +1150,14 @@ int chain_forward(ttb_ctx* ctx, int dtype, const ttb_chain_op* ops, int n_ops, i
   prm.n_ops = n_ops;
   prm.counter = counter;
   prm.status = ctx->d_status;
-  const Plan plan = plan_of(row_tiles(rows), depths, normed_k);
+  const Plan plan = plan_of(rows, depths, normed_k);
   TTB_REQUIRE(ctx, plan.chunks > 0, "chain_forward: an operation is too deep");
   prm.ring_bytes = plan.ring_bytes;
   prm.a_bytes = plan.a_bytes;
+  prm.sums_bytes = sums_of(plan.tiles, plan.group);
   for (int i = 0; i < n_ops; ++i)
     if (ops[i].kind == TTB_CHAIN_LINEAR)  // a group's weights fit in the ring
-      prm.ops[i].reserved |= std::min(kGroup, prm.ring_bytes / unit_bytes(ops[i].u.linear.K));
+      prm.ops[i].reserved |= std::min(plan.group, prm.ring_bytes / unit_bytes(ops[i].u.linear.K));
   if (flow) TTB_CUDA(ctx, cudaMemsetAsync(flow, TTB_CHAIN_UNWRITTEN & 0xff, flow_bytes, ctx->stream));
   else TTB_CUDA(ctx, cudaMemsetAsync(counter, 0, TTB_CHAIN_WORKSPACE, ctx->stream));
   switch (plan.tiles) {
