@@ -1,0 +1,149 @@
+"""fp32 as two scaled fp16 planes: the planes against the values, products of planes against fp64 on every tile (few rows, split along K, wide, pairs, ragged) and
+over the range of scales that fp32 has, and the kernels that leave planes for the next product. Tolerances: planes hold 22 bits of an element and 2^-40
+of the row's bound (2^-39 for the two roundings); the tensor cores truncate their partial sums, 1e-8 of the result a term.
+"""
+import pytest
+import torch
+
+from turbotransformers_b200 import _capi
+
+pytestmark = pytest.mark.gpu
+torch.set_grad_enabled(False)
+DEV = torch.device("cuda:0")
+
+
+def randn(*shape, seed=1, scale=1.0):
+    return torch.randn(*shape, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV) * scale
+
+
+def err(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+def split(ctx, x, bias=None):
+    """Planes [2, rows, K], their scale and {largest row sum of magnitudes, largest magnitude of the bias}."""
+    planes, scale, stats = torch.zeros(2, *x.shape, device=DEV).half(), torch.zeros(x.shape[0], device=DEV), torch.full((2, ), 7.0, device=DEV)
+    ctx.call("split_f16", x, x.shape[0], x.shape[1], planes[0], planes[1], scale, bias, 0 if bias is None else bias.numel(), stats)
+    return planes, scale, stats
+
+
+def value(planes, scale):
+    return (planes[0].double() + planes[1].double()) * scale.double()[:, None]
+
+
+def held(planes, scale, want, bound):
+    """Whether planes hold `want` to what they have bits for; bound: of a row's magnitudes, that the scale was made from."""
+    off = (value(planes, scale) - want.double()).abs()
+    return bool((off <= 2.0 ** -22 * want.double().abs() + 2.0 ** -39 * bound.double()[:, None]).all())
+
+
+@pytest.mark.parametrize("M,K", [(1, 1), (3, 77), (8, 768), (9, 3072), (1000, 40)])
+def test_planes(ctx, M, K):
+    x, bias = randn(M, K) * 2.0 ** torch.randint(-90, 90, (M, 1), generator=torch.Generator(device=DEV).manual_seed(2), device=DEV), randn(2 * M + 1, seed=3)
+    x[0, 0] = 0
+    planes, scale, stats = split(ctx, x, bias)
+    assert held(planes, scale, x, x.abs().amax(1))
+    assert torch.equal(torch.frexp(scale).mantissa, torch.full_like(scale, 0.5))  # powers of two
+    most = float(x.double().abs().sum(1).max())
+    assert abs(float(stats[0]) - most) <= 1e-5 * most and float(stats[1]) == float(bias.abs().max())
+    for odd in (float("nan"), float("inf"), 3.4e38):
+        y = x.clone()
+        y[-1, -1] = odd
+        planes, scale, _ = split(ctx, y)
+        assert bool(torch.isfinite(value(planes, scale)[-1, -1])) == (odd == 3.4e38) and held(planes[:, :-1], scale[:-1], x[:-1], x[:-1].abs().amax(1))
+    planes, scale, _ = split(ctx, torch.zeros(M, K, device=DEV))
+    assert not value(planes, scale).any()
+
+
+def product(ctx, a, w, N, K, epilogue, planes=False, **more):
+    M = a[1].numel()
+    fields = dict(A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], stats=w[2], **more)
+    if planes:
+        out, scale = torch.full((2, M, N), 7.0, device=DEV).half(), torch.zeros(M, device=DEV)
+        ctx.linear_split(M, N, K, epilogue, out=out[0], out_lo=out[1], out_scale=scale, **fields)
+        return out, scale
+    out = torch.full((M, N), 7.0, device=DEV)
+    ctx.linear_split(M, N, K, epilogue, out=out, **fields)
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 768, 768), (31, 2304, 768), (128, 768, 3072), (129, 3072, 768), (527, 100, 1024), (200, 65, 64), (1100, 3072, 768), (3000, 768, 768),
+                                   (5000, 2304, 768), (77, 770, 8)])
+def test_product(ctx, M, N, K):
+    x, w, bias, res = randn(M, K), randn(N, K, seed=2, scale=K ** -0.5), randn(N, seed=3), randn(M, N, seed=4)
+    a, b = split(ctx, x), split(ctx, w, bias)
+    exact = x.double() @ w.double().T
+    gelu = torch.nn.functional.gelu(exact + bias.double(), approximate="tanh")
+    tol = 1e-8 * K + 2e-6  # (tanh in fp32 for the second term)
+    assert err(product(ctx, a, b, N, K, _capi.EPI_NONE), exact) < 1e-8 * K + 3e-7
+    assert err(product(ctx, a, b, N, K, _capi.EPI_BIAS_RESIDUAL, bias=bias, residual=res), exact + bias.double() + res.double()) < tol
+    out = product(ctx, a, b, N, K, _capi.EPI_BIAS_GELU, bias=bias)
+    assert err(out, gelu) < tol
+    planes, scale = product(ctx, a, b, N, K, _capi.EPI_BIAS_GELU, planes=True, bias=bias)
+    bound = 32768 * a[1] * b[2][0] + b[2][1]
+    assert bool((gelu.abs() <= bound.double()[:, None]).all()) and held(planes, scale, value(planes, scale), bound)
+    assert err(value(planes, scale), gelu) < tol and bool((scale * 65504 >= bound).all())
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [5, 300])
+def test_product_over_the_range_of_scales(ctx, M):
+    """Rows and columns many powers of two apart, and a row's own elements too: every element is as close to its own terms as in tf32 planes, whose exponent is fp32's."""
+    N, K = 96, 256
+    powers = lambda n, most, seed: 2.0 ** torch.randint(-most, most, (n, 1), generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+    x, w = randn(M, K) * powers(M, 50, 5), randn(N, K, seed=2) * powers(N, 50, 6)
+    x, w = x * powers(K, 4, 7).T, w * powers(K, 4, 8).T
+    out = product(ctx, split(ctx, x), split(ctx, w), N, K, _capi.EPI_NONE)
+    terms = x.double().abs() @ w.double().abs().T
+    # of every term: both operands' planes, the product of the two second ones that is left out, and the accumulator
+    assert float(((out.double() - x.double() @ w.double().T).abs() / terms).max()) < 3 * 2.0 ** -22 + 1e-8 * K
+
+
+@pytest.mark.parametrize("M,N", [(1, 768), (37, 1024), (149, 768), (1184, 768), (1185, 768), (600, 776), (600, 2048), (1500, 264), (900, 8)])
+def test_layer_norm_leaves_the_planes_of_its_output(ctx, M, N):
+    out, y, bias, gamma, beta = randn(M, N), randn(M, N, seed=2), randn(N, seed=3), randn(N, seed=4), randn(N, seed=5)
+    want = torch.nn.functional.layer_norm((out + y + bias).double(), (N,), gamma.double(), beta.double(), 1e-12)
+    planes, scale = torch.zeros(2, M, N, device=DEV).half(), torch.zeros(M, device=DEV)
+    ctx.call("add_bias_layernorm_split", out, planes[0], planes[1], scale, y, bias, gamma, beta, M, N, 1e-12)
+    assert err(out, want) < 1e-6
+    again, s, _ = split(ctx, out)
+    assert torch.equal(planes, again) and torch.equal(scale, s)
+
+
+def test_embedding_leaves_the_planes_of_its_output(ctx):
+    for hidden in (768, 128, 1000):
+        ids, out = torch.randint(0, 100, (3, 7), generator=torch.Generator(device=DEV).manual_seed(1), device=DEV), torch.zeros(21, hidden, device=DEV)
+        planes, scale, plain = torch.zeros(2, 21, hidden, device=DEV).half(), torch.zeros(21, device=DEV), torch.zeros(21, hidden, device=DEV)
+        tables = (randn(100, hidden), randn(16, hidden, seed=2), randn(2, hidden, seed=3), randn(hidden, seed=4), randn(hidden, seed=5))
+        ctx.call("embedding_ln_split", ids, None, None, None, 3, 7, 21, *tables, hidden, 100, 16, 2, 1e-12, out, planes[0], planes[1], scale)
+        ctx.call("embedding_ln", _capi.F32, ids, None, None, None, 3, 7, 21, *tables, hidden, 100, 16, 2, 1e-12, plain)
+        again, s, _ = split(ctx, out)
+        assert torch.equal(out, plain) and torch.equal(planes, again) and torch.equal(scale, s)
+
+
+@pytest.mark.parametrize("lens", [[1], [7, 64, 33, 120], [65] * 30, [513, 3]])
+def test_attention_leaves_the_planes_of_its_output(ctx, lens):
+    T, H = sum(lens), 768
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+    rows, stats = randn(T, seed=2).abs() * 2.0 ** -12, torch.tensor([2.0, 3.0], device=DEV)
+    reach = 32768 * rows * stats[0] + stats[1]  # of a row's keys and values
+    qkv = (torch.rand(T, 3 * H, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV) * 2 - 1) * reach[:, None]
+    qkv[:, :2 * H] = randn(T, 2 * H, seed=4)
+    plain, planes, scale = torch.zeros(T, H, device=DEV), torch.zeros(2, T, H, device=DEV).half(), torch.zeros(T, device=DEV)
+    ctx.call("attention_f32", qkv, cu, len(lens), max(lens), 12, 64, None, 0, 0, 0, 0.125, plain, None)
+    ctx.call("attention_f32_split", qkv, cu, len(lens), max(lens), 12, 64, None, 0, 0, 0, 0.125, rows, stats, planes[0], planes[1], scale)
+    bound = torch.cat([reach[cu[b]:cu[b + 1]].max().expand(n) for b, n in enumerate(lens)])
+    assert held(planes, scale, plain, bound) and bool((scale * 65504 >= bound).all())
+
+
+def test_what_is_refused(ctx):
+    x = randn(16, 64)
+    a, w = split(ctx, x), split(ctx, randn(32, 64, seed=2), randn(32, seed=3))
+    out = torch.zeros(2, 16, 32, device=DEV).half()
+    for bad in (dict(A2=None), dict(row_scale=None), dict(col_scale=None), dict(lda=68), dict(K=60), dict(out_lo=out[1]), dict(W2=w[0][1].view(-1)[4:])):
+        fields = dict(dict(A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], out=out[0]), **bad)
+        with pytest.raises(_capi.TTBError):
+            ctx.linear_split(16, 32, fields.pop("K", 64), _capi.EPI_NONE, **fields)
+    with pytest.raises(_capi.TTBError):
+        ctx.call("add_bias_layernorm_split", x, a[0][0], a[0][1], a[1], x, x, x, x, 16, 60, 1e-12)
+    assert ctx.device_status() == 0

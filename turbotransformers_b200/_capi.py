@@ -26,6 +26,12 @@ class LinearArgs(C.Structure):
                 ("ldo", i64)]
 
 
+class LinearSplitArgs(C.Structure):
+    """ttb_linear_split_args of include/ttb.h."""
+    _fields_ = [(n, p) for n in ("A", "A2", "W", "W2", "row_scale", "col_scale", "bias", "residual", "stats", "out", "out_lo", "out_scale")] + [
+        (n, i64) for n in ("M", "N", "K", "lda", "ldr", "ldo")] + [("epilogue", i32)]
+
+
 class ChainLinear(C.Structure):
     """ttb_chain_linear of include/ttb.h."""
     _fields_ = [(n, p) for n in ("A", "W", "bias", "residual", "gamma", "beta", "normed", "out")] + \
@@ -110,6 +116,11 @@ SIGNATURES = {
     "ttb_linear_ex": (i32, [p, C.POINTER(LinearArgs)]),
     "ttb_linear_plan": (i32, [p, i32, i32, i32, i32, i32, i64, i64, i64, C.POINTER(i64)]),
     "ttb_split_tf32": (i32, [p, p, i64, p, p]),
+    "ttb_split_f16": (i32, [p, p, i64, i64, p, p, p, p, i64, p]),
+    "ttb_add_bias_layernorm_split": (i32, [p, p, p, p, p, p, p, p, p, i64, i64, f32]),
+    "ttb_embedding_ln_split": (i32, [p, p, p, p, p, i64, i64, i64, p, p, p, p, p, i64, i64, i64, i64, f32, p, p, p, p]),
+    "ttb_attention_f32_split": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p, p, p, p]),
+    "ttb_linear_split": (i32, [p, C.POINTER(LinearSplitArgs)]),
     "ttb_linear_layernorm": (i32, [p, i32, p, i64, p, p, p, i64, p, p, f32, i64, i64, i64, p, i64]),
     "ttb_prepack_weight_int8_affine": (i32, [p, i32, p, i32, i64, i64, p, p, p]),
     "ttb_quantize_tensor_affine": (i32, [p, i32, p, i64, i64, p, p]),
@@ -196,6 +207,13 @@ class Context:
         a = LinearArgs(dtype, out_dtype, ptr(A), ptr(A2), lda or K, ptr(W), ptr(W2), ptr(bias), ptr(residual), ldr or N, M, N, K,
                        epilogue, ptr(out), ptr(out_lo), ldo or N)
         self.check(lib().ttb_linear_ex(self.h, C.byref(a)))
+
+    def linear_split(self, M, N, K, epilogue, **fields):
+        """ttb_linear_split with the argument block filled from tensors by the fields' names."""
+        a = LinearSplitArgs(M=M, N=N, K=K, lda=K, ldr=N, ldo=N, epilogue=epilogue)
+        for name, value in fields.items():
+            setattr(a, name, value.data_ptr() if hasattr(value, "data_ptr") else value)
+        self.check(lib().ttb_linear_split(self.h, C.byref(a)))
 
     @staticmethod
     def _chain_block(ops):

@@ -42,11 +42,32 @@ std::vector<int64_t> WithLast(const Tensor& t, int64_t last) {
 // for the residual stream, an fp32 copy; see core::Tensor::lo() / f32().
 bool PreciseMode(int dt) { return dt == TTB_BF16 && core::PreciseBF16(); }
 
+bool Aligned16(std::initializer_list<const void*> ps) {
+  uintptr_t x = 0;
+  for (const void* p : ps) x |= reinterpret_cast<uintptr_t>(p);
+  return (x & 15) == 0;
+}
+
 // fp32 models on the tensor cores: an activation travels with the two planes that a product takes (core::Tensor::hi(), lo()), written by the
 // kernel that makes the activation; where nothing but a product reads it, it is the first plane itself and lo() the second. Both are
 // the planes of a rounding. With the activation as it is for the first, which the tensor cores truncate, the second would have 13 bits for 11
 // and always the activation's sign, so that what the accumulator cuts off a product no longer averages out: whole models 4 % less accurate.
 bool Fp32Planes(int dt) { return dt == TTB_F32 && core::Fp32TensorCores(); }
+// The same as two fp16 planes and a scale for each row, for products at twice the rate and half the bytes: where every width is a multiple of eight.
+struct SplitPlanes {
+  void *hi, *lo;
+  float* scale;
+};
+SplitPlanes NewSplit(Tensor* t, bool only) {
+  core::TensorExtras& ex = t->NewExtras();
+  ex.split_only = only;
+  SplitPlanes p;
+  p.hi = ex.hi.Reshape(core::kFloat16, ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/hi_plane");
+  p.lo = ex.lo.Reshape(core::kFloat16, ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/lo_plane");
+  p.scale = ex.split_scale.Reshape<float>({t->rows()}, kDLCUDA, t->device_id(), "fp32/planes_scale");
+  return p;
+}
+bool SplitWidth(int64_t n) { return n % 8 == 0 && n <= 2048; }  // of a layer norm that leaves planes
 float* NewLo(Tensor* t) { return t->NewExtras().lo.Reshape<float>(ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/lo_plane"); }
 void NewPlanes(Tensor* t, float** hi, float** lo) {
   core::TensorExtras& ex = t->NewExtras();
@@ -82,6 +103,12 @@ void LayerNormWithInt8(ttb_ctx* c, Tensor* t, const Tensor& gamma, const Tensor&
 void AddBiasLayerNormF32(ttb_ctx* c, Tensor* t, const Tensor& input, const Tensor& bias, const Tensor& gamma, const Tensor& beta, int64_t M, int64_t N,
                          const char* name) {
   float* out = t->mutableData<float>();
+  if (Fp32Planes(TTB_F32) && SplitWidth(N) && M > 0 && Aligned16({out, input.raw(), bias.raw(), gamma.raw(), beta.raw()})) {
+    const SplitPlanes p = NewSplit(t, false);
+    Check(ttb_add_bias_layernorm_split(c, out, p.hi, p.lo, p.scale, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
+          name);
+    return;
+  }
   float *hi = nullptr, *lo = nullptr;
   if (Fp32Planes(TTB_F32)) NewPlanes(t, &hi, &lo);
   Check(ttb_add_bias_layernorm_f32_planes(c, out, hi, lo, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
@@ -127,6 +154,24 @@ const float* PackedLinear::PackedTf32(bool is_trans) const {
     Check(ttb_split_tf32(c, planes, N * K, planes, planes + N * K), c, "split_tf32");
   }
   return p.data<float>();
+}
+
+PackedLinear::Split PackedLinear::PackedSplit(bool is_trans) const {
+  std::lock_guard<std::mutex> g(cache_->mu);
+  Tensor &planes = cache_->split[is_trans ? 1 : 0], &scale = cache_->split_scale[is_trans ? 1 : 0];
+  const int64_t K = in_dim(is_trans), N = out_dim(is_trans);
+  if (planes.is_null()) {
+    ttb_ctx* c = DeviceContext(weight_.device_id());
+    Tensor rows(nullptr);
+    float* w = rows.Reshape<float>({N, K}, kDLCUDA, weight_.device_id(), "linear/rows_of_weight");
+    Check(ttb_prepack_weight(c, TTB_F32, weight_.raw(), is_trans ? 1 : 0, K, N, TTB_F32, w), c, "prepack_weight");
+    float* s = scale.Reshape<float>({2 + (N + 3) / 4 * 4}, kDLCUDA, weight_.device_id(), "linear/split_weight_scales");
+    char* p = static_cast<char*>(planes.Reshape(core::kFloat16, {2, N, K}, kDLCUDA, weight_.device_id(), "linear/split_weight_planes"));
+    const bool bias = !bias_.is_null();
+    Check(ttb_split_f16(c, w, N, K, p, p + N * K * 2, s, bias ? bias_.data<float>() : nullptr, bias ? bias_.numel() : 0, s + (N + 3) / 4 * 4), c, "split_f16");
+  }
+  const char* p = static_cast<const char*>(planes.raw());
+  return {p, p + N * K * 2, scale.data<float>(), scale.data<float>() + (N + 3) / 4 * 4};
 }
 
 const float* PackedLinear::BiasF32() const {
@@ -194,7 +239,7 @@ void PackedLinear::ForwardLayerNorm(const Tensor& x, int64_t M, const void* resi
 }
 
 void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
-                           const char* name, int64_t ldo, void* out_lo, bool f32_out, Tensor* q8_of_out) const {
+                           const char* name, int64_t ldo, void* out_lo, bool f32_out, Tensor* q8_of_out, const SplitOut* split_out) const {
   const int dt = FloatType(x, name);
   SameTypeDevice(x, weight_, name);
   const int64_t K = in_dim(is_trans), N = out_dim(is_trans);
@@ -206,11 +251,33 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
   TT_ENFORCE(ldo == N || (dt != TTB_F32 && !use_int8()), "%s: a padded output pitch is only supported on the 16-bit path", name);
   TT_ENFORCE((!out_lo && !f32_out) || (dt == TTB_BF16 && !use_int8()) || (out_lo && Fp32Planes(dt) && K % 4 == 0),
              "%s: two-plane and fp32 outputs belong to the bf16 path, fp32 planes to the tensor cores", name);
+  if (dt == TTB_F32 && M > 0 && (x.split_only() || (core::Fp32TensorCores() && K % 8 == 0 && (x.split_scale() || !x.lo())))) {
+    // fp32 on the tensor cores: activation and weight as two fp16 planes each, three products accumulated in one GEMM with the elementwise kernel that followed
+    // MatMul in the reference as its epilogue (mat_mul.cpp:81-96 selects tensor-op math for the same product). An activation that brings its planes
+    // along is not split again.
+    const Split w = PackedSplit(is_trans);
+    ttb_linear_split_args args{};
+    Tensor planes(nullptr), scale(nullptr);
+    if (x.split_scale()) {
+      args.A = x.hi()->raw(); args.A2 = x.lo()->raw(); args.row_scale = x.split_scale()->data<float>();
+    } else {
+      char* a = static_cast<char*>(planes.Reshape(core::kFloat16, {2, M, K}, kDLCUDA, x.device_id(), "linear/split_activation_planes"));
+      float* s = scale.Reshape<float>({M}, kDLCUDA, x.device_id(), "linear/split_activation_scales");
+      Check(ttb_split_f16(c, x.data<float>(), M, K, a, a + M * K * 2, s, nullptr, 0, nullptr), c, name);
+      args.A = a; args.A2 = a + M * K * 2; args.row_scale = s;
+    }
+    args.W = w.hi; args.W2 = w.lo; args.col_scale = w.scale; args.stats = w.stats;
+    args.bias = static_cast<const float*>(bias); args.residual = static_cast<const float*>(residual);
+    args.out = split_out ? split_out->hi : out;
+    args.out_lo = split_out ? split_out->lo : nullptr;
+    args.out_scale = split_out ? split_out->scale : nullptr;
+    args.M = M; args.N = N; args.K = K; args.lda = K; args.ldr = N; args.ldo = N; args.epilogue = epilogue;
+    Check(ttb_linear_split(c, &args), c, name);
+    return;
+  }
+  TT_ENFORCE(!split_out && !x.split_only(), "%s: planes without a product that takes them", name);
   if (dt == TTB_F32 && (core::Fp32TensorCores() || (x.lo() && !x.hi())) && K % 4 == 0 && M > 0) {
-    // fp32 on the tensor cores: activations split into two tf32 planes, weights kept as two planes, three products
-    // accumulated in one GEMM with the elementwise kernel that followed MatMul in the reference as its epilogue
-    // (mat_mul.cpp:81-96 selects tensor-op math for the same product)
-    // (an activation that brings its planes along is not split again)
+    // the same with tf32 planes, for widths that are no multiple of eight
     Tensor planes(nullptr);
     const float* w = PackedTf32(is_trans);
     ttb_linear_args args{};
@@ -329,6 +396,15 @@ void BERTEmbedding::operator()(const Tensor& input_ids, const Tensor& position_i
     core::TensorExtras& ex = output_tensor->NewExtras();
     lo = ex.lo.Reshape(word_embedings_.dtype(), {B, L, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({B, L, H}, kDLCUDA, dev, "precise/residual_stream");
+  } else if (Fp32Planes(dt) && SplitWidth(H) && B * L > 0) {
+    const SplitPlanes p = NewSplit(output_tensor, false);
+    Check(ttb_embedding_ln_split(c, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
+                                 token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), nullptr, B, L, B * L, word_embedings_.data<float>(),
+                                 position_embeddings_.data<float>(), token_type_embeddings_.data<float>(), layer_norm_weights_.data<float>(),
+                                 layer_norm_bias_.data<float>(), H, word_embedings_.shape(0), position_embeddings_.shape(0), token_type_embeddings_.shape(0), 1e-12f,
+                                 static_cast<float*>(out), p.hi, p.lo, p.scale),
+          c, "BERTEmbedding");
+    return;
   } else if (Fp32Planes(dt)) {
     float* rest;
     NewPlanes(output_tensor, &f32, &rest);
@@ -360,6 +436,16 @@ void BERTEmbedding::Packed(const Tensor& input_ids, const std::vector<int64_t>& 
     core::TensorExtras& ex = output_tensor->NewExtras();
     lo = ex.lo.Reshape(word_embedings_.dtype(), {1, T, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({1, T, H}, kDLCUDA, dev, "precise/residual_stream");
+  } else if (Fp32Planes(dt) && SplitWidth(H) && T > 0) {
+    const SplitPlanes p = NewSplit(output_tensor, false);
+    const core::CuSeqlensHandle cu = core::CuSeqlens(dev, seq_lens);
+    Check(ttb_embedding_ln_split(c, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
+                                 token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), cu.get(), (int64_t)seq_lens.size(), 0, T,
+                                 word_embedings_.data<float>(), position_embeddings_.data<float>(), token_type_embeddings_.data<float>(),
+                                 layer_norm_weights_.data<float>(), layer_norm_bias_.data<float>(), H, word_embedings_.shape(0), position_embeddings_.shape(0),
+                                 token_type_embeddings_.shape(0), 1e-12f, static_cast<float*>(out), p.hi, p.lo, p.scale),
+          c, "BERTEmbedding/packed");
+    return;
   } else if (Fp32Planes(dt)) {
     float* rest;
     NewPlanes(output_tensor, &f32, &rest);
@@ -586,7 +672,13 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
   } else if (Fp32Planes(dt) && !att_score && !cache_keys && d == 64 && B <= 65535 && (!causal_ || !attention_mask.is_null())) {
     // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own (a causal layer's
     // mask tensor says what its rows see, as it does in the sequence below; the kernel's own causal form is the C call's)
-    Tensor qkv(nullptr);
+    Tensor qkv(nullptr), planes_in(nullptr);
+    if (!gemm_in->lo() && T > 0) {  // planes here, so that the attention kernel knows what bounds the values whether the input brought its own or not
+      planes_in.Reshape(x.dtype(), {T, H}, kDLCUDA, dev, "self/planes_in");
+      const SplitPlanes p = NewSplit(&planes_in, true);
+      Check(ttb_split_f16(c, gemm_in->data<float>(), T, H, p.hi, p.lo, p.scale, nullptr, 0, nullptr), c, "self/split_f16");
+      gemm_in = &planes_in;
+    }
     qkv.Reshape(x.dtype(), {T, 3 * H}, kDLCUDA, dev, "self/qkv_out1/Reshape");
     qkv_.Forward(*gemm_in, T, TTB_EPI_BIAS, nullptr, qkv.raw_mut(), is_trans_weight, "self/gemm012_fused");
     const core::CuSeqlensHandle cu_handle = seq_lens ? core::CuSeqlens(dev, *seq_lens) : core::UniformCuSeqlens(dev, B, maxL);
@@ -600,9 +692,16 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
       if (MaskIs2D(attention_mask)) { mbs = maxL; mrs = 0; }
       else { mrs = maxL; mbs = maxL * maxL; }
     }
-    float* hi = context.mutableData<float>();
-    float* lo = NewLo(&context);
-    Check(ttb_attention_f32_planes(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, hi, lo), c, "attention_f32");
+    if (gemm_in->split_scale() && T > 0) {  // the output as fp16 planes, within the bound that the product's operands give for the values
+      const SplitPlanes p = NewSplit(&context, true);
+      Check(ttb_attention_f32_split(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, gemm_in->split_scale()->data<float>(),
+                                    qkv_.PackedSplit(is_trans_weight).stats, p.hi, p.lo, p.scale),
+            c, "attention_f32");
+    } else {
+      float* hi = context.mutableData<float>();
+      float* lo = NewLo(&context);
+      Check(ttb_attention_f32_planes(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, hi, lo), c, "attention_f32");
+    }
   } else {
     // The reference's own sequence (multi_headed_attention.cpp:168-232,320-354), scores materialised.
     TT_ENFORCE(!cache_keys, "layer_cache decoding is provided for 16-bit models with 64-wide heads");
@@ -863,6 +962,12 @@ void BertIntermediate::Run(const Tensor& input_tensor, Tensor* output_tensor, bo
   output_tensor->Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "BertIntermediate/Reshape");
   void* out = output_tensor->raw_mut();
   void* lo = nullptr;
+  if (for_output && Fp32Planes(dt) && input_tensor.split_scale() && dense_.out_dim(false) % 8 == 0 && input_tensor.rows() > 0) {
+    const SplitPlanes p = NewSplit(output_tensor, true);
+    const PackedLinear::SplitOut split{p.hi, p.lo, p.scale};
+    dense_.Forward(input_tensor, input_tensor.rows(), TTB_EPI_BIAS_GELU, nullptr, out, false, "BertIntermediate", 0, nullptr, false, nullptr, &split);
+    return;
+  }
   if (for_output && Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0 && dense_.out_dim(false) % 4 == 0) lo = NewLo(output_tensor);
   else if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came
     lo = output_tensor->NewExtras().lo.Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "precise/lo_plane");

@@ -34,6 +34,17 @@ class PackedLinear {
   const void* Packed(bool is_trans) const;
   // fp32 weights as two tf32 planes [2][N,K] (hi, then lo), for the three-product tensor-core GEMM.
   const float* PackedTf32(bool is_trans) const;
+  // fp32 weights as two fp16 planes [N,K] with a scale for each row, and {largest sum of magnitudes of a row, largest magnitude of the bias} (ttb_split_f16).
+  struct Split {
+    const void *hi, *lo;
+    const float *scale, *stats;
+  };
+  Split PackedSplit(bool is_trans) const;
+  // An output as fp16 planes with a scale for each row.
+  struct SplitOut {
+    void *hi, *lo;
+    float* scale;
+  };
   // int8 [N,K] copy + device scale (built on first use); `col_sum` (may be null) selects the reference recipe's
   // quantiser (torch's per-tensor rule) and receives the per-output-row sums its zero-point correction needs.
   void Int8(bool is_trans, const int8_t** wq, const float** scale, const int32_t** col_sum = nullptr) const;
@@ -57,7 +68,8 @@ class PackedLinear {
                         void* out, bool is_trans, const char* name) const;
   // q8_of_out (per-row int8 mode): the tensor that owns `out`; it gets the int8 form of the output attached (q8(), q8_scale()).
   void Forward(const core::Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
-               const char* name, int64_t ldo = 0, void* out_lo = nullptr, bool f32_out = false, core::Tensor* q8_of_out = nullptr) const;
+               const char* name, int64_t ldo = 0, void* out_lo = nullptr, bool f32_out = false, core::Tensor* q8_of_out = nullptr,
+               const SplitOut* split_out = nullptr) const;
 
  private:
   core::Tensor weight_, bias_;
@@ -66,6 +78,8 @@ class PackedLinear {
     std::mutex mu;
     core::Tensor packed[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor tf32[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
+    core::Tensor split[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
+    core::Tensor split_scale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor q[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qscale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qref[2]{core::Tensor(nullptr), core::Tensor(nullptr)};

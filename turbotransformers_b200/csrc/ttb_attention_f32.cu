@@ -22,11 +22,21 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 template <int R> constexpr int kSmem = (2 * 8 * R + 2 * kKeys) * kPitch * 4;
 
-// ROUNDED: the output leaves as its two planes, in place of it. (As a choice at run time it cost 15 registers and 1.2 us of 18 at 527 rows.)
-template <int R, bool ROUNDED>
+// What the planes of the output in fp16 take: of the rows that the queries, keys and values were computed from, what they were divided by, and the weights'
+// statistics (ttb_split_f16), which bound the values and so their averages; the planes' own scale.
+struct SplitOut {
+  const float *row_scale, *stats;
+  __half *hi, *lo;
+  float* scale;
+};
+enum { OUT_VALUE = 0, OUT_TF32 = 1, OUT_F16 = 2 };
+
+// OUT: the output leaves as it is, or as its two planes, in place of it. (As a choice at run time it cost 15 registers and 1.2 us of 18 at 527 rows.)
+template <int R, int OUT>
 __global__ void __launch_bounds__(kThreads)
 attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ cu, int heads, const float* __restrict__ mask, long long mask_batch,
-                     long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo) {
+                     long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo, const SplitOut split) {
+  constexpr bool ROUNDED = OUT == OUT_TF32;
   constexpr int kRows = 8 * R;
   extern __shared__ __align__(16) float smem[];
   float *qs = smem, *ps = qs + kRows * kPitch, *ks = ps + kRows * kPitch, *vs = ks + kKeys * kPitch;
@@ -140,6 +150,13 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
     }
     __syncwarp();
   }
+  float up = 1.f;
+  if constexpr (OUT == OUT_F16) {  // one scale for all heads and rows of the sequence: no value of it is beyond this bound
+    float most = 0.f;
+    for (int j = tid & 31; j < len; j += 32) most = fmaxf(most, split.row_scale[begin + j]);
+    const float down = f16_planes_scale(warp_max(most) * 32768.f * split.stats[0] + split.stats[1], &up);
+    if (h == 0 && tid < kRows && q0 + tid < len) split.scale[begin + q0 + tid] = down;
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     float sum = l[r];
@@ -150,38 +167,51 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
     const float inv = 1.0f / sum;
     const float4 y = make_float4(acc[r][0] * inv, acc[r][1] * inv, acc[r][2] * inv, acc[r][3] * inv);
     const long long at = (long long)(begin + i) * H + h * D + kg * 4;
+    if constexpr (OUT == OUT_F16) {
+      const float v[4] = {y.x * up, y.y * up, y.z * up, y.w * up};
+      __half2 hi[2], lo[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        hi[e] = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+        const float2 f = __half22float2(hi[e]);
+        lo[e] = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
+      }
+      *reinterpret_cast<uint2*>(split.hi + at) = *reinterpret_cast<const uint2*>(hi);
+      *reinterpret_cast<uint2*>(split.lo + at) = *reinterpret_cast<const uint2*>(lo);
+      continue;
+    }
     *reinterpret_cast<float4*>(out + at) = ROUNDED ? make_float4(tf32_hi(y.x), tf32_hi(y.y), tf32_hi(y.z), tf32_hi(y.w)) : y;
     if (ROUNDED || out_lo) *reinterpret_cast<float4*>(out_lo + at) = make_float4(tf32_lo(y.x, ROUNDED), tf32_lo(y.y, ROUNDED), tf32_lo(y.z, ROUNDED), tf32_lo(y.w, ROUNDED));
   }
 }
 
-template <int R, bool ROUNDED>
+template <int R, int OUT>
 cudaError_t launch_f32(ttb_ctx* ctx, dim3 grid, const float* qkv, const int32_t* cu, int heads, const float* mask, int64_t mbs, int64_t mrs, int causal, float scale,
-                       float* out, float* out_lo) {
-  cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<R, ROUNDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<R>);
+                       float* out, float* out_lo, const SplitOut& split) {
+  cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<R, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<R>);
   if (e != cudaSuccess) return e;
-  return launch_pdl(attention_f32_kernel<R, ROUNDED>, grid, dim3(kThreads), (size_t)kSmem<R>, ctx->stream, qkv, cu, heads, mask, (long long)mbs, (long long)mrs, causal, scale, out,
-                    out_lo);
+  return launch_pdl(attention_f32_kernel<R, OUT>, grid, dim3(kThreads), (size_t)kSmem<R>, ctx->stream, qkv, cu, heads, mask, (long long)mbs, (long long)mrs, causal, scale, out,
+                    out_lo, split);
 }
 
-template <bool ROUNDED>
+template <int OUT>
 int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
-                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
+                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo, const SplitOut& split = SplitOut()) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, d == D && heads > 0 && heads <= 65535 && B >= 0 && B <= 65535 && max_seqlen >= 0 && max_seqlen < (1 << 30), "attention_f32: bad shape");
   if (B == 0 || max_seqlen == 0) return TTB_OK;
-  TTB_REQUIRE(ctx, qkv && cu_seqlens && out, "attention_f32: null pointer");
+  TTB_REQUIRE(ctx, qkv && cu_seqlens && (out || OUT == OUT_F16), "attention_f32: null pointer");
   TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo)) & 15) == 0,
               "attention_f32: buffers must be 16-byte aligned");
   DeviceGuard g(ctx->device);
   // 32 rows a CTA read a tile of keys half as often as 16; with few (sequence, head, rows) the chip has room for twice the CTAs
   const int64_t ctas = B * heads * ((max_seqlen + 31) / 32);
   if (ctas >= 2 * ctx->sm_count)
-    TTB_CUDA(ctx, (launch_f32<4, ROUNDED>(ctx, dim3((unsigned)((max_seqlen + 31) / 32), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo)));
+    TTB_CUDA(ctx, (launch_f32<4, OUT>(ctx, dim3((unsigned)((max_seqlen + 31) / 32), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
+                                causal, scale, out, out_lo, split)));
   else
-    TTB_CUDA(ctx, (launch_f32<2, ROUNDED>(ctx, dim3((unsigned)((max_seqlen + 15) / 16), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo)));
+    TTB_CUDA(ctx, (launch_f32<2, OUT>(ctx, dim3((unsigned)((max_seqlen + 15) / 16), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
+                                causal, scale, out, out_lo, split)));
   return launched(ctx, "attention_f32");
 }
 
@@ -189,11 +219,21 @@ int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int
 
 extern "C" int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
                                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
-  return attention_f32<false>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, out, out_lo);
+  return attention_f32<OUT_VALUE>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, out, out_lo);
 }
 
 extern "C" int ttb_attention_f32_planes(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
                                         const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* hi, float* lo) {
   if (ctx && B > 0 && max_seqlen > 0) TTB_REQUIRE(ctx, lo, "attention_f32_planes: null pointer");
-  return attention_f32<true>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, hi, lo);
+  return attention_f32<OUT_TF32>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, hi, lo);
+}
+
+extern "C" int ttb_attention_f32_split(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
+                                       const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, const float* row_scale,
+                                       const float* stats, void* hi, void* lo, float* out_scale) {
+  if (ctx && B > 0 && max_seqlen > 0)
+    TTB_REQUIRE(ctx, row_scale && stats && hi && lo && out_scale && ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 7) == 0,
+                "attention_f32_split: null or misaligned pointer");
+  return attention_f32<OUT_F16>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, nullptr, nullptr,
+                                SplitOut{row_scale, stats, static_cast<__half*>(hi), static_cast<__half*>(lo), out_scale});
 }

@@ -168,6 +168,26 @@ __device__ __forceinline__ float tf32_lo(float x, bool rounded) {
 template <typename T> __device__ __forceinline__ float rest_of(float v, bool) { return v - to_f(from_f<T>(v)); }
 template <> __device__ __forceinline__ float rest_of<float>(float v, bool rounded) { return tf32_lo(v, rounded); }
 
+// An fp32 matrix as two fp16 planes: a row is multiplied by the power of two `up` that brings `most`, a bound of its magnitudes, into [2^14, 2^15);
+// hi is that rounded to fp16, lo what the rounding dropped, rounded likewise: together 2^-23 of an element off at most, like two tf32 planes, or
+// 2^-40 of `most` where that is more (lo is then among fp16's subnormal numbers). Returns the inverse of `up`. (No bound, or none that is a number: 1.)
+__device__ __forceinline__ float f16_planes_scale(float most, float* up) {
+  const int e = (int)((__float_as_uint(most) >> 23) & 255);        // the biased exponent
+  const int d = (e == 0 || e == 255) ? 0 : max(-112, min(113, e - 127 - 14));
+  *up = __uint_as_float((uint32_t)(127 - d) << 23);
+  return __uint_as_float((uint32_t)(127 + d) << 23);
+}
+__device__ __forceinline__ void f16_planes8(const float* v, float up, uint4* hi, uint4* lo) {
+  __half2 *h = reinterpret_cast<__half2*>(hi), *l = reinterpret_cast<__half2*>(lo);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = v[2 * i] * up, b = v[2 * i + 1] * up;
+    h[i] = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h[i]);
+    l[i] = __floats2half2_rn(a - f.x, b - f.y);
+  }
+}
+
 // A group of 8 consecutive elements moved with 16-byte (or 2x16-byte for fp32) accesses.
 template <typename T> struct Vec8 {
   float v[8];

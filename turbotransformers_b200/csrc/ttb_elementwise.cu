@@ -30,12 +30,13 @@ constexpr int kLnRows = 2;
 
 // EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
 // same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
-// other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099).
+// other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099);
+// 4, fp32 with its two fp16 planes (ttb_split_f16; out_f32 and out_lo are those) and out_scale.
 template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
                       const TOut* __restrict__ beta, TOut* out, TOut* __restrict__ out_lo, float* __restrict__ out_f32, int64_t M, int N,
-                      float eps) {
+                      float eps, float* __restrict__ out_scale) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -87,6 +88,46 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
     float rstd[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) rstd[r] = rsqrtf(warp_sum(sq[r]) / (float)N + eps);
+    if constexpr (EXTRA == 4) {  // the planes' scale is known when all of the row is
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int64_t row = row0 + r;
+        if (row >= M) continue;
+        float top = 0.f;
+#pragma unroll
+        for (int it = 0; it < ITERS; ++it) {
+          const int col = (it * 32 + lane) * 8;
+          if (col < N) {
+            Vec8<TOut> g, b;
+            g.load(gamma + col);
+            b.load(beta + col);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              v[r][it][j] = b.v[j] + g.v[j] * rstd[r] * (v[r][it][j] - mean[r]);
+              top = fmaxf(top, fabsf(v[r][it][j]));
+            }
+          }
+        }
+        float up;
+        const float down = f16_planes_scale(warp_max(top), &up);
+        if (lane == 0) out_scale[row] = down;
+#pragma unroll
+        for (int it = 0; it < ITERS; ++it) {
+          const int col = (it * 32 + lane) * 8;
+          if (col < N) {
+            Vec8<TOut> o;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o.v[j] = v[r][it][j];
+            o.store(out + row * N + col);
+            uint4 h, l;
+            f16_planes8(v[r][it], up, &h, &l);
+            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out_f32) + row * N + col) = h;
+            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out_lo) + row * N + col) = l;
+          }
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int col = (it * 32 + lane) * 8;
@@ -496,6 +537,29 @@ layernorm_rows_generic_kernel(const TIn* x, const TIn* __restrict__ residual, co
   }
 }
 
+// out = LN(x + residual + bias) in fp32, with its two fp16 planes and their scales. N % 8 == 0, N <= 2048, 16-byte aligned rows: what a product takes.
+int launch_layernorm_split(ttb_ctx* ctx, const float* x, const float* residual, const float* bias, const float* gamma, const float* beta, float* out, __half* hi,
+                           __half* lo, float* scale, int64_t M, int64_t N, float eps) {
+  const bool few = M <= 8 * (int64_t)ctx->sm_count;  // (see launch_layernorm)
+  const int few_grid = (int)((M + 1) / 2), grid = grid_for((M + kLnRows - 1) / kLnRows, kLnWarps, ctx->sm_count);
+#define LN_SPLIT(IT)                                                                                                                                      \
+  do {                                                                                                                                                    \
+    if (few)                                                                                                                                              \
+      launch_pdl(layernorm_rows_kernel<float, float, IT, true, 4, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, out,     \
+                 reinterpret_cast<float*>(lo), reinterpret_cast<float*>(hi), M, (int)N, eps, scale);                                                       \
+    else                                                                                                                                                  \
+      launch_pdl(layernorm_rows_kernel<float, float, IT, true, 4, kLnWarps, 1>, dim3(2 * grid), dim3(kLnWarps * 32), 0, ctx->stream, x, residual, bias, gamma, \
+                 beta, out, reinterpret_cast<float*>(lo), reinterpret_cast<float*>(hi), M, (int)N, eps, scale);                                            \
+  } while (0)
+  if (N <= 256) LN_SPLIT(1);
+  else if (N <= 512) LN_SPLIT(2);
+  else if (N <= 768) LN_SPLIT(3);
+  else if (N <= 1024) LN_SPLIT(4);
+  else LN_SPLIT(8);
+#undef LN_SPLIT
+  return launched(ctx, "layernorm_split");
+}
+
 template <typename TIn, typename TOut, bool ADD>
 int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut* bias, const TOut* gamma, const TOut* beta, TOut* out,
                      TOut* out_lo, float* out_f32, int64_t M, int64_t N, float eps) {
@@ -515,25 +579,25 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   do {                                                                                                                           \
     if (few && traded)                                                                                                           \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else if (few && planes)                                                                                                      \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else if (planes)                                                                                                             \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else if (few && extra)                                                                                                       \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else if (few)                                                                                                                \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else if (extra)                                                                                                              \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
     else                                                                                                                         \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
   } while (0)
   const bool aligned = (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo) |
                                          reinterpret_cast<uintptr_t>(out_f32) | reinterpret_cast<uintptr_t>(gamma) |
@@ -737,7 +801,7 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
                     int64_t n_tokens, const T* __restrict__ word, const T* __restrict__ position,
                     const T* __restrict__ token_type, const T* __restrict__ gamma, const T* __restrict__ beta,
                     int hidden, int64_t vocab, int64_t n_pos, int64_t n_types, float eps, T* __restrict__ out,
-                    T* __restrict__ out_lo, float* __restrict__ out_f32, int* status) {
+                    T* __restrict__ out_lo, float* __restrict__ out_f32, float* __restrict__ out_scale, int* status) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -764,6 +828,26 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
     float sq = 0.f;
     for (int c = lane; c < hidden; c += 32) { float d = val(c) - mean; sq += d * d; }
     const float rstd = rsqrtf(warp_sum(sq) / (float)hidden + eps);
+    if (std::is_same<T, float>::value && out_scale) {  // fp16 planes and their scale, which is known when all of the row is
+      float top = 0.f;
+#pragma unroll 4
+      for (int c = lane; c < hidden; c += 32) {
+        const float y = to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean);
+        out[t * hidden + c] = from_f<T>(y);
+        top = fmaxf(top, fabsf(y));
+      }
+      float up;
+      const float down = f16_planes_scale(warp_max(top), &up);
+      if (lane == 0) out_scale[t] = down;
+#pragma unroll 4
+      for (int c = lane; c < hidden; c += 32) {
+        const float y = (to_f(beta[c]) + to_f(gamma[c]) * rstd * (val(c) - mean)) * up;
+        const __half h = __float2half_rn(y);
+        reinterpret_cast<__half*>(out_f32)[t * hidden + c] = h;
+        reinterpret_cast<__half*>(out_lo)[t * hidden + c] = __float2half_rn(y - __half2float(h));
+      }
+      continue;
+    }
     if (std::is_same<T, float>::value && out_f32 && out_lo) {  // (a loop of its own: stores under conditions keep the loads from going ahead)
 #pragma unroll 4
       for (int c = lane; c < hidden; c += 32) {
@@ -1372,6 +1456,21 @@ extern "C" int ttb_add_bias_layernorm_f32_planes(ttb_ctx* ctx, float* out, float
   return add_bias_layernorm_f32(ctx, out, hi, lo, input, bias, gamma, beta, M, N, eps);
 }
 
+extern "C" int ttb_add_bias_layernorm_split(ttb_ctx* ctx, float* out, void* hi, void* lo, float* scale, const float* input, const float* bias, const float* gamma,
+                                            const float* beta, int64_t M, int64_t N, float eps) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, M >= 0 && N > 0 && N % 8 == 0 && N <= 2048, "add_bias_layernorm_split: bad shape M=%lld N=%lld", (long long)M, (long long)N);
+  if (M == 0) return TTB_OK;
+  uintptr_t all = 0;
+  for (const void* q : {(const void*)out, (const void*)hi, (const void*)lo, (const void*)input, (const void*)bias, (const void*)gamma, (const void*)beta}) {
+    TTB_REQUIRE(ctx, q, "add_bias_layernorm_split: null pointer");
+    all |= reinterpret_cast<uintptr_t>(q);
+  }
+  TTB_REQUIRE(ctx, scale && (all & 15) == 0, "add_bias_layernorm_split: null or misaligned pointer");
+  DeviceGuard g(ctx->device);
+  return launch_layernorm_split(ctx, out, input, bias, gamma, beta, out, (__half*)hi, (__half*)lo, scale, M, N, eps);
+}
+
 extern "C" int ttb_layernorm(ttb_ctx* ctx, int dtype, const void* in, void* out, const void* gamma, const void* beta,
                              int64_t M, int64_t N, float eps) {
   if (!ctx) return TTB_ERR_INVALID;
@@ -1489,11 +1588,11 @@ extern "C" int ttb_embedding_ln(ttb_ctx* ctx, int dtype, const int64_t* ids, con
                                  gamma, beta, hidden, vocab, n_positions, n_types, eps, out, nullptr, nullptr);
 }
 
-extern "C" int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64_t* position_ids,
+static int embedding_ln(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64_t* position_ids,
                                        const int64_t* token_type_ids, const int32_t* cu_seqlens, int64_t B, int64_t seq_len,
                                        int64_t n_tokens, const void* word, const void* position, const void* token_type,
                                        const void* gamma, const void* beta, int64_t hidden, int64_t vocab, int64_t n_positions,
-                                       int64_t n_types, float eps, void* out, void* out_lo, float* out_f32) {
+                                       int64_t n_types, float eps, void* out, void* out_lo, float* out_f32, float* out_scale) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, n_tokens >= 0 && hidden > 0 && vocab > 0 && n_positions > 0 && n_types > 0, "embedding_ln: bad shape");
   if (n_tokens == 0) return TTB_OK;
@@ -1527,8 +1626,26 @@ extern "C" int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* i
                      (launch_pdl(embedding_ln_kernel<T>, dim3(grid), dim3(kRowsPerBlock * 32), 0, ctx->stream, 
                          ids, position_ids, token_type_ids, cu_seqlens, (int)B, (int)(seq_len > 0 ? seq_len : 1), n_tokens,
                          (const T*)word, (const T*)position, (const T*)token_type, (const T*)gamma, (const T*)beta,
-                         (int)hidden, vocab, n_positions, n_types, eps, (T*)out, (T*)out_lo, out_f32, ctx->d_status)));
+                         (int)hidden, vocab, n_positions, n_types, eps, (T*)out, (T*)out_lo, out_f32, out_scale, ctx->d_status)));
   return launched(ctx, "embedding_ln");
+}
+
+extern "C" int ttb_embedding_ln_planes(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64_t* position_ids,
+                                       const int64_t* token_type_ids, const int32_t* cu_seqlens, int64_t B, int64_t seq_len,
+                                       int64_t n_tokens, const void* word, const void* position, const void* token_type,
+                                       const void* gamma, const void* beta, int64_t hidden, int64_t vocab, int64_t n_positions,
+                                       int64_t n_types, float eps, void* out, void* out_lo, float* out_f32) {
+  return embedding_ln(ctx, dtype, ids, position_ids, token_type_ids, cu_seqlens, B, seq_len, n_tokens, word, position, token_type, gamma, beta, hidden, vocab, n_positions,
+                      n_types, eps, out, out_lo, out_f32, nullptr);
+}
+
+extern "C" int ttb_embedding_ln_split(ttb_ctx* ctx, const int64_t* ids, const int64_t* position_ids, const int64_t* token_type_ids, const int32_t* cu_seqlens,
+                                      int64_t B, int64_t seq_len, int64_t n_tokens, const float* word, const float* position, const float* token_type,
+                                      const float* gamma, const float* beta, int64_t hidden, int64_t vocab, int64_t n_positions, int64_t n_types, float eps,
+                                      float* out, void* hi, void* lo, float* scale) {
+  if (ctx && n_tokens > 0) TTB_REQUIRE(ctx, hi && lo && scale, "embedding_ln_split: null pointer");
+  return embedding_ln(ctx, TTB_F32, ids, position_ids, token_type_ids, cu_seqlens, B, seq_len, n_tokens, word, position, token_type, gamma, beta, hidden, vocab,
+                      n_positions, n_types, eps, out, lo, static_cast<float*>(hi), scale);
 }
 
 extern "C" int ttb_seq_pool(ttb_ctx* ctx, int dtype, const void* in, int64_t B, int64_t L, int64_t H, int pool_type,

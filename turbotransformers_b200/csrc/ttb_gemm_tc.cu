@@ -17,6 +17,11 @@
 // of two A maps and of two W maps. That is how operands wider than the tensor core's formats are used at full accuracy:
 //   bf16 activations kept as hi + lo planes :  A_hi.W + A_lo.W                       (2 passes)
 //   fp32 as three tf32 products             :  A_hi.W_hi + A_lo.W_hi + A_hi.W_lo     (3 passes)
+//   fp32 as three fp16 products             :  the same, of rows that are scaled into fp16's range; the epilogue takes the scales out again
+// fp16 planes hold as many bits as tf32 ones (an element to 2^-23, or to 2^-40 of its row's largest) at half the bytes and twice the rate, and a sum is
+// half as many instructions, each of which truncates it: us, tf32 / fp16 planes, and error against 64 bits: 128 x 2304 x 768 11.6 / 10.2, 527 x 768 x 3072 33.8 /
+// 19.6, 1.1e-5 / 5.6e-6; 3000 x 2304 x 768 44.7 / 27.7, 2.8e-6 / 1.5e-6; 3000 x 768 x 3072 63.1 / 32.1. (128 x 768 x 768 9.5 / 10.2, 8.3e-7 / 1.5e-6: there
+// is less to split along K.) BERT-base fp32: 1 x 128 1085 -> 941, 7.5e-6 -> 4.8e-6; 8 ragged requests 1748 -> 1277, 1.7e-5 -> 8.6e-6.
 // Products of few tiles with a long K are split along K over the CTAs of a cluster: every CTA accumulates its K range
 // in its own TMEM, the others hand their partial tile to the first CTA through distributed shared memory, and that CTA
 // adds them in rank order and runs the epilogue, so the result does not depend on timing.
@@ -84,9 +89,10 @@ enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
 // columns, bound by the MMAs, run the products as passes over K: with slots twice the size they have too few of them (bf16
 // 9000 x 2304 x 768 50.6 us in passes, 60.1 from shared slots).
 template <int BN, bool TWO, int KIND, typename OutT, int VAR> struct Planes {
-  static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR == 1)));
+  static constexpr bool split = KIND == KIND_F16 && VAR >= 5;  // VAR_SPLIT, VAR_SPLIT_PLANES
+  static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || split || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR == 1)));
   static constexpr int A = shared ? 2 : 1;
-  static constexpr int B = (shared && KIND == KIND_TF32) ? 2 : 1;
+  static constexpr int B = (shared && (KIND == KIND_TF32 || split)) ? 2 : 1;
 };
 
 struct GemmParams {
@@ -100,7 +106,10 @@ struct GemmParams {
   const void* bias;        // OutT[N] or null
   const void* residual;    // OutT[M, ldr] or null
   long long ldr;
-  const float* row_scale;  // int8, symmetric: per-row activation scale
+  const float* row_scale;  // int8, symmetric: per-row activation scale; fp32 as fp16 planes: what a row of them was divided by
+  const float* col_scale;  // fp32 as fp16 planes: the same of W's rows
+  const float* stats;      // planes out: {largest sum of magnitudes of a row of W, largest magnitude of the bias}
+  float* out_scale;        // planes out: [M], what a row of them was divided by
   const float* w_scale;    // int8: device scalar, weight scale
   const float* act_qparams;  // int8, affine per tensor: device [scale, zero point]; null selects the symmetric form
   const int* col_sum;        // int8, affine: sum over k of Wq[n, k]
@@ -188,7 +197,8 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 //   VAR_PLAIN, VAR_TWO_PLANES (output written with a second plane, what a product drops of the first), VAR_TF32_PLANES (fp32 output rounded to tf32, and
 //   what that dropped; as a choice at run time of the one before, 3 us of 30 at 527 x 3072 x 768), VAR_AFFINE (int8 with a per-tensor zero point),
 //   VAR_WORDS (STORE_WORDS; carried by every kernel it cost packed fp16 batches 1 %: 4120 -> 4164 us, 4149 against 4159 without)
-enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3, VAR_TF32_PLANES = 4 };
+//   VAR_SPLIT, VAR_SPLIT_PLANES (operands are fp32 as two scaled fp16 planes; the output is fp32, or such planes again)
+enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3, VAR_TF32_PLANES = 4, VAR_SPLIT = 5, VAR_SPLIT_PLANES = 6 };
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR, bool LN = false>
 __global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
@@ -416,6 +426,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     const int zero_point = affine ? (int)p.act_qparams[1] : 0;
     constexpr bool rounded = (VAR == VAR_TF32_PLANES), two_planes = (VAR == VAR_TWO_PLANES) || rounded;
     static_assert(!rounded || EB == 4, "planes as tf32 are fp32 words");
+    constexpr bool split = P::split, planes16 = VAR == VAR_SPLIT_PLANES;  // the latter's tiles leave from registers: a row's 32 columns are 64 bytes of each plane
+    static_assert(!split || EB == 4, "computed in fp32");
     const bool vec_ok = (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                         ((reinterpret_cast<uintptr_t>(p.out_lo) & 15) == 0) &&
                         (!bias || (reinterpret_cast<uintptr_t>(bias) & 15) == 0) &&
@@ -630,6 +642,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       uint4 bias_q[QN], res_q[QN];
       const bool fetched = BN == 32 && half == 0 && vec_ok && row < p.M && n_blk * BN + 32 <= p.N && !(SK && rank != 0);
       if (fetched) {
+        if (split) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col_scale + n_blk * BN));  // (registers for them are not left)
         if (p.epilogue != TTB_EPI_NONE) {
           const uint4* bp = reinterpret_cast<const uint4*>(bias + n_blk * BN);
 #pragma unroll
@@ -641,12 +654,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
           for (int i = 0; i < QN; ++i) res_q[i] = rp[i];
         }
       }
-      const float rs = (KIND != KIND_I8) ? 1.0f : (affine ? act_scale * w_scale : (row < p.M ? p.row_scale[row] * w_scale : 1.0f));
+      const float rs = split ? (row < p.M ? p.row_scale[row] : 1.0f) : (KIND != KIND_I8) ? 1.0f : (affine ? act_scale * w_scale : (row < p.M ? p.row_scale[row] * w_scale : 1.0f));
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) break;
       tc_fence_after();
       if (!SK) prefetch_residual(tile + tile_step);  // the next tile's rows, a whole mainloop ahead
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * C::ISSUERS * BN);
-      if (use_tma || half == 1) {
+      if (use_tma || (half == 1 && !(planes16 && BN >= 64))) {
         if (!staged_work) {  // nothing to do for this warp on this tile: just hand the accumulator back
           tc_fence_before();
           __syncwarp();
@@ -706,6 +719,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
             } else {
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] = dequant(r0[j], rs, 0);
+              if constexpr (split) {  // (one power of two after the other: their product may be out of range where the result is not)
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                  const float4 cs = (colh + g * 4 < p.N) ? __ldg(reinterpret_cast<const float4*>(p.col_scale + colh + g * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                  v[g * 4 + 0] = v[g * 4 + 0] * rs * cs.x;
+                  v[g * 4 + 1] = v[g * 4 + 1] * rs * cs.y;
+                  v[g * 4 + 2] = v[g * 4 + 2] * rs * cs.z;
+                  v[g * 4 + 3] = v[g * 4 + 3] * rs * cs.w;
+                }
+              }
             }
             if (p.epilogue != TTB_EPI_NONE) {
 #pragma unroll
@@ -823,8 +846,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       // ---- direct path (narrow tiles or unaligned output): the first warp of each lane quarter walks the tile
       bool gave_up = false;
       float row_max = 0.f;
+      constexpr bool by_half = planes16 && BN >= 64;  // both warps of a lane quarter walk the tile
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = by_half ? half * (BN / 64) : 0; c < (by_half ? (half + 1) * (BN / 64) : BN / 32); ++c) {
         uint32_t r[32];
         load_sums(taddr + (uint32_t)(c * 32), r);
         const int col0 = n_blk * BN + c * 32;
@@ -855,6 +879,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = dequant(r[j], rs, (affine && col0 + j < p.N) ? p.col_sum[col0 + j] : 0);
         const bool full = vec_ok && (col0 + 32 <= p.N);
+        if constexpr (split) {
+          if (full) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 cs = reinterpret_cast<const float4*>(p.col_scale + col0)[i];
+              v[i * 4 + 0] = v[i * 4 + 0] * rs * cs.x;
+              v[i * 4 + 1] = v[i * 4 + 1] * rs * cs.y;
+              v[i * 4 + 2] = v[i * 4 + 2] * rs * cs.z;
+              v[i * 4 + 3] = v[i * 4 + 3] * rs * cs.w;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = v[j] * rs * (col0 + j < p.N ? p.col_scale[col0 + j] : 0.f);
+          }
+        }
         if (p.epilogue != TTB_EPI_NONE) {
           float b[32];
           if (BN == 32 && full) {
@@ -894,6 +933,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (col0 + j < p.N) row_max = fmaxf(row_max, fabsf(v[j]));
+        }
+        if constexpr (planes16) {
+          float up;
+          const float down = f16_planes_scale(rs * 32768.f * p.stats[0] + p.stats[1], &up);
+          if (n_blk == 0 && c == 0) p.out_scale[row] = down;
+          __half* hi = static_cast<__half*>(p.out) + (long long)row * p.ldo + col0;
+          __half* lo = static_cast<__half*>(p.out_lo) + (long long)row * p.ldo + col0;
+          if (full) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint4 h, l;
+              f16_planes8(&v[i * 8], up, &h, &l);
+              reinterpret_cast<uint4*>(hi)[i] = h;
+              reinterpret_cast<uint4*>(lo)[i] = l;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (col0 + j < p.N) {
+                hi[j] = __float2half_rn(v[j] * up);
+                lo[j] = __float2half_rn(v[j] * up - __half2float(__float2half_rn(v[j] * up)));
+              }
+          }
+          continue;
         }
 #pragma unroll 1
         for (int plane = 0; plane < (two_planes ? 2 : 1); ++plane) {
@@ -1052,11 +1115,11 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   GemmParams q = p;
   q.a_rows = a_rows;
   CUtensorMap tmO = tmA0, tmO2 = tmA0;  // placeholders when the direct-store epilogue is used
-  const bool tma = BN >= 64 && whole_rows<OutT>(p);
+  const bool tma = BN >= 64 && VAR != VAR_SPLIT_PLANES && whole_rows<OutT>(p);
   // Ragged or misaligned rows without bias, residual or second plane (a 50257-wide vocabulary): word stores.
   // 8192 x 50257 x 768 in fp16 into a contiguous tensor: 845 us, against about 560 into padded rows and 585 for the pass that
   // compacted them. What is left over the padded form are the partial 32-byte sectors at both ends of each 128 bytes.
-  const bool words = BN >= 64 && !tma && p.epilogue == TTB_EPI_NONE && !p.out_lo;
+  const bool words = BN >= 64 && !tma && p.epilogue == TTB_EPI_NONE && !p.out_lo && !P::split;
   if constexpr (VAR == VAR_PLAIN && BN >= 64) {
     if (words) return launch_tc<BN, KIND, OutT, TWO, SK, VAR_WORDS>(ctx, op, p);
   }
@@ -1351,7 +1414,7 @@ TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, b
 
 template <int KIND, typename OutT, int VAR = VAR_PLAIN>
 int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
-  const TilePlan plan = choose_tile<KIND, OutT, VAR>(ctx, p.M, p.N, p.K, p.npass, !whole_rows<OutT>(p));
+  const TilePlan plan = choose_tile<KIND, OutT, VAR>(ctx, p.M, p.N, p.K, p.npass, VAR != VAR_SPLIT_PLANES && !whole_rows<OutT>(p));
   p.split_k = plan.split_k;
   if (plan.pair) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
   if (plan.split_k > 1) return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
@@ -1492,6 +1555,41 @@ __global__ void __launch_bounds__(256) int8_row_sum_kernel(const int8_t* __restr
   if (lane == 0) col_sum[n] = acc;
 }
 
+// Rows of fp32 -> two fp16 planes of a row times the power of two that brings its largest magnitude below 2^15, and its inverse. A warp a row.
+// stats: receives the largest sum of magnitudes of a row, and the largest magnitude of the bias (atomic maxima), or null.
+__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, int64_t rows, int K, __half* __restrict__ hi, __half* __restrict__ lo,
+                                                        float* __restrict__ scale, const float* __restrict__ bias, int64_t n_bias, float* __restrict__ stats) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const float* src = x + row * K;
+  float top = 0.f, sum = 0.f;
+  for (int k = lane; k < K; k += 32) {
+    const float a = fabsf(src[k]);
+    top = fmaxf(top, a);
+    sum += a;
+  }
+  top = warp_max(top);
+  sum = warp_sum(sum);
+  float up;
+  const float down = f16_planes_scale(top, &up);
+  if (lane == 0) {
+    scale[row] = down;
+    if (stats) {  // (non-negative floats order like their bits)
+      atomicMax(reinterpret_cast<int*>(stats), __float_as_int(sum));
+      for (int64_t i = row; i < n_bias; i += rows) atomicMax(reinterpret_cast<int*>(stats + 1), __float_as_int(fabsf(bias[i])));
+    }
+  }
+  for (int k = lane; k < K; k += 32) {
+    const float v = src[k] * up;
+    const __half h = __float2half_rn(v);
+    hi[row * K + k] = h;
+    lo[row * K + k] = __float2half_rn(v - __half2float(h));
+  }
+}
+
 // fp32 -> two tf32-representable planes: hi = x rounded to 10 mantissa bits, lo = (x - hi) rounded likewise. hi + lo
 // is x to 2^-23, which is what three tf32 products recover.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, int64_t n, float* __restrict__ hi, float* __restrict__ lo) {
@@ -1554,6 +1652,42 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
   return pick_tile<KIND_BF16, __nv_bfloat16>(ctx, op, p);
 }
 
+extern "C" int ttb_linear_split(ttb_ctx* ctx, const ttb_linear_split_args* a) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, a != nullptr, "linear_split: null argument block");
+  const bool planes = a->out_lo != nullptr;
+  int s = check_linear(ctx, "linear_split", a->A, a->W, a->bias, a->residual, a->M, a->N, a->K, a->epilogue, a->out, a->ldo, 8);
+  if (s || a->M == 0) return s;
+  TTB_REQUIRE(ctx, a->A2 && a->W2 && a->row_scale && a->col_scale && (!planes || (a->out_scale && a->stats)), "linear_split: null pointer");
+  TTB_REQUIRE(ctx, a->lda >= a->K && a->lda % 8 == 0, "linear_split: lda must be >= K and a multiple of 8");
+  TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(a->A2) | reinterpret_cast<uintptr_t>(a->W2) | reinterpret_cast<uintptr_t>(a->col_scale)) & 15) == 0,
+              "linear_split: operands must be 16-byte aligned");
+  DeviceGuard g(ctx->device);
+  GemmParams p{};
+  p.M = (int)a->M; p.N = (int)a->N; p.K = (int)a->K;
+  p.npass = 3;
+  p.pass_a = 2;  // (A, W), (A2, W), (A, W2)
+  p.pass_b = 4;
+  p.out = a->out; p.ldo = a->ldo; p.out_lo = a->out_lo;
+  p.bias = a->bias; p.residual = a->residual; p.ldr = a->ldr;
+  p.row_scale = a->row_scale; p.col_scale = a->col_scale; p.stats = a->stats; p.out_scale = a->out_scale;
+  p.epilogue = a->epilogue; p.staged = STORE_DIRECT; p.split_k = 1; p.status = ctx->d_status;
+  const Operands op{a->A, a->A2, a->lda, a->W, a->W2};
+  return planes ? pick_tile<KIND_F16, float, VAR_SPLIT_PLANES>(ctx, op, p) : pick_tile<KIND_F16, float, VAR_SPLIT>(ctx, op, p);
+}
+
+extern "C" int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale, const float* bias, int64_t n_bias, float* stats) {
+  if (!ctx) return TTB_ERR_INVALID;
+  TTB_REQUIRE(ctx, rows >= 0 && K > 0 && K < (1ll << 31) && rows < (1ll << 33) && n_bias >= 0, "split_f16: bad shape");
+  if (rows == 0) return TTB_OK;
+  TTB_REQUIRE(ctx, x && hi && lo && scale && (!bias || stats), "split_f16: null pointer");
+  DeviceGuard g(ctx->device);
+  if (stats) TTB_CUDA(ctx, cudaMemsetAsync(stats, 0, 2 * sizeof(float), ctx->stream));
+  launch_pdl(split_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, ctx->stream, x, rows, (int)K, (__half*)hi, (__half*)lo, scale, bias, bias ? n_bias : (int64_t)0,
+             stats);
+  return launched(ctx, "split_f16");
+}
+
 extern "C" int ttb_linear_plan(ttb_ctx* ctx, int dtype, int out_dtype, int products, int two_plane_out, int whole, int64_t M, int64_t N, int64_t K,
                                int64_t* plan) {
   if (!ctx) return TTB_ERR_INVALID;
@@ -1562,7 +1696,9 @@ extern "C" int ttb_linear_plan(ttb_ctx* ctx, int dtype, int out_dtype, int produ
   DeviceGuard g(ctx->device);
   TilePlan t{};
   const bool words = !whole;
-  if (dtype == TTB_F32 && out_dtype == TTB_F32 && products >= 1 && products <= 3) t = choose_tile<KIND_TF32, float, VAR_PLAIN>(ctx, M, N, K, products, words);
+  if (dtype == TTB_F16 && out_dtype == TTB_F32 && products == 3) {  // fp32 as fp16 planes
+    t = two_plane_out ? choose_tile<KIND_F16, float, VAR_SPLIT_PLANES>(ctx, M, N, K, 3, false) : choose_tile<KIND_F16, float, VAR_SPLIT>(ctx, M, N, K, 3, words);
+  } else if (dtype == TTB_F32 && out_dtype == TTB_F32 && products >= 1 && products <= 3) t = choose_tile<KIND_TF32, float, VAR_PLAIN>(ctx, M, N, K, products, words);
   else if (dtype == TTB_I8 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_I8, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
   else if (dtype == TTB_F16 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_F16, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
   else if (dtype == TTB_BF16 && out_dtype == TTB_F32 && (products == 1 || products == 2)) t = choose_tile<KIND_BF16, float, VAR_PLAIN>(ctx, M, N, K, products, words);
