@@ -1,26 +1,37 @@
 // Self-attention of fp32 models over packed tokens, in one kernel (ttb_attention_f32).
 //
 // It takes the place of five (SplitAddBiasTransposeForScore, the score product, ApplyMaskAndSoftmax, the value product, TransposeForScore)
-// that pad every sequence to the longest and write the scores out. Products and softmax stay in fp32 on the CUDA cores, as they were: scores that
-// are rounded to a tensor-core format would cost accuracy, and at the sizes of fp32 requests the launches and the padding, not the
-// arithmetic, were the time. A CTA has 8 R query rows of one (sequence, head) and goes over the keys in tiles of 64 with an online
-// softmax; a thread computes R x 4 scores, then R x 4 outputs, from 16-byte reads of shared memory (rows of 68 floats: the lanes of a read
-// hit different banks). BERT-base fp32, us a pass, with the planes below, against
-// those five: 8 requests of 10 to 120 tokens 2591 -> 1730, 16 of 8 to 512 13283 -> 5670, 1 x 128 1187 -> 1084, 8 x 512 8826 -> 6050, 32 x 512 32363 ->
-// 22300 (with the layer norms of few rows; its Linears are what is left); one layer's attention over 1 x 4096 tokens 2693 -> 1705. The output may leave as the two planes that the next product takes.
+// that pad every sequence to the longest and write the scores out. Both products run on mma.sync m16n8k16 with every fp32 operand as two fp16 planes (three
+// products, 22 bits of an element, like the Linears'): on the CUDA cores, from shared memory, they were bound by its bandwidth (4 wavefronts a 16-byte read for
+// 32 multiply-adds: 58 % of its peak, 8 us for 16 rows against 64 keys). A row of queries or keys is scaled by its own largest element, a tile of values by its own, the
+// probabilities by 2^14; the scales come out again in fp32. Softmax, sums and the outputs' accumulation from tile to tile are fp32. Of a tile's products the small
+// ones are added up first, since the tensor core truncates the sum with every addition: 128 keys 2.1e-7 from 64 bits (all in turn 5.0e-7, on the CUDA cores 3.4e-7),
+// 512 keys 2.4e-7 (5.3e-7, 5.0e-7).
+// A CTA of four warps has 16 WR query rows of one (sequence, head), and WK of its warps share a tile of 64 keys: few rows for few CTAs, since the keys' way and their
+// conversion are then the time. us, 12 heads, CUDA cores / now: 8 sequences of up to 120 20.1 / 10.4, 1 x 300 42 / 19, 1 x 512 71 / 28, 3 of up to 445 68 / 33, 9 x 182 41 /
+// 23, 8 x 512 206 / 101.
 #include "ttb_common.cuh"
 
 using namespace ttb;
 
 namespace {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 128, kWarps = 4;
 constexpr int D = 64;
 constexpr int kKeys = 64;
-constexpr int kPitch = 68;
+constexpr int kPitch = 72;      // halves between the rows of a tile in shared memory: eight rows' sixteen bytes are in different banks
+constexpr int kOutPitch = 68;   // floats between the rows of a warp's output, with {maximum, sum} behind the 64
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kProbScale = 16384.f;
 
-template <int R> constexpr int kSmem = (2 * 8 * R + 2 * kKeys) * kPitch * 4;
+struct Tiles {
+  __half k[2][kKeys * kPitch], v[2][kKeys * kPitch];  // hi, lo
+  float k_scale[kKeys];
+};
+union Shared {
+  Tiles t;
+  float out[kWarps][16 * kOutPitch];
+};
 
 // What the planes of the output in fp16 take: of the rows that the queries, keys and values were computed from, what they were divided by, and the weights'
 // statistics (ttb_split_f16), which bound the values and so their averages; the planes' own scale.
@@ -31,167 +42,271 @@ struct SplitOut {
 };
 enum { OUT_VALUE = 0, OUT_TF32 = 1, OUT_F16 = 2 };
 
-// OUT: the output leaves as it is, or as its two planes, in place of it. (As a choice at run time it cost 15 registers and 1.2 us of 18 at 527 rows.)
-template <int R, int OUT>
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two neighbouring elements as halves of the planes.
+__device__ __forceinline__ void planes2(float x, float y, uint32_t* hi, uint32_t* lo) {
+  const __half2 h = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+  *hi = *reinterpret_cast<const uint32_t*>(&h);
+  *lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// OUT: the output leaves as it is, or as its two planes, in place of it.
+template <int WR, int OUT>
 __global__ void __launch_bounds__(kThreads)
 attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ cu, int heads, const float* __restrict__ mask, long long mask_batch,
                      long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo, const SplitOut split) {
   constexpr bool ROUNDED = OUT == OUT_TF32;
-  constexpr int kRows = 8 * R;
-  extern __shared__ __align__(16) float smem[];
-  float *qs = smem, *ps = qs + kRows * kPitch, *ks = ps + kRows * kPitch, *vs = ks + kKeys * kPitch;
+  constexpr int WK = kWarps / WR, kRows = 16 * WR, kMine = kKeys / WK, NT = kMine / 8;  // keys of a tile for a warp, in eights
+  __shared__ __align__(16) Shared sm;
+  __shared__ int v_most[2];
   pdl_trigger();
   pdl_wait();
   const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * kRows;
   const int begin = cu[b], len = cu[b + 1] - begin;
   if (q0 >= len) return;
-  const int tid = threadIdx.x, kg = tid & 15, rg = tid >> 4;  // keys or dimensions, rows
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wr = warp % WR, wk = warp / WR;
   const int H = heads * D;
   const long long pitch = 3ll * H;
   const float* base = qkv + (long long)begin * pitch + h * D;
-  for (int i = tid; i < kRows * 16; i += kThreads) {
-    const int r = i >> 4, c = (i & 15) * 4;
-    *reinterpret_cast<float4*>(qs + r * kPitch + c) =
-        q0 + r < len ? *reinterpret_cast<const float4*>(base + (q0 + r) * pitch + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  float m[R], l[R], acc[R][4];
+  const int row0 = q0 + wr * 16 + g;  // of the thread's rows row0 and row0 + 8
+  // the warp's queries as fragments
+  uint32_t qh[4][4], ql[4][4];
+  float q_scale[2];
+  {
+    float2 x[4][4];
+    float top[2] = {0.f, 0.f};
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    m[r] = -INFINITY;
-    l[r] = 0.f;
+    for (int s = 0; s < 4; ++s)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[r][e] = 0.f;
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + (e & 1) * 8;
+        x[s][e] = row < len ? *reinterpret_cast<const float2*>(base + row * pitch + s * 16 + (e >> 1) * 8 + t * 2) : make_float2(0.f, 0.f);
+        top[e & 1] = fmaxf(top[e & 1], fmaxf(fabsf(x[s][e].x), fabsf(x[s][e].y)));
+      }
+    float up[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], o));
+      q_scale[r] = f16_planes_scale(top[r], &up[r]);
+    }
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) planes2(x[s][e].x * up[e & 1], x[s][e].y * up[e & 1], &qh[s][e], &ql[s][e]);
   }
+  if (tid < 2) v_most[tid] = 0;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[8][4];
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
   const int keys = causal ? min(len, q0 + kRows) : len;
-  for (int j0 = 0; j0 < keys; j0 += kKeys) {
+  int turn = 0;
+  for (int j0 = 0; j0 < keys; j0 += kKeys, turn ^= 1) {
+    // a thread's keys and values: four elements of rows (tid / 16), + 8, ...
+    const int col = (tid & 15) * 4, first = tid >> 4;
+    float4 k[8], v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      k[i] = v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j0 + first + i * 8 < keys) {
+        const float* src = base + (j0 + first + i * 8) * pitch + H + col;
+        k[i] = *reinterpret_cast<const float4*>(src);
+        v[i] = *reinterpret_cast<const float4*>(src + H);
+      }
+    }
     __syncthreads();  // the tile before has been read
-    // four rows of keys and of values in flight per thread
+    float most = 0.f;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      float4 k[4], v[4];
+    for (int i = 0; i < 8; ++i) {
+      float top = fmaxf(fmaxf(fabsf(k[i].x), fabsf(k[i].y)), fmaxf(fabsf(k[i].z), fabsf(k[i].w)));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = (half * 4 + i) * 8 + rg;
-        k[i] = v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (j0 + r < keys) {
-          const float* src = base + (j0 + r) * pitch + H + kg * 4;
-          k[i] = *reinterpret_cast<const float4*>(src);
-          v[i] = *reinterpret_cast<const float4*>(src + H);
+      for (int o = 1; o < 16; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      float up;
+      const float down = f16_planes_scale(top, &up);
+      const int r = first + i * 8;
+      if (col == 0) sm.t.k_scale[r] = down * scale;
+      uint2 hi, lo;
+      planes2(k[i].x * up, k[i].y * up, &hi.x, &lo.x);
+      planes2(k[i].z * up, k[i].w * up, &hi.y, &lo.y);
+      *reinterpret_cast<uint2*>(&sm.t.k[0][r * kPitch + col]) = hi;
+      *reinterpret_cast<uint2*>(&sm.t.k[1][r * kPitch + col]) = lo;
+      most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+    }
+    most = warp_max(most);
+    if (lane == 0) atomicMax(&v_most[turn], __float_as_int(most));  // (non-negative floats order like their bits)
+    __syncthreads();
+    float v_up;
+    const float v_down = f16_planes_scale(__int_as_float(v_most[turn]), &v_up);
+    if (tid == 0) v_most[turn ^ 1] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = first + i * 8;
+      uint2 hi, lo;
+      planes2(v[i].x * v_up, v[i].y * v_up, &hi.x, &lo.x);
+      planes2(v[i].z * v_up, v[i].w * v_up, &hi.y, &lo.y);
+      *reinterpret_cast<uint2*>(&sm.t.v[0][r * kPitch + col]) = hi;
+      *reinterpret_cast<uint2*>(&sm.t.v[1][r * kPitch + col]) = lo;
+    }
+    __syncthreads();
+    const int mine = wk * kMine;  // the warp's keys of the tile
+    if (j0 + mine >= keys) continue;
+    float s[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+    // the small products first: a sum is truncated with every one that is added to it
+#pragma unroll
+    for (int n = 0; n < NT; n += 2) {
+      const int at = (mine + n * 8 + (lane & 7) + (lane >> 4) * 8) * kPitch + ((lane >> 3) & 1) * 8;
+      uint32_t kh[4][4];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        uint32_t kl[4];
+        ldmatrix4(kh[d], &sm.t.k[0][at + d * 16]);
+        ldmatrix4(kl, &sm.t.k[1][at + d * 16]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          mma16816(s[n + u], ql[d], kh[d][2 * u], kh[d][2 * u + 1]);
+          mma16816(s[n + u], qh[d], kl[2 * u], kl[2 * u + 1]);
         }
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = (half * 4 + i) * 8 + rg;
-        *reinterpret_cast<float4*>(ks + r * kPitch + kg * 4) = k[i];
-        *reinterpret_cast<float4*>(vs + r * kPitch + kg * 4) = v[i];
-      }
+      for (int d = 0; d < 4; ++d)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) mma16816(s[n + u], qh[d], kh[d][2 * u], kh[d][2 * u + 1]);
     }
-    __syncthreads();
-    // scores of rows rg * R .. and keys kg, kg + 16, ...
-    float s[R][4];
+    float top[2] = {m[0], m[1]};
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s[r][e] = 0.f;
-#pragma unroll 4
-    for (int d = 0; d < D; d += 4) {
-      float4 q[R], k[4];
-#pragma unroll
-      for (int r = 0; r < R; ++r) q[r] = *reinterpret_cast<const float4*>(qs + (rg * R + r) * kPitch + d);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) k[e] = *reinterpret_cast<const float4*>(ks + (kg + 16 * e) * kPitch + d);
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[r][e] = fmaf(q[r].x, k[e].x, fmaf(q[r].y, k[e].y, fmaf(q[r].z, k[e].z, fmaf(q[r].w, k[e].w, s[r][e]))));
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = q0 + rg * R + r;
-      float top = m[r];
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int j = j0 + kg + 16 * e;
-        s[r][e] *= scale;
-        if (mask && i < len && j < len) s[r][e] += mask[b * mask_batch + i * mask_row + j];
-        if (j >= keys || (causal && j > i)) s[r][e] = -INFINITY;
-        top = fmaxf(top, s[r][e]);
+        const int at = mine + n * 8 + t * 2 + (e & 1), j = j0 + at, i = row0 + (e >> 1) * 8;
+        float x = s[n][e] * q_scale[e >> 1] * sm.t.k_scale[at];
+        if (mask && i < len && j < len) x += mask[b * mask_batch + i * mask_row + j];
+        if (j >= keys || (causal && j > i)) x = -INFINITY;
+        s[n][e] = x;
+        top[e >> 1] = fmaxf(top[e >> 1], x);
       }
+    float keep[2], centre[2];
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      const float centre = top == -INFINITY ? 0.f : top, keep = exp2f((m[r] - centre) * kLog2e);
-      m[r] = top;
-      l[r] *= keep;
+    for (int r = 0; r < 2; ++r) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[r][e] *= keep;
-        const float p = expf(s[r][e] - centre);
-        l[r] += p;  // this thread's keys; the sixteen threads' sums meet at the end
-        ps[(rg * R + r) * kPitch + kg + 16 * e] = p;
-      }
+      for (int o = 1; o < 4; o <<= 1) top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], o));
+      centre[r] = top[r] == -INFINITY ? 0.f : top[r];
+      keep[r] = exp2f((m[r] - centre[r]) * kLog2e);
+      m[r] = top[r];
+      l[r] *= keep[r];
     }
-    __syncwarp();  // a row's probabilities are written and read by one half-warp
-    // outputs of rows rg * R .. and dimensions kg * 4 ..
-    const int last = min(kKeys, (keys - j0 + 3) & ~3);
-#pragma unroll 2
-    for (int j = 0; j < last; j += 4) {
-      float4 p[R], v[4];
+    uint32_t ph[NT / 2][4], pl[NT / 2][4];
 #pragma unroll
-      for (int r = 0; r < R; ++r) p[r] = *reinterpret_cast<const float4*>(ps + (rg * R + r) * kPitch + j);
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const float4*>(vs + (j + e) * kPitch + kg * 4);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        acc[r][0] = fmaf(p[r].x, v[0].x, fmaf(p[r].y, v[1].x, fmaf(p[r].z, v[2].x, fmaf(p[r].w, v[3].x, acc[r][0]))));
-        acc[r][1] = fmaf(p[r].x, v[0].y, fmaf(p[r].y, v[1].y, fmaf(p[r].z, v[2].y, fmaf(p[r].w, v[3].y, acc[r][1]))));
-        acc[r][2] = fmaf(p[r].x, v[0].z, fmaf(p[r].y, v[1].z, fmaf(p[r].z, v[2].z, fmaf(p[r].w, v[3].z, acc[r][2]))));
-        acc[r][3] = fmaf(p[r].x, v[0].w, fmaf(p[r].y, v[1].w, fmaf(p[r].z, v[2].w, fmaf(p[r].w, v[3].w, acc[r][3]))));
+      for (int r = 0; r < 2; ++r) {
+        const float x = expf(s[n][r * 2] - centre[r]), y = expf(s[n][r * 2 + 1] - centre[r]);
+        l[r] += x + y;
+        planes2(x * kProbScale, y * kProbScale, &ph[n / 2][(n & 1) * 2 + r], &pl[n / 2][(n & 1) * 2 + r]);
       }
+    const float factor = v_down * (1.f / kProbScale);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {  // sixteen dimensions
+      float o[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[u][e] = 0.f;
+      uint32_t vh[NT / 2][4];
+#pragma unroll
+      for (int n = 0; n < NT / 2; ++n) {  // sixteen keys
+        const int at = (mine + n * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kPitch + d * 16 + (lane >> 4) * 8;
+        uint32_t vl[4];
+        ldmatrix4_trans(vh[n], &sm.t.v[0][at]);
+        ldmatrix4_trans(vl, &sm.t.v[1][at]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          mma16816(o[u], pl[n], vh[n][2 * u], vh[n][2 * u + 1]);
+          mma16816(o[u], ph[n], vl[2 * u], vl[2 * u + 1]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < NT / 2; ++n)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) mma16816(o[u], ph[n], vh[n][2 * u], vh[n][2 * u + 1]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[d * 2 + u][e] = fmaf(o[u][e], factor, acc[d * 2 + u][e] * keep[e >> 1]);
     }
-    __syncwarp();
   }
+  __syncthreads();  // the last tile has been read: the warps' results take its place
+  {
+    float* mine = sm.out[warp];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], o);
+      if (t == 0) *reinterpret_cast<float2*>(mine + (g + r * 8) * kOutPitch + D) = make_float2(m[r], l[r]);
+#pragma unroll
+      for (int n = 0; n < 8; ++n) *reinterpret_cast<float2*>(mine + (g + r * 8) * kOutPitch + n * 8 + t * 2) = make_float2(acc[n][r * 2], acc[n][r * 2 + 1]);
+    }
+  }
+  __syncthreads();
   float up = 1.f;
   if constexpr (OUT == OUT_F16) {  // one scale for all heads and rows of the sequence: no value of it is beyond this bound
     float most = 0.f;
-    for (int j = tid & 31; j < len; j += 32) most = fmaxf(most, split.row_scale[begin + j]);
+    for (int j = lane; j < len; j += 32) most = fmaxf(most, split.row_scale[begin + j]);
     const float down = f16_planes_scale(warp_max(most) * 32768.f * split.stats[0] + split.stats[1], &up);
     if (h == 0 && tid < kRows && q0 + tid < len) split.scale[begin + q0 + tid] = down;
   }
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    float sum = l[r];
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const int i = q0 + rg * R + r;
+  for (int n = 0; n < 2 * WR; ++n) {
+    const int r = (n * kThreads + tid) >> 4, c = (tid & 15) * 4, i = q0 + r;
     if (i >= len) continue;
-    const float inv = 1.0f / sum;
-    const float4 y = make_float4(acc[r][0] * inv, acc[r][1] * inv, acc[r][2] * inv, acc[r][3] * inv);
-    const long long at = (long long)(begin + i) * H + h * D + kg * 4;
-    if constexpr (OUT == OUT_F16) {
-      const float v[4] = {y.x * up, y.y * up, y.z * up, y.w * up};
-      __half2 hi[2], lo[2];
+    // the warps that shared this row's keys, in their order
+    float top = -INFINITY, sum = 0.f;
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        hi[e] = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-        const float2 f = __half22float2(hi[e]);
-        lo[e] = __floats2half2_rn(v[2 * e] - f.x, v[2 * e + 1] - f.y);
-      }
-      *reinterpret_cast<uint2*>(split.hi + at) = *reinterpret_cast<const uint2*>(hi);
-      *reinterpret_cast<uint2*>(split.lo + at) = *reinterpret_cast<const uint2*>(lo);
+    for (int w = 0; w < WK; ++w) top = fmaxf(top, sm.out[r / 16 + w * WR][(r & 15) * kOutPitch + D]);
+    const float centre = top == -INFINITY ? 0.f : top;
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < WK; ++w) {
+      const float* theirs = sm.out[r / 16 + w * WR] + (r & 15) * kOutPitch;
+      const float f = exp2f((theirs[D] - centre) * kLog2e);
+      const float4 x = *reinterpret_cast<const float4*>(theirs + c);
+      sum = fmaf(theirs[D + 1], f, sum);
+      y = make_float4(fmaf(x.x, f, y.x), fmaf(x.y, f, y.y), fmaf(x.z, f, y.z), fmaf(x.w, f, y.w));
+    }
+    const float inv = 1.0f / sum;
+    y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+    const long long at = (long long)(begin + i) * H + h * D + c;
+    if constexpr (OUT == OUT_F16) {
+      uint2 hi, lo;
+      planes2(y.x * up, y.y * up, &hi.x, &lo.x);
+      planes2(y.z * up, y.w * up, &hi.y, &lo.y);
+      *reinterpret_cast<uint2*>(split.hi + at) = hi;
+      *reinterpret_cast<uint2*>(split.lo + at) = lo;
       continue;
     }
     *reinterpret_cast<float4*>(out + at) = ROUNDED ? make_float4(tf32_hi(y.x), tf32_hi(y.y), tf32_hi(y.z), tf32_hi(y.w)) : y;
     if (ROUNDED || out_lo) *reinterpret_cast<float4*>(out_lo + at) = make_float4(tf32_lo(y.x, ROUNDED), tf32_lo(y.y, ROUNDED), tf32_lo(y.z, ROUNDED), tf32_lo(y.w, ROUNDED));
   }
-}
-
-template <int R, int OUT>
-cudaError_t launch_f32(ttb_ctx* ctx, dim3 grid, const float* qkv, const int32_t* cu, int heads, const float* mask, int64_t mbs, int64_t mrs, int causal, float scale,
-                       float* out, float* out_lo, const SplitOut& split) {
-  cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<R, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<R>);
-  if (e != cudaSuccess) return e;
-  return launch_pdl(attention_f32_kernel<R, OUT>, grid, dim3(kThreads), (size_t)kSmem<R>, ctx->stream, qkv, cu, heads, mask, (long long)mbs, (long long)mrs, causal, scale, out,
-                    out_lo, split);
 }
 
 template <int OUT>
@@ -204,14 +319,17 @@ int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int
   TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo)) & 15) == 0,
               "attention_f32: buffers must be 16-byte aligned");
   DeviceGuard g(ctx->device);
-  // 32 rows a CTA read a tile of keys half as often as 16; with few (sequence, head, rows) the chip has room for twice the CTAs
-  const int64_t ctas = B * heads * ((max_seqlen + 31) / 32);
-  if (ctas >= 2 * ctx->sm_count)
-    TTB_CUDA(ctx, (launch_f32<4, OUT>(ctx, dim3((unsigned)((max_seqlen + 31) / 32), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo, split)));
-  else
-    TTB_CUDA(ctx, (launch_f32<2, OUT>(ctx, dim3((unsigned)((max_seqlen + 15) / 16), (unsigned)heads, (unsigned)B), qkv, cu_seqlens, (int)heads, mask, mask_batch_stride, mask_row_stride,
-                                causal, scale, out, out_lo, split)));
+  auto blocks = [&](int rows) { return dim3((unsigned)((max_seqlen + rows - 1) / rows), (unsigned)heads, (unsigned)B); };
+  auto ctas = [&](int64_t rows) { return B * heads * ((max_seqlen + rows - 1) / rows); };
+#define ATTENTION_F32(WR)                                                                                                                                  \
+  launch_pdl(attention_f32_kernel<WR, OUT>, blocks(16 * WR), dim3(kThreads), 0, ctx->stream, qkv, cu_seqlens, (int)heads, mask, (long long)mask_batch_stride, \
+             (long long)mask_row_stride, causal, scale, out, out_lo, split)
+  // The most rows a CTA with which the chip is still full: us with 16, 32, 64 rows: 192 CTAs of 64 rows (384 of 32) 10.4, 12.4, 15.6; 324 (648) 36, 27.5, 23.1; 252
+  // (504) 37.7, 32.8, 44.6; 96 (192) 28.6, 36, 44.7; 768 181, 128, 101.
+  if (ctas(64) >= 2 * ctx->sm_count) ATTENTION_F32(4);
+  else if (ctas(32) >= 3 * ctx->sm_count) ATTENTION_F32(2);
+  else ATTENTION_F32(1);
+#undef ATTENTION_F32
   return launched(ctx, "attention_f32");
 }
 
