@@ -156,19 +156,22 @@ const float* PackedLinear::PackedTf32(bool is_trans) const {
   return p.data<float>();
 }
 
-PackedLinear::Split PackedLinear::PackedSplit(bool is_trans) const {
+PackedLinear::Split PackedLinear::PackedSplit(bool is_trans, bool stats) const {
   std::lock_guard<std::mutex> g(cache_->mu);
   Tensor &planes = cache_->split[is_trans ? 1 : 0], &scale = cache_->split_scale[is_trans ? 1 : 0];
   const int64_t K = in_dim(is_trans), N = out_dim(is_trans);
-  if (planes.is_null()) {
+  bool& has_stats = cache_->split_stats[is_trans ? 1 : 0];
+  if (planes.is_null() || (stats && !has_stats)) {
     ttb_ctx* c = DeviceContext(weight_.device_id());
     Tensor rows(nullptr);
     float* w = rows.Reshape<float>({N, K}, kDLCUDA, weight_.device_id(), "linear/rows_of_weight");
     Check(ttb_prepack_weight(c, TTB_F32, weight_.raw(), is_trans ? 1 : 0, K, N, TTB_F32, w), c, "prepack_weight");
     float* s = scale.Reshape<float>({2 + (N + 3) / 4 * 4}, kDLCUDA, weight_.device_id(), "linear/split_weight_scales");
     char* p = static_cast<char*>(planes.Reshape(core::kFloat16, {2, N, K}, kDLCUDA, weight_.device_id(), "linear/split_weight_planes"));
-    const bool bias = !bias_.is_null();
-    Check(ttb_split_f16(c, w, N, K, p, p + N * K * 2, s, bias ? bias_.data<float>() : nullptr, bias ? bias_.numel() : 0, s + (N + 3) / 4 * 4), c, "split_f16");
+    const bool bias = stats && !bias_.is_null();
+    Check(ttb_split_f16(c, w, N, K, p, p + N * K * 2, s, bias ? bias_.data<float>() : nullptr, bias ? bias_.numel() : 0, stats ? s + (N + 3) / 4 * 4 : nullptr), c,
+          "split_f16");
+    has_stats = stats;
   }
   const char* p = static_cast<const char*>(planes.raw());
   return {p, p + N * K * 2, scale.data<float>(), scale.data<float>() + (N + 3) / 4 * 4};
@@ -255,7 +258,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     // fp32 on the tensor cores: activation and weight as two fp16 planes each, three products accumulated in one GEMM with the elementwise kernel that followed
     // MatMul in the reference as its epilogue (mat_mul.cpp:81-96 selects tensor-op math for the same product). An activation that brings its planes
     // along is not split again.
-    const Split w = PackedSplit(is_trans);
+    const Split w = PackedSplit(is_trans, split_out != nullptr);
     ttb_linear_split_args args{};
     Tensor planes(nullptr), scale(nullptr);
     if (x.split_scale()) {
@@ -673,6 +676,7 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
     // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own (a causal layer's
     // mask tensor says what its rows see, as it does in the sequence below; the kernel's own causal form is the C call's)
     Tensor qkv(nullptr), planes_in(nullptr);
+    if (H % 8 == 0 && T > 0) qkv_.PackedSplit(is_trans_weight, true);
     if (!gemm_in->lo() && T > 0) {  // planes here, so that the attention kernel knows what bounds the values whether the input brought its own or not
       planes_in.Reshape(x.dtype(), {T, H}, kDLCUDA, dev, "self/planes_in");
       const SplitPlanes p = NewSplit(&planes_in, true);
@@ -695,7 +699,7 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
     if (gemm_in->split_scale() && T > 0) {  // the output as fp16 planes, within the bound that the product's operands give for the values
       const SplitPlanes p = NewSplit(&context, true);
       Check(ttb_attention_f32_split(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, gemm_in->split_scale()->data<float>(),
-                                    qkv_.PackedSplit(is_trans_weight).stats, p.hi, p.lo, p.scale),
+                                    qkv_.PackedSplit(is_trans_weight, true).stats, p.hi, p.lo, p.scale),
             c, "attention_f32");
     } else {
       float* hi = context.mutableData<float>();

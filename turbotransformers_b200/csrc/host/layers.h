@@ -39,7 +39,8 @@ class PackedLinear {
     const void *hi, *lo;
     const float *scale, *stats;
   };
-  Split PackedSplit(bool is_trans) const;
+  // (The statistics are there where they have been asked for.)
+  Split PackedSplit(bool is_trans, bool stats) const;
   // An output as fp16 planes with a scale for each row.
   struct SplitOut {
     void *hi, *lo;
@@ -80,6 +81,7 @@ class PackedLinear {
     core::Tensor tf32[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor split[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor split_scale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
+    bool split_stats[2] = {false, false};
     core::Tensor q[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qscale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qref[2]{core::Tensor(nullptr), core::Tensor(nullptr)};

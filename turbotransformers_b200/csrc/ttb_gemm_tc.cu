@@ -1565,11 +1565,20 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   const float* src = x + row * K;
+  const bool eights = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0;
   float top = 0.f, sum = 0.f;
-  for (int k = lane; k < K; k += 32) {
-    const float a = fabsf(src[k]);
-    top = fmaxf(top, a);
-    sum += a;
+  auto count = [&](float v) {
+    top = fmaxf(top, fabsf(v));
+    sum += fabsf(v);
+  };
+  if (eights) {
+#pragma unroll 4
+    for (int k = lane * 4; k < K; k += 128) {
+      const float4 v = *reinterpret_cast<const float4*>(src + k);
+      count(v.x); count(v.y); count(v.z); count(v.w);
+    }
+  } else {
+    for (int k = lane; k < K; k += 32) count(src[k]);
   }
   top = warp_max(top);
   sum = warp_sum(sum);
@@ -1581,6 +1590,18 @@ __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict_
       atomicMax(reinterpret_cast<int*>(stats), __float_as_int(sum));
       for (int64_t i = row; i < n_bias; i += rows) atomicMax(reinterpret_cast<int*>(stats + 1), __float_as_int(fabsf(bias[i])));
     }
+  }
+  if (eights) {
+#pragma unroll 2
+    for (int k = lane * 8; k < K; k += 256) {
+      Vec8<float> v;
+      v.load(src + k);
+      uint4 h, l;
+      f16_planes8(v.v, up, &h, &l);
+      *reinterpret_cast<uint4*>(hi + row * K + k) = h;
+      *reinterpret_cast<uint4*>(lo + row * K + k) = l;
+    }
+    return;
   }
   for (int k = lane; k < K; k += 32) {
     const float v = src[k] * up;
