@@ -1017,90 +1017,74 @@ __global__ void prepare_masks_kernel(int64_t B, int64_t L, const int64_t* __rest
 }
 
 // ------------------------------------------------------------------------------------------------
-// Transposes between token-major [.., L, heads, d] and head-major [B, heads, L, d]; optional bias,
-// optional packed<->padded mapping through cu_seqlens. One thread moves 1 element; consecutive threads
-// walk d, so both sides are accessed in d-long contiguous runs.
+// Transposes between token-major [B, L, W, heads, d] and W head-major [B, heads, L, d], to the heads with a bias added; through
+// cu_seqlens the tokens are packed ([sumL, W, heads, d], what is past a sequence's end is zero at the heads). Bound by memory, and where
+// that is small by instructions: a thread moves VEC elements (16 bytes where d and the pointers allow it, else one), and a warp's 32
+// of these lie in one token's row, so that what has to be divided is divided once a warp, in 32 bits where it fits. 900 tokens of
+// 512 fp16: 2.5 us; 7.6 with one element a thread, whose place took six 64-bit divisions.
 // ------------------------------------------------------------------------------------------------
-// mode 0: qkv [B,L,3,h,d] + bias -> q,k,v [B,h,L,d]     (cu == nullptr: fixed length; else packed -> padded, zero-filled)
+__device__ __forceinline__ int64_t quotient(int64_t a, int64_t b) {  // a, b >= 0
+  return ((a | b) >> 32) == 0 ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b;
+}
+
 template <typename T>
+struct Heads {
+  T* at[3];
+};
+template <typename T, int VEC>
+struct alignas(sizeof(T) * VEC) Group {
+  T e[VEC];
+};
+
+template <typename T, int VEC, int W, bool TO_HEADS>
 __global__ void __launch_bounds__(256)
-split_add_bias_transpose_kernel(const T* __restrict__ qkv, const T* __restrict__ bias, const int32_t* __restrict__ cu,
-                                int64_t B, int64_t L, int heads, int d, T* __restrict__ q, T* __restrict__ k,
-                                T* __restrict__ v) {
+transpose_heads_kernel(const T* __restrict__ in, const T* __restrict__ bias, const int32_t* __restrict__ cu, int64_t B, int64_t L, int heads, int d, T* __restrict__ out,
+                       Heads<T> parts) {
+  static_assert(TO_HEADS || W == 1, "one tensor of heads goes back to tokens");
+  using G = Group<T, VEC>;
   pdl_trigger();
   pdl_wait();
-  const int64_t H = (int64_t)heads * d;
-  const int64_t n = B * L * 3 * H;  // over the padded output index space
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int dd = (int)(i % d);
-    const int hh = (int)((i / d) % heads);
-    const int w = (int)((i / H) % 3);
-    const int64_t l = (i / (3 * H)) % L;
-    const int64_t b = i / (3 * H * L);
-    T* dst = (w == 0 ? q : (w == 1 ? k : v)) + ((b * heads + hh) * L + l) * d + dd;
-    int64_t src_tok;
+  const int64_t H = (int64_t)heads * d, groups = W * H / VEC, pieces = (groups + 31) / 32, n = B * L * pieces;
+  const int d_groups = d / VEC;
+  for (int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); i < n; i += (int64_t)gridDim.x * 8) {
+    const int64_t t = quotient(i, pieces), b = quotient(t, L), l = t - b * L, g = (i - t * pieces) * 32 + (threadIdx.x & 31);
+    if (g >= groups) continue;
+    const int64_t head = quotient(g, d_groups), w = W == 1 ? 0 : head / heads;
+    const int64_t by_head = ((b * heads + (head - w * heads)) * L + l) * d + (g - head * d_groups) * VEC;
+    int64_t token = t;
+    bool padding = false;
     if (cu) {
-      const int64_t len = cu[b + 1] - cu[b];
-      if (l >= len) { *dst = from_f<T>(0.f); continue; }
-      src_tok = cu[b] + l;
-    } else {
-      src_tok = b * L + l;
+      token = cu[b] + l;
+      padding = l >= cu[b + 1] - cu[b];
     }
-    const int64_t c = (int64_t)w * H + (int64_t)hh * d + dd;
-    *dst = from_f<T>(to_f(qkv[src_tok * 3 * H + c]) + to_f(bias[c]));
+    if constexpr (TO_HEADS) {
+      G v;
+      if (padding) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) v.e[j] = from_f<T>(0.f);
+      } else {
+        v = *reinterpret_cast<const G*>(in + token * W * H + g * VEC);
+        const G add = *reinterpret_cast<const G*>(bias + g * VEC);
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) v.e[j] = from_f<T>(to_f(v.e[j]) + to_f(add.e[j]));
+      }
+      *reinterpret_cast<G*>((w == 0 ? parts.at[0] : (w == 1 ? parts.at[1] : parts.at[2])) + by_head) = v;
+    } else if (!padding) {
+      *reinterpret_cast<G*>(out + token * H + g * VEC) = *reinterpret_cast<const G*>(in + by_head);
+    }
   }
 }
 
-// [B,h,L,d] -> [B,L,h*d] (cu == nullptr) or padded -> packed [sumL, h*d] (cu given; index space = padded)
-template <typename T>
-__global__ void __launch_bounds__(256)
-transpose_for_score_kernel(const T* __restrict__ in, const int32_t* __restrict__ cu, int64_t B, int64_t L, int heads,
-                           int d, T* __restrict__ out) {
-  pdl_trigger();
-  pdl_wait();
-  const int64_t H = (int64_t)heads * d;
-  const int64_t n = B * L * H;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int dd = (int)(i % d);
-    const int hh = (int)((i / d) % heads);
-    const int64_t l = (i / H) % L;
-    const int64_t b = i / (H * L);
-    int64_t dst_tok;
-    if (cu) {
-      if (l >= cu[b + 1] - cu[b]) continue;
-      dst_tok = cu[b] + l;
-    } else {
-      dst_tok = b * L + l;
-    }
-    out[dst_tok * H + (int64_t)hh * d + dd] = in[((b * heads + hh) * L + l) * d + dd];
-  }
-}
-
-// [B,L,h,d] + bias -> [B,h,L,d] (cu == nullptr) or packed [sumL,h,d] + bias -> padded, zero-filled
-template <typename T>
-__global__ void __launch_bounds__(256)
-add_bias_transpose_kernel(const T* __restrict__ in, const T* __restrict__ bias, const int32_t* __restrict__ cu, int64_t B,
-                          int64_t L, int heads, int d, T* __restrict__ out) {
-  pdl_trigger();
-  pdl_wait();
-  const int64_t H = (int64_t)heads * d;
-  const int64_t n = B * L * H;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int dd = (int)(i % d);
-    const int hh = (int)((i / d) % heads);
-    const int64_t l = (i / H) % L;
-    const int64_t b = i / (H * L);
-    T* dst = out + ((b * heads + hh) * L + l) * d + dd;
-    int64_t src_tok;
-    if (cu) {
-      if (l >= cu[b + 1] - cu[b]) { *dst = from_f<T>(0.f); continue; }
-      src_tok = cu[b] + l;
-    } else {
-      src_tok = b * L + l;
-    }
-    const int64_t c = (int64_t)hh * d + dd;
-    *dst = from_f<T>(to_f(in[src_tok * H + c]) + to_f(bias[c]));
-  }
+template <typename T, int W, bool TO_HEADS>
+void transpose_heads(ttb_ctx* ctx, const T* in, const T* bias, const int32_t* cu, int64_t B, int64_t L, int64_t heads, int64_t d, T* out, Heads<T> parts) {
+  constexpr int kVec = 16 / sizeof(T);
+  uintptr_t at = reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(out);
+  for (T* p : parts.at) at |= reinterpret_cast<uintptr_t>(p);
+  const bool wide = d % kVec == 0 && (at & 15) == 0;
+  const int64_t groups = W * heads * d / (wide ? kVec : 1);
+  const dim3 grid(grid_for(B * L * ((groups + 31) / 32), 8, ctx->sm_count));
+  if (wide) launch_pdl(transpose_heads_kernel<T, kVec, W, TO_HEADS>, grid, dim3(256), 0, ctx->stream, in, bias, cu, B, L, (int)heads, (int)d, out, parts);
+  else launch_pdl(transpose_heads_kernel<T, 1, W, TO_HEADS>, grid, dim3(256), 0, ctx->stream, in, bias, cu, B, L, (int)heads, (int)d, out, parts);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1706,10 +1690,7 @@ extern "C" int ttb_split_add_bias_transpose_pad(ttb_ctx* ctx, int dtype, const v
   if (B * maxL == 0) return TTB_OK;
   TTB_REQUIRE(ctx, qkv && bias && q && k && v, "split_add_bias_transpose: null pointer");
   DeviceGuard g(ctx->device);
-  const int grid = grid_for(B * maxL * 3 * heads * d, 256, ctx->sm_count);
-  TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (launch_pdl(split_add_bias_transpose_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)qkv, (const T*)bias, cu_seqlens, B, maxL,
-                                                                                      (int)heads, (int)d, (T*)q, (T*)k, (T*)v)));
+  TTB_DISPATCH_FLOAT(ctx, dtype, T, (transpose_heads<T, 3, true>(ctx, (const T*)qkv, (const T*)bias, cu_seqlens, B, maxL, heads, d, nullptr, {{(T*)q, (T*)k, (T*)v}})));
   return launched(ctx, "split_add_bias_transpose");
 }
 
@@ -1726,9 +1707,7 @@ extern "C" int ttb_transpose_for_score_pad(ttb_ctx* ctx, int dtype, const void* 
   if (B * maxL == 0) return TTB_OK;
   TTB_REQUIRE(ctx, in && out, "transpose_for_score: null pointer");
   DeviceGuard g(ctx->device);
-  const int grid = grid_for(B * maxL * heads * d, 256, ctx->sm_count);
-  TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (launch_pdl(transpose_for_score_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)in, cu_seqlens, B, maxL, (int)heads, (int)d, (T*)out)));
+  TTB_DISPATCH_FLOAT(ctx, dtype, T, (transpose_heads<T, 1, false>(ctx, (const T*)in, nullptr, cu_seqlens, B, maxL, heads, d, (T*)out, Heads<T>{})));
   return launched(ctx, "transpose_for_score");
 }
 
@@ -1746,10 +1725,7 @@ extern "C" int ttb_add_bias_transpose_for_score_pad(ttb_ctx* ctx, int dtype, con
   if (B * maxL == 0) return TTB_OK;
   TTB_REQUIRE(ctx, in && bias && out, "add_bias_transpose_for_score: null pointer");
   DeviceGuard g(ctx->device);
-  const int grid = grid_for(B * maxL * heads * d, 256, ctx->sm_count);
-  TTB_DISPATCH_FLOAT(ctx, dtype, T,
-                     (launch_pdl(add_bias_transpose_kernel<T>, dim3(grid), dim3(256), 0, ctx->stream, (const T*)in, (const T*)bias, cu_seqlens, B, maxL, (int)heads,
-                                                                                (int)d, (T*)out)));
+  TTB_DISPATCH_FLOAT(ctx, dtype, T, (transpose_heads<T, 1, true>(ctx, (const T*)in, (const T*)bias, cu_seqlens, B, maxL, heads, d, nullptr, {{(T*)out, nullptr, nullptr}})));
   return launched(ctx, "add_bias_transpose_for_score");
 }
 
