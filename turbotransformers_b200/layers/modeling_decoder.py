@@ -79,6 +79,10 @@ class TransformerDecoderLayer:
         return TransformerDecoderLayer(self_attn, context_attn, feed_forward)
 
 
+_CACHE_NAMES = ("self_keys", "self_values", "memory_keys", "memory_values")
+_CACHED = set(_CACHE_NAMES)
+
+
 def _unmodified(layer) -> bool:
     """Whether a layer and its parts run this module's own calls. A caller's class in the place of any of them, such as an
     attention that wraps __call__, expects torch tensors for the layer's input, the memory and the masks."""
@@ -162,11 +166,10 @@ class TransformerDecoder:
             return None
         parts = [(l.self_attn, l.context_attn, l.feed_forward) for l in self.transformer_layers]
         caches = [self.state["cache"][f"layer_{i}"] for i in range(len(parts))]
-        names = ("self_keys", "self_values", "memory_keys", "memory_values")
-        if not all(set(c) == set(names) for c in caches) or not all(
-                type(s) is MultiHeadedAttention and type(c) is MultiHeadedAttention and type(f) is PositionwiseFeedForward for s, c, f in parts):
-            return None
-        held = [tuple(_empty() if c[k] is None else try_convert(c[k]) for k in names) for c in caches]
+        for (s, c, f), cache in zip(parts, caches):
+            if set(cache) != _CACHED or type(s) is not MultiHeadedAttention or type(c) is not MultiHeadedAttention or type(f) is not PositionwiseFeedForward:
+                return None
+        held = [tuple([_empty() if c[k] is None else try_convert(c[k]) for k in _CACHE_NAMES]) for c in caches]
         # a memory entry is only read where both of a layer are filled; otherwise both are projected, whichever was given
         projected = [h[2].is_null() or h[3].is_null() for h in held]
         memory = memory_bank.transpose(0, 1).contiguous() if any(projected) else None

@@ -15,7 +15,7 @@ AnyTensor = Union[cxx.Tensor, torch.Tensor]
 
 def convert2tt_tensor(t: torch.Tensor):
     """Zero-copy alias of a torch tensor (the layer never writes it)."""
-    return cxx.Tensor.from_dlpack(dlpack.to_dlpack(t.detach()))
+    return cxx.Tensor.from_dlpack(dlpack.to_dlpack(t if type(t) is torch.Tensor and not t.requires_grad else t.detach()))
 
 
 def try_convert(t, device: Optional[torch.device] = None):
@@ -42,5 +42,6 @@ def create_empty_if_none(output):
 def use_current_stream(t=None):
     """Point the device's kernel stream at torch's current stream so both stay ordered."""
     dev = t.device.index if isinstance(t, torch.Tensor) and t.is_cuda else torch.cuda.current_device()
-    cxx.set_stream(dev, torch.cuda.current_stream(dev).cuda_stream)
+    # (the stream's number as it is: torch.cuda.current_stream makes an object of it first, 4 us a call, two calls a decoding step)
+    cxx.set_stream(dev, torch._C._cuda_getCurrentRawStream(dev))
     return dev
