@@ -30,13 +30,12 @@ constexpr int kLnRows = 2;
 
 // EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
 // same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
-// other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099);
-// 4, fp32 with its two fp16 planes (ttb_split_f16; out_f32 and out_lo are those) and out_scale.
+// other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099).
 template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
                       const TOut* __restrict__ beta, TOut* out, TOut* __restrict__ out_lo, float* __restrict__ out_f32, int64_t M, int N,
-                      float eps, float* __restrict__ out_scale) {
+                      float eps) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -88,46 +87,6 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
     float rstd[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) rstd[r] = rsqrtf(warp_sum(sq[r]) / (float)N + eps);
-    if constexpr (EXTRA == 4) {  // the planes' scale is known when all of the row is
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) {
-        const int64_t row = row0 + r;
-        if (row >= M) continue;
-        float top = 0.f;
-#pragma unroll
-        for (int it = 0; it < ITERS; ++it) {
-          const int col = (it * 32 + lane) * 8;
-          if (col < N) {
-            Vec8<TOut> g, b;
-            g.load(gamma + col);
-            b.load(beta + col);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              v[r][it][j] = b.v[j] + g.v[j] * rstd[r] * (v[r][it][j] - mean[r]);
-              top = fmaxf(top, fabsf(v[r][it][j]));
-            }
-          }
-        }
-        float up;
-        const float down = f16_planes_scale(warp_max(top), &up);
-        if (lane == 0) out_scale[row] = down;
-#pragma unroll
-        for (int it = 0; it < ITERS; ++it) {
-          const int col = (it * 32 + lane) * 8;
-          if (col < N) {
-            Vec8<TOut> o;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o.v[j] = v[r][it][j];
-            o.store(out + row * N + col);
-            uint4 h, l;
-            f16_planes8(v[r][it], up, &h, &l);
-            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out_f32) + row * N + col) = h;
-            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out_lo) + row * N + col) = l;
-          }
-        }
-      }
-      continue;
-    }
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int col = (it * 32 + lane) * 8;
@@ -537,26 +496,88 @@ layernorm_rows_generic_kernel(const TIn* x, const TIn* __restrict__ residual, co
   }
 }
 
-// out = LN(x + residual + bias) in fp32, with its two fp16 planes and their scales. N % 8 == 0, N <= 2048, 16-byte aligned rows: what a product takes.
+// out = LN(x + residual + bias) in fp32, with its two fp16 planes (ttb_split_f16) and their scales. N % 8 == 0, N <= 2048, 16-byte aligned rows: what a
+// product takes. x may be out.
+// Bound by latency: the loads, three sums or maxima over the row that wait for one another, the stores. A CTA has one row and a thread 8 elements of it, all of
+// whose loads are sent at once. us a launch of 768 columns back to back, with a warp a row / now: 128 rows 3.7 / 2.45, 1100 9.1 / 5.0, 3000 9.6 / 7.4, 9000
+// 17.4 / 16.9, but 527 rows 4.1 / 4.8; in the pass, where the loads come from the product before, those gain too: BERT-base fp32, 1 x 128 856 -> 804, 8 ragged
+// requests (527 rows) 1113 -> 1051. (Two and four rows a CTA: 128 rows 2.8 and 3.5, 9000 21 and 27.)
+__global__ void __launch_bounds__(256)
+layernorm_split_kernel(const float* x, const float* __restrict__ residual, const float* __restrict__ bias, const float* __restrict__ gamma,
+                       const float* __restrict__ beta, float* out, __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ scale, int64_t M, int N,
+                       float eps) {
+  __shared__ float part[3][8];
+  pdl_trigger();
+  pdl_wait();
+  const int col = threadIdx.x * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const bool mine = col < N;
+  Vec8<float> g{}, b{}, add{};
+  if (mine) {
+    add.load(bias + col);
+    g.load(gamma + col);
+    b.load(beta + col);
+  }
+  for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {
+    Vec8<float> v{};
+    float sum = 0.f;
+    if (mine) {
+      Vec8<float> r;
+      v.load(x + row * N + col);
+      r.load(residual + row * N + col);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v.v[j] = v.v[j] + r.v[j] + add.v[j];
+        sum += v.v[j];
+      }
+    }
+    // (each of the three has its own words, which the next row writes behind the barrier that all have read them before)
+    sum = warp_sum(sum);
+    if (lane == 0) part[0][warp] = sum;
+    __syncthreads();
+    sum = part[0][0];
+    for (int w = 1; w < warps; ++w) sum += part[0][w];
+    const float mean = sum / (float)N;
+    float sq = 0.f;
+    if (mine) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v.v[j] -= mean;
+        sq += v.v[j] * v.v[j];
+      }
+    }
+    sq = warp_sum(sq);
+    if (lane == 0) part[1][warp] = sq;
+    __syncthreads();
+    sq = part[1][0];
+    for (int w = 1; w < warps; ++w) sq += part[1][w];
+    const float rstd = rsqrtf(sq / (float)N + eps);
+    float top = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v.v[j] = b.v[j] + g.v[j] * rstd * v.v[j];
+      top = fmaxf(top, fabsf(v.v[j]));
+    }
+    top = warp_max(top);
+    if (lane == 0) part[2][warp] = top;
+    __syncthreads();
+    top = part[2][0];
+    for (int w = 1; w < warps; ++w) top = fmaxf(top, part[2][w]);
+    float up;
+    const float down = f16_planes_scale(top, &up);
+    if (threadIdx.x == 0) scale[row] = down;
+    if (mine) {
+      v.store(out + row * N + col);
+      uint4 h, l;
+      f16_planes8(v.v, up, &h, &l);
+      *reinterpret_cast<uint4*>(hi + row * N + col) = h;
+      *reinterpret_cast<uint4*>(lo + row * N + col) = l;
+    }
+  }
+}
 int launch_layernorm_split(ttb_ctx* ctx, const float* x, const float* residual, const float* bias, const float* gamma, const float* beta, float* out, __half* hi,
                            __half* lo, float* scale, int64_t M, int64_t N, float eps) {
-  const bool few = M <= 8 * (int64_t)ctx->sm_count;  // (see launch_layernorm)
-  const int few_grid = (int)((M + 1) / 2), grid = grid_for((M + kLnRows - 1) / kLnRows, kLnWarps, ctx->sm_count);
-#define LN_SPLIT(IT)                                                                                                                                      \
-  do {                                                                                                                                                    \
-    if (few)                                                                                                                                              \
-      launch_pdl(layernorm_rows_kernel<float, float, IT, true, 4, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, out,     \
-                 reinterpret_cast<float*>(lo), reinterpret_cast<float*>(hi), M, (int)N, eps, scale);                                                       \
-    else                                                                                                                                                  \
-      launch_pdl(layernorm_rows_kernel<float, float, IT, true, 4, kLnWarps, 1>, dim3(2 * grid), dim3(kLnWarps * 32), 0, ctx->stream, x, residual, bias, gamma, \
-                 beta, out, reinterpret_cast<float*>(lo), reinterpret_cast<float*>(hi), M, (int)N, eps, scale);                                            \
-  } while (0)
-  if (N <= 256) LN_SPLIT(1);
-  else if (N <= 512) LN_SPLIT(2);
-  else if (N <= 768) LN_SPLIT(3);
-  else if (N <= 1024) LN_SPLIT(4);
-  else LN_SPLIT(8);
-#undef LN_SPLIT
+  launch_pdl(layernorm_split_kernel, dim3(grid_for(M, 1, ctx->sm_count)), dim3((N / 8 + 31) / 32 * 32), 0, ctx->stream, x, residual, bias, gamma, beta, out, hi, lo,
+             scale, M, (int)N, eps);
   return launched(ctx, "layernorm_split");
 }
 
@@ -579,25 +600,25 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   do {                                                                                                                           \
     if (few && traded)                                                                                                           \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (few && planes)                                                                                                      \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanes, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (planes)                                                                                                             \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, kPlanesTraded, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (few && extra)                                                                                                       \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (few)                                                                                                                \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, 2, 1>, dim3(few_grid), dim3(64), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else if (extra)                                                                                                              \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 1, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
     else                                                                                                                         \
       launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, 0, kLnWarps, kLnRows>, dim3(grid), dim3(block), 0, ctx->stream, x, residual, bias, gamma, beta, \
-                 out, out_lo, out_f32, M, (int)N, eps, (float*)nullptr);                                                                          \
+                 out, out_lo, out_f32, M, (int)N, eps);                                                                          \
   } while (0)
   const bool aligned = (N % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo) |
                                          reinterpret_cast<uintptr_t>(out_f32) | reinterpret_cast<uintptr_t>(gamma) |
