@@ -88,7 +88,7 @@ DLManagedTensor* NewDLPackTensor(const std::vector<int64_t>& shape, DLDeviceType
 // TTB_BF16_PRECISE=0 or SetPreciseBF16(false) selects plain bf16 storage, which is faster and 8 bits accurate).
 bool PreciseBF16();
 void SetPreciseBF16(bool on);
-// Whether fp32 models run their Linears on the tensor cores as three tf32 products (default on; TTB_FP32_GEMM=simt or
+// Whether fp32 models run their Linears on the tensor cores as three products of planes (default on; TTB_FP32_GEMM=simt or
 // SetFp32TensorCores(false) selects the exact-order CUDA-core GEMM).
 bool Fp32TensorCores();
 void SetFp32TensorCores(bool on);

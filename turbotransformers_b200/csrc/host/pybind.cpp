@@ -112,7 +112,7 @@ PYBIND11_MODULE(turbo_transformers_cxx, m) {
         "bf16 models: keep an fp32 residual stream and hi + lo activation planes between layers (default on).");
   m.def("bf16_precise", []() { return core::PreciseBF16(); });
   m.def("set_fp32_tensor_cores", [](bool on) { core::SetFp32TensorCores(on); },
-        "fp32 models: run Linears on the tensor cores as three tf32 products (default on); off = exact-order CUDA-core GEMM.");
+        "fp32 models: run Linears on the tensor cores as three products of fp16 planes (default on); off = exact-order CUDA-core GEMM.");
   m.def("fp32_tensor_cores", []() { return core::Fp32TensorCores(); });
   m.def("bytes_allocated_total", [](int device) {
     ttb_ctx* c = core::DeviceContext(device);

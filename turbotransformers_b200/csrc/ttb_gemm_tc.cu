@@ -83,7 +83,7 @@ template <int BN, bool TWO = false, bool SK = false, int PA = 1, int PB = 1> str
 // bytes of one row per instruction whatever the row's alignment.
 enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
 
-// Products over two planes of an operand (bf16 hi + lo; fp32 as three tf32 products). On tiles of up to 128 columns, which are bound
+// Products over two planes of an operand (bf16 hi + lo; fp32 as three products). On tiles of up to 128 columns, which are bound
 // by their loads, a ring slot holds both planes of a k-block and all its products are issued from there, so that no plane is
 // fetched twice: fp32 520 x 768 x 3072 51.2 -> 44.7 us, 128 x 768 x 3072 27 -> 17.9, bf16 3200 x 768 x 3072 45 -> 39. Tiles of 256
 // columns, bound by the MMAs, run the products as passes over K: with slots twice the size they have too few of them (bf16
