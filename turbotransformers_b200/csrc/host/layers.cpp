@@ -241,6 +241,11 @@ void PackedLinear::ForwardLayerNorm(const Tensor& x, int64_t M, const void* resi
   Check(ttb_linear_layernorm(c, dt, x.raw(), K, Packed(is_trans), bias_.raw(), residual, N, gamma.raw(), beta.raw(), eps, M, N, K, out, N), c, name);
 }
 
+bool PackedLinear::TakesSplit(const Tensor& x, int64_t M, bool is_trans) const {
+  return core::ToTTBDtype(x.dtype()) == TTB_F32 && M > 0 &&
+         (x.split_only() || (core::Fp32TensorCores() && in_dim(is_trans) % 8 == 0 && (x.split_scale() || !x.lo())));
+}
+
 void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
                            const char* name, int64_t ldo, void* out_lo, bool f32_out, Tensor* q8_of_out, const SplitOut* split_out) const {
   const int dt = FloatType(x, name);
@@ -254,7 +259,8 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
   TT_ENFORCE(ldo == N || (dt != TTB_F32 && !use_int8()), "%s: a padded output pitch is only supported on the 16-bit path", name);
   TT_ENFORCE((!out_lo && !f32_out) || (dt == TTB_BF16 && !use_int8()) || (out_lo && Fp32Planes(dt) && K % 4 == 0),
              "%s: two-plane and fp32 outputs belong to the bf16 path, fp32 planes to the tensor cores", name);
-  if (dt == TTB_F32 && M > 0 && (x.split_only() || (core::Fp32TensorCores() && K % 8 == 0 && (x.split_scale() || !x.lo())))) {
+  if (TakesSplit(x, M, is_trans)) {
+    TT_ENFORCE(!out_lo, "%s: a product of fp16 planes leaves no tf32 planes", name);
     // fp32 on the tensor cores: activation and weight as two fp16 planes each, three products accumulated in one GEMM with the elementwise kernel that followed
     // MatMul in the reference as its epilogue (mat_mul.cpp:81-96 selects tensor-op math for the same product). An activation that brings its planes
     // along is not split again.
@@ -972,7 +978,9 @@ void BertIntermediate::Run(const Tensor& input_tensor, Tensor* output_tensor, bo
     dense_.Forward(input_tensor, input_tensor.rows(), TTB_EPI_BIAS_GELU, nullptr, out, false, "BertIntermediate", 0, nullptr, false, nullptr, &split);
     return;
   }
-  if (for_output && Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0 && dense_.out_dim(false) % 4 == 0) lo = NewLo(output_tensor);
+  // (a product of fp16 planes leaves the activation as it is otherwise, and what takes it next splits it)
+  if (for_output && Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0 && dense_.out_dim(false) % 4 == 0 && !dense_.TakesSplit(input_tensor, input_tensor.rows(), false))
+    lo = NewLo(output_tensor);
   else if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came
     lo = output_tensor->NewExtras().lo.Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "precise/lo_plane");
   // int8 (per-row scheme): BertOutput's Linear takes this activation as int8, so it leaves with its int8 form attached

@@ -67,6 +67,8 @@ class PackedLinear {
   // it, else Forward with the residual epilogue followed by the layer norm kernel.
   void ForwardLayerNorm(const core::Tensor& x, int64_t M, const void* residual, const core::Tensor& gamma, const core::Tensor& beta, float eps,
                         void* out, bool is_trans, const char* name) const;
+  // Whether Forward runs as products of fp16 planes (PackedSplit).
+  bool TakesSplit(const core::Tensor& x, int64_t M, bool is_trans) const;
   // q8_of_out (per-row int8 mode): the tensor that owns `out`; it gets the int8 form of the output attached (q8(), q8_scale()).
   void Forward(const core::Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
                const char* name, int64_t ldo = 0, void* out_lo = nullptr, bool f32_out = false, core::Tensor* q8_of_out = nullptr,
