@@ -14,8 +14,9 @@ AnyTensor = Union[cxx.Tensor, torch.Tensor]
 
 
 def convert2tt_tensor(t: torch.Tensor):
-    """Zero-copy alias of a torch tensor (the layer never writes it)."""
-    return cxx.Tensor.from_dlpack(dlpack.to_dlpack(t if type(t) is torch.Tensor and not t.requires_grad else t.detach()))
+    """Zero-copy alias of a torch tensor (the layer never writes it), of its memory and shape as they are now: the exchange points into
+    the tensor object that is handed over, so that it is given one of its own, whatever is done to the caller's (resize_, set_, .data) while the alias lives."""
+    return cxx.Tensor.from_dlpack(dlpack.to_dlpack(t.detach()))
 
 
 def try_convert(t, device: Optional[torch.device] = None):
