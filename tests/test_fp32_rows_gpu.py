@@ -1,0 +1,49 @@
+"""fp32 layers: what a row of activations comes out as does not depend on how large or small other rows are, nor on how far a weight could take it at most.
+Against plain PyTorch in fp64, with the tolerances that the layers have for rows by themselves.
+"""
+import copy
+
+import pytest
+import torch
+
+import turbotransformers_b200 as tt
+from turbotransformers_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+torch.set_grad_enabled(False)
+DEV = torch.device("cuda:0")
+
+
+def err(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+def layer(bias=0.0):
+    from transformers.models.bert.modeling_bert import BertLayer
+    cfg = synthetic.bert_config("bert-mini", 1)
+    cfg.hidden_act, cfg._attn_implementation = "gelu_new", "eager"
+    layer = synthetic.reinit_(BertLayer(cfg).eval(), 1).to(DEV)
+    for name, p in layer.named_parameters():
+        if name.endswith("bias"):
+            p.mul_(bias)
+    return layer
+
+
+def rows(L, seed=1):
+    return torch.randn(1, L, 256, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV)
+
+
+def attention(block, x, mask=None):
+    out = tt.BertAttention.from_torch(block.attention)(x, mask)[0]
+    double = copy.deepcopy(block.attention).double()
+    return out, double(x.double(), None if mask is None else mask.double())[0]
+
+
+@pytest.mark.parametrize("size", [1.0, 1e-2, 1e-4])
+@pytest.mark.parametrize("L", [2, 65, 300])
+def test_a_row_of_zeros_among_small_ones(built, L, size):
+    block, x = layer(), rows(L) * size
+    x[0, L // 2] = 0
+    out, want = attention(block, x)
+    others = torch.arange(L, device=DEV) != L // 2
+    assert err(out[:, others], want[:, others]) < 2e-6

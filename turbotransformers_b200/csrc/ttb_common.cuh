@@ -170,10 +170,11 @@ template <> __device__ __forceinline__ float rest_of<float>(float v, bool rounde
 
 // An fp32 matrix as two fp16 planes: a row is multiplied by the power of two `up` that brings `most`, a bound of its magnitudes, into [2^14, 2^15);
 // hi is that rounded to fp16, lo what the rounding dropped, rounded likewise: together 2^-23 of an element off at most, like two tf32 planes, or
-// 2^-40 of `most` where that is more (lo is then among fp16's subnormal numbers). Returns the inverse of `up`. (No bound, or none that is a number: 1.)
+// 2^-39 of `most` where that is more (lo is then among fp16's subnormal numbers). Returns the inverse of `up`, between 2^-112 and 2^113: a row below 2^-98, or
+// one of zeros, is multiplied by 2^112 (as the bound of something else it says that there is next to nothing). A bound that is no number: 1.
 __device__ __forceinline__ float f16_planes_scale(float most, float* up) {
   const int e = (int)((__float_as_uint(most) >> 23) & 255);        // the biased exponent
-  const int d = (e == 0 || e == 255) ? 0 : max(-112, min(113, e - 127 - 14));
+  const int d = e == 255 ? 0 : max(-112, e - 127 - 14);
   *up = __uint_as_float((uint32_t)(127 - d) << 23);
   return __uint_as_float((uint32_t)(127 + d) << 23);
 }
