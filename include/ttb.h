@@ -259,21 +259,19 @@ int ttb_linear_layernorm(ttb_ctx* ctx, int dtype, const void* A, int64_t lda, co
 /* hi[i] = x[i] rounded to tf32 (10 mantissa bits), lo[i] = x[i] - hi[i] rounded likewise; x may be hi (in place).
  * The operand planes of the F32 form of ttb_linear_ex. 16-byte aligned pointers. */
 int ttb_split_tf32(ttb_ctx* ctx, const float* x, int64_t n, float* hi, float* lo);
-/* The same for products on the fp16 tensor cores, at twice the rate and half the bytes: every row of x[rows, K] times a power of two as two fp16
- * planes, hi + lo, and scale[rows], the inverse of that power (of two rows' planes, their products and scales multiply). The planes hold an
- * element to 2^-23 of itself, or to 2^-40 of the row's largest where that is more. stats (or NULL): receives {the largest sum of magnitudes of a row, the
- * largest magnitude of bias[n_bias] (or 0)}, which bound what a product makes of a row (ttb_linear_split with out_lo). */
+/* The same for products on the fp16 tensor cores, at twice the rate and half the bytes: every row of x[rows, K] times a power of two (2^112 at most) as two
+ * fp16 planes, hi + lo, and scale[rows], the inverse of that power (of two rows' planes, their products and scales multiply). The planes hold an
+ * element to 2^-23 of itself, or to 2^-39 of the row's largest where that is more. stats (or NULL): receives {the largest sum of magnitudes of a row, the
+ * largest magnitude of bias[n_bias] (or 0)}, which bound what a product makes of a row. */
 int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale, const float* bias, int64_t n_bias, float* stats);
 
 /* out[M,N] = epilogue(A . W^T) in fp32, both operands as planes of ttb_split_f16: hi.hi + lo.hi + hi.lo, accumulated in fp32 (ttb_linear_ex does it with tf32
- * planes). lda in elements, a multiple of 8, like K. With out_lo, the output leaves as such planes, out (hi) and out_lo, with out_scale[M]; `stats` is W's. */
+ * planes). lda in elements, a multiple of 8, like K. */
 typedef struct ttb_linear_split_args {
   const void *A, *A2, *W, *W2;          /* fp16: A[M, lda], A2 (lo); W[N, K], W2 (lo) */
   const float *row_scale, *col_scale;   /* [M], [N] */
   const float *bias, *residual;         /* fp32 */
-  const float* stats;
-  void *out, *out_lo;                   /* fp32 [M, ldo], or two fp16 planes */
-  float* out_scale;
+  float* out;                           /* [M, ldo] */
   int64_t M, N, K, lda, ldr, ldo;
   int32_t epilogue;
 } ttb_linear_split_args;

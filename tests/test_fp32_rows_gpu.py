@@ -8,6 +8,8 @@ import torch
 
 import turbotransformers_b200 as tt
 from turbotransformers_b200 import synthetic
+from turbotransformers_b200._cxx import cxx
+from turbotransformers_b200.layers.modeling_bert import feed_forward as feed_forward_of
 
 pytestmark = pytest.mark.gpu
 torch.set_grad_enabled(False)
@@ -47,3 +49,33 @@ def test_a_row_of_zeros_among_small_ones(built, L, size):
     out, want = attention(block, x)
     others = torch.arange(L, device=DEV) != L // 2
     assert err(out[:, others], want[:, others]) < 2e-6
+
+
+def feed_forward(block, x):
+    """The layer's feed-forward behind its attention's output for x: as this framework runs it, and in 64 bits on the same attention output."""
+    mine = tt.BertLayer.from_torch(block)
+    y = mine.attention(x, return_type=tt.ReturnType.turbo_transformers)[0]
+    exact = torch.from_numpy(cxx.tensor2nparrayf(y)).to(DEV).double().view(x.shape)
+    double = copy.deepcopy(block).double()
+    return feed_forward_of(mine.intermediate, mine.output, y, None), double.output(double.intermediate(exact), exact), mine
+
+
+@pytest.mark.parametrize("L", [9, 300])
+def test_a_weight_that_meets_nothing(built, L):
+    """A weight of 2^24 whose activations are zeros could take the inner activation far, and takes it nowhere."""
+    block = layer(bias=1.0)
+    block.attention.output.LayerNorm.weight[7] = block.attention.output.LayerNorm.bias[7] = 0
+    block.intermediate.dense.weight[5] = 0
+    block.intermediate.dense.weight[5, 7] = 2.0 ** 24
+    out, want, _ = feed_forward(block, rows(L))
+    assert err(out, want) < 2e-6
+
+
+def test_a_bias_that_is_changed_in_place(built):
+    """The runtime reads the caller's bias where it is, at each pass."""
+    block, x = layer(bias=1.0), rows(70)
+    _, _, mine = feed_forward(block, x)
+    block.intermediate.dense.bias.mul_(1e6)
+    y = mine.attention(x, return_type=tt.ReturnType.turbo_transformers)[0]
+    _, want, _ = feed_forward(block, x)
+    assert err(feed_forward_of(mine.intermediate, mine.output, y, None), want) < 2e-6

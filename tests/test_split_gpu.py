@@ -1,6 +1,6 @@
 """fp32 as two scaled fp16 planes: the planes against the values, products of planes against fp64 on every tile (few rows, split along K, wide, pairs, ragged) and
-over the range of scales that fp32 has, and the kernels that leave planes for the next product. Tolerances: planes hold 22 bits of an element and 2^-40
-of the row's bound (2^-39 for the two roundings); the tensor cores truncate their partial sums, 1e-8 of the result a term.
+over the range of scales that fp32 has, and the kernels that leave planes for the next product. Tolerances: planes hold 22 bits of an element and 2^-39
+of the row's largest; the tensor cores truncate their partial sums, 1e-8 of the result a term.
 """
 import pytest
 import torch
@@ -37,7 +37,7 @@ def held(planes, scale, want, bound):
     return bool((off <= 2.0 ** -22 * want.double().abs() + 2.0 ** -39 * bound.double()[:, None]).all())
 
 
-@pytest.mark.parametrize("M,K", [(1, 1), (3, 77), (8, 768), (9, 3072), (1000, 40)])
+@pytest.mark.parametrize("M,K", [(1, 1), (3, 77), (8, 768), (9, 3072), (1000, 40), (1, 8), (2, 264), (5, 8192), (3, 8200), (5000, 768)])
 def test_planes(ctx, M, K):
     x, bias = randn(M, K) * 2.0 ** torch.randint(-90, 90, (M, 1), generator=torch.Generator(device=DEV).manual_seed(2), device=DEV), randn(2 * M + 1, seed=3)
     x[0, 0] = 0
@@ -55,15 +55,10 @@ def test_planes(ctx, M, K):
     assert not value(planes, scale).any()
 
 
-def product(ctx, a, w, N, K, epilogue, planes=False, **more):
+def product(ctx, a, w, N, K, epilogue, **more):
     M = a[1].numel()
-    fields = dict(A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], stats=w[2], **more)
-    if planes:
-        out, scale = torch.full((2, M, N), 7.0, device=DEV).half(), torch.zeros(M, device=DEV)
-        ctx.linear_split(M, N, K, epilogue, out=out[0], out_lo=out[1], out_scale=scale, **fields)
-        return out, scale
     out = torch.full((M, N), 7.0, device=DEV)
-    ctx.linear_split(M, N, K, epilogue, out=out, **fields)
+    ctx.linear_split(M, N, K, epilogue, out=out, A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], **more)
     return out
 
 
@@ -71,18 +66,13 @@ def product(ctx, a, w, N, K, epilogue, planes=False, **more):
                                    (5000, 2304, 768), (77, 770, 8)])
 def test_product(ctx, M, N, K):
     x, w, bias, res = randn(M, K), randn(N, K, seed=2, scale=K ** -0.5), randn(N, seed=3), randn(M, N, seed=4)
-    a, b = split(ctx, x), split(ctx, w, bias)
+    a, b = split(ctx, x), split(ctx, w)
     exact = x.double() @ w.double().T
     gelu = torch.nn.functional.gelu(exact + bias.double(), approximate="tanh")
     tol = 1e-8 * K + 2e-6  # (tanh in fp32 for the second term)
     assert err(product(ctx, a, b, N, K, _capi.EPI_NONE), exact) < 1e-8 * K + 3e-7
     assert err(product(ctx, a, b, N, K, _capi.EPI_BIAS_RESIDUAL, bias=bias, residual=res), exact + bias.double() + res.double()) < tol
-    out = product(ctx, a, b, N, K, _capi.EPI_BIAS_GELU, bias=bias)
-    assert err(out, gelu) < tol
-    planes, scale = product(ctx, a, b, N, K, _capi.EPI_BIAS_GELU, planes=True, bias=bias)
-    bound = 32768 * a[1] * b[2][0] + b[2][1]
-    assert bool((gelu.abs() <= bound.double()[:, None]).all()) and held(planes, scale, value(planes, scale), bound)
-    assert err(value(planes, scale), gelu) < tol and bool((scale * 65504 >= bound).all())
+    assert err(product(ctx, a, b, N, K, _capi.EPI_BIAS_GELU, bias=bias), gelu) < tol
     assert ctx.device_status() == 0
 
 
@@ -138,10 +128,10 @@ def test_attention_leaves_the_planes_of_its_output(ctx, lens):
 
 def test_what_is_refused(ctx):
     x = randn(16, 64)
-    a, w = split(ctx, x), split(ctx, randn(32, 64, seed=2), randn(32, seed=3))
-    out = torch.zeros(2, 16, 32, device=DEV).half()
-    for bad in (dict(A2=None), dict(row_scale=None), dict(col_scale=None), dict(lda=68), dict(K=60), dict(out_lo=out[1]), dict(W2=w[0][1].view(-1)[4:])):
-        fields = dict(dict(A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], out=out[0]), **bad)
+    a, w = split(ctx, x), split(ctx, randn(32, 64, seed=2))
+    out = torch.zeros(16, 32, device=DEV)
+    for bad in (dict(A2=None), dict(row_scale=None), dict(col_scale=None), dict(lda=68), dict(K=60), dict(W2=w[0][1].view(-1)[4:])):
+        fields = dict(dict(A=a[0][0], A2=a[0][1], row_scale=a[1], W=w[0][0], W2=w[0][1], col_scale=w[1], out=out), **bad)
         with pytest.raises(_capi.TTBError):
             ctx.linear_split(16, 32, fields.pop("K", 64), _capi.EPI_NONE, **fields)
     with pytest.raises(_capi.TTBError):

@@ -28,7 +28,7 @@ class LinearArgs(C.Structure):
 
 class LinearSplitArgs(C.Structure):
     """ttb_linear_split_args of include/ttb.h."""
-    _fields_ = [(n, p) for n in ("A", "A2", "W", "W2", "row_scale", "col_scale", "bias", "residual", "stats", "out", "out_lo", "out_scale")] + [
+    _fields_ = [(n, p) for n in ("A", "A2", "W", "W2", "row_scale", "col_scale", "bias", "residual", "out")] + [
         (n, i64) for n in ("M", "N", "K", "lda", "ldr", "ldo")] + [("epilogue", i32)]
 
 

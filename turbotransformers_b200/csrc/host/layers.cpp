@@ -247,7 +247,7 @@ bool PackedLinear::TakesSplit(const Tensor& x, int64_t M, bool is_trans) const {
 }
 
 void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
-                           const char* name, int64_t ldo, void* out_lo, bool f32_out, Tensor* q8_of_out, const SplitOut* split_out) const {
+                           const char* name, int64_t ldo, void* out_lo, bool f32_out, Tensor* q8_of_out) const {
   const int dt = FloatType(x, name);
   SameTypeDevice(x, weight_, name);
   const int64_t K = in_dim(is_trans), N = out_dim(is_trans);
@@ -264,7 +264,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     // fp32 on the tensor cores: activation and weight as two fp16 planes each, three products accumulated in one GEMM with the elementwise kernel that followed
     // MatMul in the reference as its epilogue (mat_mul.cpp:81-96 selects tensor-op math for the same product). An activation that brings its planes
     // along is not split again.
-    const Split w = PackedSplit(is_trans, split_out != nullptr);
+    const Split w = PackedSplit(is_trans, false);
     ttb_linear_split_args args{};
     Tensor planes(nullptr), scale(nullptr);
     if (x.split_scale()) {
@@ -275,16 +275,14 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
       Check(ttb_split_f16(c, x.data<float>(), M, K, a, a + M * K * 2, s, nullptr, 0, nullptr), c, name);
       args.A = a; args.A2 = a + M * K * 2; args.row_scale = s;
     }
-    args.W = w.hi; args.W2 = w.lo; args.col_scale = w.scale; args.stats = w.stats;
+    args.W = w.hi; args.W2 = w.lo; args.col_scale = w.scale;
     args.bias = static_cast<const float*>(bias); args.residual = static_cast<const float*>(residual);
-    args.out = split_out ? split_out->hi : out;
-    args.out_lo = split_out ? split_out->lo : nullptr;
-    args.out_scale = split_out ? split_out->scale : nullptr;
+    args.out = static_cast<float*>(out);
     args.M = M; args.N = N; args.K = K; args.lda = K; args.ldr = N; args.ldo = N; args.epilogue = epilogue;
     Check(ttb_linear_split(c, &args), c, name);
     return;
   }
-  TT_ENFORCE(!split_out && !x.split_only(), "%s: planes without a product that takes them", name);
+  TT_ENFORCE(!x.split_only(), "%s: planes without a product that takes them", name);
   if (dt == TTB_F32 && (core::Fp32TensorCores() || (x.lo() && !x.hi())) && K % 4 == 0 && M > 0) {
     // the same with tf32 planes, for widths that are no multiple of eight
     Tensor planes(nullptr);
@@ -972,13 +970,8 @@ void BertIntermediate::Run(const Tensor& input_tensor, Tensor* output_tensor, bo
   output_tensor->Reshape(input_tensor.dtype(), shape, kDLCUDA, input_tensor.device_id(), "BertIntermediate/Reshape");
   void* out = output_tensor->raw_mut();
   void* lo = nullptr;
-  if (for_output && Fp32Planes(dt) && input_tensor.split_scale() && dense_.out_dim(false) % 8 == 0 && input_tensor.rows() > 0) {
-    const SplitPlanes p = NewSplit(output_tensor, true);
-    const PackedLinear::SplitOut split{p.hi, p.lo, p.scale};
-    dense_.Forward(input_tensor, input_tensor.rows(), TTB_EPI_BIAS_GELU, nullptr, out, false, "BertIntermediate", 0, nullptr, false, nullptr, &split);
-    return;
-  }
-  // (a product of fp16 planes leaves the activation as it is otherwise, and what takes it next splits it)
+  // A product of fp16 planes leaves the activation as it is, and what takes it next splits it: the planes' scale is that of a row's largest, which no
+  // tile of the product knows. (A bound in its place, the row of the input's largest times the weight's largest row sum, may be far from any value.)
   if (for_output && Fp32Planes(dt) && dense_.in_dim(false) % 4 == 0 && dense_.out_dim(false) % 4 == 0 && !dense_.TakesSplit(input_tensor, input_tensor.rows(), false))
     lo = NewLo(output_tensor);
   else if (PreciseMode(dt) && input_tensor.lo() && !dense_.use_int8())  // the activation leaves as two planes, like it came

@@ -41,11 +41,6 @@ class PackedLinear {
   };
   // (The statistics are there where they have been asked for.)
   Split PackedSplit(bool is_trans, bool stats) const;
-  // An output as fp16 planes with a scale for each row.
-  struct SplitOut {
-    void *hi, *lo;
-    float* scale;
-  };
   // int8 [N,K] copy + device scale (built on first use); `col_sum` (may be null) selects the reference recipe's
   // quantiser (torch's per-tensor rule) and receives the per-output-row sums its zero-point correction needs.
   void Int8(bool is_trans, const int8_t** wq, const float** scale, const int32_t** col_sum = nullptr) const;
@@ -71,8 +66,7 @@ class PackedLinear {
   bool TakesSplit(const core::Tensor& x, int64_t M, bool is_trans) const;
   // q8_of_out (per-row int8 mode): the tensor that owns `out`; it gets the int8 form of the output attached (q8(), q8_scale()).
   void Forward(const core::Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
-               const char* name, int64_t ldo = 0, void* out_lo = nullptr, bool f32_out = false, core::Tensor* q8_of_out = nullptr,
-               const SplitOut* split_out = nullptr) const;
+               const char* name, int64_t ldo = 0, void* out_lo = nullptr, bool f32_out = false, core::Tensor* q8_of_out = nullptr) const;
 
  private:
   core::Tensor weight_, bias_;

@@ -89,7 +89,7 @@ enum { STORE_DIRECT = 0, STORE_TMA = 1, STORE_WORDS = 2 };
 // columns, bound by the MMAs, run the products as passes over K: with slots twice the size they have too few of them (bf16
 // 9000 x 2304 x 768 50.6 us in passes, 60.1 from shared slots).
 template <int BN, bool TWO, int KIND, typename OutT, int VAR> struct Planes {
-  static constexpr bool split = KIND == KIND_F16 && VAR >= 5;  // VAR_SPLIT, VAR_SPLIT_PLANES
+  static constexpr bool split = KIND == KIND_F16 && VAR == 5;  // VAR_SPLIT
   static constexpr bool shared = !TWO && BN <= 128 && (KIND == KIND_TF32 || split || (KIND == KIND_BF16 && (sizeof(OutT) == 4 || VAR == 1)));
   static constexpr int A = shared ? 2 : 1;
   static constexpr int B = (shared && (KIND == KIND_TF32 || split)) ? 2 : 1;
@@ -108,8 +108,6 @@ struct GemmParams {
   long long ldr;
   const float* row_scale;  // int8, symmetric: per-row activation scale; fp32 as fp16 planes: what a row of them was divided by
   const float* col_scale;  // fp32 as fp16 planes: the same of W's rows
-  const float* stats;      // planes out: {largest sum of magnitudes of a row of W, largest magnitude of the bias}
-  float* out_scale;        // planes out: [M], what a row of them was divided by
   const float* w_scale;    // int8: device scalar, weight scale
   const float* act_qparams;  // int8, affine per tensor: device [scale, zero point]; null selects the symmetric form
   const int* col_sum;        // int8, affine: sum over k of Wq[n, k]
@@ -197,8 +195,8 @@ template <typename OutT> __device__ __forceinline__ void load32(const OutT* p, f
 //   VAR_PLAIN, VAR_TWO_PLANES (output written with a second plane, what a product drops of the first), VAR_TF32_PLANES (fp32 output rounded to tf32, and
 //   what that dropped; as a choice at run time of the one before, 3 us of 30 at 527 x 3072 x 768), VAR_AFFINE (int8 with a per-tensor zero point),
 //   VAR_WORDS (STORE_WORDS; carried by every kernel it cost packed fp16 batches 1 %: 4120 -> 4164 us, 4149 against 4159 without)
-//   VAR_SPLIT, VAR_SPLIT_PLANES (operands are fp32 as two scaled fp16 planes; the output is fp32, or such planes again)
-enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3, VAR_TF32_PLANES = 4, VAR_SPLIT = 5, VAR_SPLIT_PLANES = 6 };
+//   VAR_SPLIT (operands are fp32 as two scaled fp16 planes)
+enum { VAR_PLAIN = 0, VAR_TWO_PLANES = 1, VAR_AFFINE = 2, VAR_WORDS = 3, VAR_TF32_PLANES = 4, VAR_SPLIT = 5 };
 
 template <int BN, int KIND, typename OutT, bool TWO, bool SK, int VAR, bool LN = false>
 __global__ void __launch_bounds__(Cfg<BN, TWO, SK>::THREADS, 1)
@@ -426,7 +424,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
     const int zero_point = affine ? (int)p.act_qparams[1] : 0;
     constexpr bool rounded = (VAR == VAR_TF32_PLANES), two_planes = (VAR == VAR_TWO_PLANES) || rounded;
     static_assert(!rounded || EB == 4, "planes as tf32 are fp32 words");
-    constexpr bool split = P::split, planes16 = VAR == VAR_SPLIT_PLANES;  // the latter's tiles leave from registers: a row's 32 columns are 64 bytes of each plane
+    constexpr bool split = P::split;
     static_assert(!split || EB == 4, "computed in fp32");
     const bool vec_ok = (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0) &&
                         ((reinterpret_cast<uintptr_t>(p.out_lo) & 15) == 0) &&
@@ -659,7 +657,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       tc_fence_after();
       if (!SK) prefetch_residual(tile + tile_step);  // the next tile's rows, a whole mainloop ahead
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * C::ISSUERS * BN);
-      if (use_tma || (half == 1 && !(planes16 && BN >= 64))) {
+      if (use_tma || half == 1) {
         if (!staged_work) {  // nothing to do for this warp on this tile: just hand the accumulator back
           tc_fence_before();
           __syncwarp();
@@ -846,9 +844,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
       // ---- direct path (narrow tiles or unaligned output): the first warp of each lane quarter walks the tile
       bool gave_up = false;
       float row_max = 0.f;
-      constexpr bool by_half = planes16 && BN >= 64;  // both warps of a lane quarter walk the tile
 #pragma unroll 1
-      for (int c = by_half ? half * (BN / 64) : 0; c < (by_half ? (half + 1) * (BN / 64) : BN / 32); ++c) {
+      for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
         load_sums(taddr + (uint32_t)(c * 32), r);
         const int col0 = n_blk * BN + c * 32;
@@ -933,30 +930,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__
 #pragma unroll
           for (int j = 0; j < 32; ++j)
             if (col0 + j < p.N) row_max = fmaxf(row_max, fabsf(v[j]));
-        }
-        if constexpr (planes16) {
-          float up;
-          const float down = f16_planes_scale(rs * 32768.f * p.stats[0] + p.stats[1], &up);
-          if (n_blk == 0 && c == 0) p.out_scale[row] = down;
-          __half* hi = static_cast<__half*>(p.out) + (long long)row * p.ldo + col0;
-          __half* lo = static_cast<__half*>(p.out_lo) + (long long)row * p.ldo + col0;
-          if (full) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint4 h, l;
-              f16_planes8(&v[i * 8], up, &h, &l);
-              reinterpret_cast<uint4*>(hi)[i] = h;
-              reinterpret_cast<uint4*>(lo)[i] = l;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (col0 + j < p.N) {
-                hi[j] = __float2half_rn(v[j] * up);
-                lo[j] = __float2half_rn(v[j] * up - __half2float(__float2half_rn(v[j] * up)));
-              }
-          }
-          continue;
         }
 #pragma unroll 1
         for (int plane = 0; plane < (two_planes ? 2 : 1); ++plane) {
@@ -1115,7 +1088,7 @@ int launch_tc(ttb_ctx* ctx, const Operands& op, const GemmParams& p) {
   GemmParams q = p;
   q.a_rows = a_rows;
   CUtensorMap tmO = tmA0, tmO2 = tmA0;  // placeholders when the direct-store epilogue is used
-  const bool tma = BN >= 64 && VAR != VAR_SPLIT_PLANES && whole_rows<OutT>(p);
+  const bool tma = BN >= 64 && whole_rows<OutT>(p);
   // Ragged or misaligned rows without bias, residual or second plane (a 50257-wide vocabulary): word stores.
   // 8192 x 50257 x 768 in fp16 into a contiguous tensor: 845 us, against about 560 into padded rows and 585 for the pass that
   // compacted them. What is left over the padded form are the partial 32-byte sectors at both ends of each 128 bytes.
@@ -1414,7 +1387,7 @@ TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, b
 
 template <int KIND, typename OutT, int VAR = VAR_PLAIN>
 int pick_tile(ttb_ctx* ctx, const Operands& op, GemmParams& p) {
-  const TilePlan plan = choose_tile<KIND, OutT, VAR>(ctx, p.M, p.N, p.K, p.npass, VAR != VAR_SPLIT_PLANES && !whole_rows<OutT>(p));
+  const TilePlan plan = choose_tile<KIND, OutT, VAR>(ctx, p.M, p.N, p.K, p.npass, !whole_rows<OutT>(p));
   p.split_k = plan.split_k;
   if (plan.pair) return launch_tc<256, KIND, OutT, true, false, VAR>(ctx, op, p);
   if (plan.split_k > 1) return launch_tc<32, KIND, OutT, false, true, VAR>(ctx, op, p);
@@ -1555,7 +1528,39 @@ __global__ void __launch_bounds__(256) int8_row_sum_kernel(const int8_t* __restr
   if (lane == 0) col_sum[n] = acc;
 }
 
-// Rows of fp32 -> two fp16 planes of a row times the power of two that brings its largest magnitude below 2^15, and its inverse. A warp a row.
+// Rows of fp32 -> two fp16 planes of a row times the power of two that brings its largest magnitude below 2^15, and its inverse. Bound by latency, of
+// activations between two products, and then by memory: a CTA has a row, a thread eight elements of it, which it reads once. us a launch, a warp a row and two
+// reads / now: 128 rows of 768 2.5 / 1.5, of 3072 5.4 / 2.6; 527 rows 2.8 / 2.4, 5.8 / 3.1; 3000 rows 6.2 / 4.7, 21.5 / 9.3.
+__global__ void __launch_bounds__(1024) split_f16_rows_kernel(const float* __restrict__ x, int64_t rows, int K, __half* __restrict__ hi, __half* __restrict__ lo,
+                                                              float* __restrict__ scale) {
+  __shared__ float part[2][32];
+  pdl_trigger();
+  pdl_wait();
+  const int col = threadIdx.x * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  int turn = 0;  // (the next row's maxima are other words: warps may still read these)
+  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, turn ^= 1) {
+    Vec8<float> v{};
+    if (col < K) v.load(x + row * K + col);
+    float top = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) top = fmaxf(top, fabsf(v.v[j]));
+    top = warp_max(top);
+    if (lane == 0) part[turn][warp] = top;
+    __syncthreads();
+    top = warp_max(lane < warps ? part[turn][lane] : 0.f);
+    float up;
+    const float down = f16_planes_scale(top, &up);
+    if (threadIdx.x == 0) scale[row] = down;
+    if (col < K) {
+      uint4 h, l;
+      f16_planes8(v.v, up, &h, &l);
+      *reinterpret_cast<uint4*>(hi + row * K + col) = h;
+      *reinterpret_cast<uint4*>(lo + row * K + col) = l;
+    }
+  }
+}
+
+// The same for rows of any width and alignment, a warp a row.
 // stats: receives the largest sum of magnitudes of a row, and the largest magnitude of the bias (atomic maxima), or null.
 __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, int64_t rows, int K, __half* __restrict__ hi, __half* __restrict__ lo,
                                                         float* __restrict__ scale, const float* __restrict__ bias, int64_t n_bias, float* __restrict__ stats) {
@@ -1676,10 +1681,9 @@ extern "C" int ttb_linear_ex(ttb_ctx* ctx, const ttb_linear_args* a) {
 extern "C" int ttb_linear_split(ttb_ctx* ctx, const ttb_linear_split_args* a) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, a != nullptr, "linear_split: null argument block");
-  const bool planes = a->out_lo != nullptr;
   int s = check_linear(ctx, "linear_split", a->A, a->W, a->bias, a->residual, a->M, a->N, a->K, a->epilogue, a->out, a->ldo, 8);
   if (s || a->M == 0) return s;
-  TTB_REQUIRE(ctx, a->A2 && a->W2 && a->row_scale && a->col_scale && (!planes || (a->out_scale && a->stats)), "linear_split: null pointer");
+  TTB_REQUIRE(ctx, a->A2 && a->W2 && a->row_scale && a->col_scale, "linear_split: null pointer");
   TTB_REQUIRE(ctx, a->lda >= a->K && a->lda % 8 == 0, "linear_split: lda must be >= K and a multiple of 8");
   TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(a->A2) | reinterpret_cast<uintptr_t>(a->W2) | reinterpret_cast<uintptr_t>(a->col_scale)) & 15) == 0,
               "linear_split: operands must be 16-byte aligned");
@@ -1689,12 +1693,12 @@ extern "C" int ttb_linear_split(ttb_ctx* ctx, const ttb_linear_split_args* a) {
   p.npass = 3;
   p.pass_a = 2;  // (A, W), (A2, W), (A, W2)
   p.pass_b = 4;
-  p.out = a->out; p.ldo = a->ldo; p.out_lo = a->out_lo;
+  p.out = a->out; p.ldo = a->ldo;
   p.bias = a->bias; p.residual = a->residual; p.ldr = a->ldr;
-  p.row_scale = a->row_scale; p.col_scale = a->col_scale; p.stats = a->stats; p.out_scale = a->out_scale;
+  p.row_scale = a->row_scale; p.col_scale = a->col_scale;
   p.epilogue = a->epilogue; p.staged = STORE_DIRECT; p.split_k = 1; p.status = ctx->d_status;
   const Operands op{a->A, a->A2, a->lda, a->W, a->W2};
-  return planes ? pick_tile<KIND_F16, float, VAR_SPLIT_PLANES>(ctx, op, p) : pick_tile<KIND_F16, float, VAR_SPLIT>(ctx, op, p);
+  return pick_tile<KIND_F16, float, VAR_SPLIT>(ctx, op, p);
 }
 
 extern "C" int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale, const float* bias, int64_t n_bias, float* stats) {
@@ -1704,6 +1708,12 @@ extern "C" int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t
   TTB_REQUIRE(ctx, x && hi && lo && scale && (!bias || stats), "split_f16: null pointer");
   DeviceGuard g(ctx->device);
   if (stats) TTB_CUDA(ctx, cudaMemsetAsync(stats, 0, 2 * sizeof(float), ctx->stream));
+  const bool eights = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0;
+  if (eights && K <= 8192 && !stats) {
+    launch_pdl(split_f16_rows_kernel, dim3((unsigned)std::min<int64_t>(rows, 16 * (int64_t)ctx->sm_count)), dim3((unsigned)((K / 8 + 31) / 32 * 32)), 0, ctx->stream, x, rows,
+               (int)K, (__half*)hi, (__half*)lo, scale);
+    return launched(ctx, "split_f16");
+  }
   launch_pdl(split_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, ctx->stream, x, rows, (int)K, (__half*)hi, (__half*)lo, scale, bias, bias ? n_bias : (int64_t)0,
              stats);
   return launched(ctx, "split_f16");
@@ -1717,9 +1727,8 @@ extern "C" int ttb_linear_plan(ttb_ctx* ctx, int dtype, int out_dtype, int produ
   DeviceGuard g(ctx->device);
   TilePlan t{};
   const bool words = !whole;
-  if (dtype == TTB_F16 && out_dtype == TTB_F32 && products == 3) {  // fp32 as fp16 planes
-    t = two_plane_out ? choose_tile<KIND_F16, float, VAR_SPLIT_PLANES>(ctx, M, N, K, 3, false) : choose_tile<KIND_F16, float, VAR_SPLIT>(ctx, M, N, K, 3, words);
-  } else if (dtype == TTB_F32 && out_dtype == TTB_F32 && products >= 1 && products <= 3) t = choose_tile<KIND_TF32, float, VAR_PLAIN>(ctx, M, N, K, products, words);
+  if (dtype == TTB_F16 && out_dtype == TTB_F32 && products == 3) t = choose_tile<KIND_F16, float, VAR_SPLIT>(ctx, M, N, K, 3, words);  // fp32 as fp16 planes
+  else if (dtype == TTB_F32 && out_dtype == TTB_F32 && products >= 1 && products <= 3) t = choose_tile<KIND_TF32, float, VAR_PLAIN>(ctx, M, N, K, products, words);
   else if (dtype == TTB_I8 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_I8, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
   else if (dtype == TTB_F16 && out_dtype == TTB_F16 && products == 1) t = choose_tile<KIND_F16, __half, VAR_PLAIN>(ctx, M, N, K, 1, words);
   else if (dtype == TTB_BF16 && out_dtype == TTB_F32 && (products == 1 || products == 2)) t = choose_tile<KIND_BF16, float, VAR_PLAIN>(ctx, M, N, K, products, words);
