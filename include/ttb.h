@@ -261,9 +261,8 @@ int ttb_linear_layernorm(ttb_ctx* ctx, int dtype, const void* A, int64_t lda, co
 int ttb_split_tf32(ttb_ctx* ctx, const float* x, int64_t n, float* hi, float* lo);
 /* The same for products on the fp16 tensor cores, at twice the rate and half the bytes: every row of x[rows, K] times a power of two (2^112 at most) as two
  * fp16 planes, hi + lo, and scale[rows], the inverse of that power (of two rows' planes, their products and scales multiply). The planes hold an
- * element to 2^-23 of itself, or to 2^-39 of the row's largest where that is more. stats (or NULL): receives {the largest sum of magnitudes of a row, the
- * largest magnitude of bias[n_bias] (or 0)}, which bound what a product makes of a row. */
-int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale, const float* bias, int64_t n_bias, float* stats);
+ * element to 2^-23 of itself, or to 2^-39 of the row's largest where that is more. */
+int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale);
 
 /* out[M,N] = epilogue(A . W^T) in fp32, both operands as planes of ttb_split_f16: hi.hi + lo.hi + hi.lo, accumulated in fp32 (ttb_linear_ex does it with tf32
  * planes). lda in elements, a multiple of 8, like K. */
@@ -277,15 +276,12 @@ typedef struct ttb_linear_split_args {
 } ttb_linear_split_args;
 int ttb_linear_split(ttb_ctx* ctx, const ttb_linear_split_args* args);
 /* Kernels that leave such planes, hi and lo with scale[rows], for the next product: out = LayerNorm(out + input + bias) in place (N % 8 == 0, N <= 2048, 16-byte
- * aligned); ttb_embedding_ln in F32; ttb_attention_f32 in place of its output, where row_scale and stats are those of the product that made qkv. */
+ * aligned); ttb_embedding_ln in F32. */
 int ttb_add_bias_layernorm_split(ttb_ctx* ctx, float* out, void* hi, void* lo, float* scale, const float* input, const float* bias, const float* gamma,
                                  const float* beta, int64_t M, int64_t N, float eps);
 int ttb_embedding_ln_split(ttb_ctx* ctx, const int64_t* ids, const int64_t* position_ids, const int64_t* token_type_ids, const int32_t* cu_seqlens, int64_t B,
                            int64_t seq_len, int64_t n_tokens, const float* word, const float* position, const float* token_type, const float* gamma, const float* beta,
                            int64_t hidden, int64_t vocab, int64_t n_positions, int64_t n_types, float eps, float* out, void* hi, void* lo, float* scale);
-int ttb_attention_f32_split(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
-                            int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, const float* row_scale, const float* stats, void* hi,
-                            void* lo, float* out_scale);
 
 /* int8 x int8 -> int32 (tcgen05 kind::i8), out = epilogue(acc * row_scale[m] * *w_scale + bias), out dtype
  * F16/BF16. Replaces the torch dynamic-quantised Linear + FusedAddBiasGELU / FusedAddBiasLayerNorm glue of

@@ -51,6 +51,17 @@ def test_a_row_of_zeros_among_small_ones(built, L, size):
     assert err(out[:, others], want[:, others]) < 2e-6
 
 
+@pytest.mark.parametrize("L", [9, 300])
+def test_a_value_weight_that_meets_nothing(built, L):
+    """The same as below of the attention's values and output."""
+    block, x = layer(bias=1.0), rows(L)
+    x[..., 7] = 0
+    block.attention.self.value.weight[5] = 0
+    block.attention.self.value.weight[5, 7] = 2.0 ** 24
+    out, want = attention(block, x)
+    assert err(out, want) < 2e-6
+
+
 def feed_forward(block, x):
     """The layer's feed-forward behind its attention's output for x: as this framework runs it, and in 64 bits on the same attention output."""
     mine = tt.BertLayer.from_torch(block)

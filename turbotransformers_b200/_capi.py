@@ -116,10 +116,9 @@ SIGNATURES = {
     "ttb_linear_ex": (i32, [p, C.POINTER(LinearArgs)]),
     "ttb_linear_plan": (i32, [p, i32, i32, i32, i32, i32, i64, i64, i64, C.POINTER(i64)]),
     "ttb_split_tf32": (i32, [p, p, i64, p, p]),
-    "ttb_split_f16": (i32, [p, p, i64, i64, p, p, p, p, i64, p]),
+    "ttb_split_f16": (i32, [p, p, i64, i64, p, p, p]),
     "ttb_add_bias_layernorm_split": (i32, [p, p, p, p, p, p, p, p, p, i64, i64, f32]),
     "ttb_embedding_ln_split": (i32, [p, p, p, p, p, i64, i64, i64, p, p, p, p, p, i64, i64, i64, i64, f32, p, p, p, p]),
-    "ttb_attention_f32_split": (i32, [p, p, p, i64, i64, i64, i64, p, i64, i64, i32, f32, p, p, p, p, p]),
     "ttb_linear_split": (i32, [p, C.POINTER(LinearSplitArgs)]),
     "ttb_linear_layernorm": (i32, [p, i32, p, i64, p, p, p, i64, p, p, f32, i64, i64, i64, p, i64]),
     "ttb_prepack_weight_int8_affine": (i32, [p, i32, p, i32, i64, i64, p, p, p]),

@@ -163,12 +163,11 @@ class Tensor {
   //         that travels between two of the runtime's own products only, or with hi, what rounding to tf32 dropped
   //   f32 : same shape in fp32, the unrounded value (the residual stream of a bf16 model)
   //   hi  : of an fp32 activation, the value rounded to tf32 (the tensor itself is the unrounded value, hi + lo what a product reads)
-  //   split_scale : of an fp32 activation, [rows]: hi and lo are then its fp16 planes (ttb_split_f16). Where split_only, the tensor itself is not written
+  //   split_scale : of an fp32 activation, [rows]: hi and lo are then its fp16 planes (ttb_split_f16).
   const Tensor* lo() const;
   const Tensor* f32() const;
   const Tensor* hi() const;
   const Tensor* split_scale() const;
-  bool split_only() const;
   const Tensor* q8() const;
   const Tensor* q8_scale() const;
   TensorExtras& NewExtras();
@@ -189,7 +188,6 @@ struct TensorExtras {
   Tensor f32{nullptr};
   Tensor hi{nullptr};
   Tensor split_scale{nullptr};
-  bool split_only = false;
   // int8 models: the per-row symmetric int8 form of this activation and its row scales, written by the layer norm that
   // produced it so that the next int8 Linear does not quantise it again
   Tensor q8{nullptr};
@@ -199,7 +197,6 @@ inline const Tensor* Tensor::lo() const { return extras_ && !extras_->lo.is_null
 inline const Tensor* Tensor::f32() const { return extras_ && !extras_->f32.is_null() ? &extras_->f32 : nullptr; }
 inline const Tensor* Tensor::hi() const { return extras_ && !extras_->hi.is_null() ? &extras_->hi : nullptr; }
 inline const Tensor* Tensor::split_scale() const { return extras_ && !extras_->split_scale.is_null() ? &extras_->split_scale : nullptr; }
-inline bool Tensor::split_only() const { return extras_ && extras_->split_only; }
 inline const Tensor* Tensor::q8() const { return extras_ && !extras_->q8.is_null() ? &extras_->q8 : nullptr; }
 inline const Tensor* Tensor::q8_scale() const { return extras_ && !extras_->q8_scale.is_null() ? &extras_->q8_scale : nullptr; }
 inline TensorExtras& Tensor::NewExtras() {

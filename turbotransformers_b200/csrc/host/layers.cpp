@@ -58,9 +58,8 @@ struct SplitPlanes {
   void *hi, *lo;
   float* scale;
 };
-SplitPlanes NewSplit(Tensor* t, bool only) {
+SplitPlanes NewSplit(Tensor* t) {
   core::TensorExtras& ex = t->NewExtras();
-  ex.split_only = only;
   SplitPlanes p;
   p.hi = ex.hi.Reshape(core::kFloat16, ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/hi_plane");
   p.lo = ex.lo.Reshape(core::kFloat16, ShapeOf(*t), kDLCUDA, t->device_id(), "fp32/lo_plane");
@@ -104,7 +103,7 @@ void AddBiasLayerNormF32(ttb_ctx* c, Tensor* t, const Tensor& input, const Tenso
                          const char* name) {
   float* out = t->mutableData<float>();
   if (Fp32Planes(TTB_F32) && SplitWidth(N) && M > 0 && Aligned16({out, input.raw(), bias.raw(), gamma.raw(), beta.raw()})) {
-    const SplitPlanes p = NewSplit(t, false);
+    const SplitPlanes p = NewSplit(t);
     Check(ttb_add_bias_layernorm_split(c, out, p.hi, p.lo, p.scale, input.data<float>(), bias.data<float>(), gamma.data<float>(), beta.data<float>(), M, N, 1e-12f), c,
           name);
     return;
@@ -156,25 +155,21 @@ const float* PackedLinear::PackedTf32(bool is_trans) const {
   return p.data<float>();
 }
 
-PackedLinear::Split PackedLinear::PackedSplit(bool is_trans, bool stats) const {
+PackedLinear::Split PackedLinear::PackedSplit(bool is_trans) const {
   std::lock_guard<std::mutex> g(cache_->mu);
   Tensor &planes = cache_->split[is_trans ? 1 : 0], &scale = cache_->split_scale[is_trans ? 1 : 0];
   const int64_t K = in_dim(is_trans), N = out_dim(is_trans);
-  bool& has_stats = cache_->split_stats[is_trans ? 1 : 0];
-  if (planes.is_null() || (stats && !has_stats)) {
+  if (planes.is_null()) {
     ttb_ctx* c = DeviceContext(weight_.device_id());
     Tensor rows(nullptr);
     float* w = rows.Reshape<float>({N, K}, kDLCUDA, weight_.device_id(), "linear/rows_of_weight");
     Check(ttb_prepack_weight(c, TTB_F32, weight_.raw(), is_trans ? 1 : 0, K, N, TTB_F32, w), c, "prepack_weight");
-    float* s = scale.Reshape<float>({2 + (N + 3) / 4 * 4}, kDLCUDA, weight_.device_id(), "linear/split_weight_scales");
+    float* s = scale.Reshape<float>({N}, kDLCUDA, weight_.device_id(), "linear/split_weight_scales");
     char* p = static_cast<char*>(planes.Reshape(core::kFloat16, {2, N, K}, kDLCUDA, weight_.device_id(), "linear/split_weight_planes"));
-    const bool bias = stats && !bias_.is_null();
-    Check(ttb_split_f16(c, w, N, K, p, p + N * K * 2, s, bias ? bias_.data<float>() : nullptr, bias ? bias_.numel() : 0, stats ? s + (N + 3) / 4 * 4 : nullptr), c,
-          "split_f16");
-    has_stats = stats;
+    Check(ttb_split_f16(c, w, N, K, p, p + N * K * 2, s), c, "split_f16");
   }
   const char* p = static_cast<const char*>(planes.raw());
-  return {p, p + N * K * 2, scale.data<float>(), scale.data<float>() + (N + 3) / 4 * 4};
+  return {p, p + N * K * 2, scale.data<float>()};
 }
 
 const float* PackedLinear::BiasF32() const {
@@ -243,7 +238,7 @@ void PackedLinear::ForwardLayerNorm(const Tensor& x, int64_t M, const void* resi
 
 bool PackedLinear::TakesSplit(const Tensor& x, int64_t M, bool is_trans) const {
   return core::ToTTBDtype(x.dtype()) == TTB_F32 && M > 0 &&
-         (x.split_only() || (core::Fp32TensorCores() && in_dim(is_trans) % 8 == 0 && (x.split_scale() || !x.lo())));
+         core::Fp32TensorCores() && in_dim(is_trans) % 8 == 0 && (x.split_scale() || !x.lo());
 }
 
 void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void* residual, void* out, bool is_trans,
@@ -264,7 +259,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     // fp32 on the tensor cores: activation and weight as two fp16 planes each, three products accumulated in one GEMM with the elementwise kernel that followed
     // MatMul in the reference as its epilogue (mat_mul.cpp:81-96 selects tensor-op math for the same product). An activation that brings its planes
     // along is not split again.
-    const Split w = PackedSplit(is_trans, false);
+    const Split w = PackedSplit(is_trans);
     ttb_linear_split_args args{};
     Tensor planes(nullptr), scale(nullptr);
     if (x.split_scale()) {
@@ -272,7 +267,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     } else {
       char* a = static_cast<char*>(planes.Reshape(core::kFloat16, {2, M, K}, kDLCUDA, x.device_id(), "linear/split_activation_planes"));
       float* s = scale.Reshape<float>({M}, kDLCUDA, x.device_id(), "linear/split_activation_scales");
-      Check(ttb_split_f16(c, x.data<float>(), M, K, a, a + M * K * 2, s, nullptr, 0, nullptr), c, name);
+      Check(ttb_split_f16(c, x.data<float>(), M, K, a, a + M * K * 2, s), c, name);
       args.A = a; args.A2 = a + M * K * 2; args.row_scale = s;
     }
     args.W = w.hi; args.W2 = w.lo; args.col_scale = w.scale;
@@ -282,7 +277,6 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     Check(ttb_linear_split(c, &args), c, name);
     return;
   }
-  TT_ENFORCE(!x.split_only(), "%s: planes without a product that takes them", name);
   if (dt == TTB_F32 && (core::Fp32TensorCores() || (x.lo() && !x.hi())) && K % 4 == 0 && M > 0) {
     // the same with tf32 planes, for widths that are no multiple of eight
     Tensor planes(nullptr);
@@ -404,7 +398,7 @@ void BERTEmbedding::operator()(const Tensor& input_ids, const Tensor& position_i
     lo = ex.lo.Reshape(word_embedings_.dtype(), {B, L, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({B, L, H}, kDLCUDA, dev, "precise/residual_stream");
   } else if (Fp32Planes(dt) && SplitWidth(H) && B * L > 0) {
-    const SplitPlanes p = NewSplit(output_tensor, false);
+    const SplitPlanes p = NewSplit(output_tensor);
     Check(ttb_embedding_ln_split(c, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
                                  token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), nullptr, B, L, B * L, word_embedings_.data<float>(),
                                  position_embeddings_.data<float>(), token_type_embeddings_.data<float>(), layer_norm_weights_.data<float>(),
@@ -444,7 +438,7 @@ void BERTEmbedding::Packed(const Tensor& input_ids, const std::vector<int64_t>& 
     lo = ex.lo.Reshape(word_embedings_.dtype(), {1, T, H}, kDLCUDA, dev, "precise/lo_plane");
     f32 = ex.f32.Reshape<float>({1, T, H}, kDLCUDA, dev, "precise/residual_stream");
   } else if (Fp32Planes(dt) && SplitWidth(H) && T > 0) {
-    const SplitPlanes p = NewSplit(output_tensor, false);
+    const SplitPlanes p = NewSplit(output_tensor);
     const core::CuSeqlensHandle cu = core::CuSeqlens(dev, seq_lens);
     Check(ttb_embedding_ln_split(c, input_ids.data<int64_t>(), position_ids.is_null() ? nullptr : position_ids.data<int64_t>(),
                                  token_type_ids.is_null() ? nullptr : token_type_ids.data<int64_t>(), cu.get(), (int64_t)seq_lens.size(), 0, T,
@@ -679,14 +673,7 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
   } else if (Fp32Planes(dt) && !att_score && !cache_keys && d == 64 && B <= 65535 && (!causal_ || !attention_mask.is_null())) {
     // fp32 without a request for the scores: one kernel on the packed rows, whose keys are each sequence's own (a causal layer's
     // mask tensor says what its rows see, as it does in the sequence below; the kernel's own causal form is the C call's)
-    Tensor qkv(nullptr), planes_in(nullptr);
-    if (H % 8 == 0 && T > 0) qkv_.PackedSplit(is_trans_weight, true);
-    if (!gemm_in->lo() && T > 0) {  // planes here, so that the attention kernel knows what bounds the values whether the input brought its own or not
-      planes_in.Reshape(x.dtype(), {T, H}, kDLCUDA, dev, "self/planes_in");
-      const SplitPlanes p = NewSplit(&planes_in, true);
-      Check(ttb_split_f16(c, gemm_in->data<float>(), T, H, p.hi, p.lo, p.scale, nullptr, 0, nullptr), c, "self/split_f16");
-      gemm_in = &planes_in;
-    }
+    Tensor qkv(nullptr);
     qkv.Reshape(x.dtype(), {T, 3 * H}, kDLCUDA, dev, "self/qkv_out1/Reshape");
     qkv_.Forward(*gemm_in, T, TTB_EPI_BIAS, nullptr, qkv.raw_mut(), is_trans_weight, "self/gemm012_fused");
     const core::CuSeqlensHandle cu_handle = seq_lens ? core::CuSeqlens(dev, *seq_lens) : core::UniformCuSeqlens(dev, B, maxL);
@@ -700,16 +687,9 @@ void MultiHeadedAttention::Run(const Tensor& x, const Tensor& attention_mask, co
       if (MaskIs2D(attention_mask)) { mbs = maxL; mrs = 0; }
       else { mrs = maxL; mbs = maxL * maxL; }
     }
-    if (gemm_in->split_scale() && T > 0) {  // the output as fp16 planes, within the bound that the product's operands give for the values
-      const SplitPlanes p = NewSplit(&context, true);
-      Check(ttb_attention_f32_split(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, gemm_in->split_scale()->data<float>(),
-                                    qkv_.PackedSplit(is_trans_weight, true).stats, p.hi, p.lo, p.scale),
-            c, "attention_f32");
-    } else {
-      float* hi = context.mutableData<float>();
-      float* lo = NewLo(&context);
-      Check(ttb_attention_f32_planes(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, hi, lo), c, "attention_f32");
-    }
+    // (as it is: the planes' scale is that of a row's largest over all heads, which a CTA does not know, and the product splits it)
+    Check(ttb_attention_f32(c, qkv.data<float>(), cu_handle.get(), B, maxL, heads, d, mask, mbs, mrs, 0, scale, context.mutableData<float>(), nullptr), c,
+          "attention_f32");
   } else {
     // The reference's own sequence (multi_headed_attention.cpp:168-232,320-354), scores materialised.
     TT_ENFORCE(!cache_keys, "layer_cache decoding is provided for 16-bit models with 64-wide heads");

@@ -34,13 +34,12 @@ class PackedLinear {
   const void* Packed(bool is_trans) const;
   // fp32 weights as two tf32 planes [2][N,K] (hi, then lo), for the three-product tensor-core GEMM of widths that are no multiple of eight.
   const float* PackedTf32(bool is_trans) const;
-  // fp32 weights as two fp16 planes [N,K] with a scale for each row, and {largest sum of magnitudes of a row, largest magnitude of the bias} (ttb_split_f16).
+  // fp32 weights as two fp16 planes [N,K] with a scale for each row (ttb_split_f16).
   struct Split {
     const void *hi, *lo;
-    const float *scale, *stats;
+    const float* scale;
   };
-  // (The statistics are there where they have been asked for.)
-  Split PackedSplit(bool is_trans, bool stats) const;
+  Split PackedSplit(bool is_trans) const;
   // int8 [N,K] copy + device scale (built on first use); `col_sum` (may be null) selects the reference recipe's
   // quantiser (torch's per-tensor rule) and receives the per-output-row sums its zero-point correction needs.
   void Int8(bool is_trans, const int8_t** wq, const float** scale, const int32_t** col_sum = nullptr) const;
@@ -77,7 +76,6 @@ class PackedLinear {
     core::Tensor tf32[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor split[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor split_scale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
-    bool split_stats[2] = {false, false};
     core::Tensor q[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qscale[2]{core::Tensor(nullptr), core::Tensor(nullptr)};
     core::Tensor qref[2]{core::Tensor(nullptr), core::Tensor(nullptr)};

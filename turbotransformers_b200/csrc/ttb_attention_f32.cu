@@ -33,15 +33,6 @@ union Shared {
   float out[kWarps][16 * kOutPitch];
 };
 
-// What the planes of the output in fp16 take: of the rows that the queries, keys and values were computed from, what they were divided by, and the weights'
-// statistics (ttb_split_f16), which bound the values and so their averages; the planes' own scale.
-struct SplitOut {
-  const float *row_scale, *stats;
-  __half *hi, *lo;
-  float* scale;
-};
-enum { OUT_VALUE = 0, OUT_TF32 = 1, OUT_F16 = 2 };
-
 __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
@@ -64,12 +55,11 @@ __device__ __forceinline__ void planes2(float x, float y, uint32_t* hi, uint32_t
   *lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-// OUT: the output leaves as it is, or as its two planes, in place of it.
-template <int WR, int OUT>
+// ROUNDED: the output leaves as its two tf32 planes.
+template <int WR, bool ROUNDED>
 __global__ void __launch_bounds__(kThreads)
 attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ cu, int heads, const float* __restrict__ mask, long long mask_batch,
-                     long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo, const SplitOut split) {
-  constexpr bool ROUNDED = OUT == OUT_TF32;
+                     long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo) {
   constexpr int WK = kWarps / WR, kRows = 16 * WR, kMine = kKeys / WK, NT = kMine / 8;  // keys of a tile for a warp, in eights
   __shared__ __align__(16) Shared sm;
   __shared__ int v_most[2];
@@ -268,13 +258,6 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
     }
   }
   __syncthreads();
-  float up = 1.f;
-  if constexpr (OUT == OUT_F16) {  // one scale for all heads and rows of the sequence: no value of it is beyond this bound
-    float most = 0.f;
-    for (int j = lane; j < len; j += 32) most = fmaxf(most, split.row_scale[begin + j]);
-    const float down = f16_planes_scale(warp_max(most) * 32768.f * split.stats[0] + split.stats[1], &up);
-    if (h == 0 && tid < kRows && q0 + tid < len) split.scale[begin + q0 + tid] = down;
-  }
 #pragma unroll
   for (int n = 0; n < 2 * WR; ++n) {
     const int r = (n * kThreads + tid) >> 4, c = (tid & 15) * 4, i = q0 + r;
@@ -296,34 +279,26 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
     const float inv = 1.0f / sum;
     y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
     const long long at = (long long)(begin + i) * H + h * D + c;
-    if constexpr (OUT == OUT_F16) {
-      uint2 hi, lo;
-      planes2(y.x * up, y.y * up, &hi.x, &lo.x);
-      planes2(y.z * up, y.w * up, &hi.y, &lo.y);
-      *reinterpret_cast<uint2*>(split.hi + at) = hi;
-      *reinterpret_cast<uint2*>(split.lo + at) = lo;
-      continue;
-    }
     *reinterpret_cast<float4*>(out + at) = ROUNDED ? make_float4(tf32_hi(y.x), tf32_hi(y.y), tf32_hi(y.z), tf32_hi(y.w)) : y;
     if (ROUNDED || out_lo) *reinterpret_cast<float4*>(out_lo + at) = make_float4(tf32_lo(y.x, ROUNDED), tf32_lo(y.y, ROUNDED), tf32_lo(y.z, ROUNDED), tf32_lo(y.w, ROUNDED));
   }
 }
 
-template <int OUT>
+template <bool ROUNDED>
 int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
-                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo, const SplitOut& split = SplitOut()) {
+                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
   if (!ctx) return TTB_ERR_INVALID;
   TTB_REQUIRE(ctx, d == D && heads > 0 && heads <= 65535 && B >= 0 && B <= 65535 && max_seqlen >= 0 && max_seqlen < (1 << 30), "attention_f32: bad shape");
   if (B == 0 || max_seqlen == 0) return TTB_OK;
-  TTB_REQUIRE(ctx, qkv && cu_seqlens && (out || OUT == OUT_F16), "attention_f32: null pointer");
+  TTB_REQUIRE(ctx, qkv && cu_seqlens && out, "attention_f32: null pointer");
   TTB_REQUIRE(ctx, ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_lo)) & 15) == 0,
               "attention_f32: buffers must be 16-byte aligned");
   DeviceGuard g(ctx->device);
   auto blocks = [&](int rows) { return dim3((unsigned)((max_seqlen + rows - 1) / rows), (unsigned)heads, (unsigned)B); };
   auto ctas = [&](int64_t rows) { return B * heads * ((max_seqlen + rows - 1) / rows); };
 #define ATTENTION_F32(WR)                                                                                                                                  \
-  launch_pdl(attention_f32_kernel<WR, OUT>, blocks(16 * WR), dim3(kThreads), 0, ctx->stream, qkv, cu_seqlens, (int)heads, mask, (long long)mask_batch_stride, \
-             (long long)mask_row_stride, causal, scale, out, out_lo, split)
+  launch_pdl(attention_f32_kernel<WR, ROUNDED>, blocks(16 * WR), dim3(kThreads), 0, ctx->stream, qkv, cu_seqlens, (int)heads, mask, (long long)mask_batch_stride, \
+             (long long)mask_row_stride, causal, scale, out, out_lo)
   // The most rows a CTA with which the chip is still full: us with 16, 32, 64 rows: 192 CTAs of 64 rows (384 of 32) 10.4, 12.4, 15.6; 324 (648) 36, 27.5, 23.1; 252
   // (504) 37.7, 32.8, 44.6; 96 (192) 28.6, 36, 44.7; 768 181, 128, 101.
   if (ctas(64) >= 2 * ctx->sm_count) ATTENTION_F32(4);
@@ -337,21 +312,11 @@ int attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int
 
 extern "C" int ttb_attention_f32(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d, const float* mask,
                                  int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* out, float* out_lo) {
-  return attention_f32<OUT_VALUE>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, out, out_lo);
+  return attention_f32<false>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, out, out_lo);
 }
 
 extern "C" int ttb_attention_f32_planes(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
                                         const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, float* hi, float* lo) {
   if (ctx && B > 0 && max_seqlen > 0) TTB_REQUIRE(ctx, lo, "attention_f32_planes: null pointer");
-  return attention_f32<OUT_TF32>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, hi, lo);
-}
-
-extern "C" int ttb_attention_f32_split(ttb_ctx* ctx, const float* qkv, const int32_t* cu_seqlens, int64_t B, int64_t max_seqlen, int64_t heads, int64_t d,
-                                       const float* mask, int64_t mask_batch_stride, int64_t mask_row_stride, int causal, float scale, const float* row_scale,
-                                       const float* stats, void* hi, void* lo, float* out_scale) {
-  if (ctx && B > 0 && max_seqlen > 0)
-    TTB_REQUIRE(ctx, row_scale && stats && hi && lo && out_scale && ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 7) == 0,
-                "attention_f32_split: null or misaligned pointer");
-  return attention_f32<OUT_F16>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, nullptr, nullptr,
-                                SplitOut{row_scale, stats, static_cast<__half*>(hi), static_cast<__half*>(lo), out_scale});
+  return attention_f32<true>(ctx, qkv, cu_seqlens, B, max_seqlen, heads, d, mask, mask_batch_stride, mask_row_stride, causal, scale, hi, lo);
 }

@@ -1561,53 +1561,20 @@ __global__ void __launch_bounds__(1024) split_f16_rows_kernel(const float* __res
 }
 
 // The same for rows of any width and alignment, a warp a row.
-// stats: receives the largest sum of magnitudes of a row, and the largest magnitude of the bias (atomic maxima), or null.
 __global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, int64_t rows, int K, __half* __restrict__ hi, __half* __restrict__ lo,
-                                                        float* __restrict__ scale, const float* __restrict__ bias, int64_t n_bias, float* __restrict__ stats) {
+                                                        float* __restrict__ scale) {
   pdl_trigger();
   pdl_wait();
   const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   const float* src = x + row * K;
-  const bool eights = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0;
-  float top = 0.f, sum = 0.f;
-  auto count = [&](float v) {
-    top = fmaxf(top, fabsf(v));
-    sum += fabsf(v);
-  };
-  if (eights) {
+  float top = 0.f;
 #pragma unroll 4
-    for (int k = lane * 4; k < K; k += 128) {
-      const float4 v = *reinterpret_cast<const float4*>(src + k);
-      count(v.x); count(v.y); count(v.z); count(v.w);
-    }
-  } else {
-    for (int k = lane; k < K; k += 32) count(src[k]);
-  }
-  top = warp_max(top);
-  sum = warp_sum(sum);
+  for (int k = lane; k < K; k += 32) top = fmaxf(top, fabsf(src[k]));
   float up;
-  const float down = f16_planes_scale(top, &up);
-  if (lane == 0) {
-    scale[row] = down;
-    if (stats) {  // (non-negative floats order like their bits)
-      atomicMax(reinterpret_cast<int*>(stats), __float_as_int(sum));
-      for (int64_t i = row; i < n_bias; i += rows) atomicMax(reinterpret_cast<int*>(stats + 1), __float_as_int(fabsf(bias[i])));
-    }
-  }
-  if (eights) {
-#pragma unroll 2
-    for (int k = lane * 8; k < K; k += 256) {
-      Vec8<float> v;
-      v.load(src + k);
-      uint4 h, l;
-      f16_planes8(v.v, up, &h, &l);
-      *reinterpret_cast<uint4*>(hi + row * K + k) = h;
-      *reinterpret_cast<uint4*>(lo + row * K + k) = l;
-    }
-    return;
-  }
+  const float down = f16_planes_scale(warp_max(top), &up);
+  if (lane == 0) scale[row] = down;
   for (int k = lane; k < K; k += 32) {
     const float v = src[k] * up;
     const __half h = __float2half_rn(v);
@@ -1701,21 +1668,18 @@ extern "C" int ttb_linear_split(ttb_ctx* ctx, const ttb_linear_split_args* a) {
   return pick_tile<KIND_F16, float, VAR_SPLIT>(ctx, op, p);
 }
 
-extern "C" int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale, const float* bias, int64_t n_bias, float* stats) {
+extern "C" int ttb_split_f16(ttb_ctx* ctx, const float* x, int64_t rows, int64_t K, void* hi, void* lo, float* scale) {
   if (!ctx) return TTB_ERR_INVALID;
-  TTB_REQUIRE(ctx, rows >= 0 && K > 0 && K < (1ll << 31) && rows < (1ll << 33) && n_bias >= 0, "split_f16: bad shape");
+  TTB_REQUIRE(ctx, rows >= 0 && K > 0 && K < (1ll << 31) && rows < (1ll << 33), "split_f16: bad shape");
   if (rows == 0) return TTB_OK;
-  TTB_REQUIRE(ctx, x && hi && lo && scale && (!bias || stats), "split_f16: null pointer");
+  TTB_REQUIRE(ctx, x && hi && lo && scale, "split_f16: null pointer");
   DeviceGuard g(ctx->device);
-  if (stats) TTB_CUDA(ctx, cudaMemsetAsync(stats, 0, 2 * sizeof(float), ctx->stream));
   const bool eights = K % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0;
-  if (eights && K <= 8192 && !stats) {
+  if (eights && K <= 8192)  // (what a CTA's threads hold at once)
     launch_pdl(split_f16_rows_kernel, dim3((unsigned)std::min<int64_t>(rows, 16 * (int64_t)ctx->sm_count)), dim3((unsigned)((K / 8 + 31) / 32 * 32)), 0, ctx->stream, x, rows,
                (int)K, (__half*)hi, (__half*)lo, scale);
-    return launched(ctx, "split_f16");
-  }
-  launch_pdl(split_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, ctx->stream, x, rows, (int)K, (__half*)hi, (__half*)lo, scale, bias, bias ? n_bias : (int64_t)0,
-             stats);
+  else
+    launch_pdl(split_f16_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, ctx->stream, x, rows, (int)K, (__half*)hi, (__half*)lo, scale);
   return launched(ctx, "split_f16");
 }
 
