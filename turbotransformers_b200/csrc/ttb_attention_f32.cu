@@ -2,14 +2,16 @@
 //
 // It takes the place of five (SplitAddBiasTransposeForScore, the score product, ApplyMaskAndSoftmax, the value product, TransposeForScore)
 // that pad every sequence to the longest and write the scores out. Both products run on mma.sync m16n8k16 with every fp32 operand as two fp16 planes (three
-// products, 22 bits of an element, like the Linears'): on the CUDA cores, from shared memory, they were bound by its bandwidth (4 wavefronts a 16-byte read for
-// 32 multiply-adds: 58 % of its peak, 8 us for 16 rows against 64 keys). A row of queries or keys is scaled by its own largest element, a tile of values by its own, the
-// probabilities by 2^14; the scales come out again in fp32. Softmax, sums and the outputs' accumulation from tile to tile are fp32. Of a tile's products the small
-// ones are added up first, since the tensor core truncates the sum with every addition: 128 keys 2.1e-7 from 64 bits (all in turn 5.0e-7, on the CUDA cores 3.4e-7),
-// 512 keys 2.4e-7 (5.3e-7, 5.0e-7).
+// products, 22 bits of an element): on the CUDA cores, from shared memory, they were bound by its bandwidth (4 wavefronts a 16-byte read for
+// 32 multiply-adds: 58 % of its peak, 8 us for 16 rows against 64 keys). A row of queries, keys or values is scaled by its own largest element, a row of
+// probabilities, times their values' scales, by its own in each tile; the scales come out again in fp32. So a key that a row does not see leaves no trace in it, however
+// large it is. (One scale for a tile of values was 7 % faster, and a hidden key of 1e9 made the others 6e-3 wrong.) The second planes are 2^11 times what the first ones
+// leave, so that an element has all its bits down to 2^-28 of its row's largest. Softmax, sums and the outputs' accumulation from tile to tile are fp32. Of a tile's
+// products the small ones are added up first, since the tensor core truncates the sum with every addition. Error against 64 bits, CUDA cores with fp32 operands / now:
+// 128 keys 3.4e-7 / 2.2e-7, 512 keys 5.0e-7 / 2.4e-7; worst of all outputs, of its terms' magnitudes, with rows and dimensions up to 2^16 apart 1.3e-6 / 6.3e-7.
 // A CTA of four warps has 16 WR query rows of one (sequence, head), and WK of its warps share a tile of 64 keys: few rows for few CTAs, since the keys' way and their
-// conversion are then the time. us, 12 heads, CUDA cores / now: 8 sequences of up to 120 20.1 / 10.4, 1 x 300 42 / 19, 1 x 512 71 / 28, 3 of up to 445 68 / 33, 9 x 182 41 /
-// 23, 8 x 512 206 / 101.
+// conversion are then the time. us, 12 heads, CUDA cores / now: 8 sequences of up to 120 19.6 / 10.8, 1 x 128 15.4 / 9.8, 1 x 300 43 / 20.4, 1 x 512 71 / 31, 9 x 182 40 / 24,
+// 6 x 512 149 / 82.
 #include "ttb_common.cuh"
 
 using namespace ttb;
@@ -22,11 +24,11 @@ constexpr int kKeys = 64;
 constexpr int kPitch = 72;      // halves between the rows of a tile in shared memory: eight rows' sixteen bytes are in different banks
 constexpr int kOutPitch = 68;   // floats between the rows of a warp's output, with {maximum, sum} behind the 64
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kProbScale = 16384.f;
+constexpr float kLoUp = 2048.f, kLoDown = 1.f / kLoUp;  // the second planes are multiplied by 2^11: see planes2
 
 struct Tiles {
   __half k[2][kKeys * kPitch], v[2][kKeys * kPitch];  // hi, lo
-  float k_scale[kKeys];
+  float k_scale[kKeys], v_scale[kKeys];
 };
 union Shared {
   Tiles t;
@@ -46,14 +48,20 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Two neighbouring elements as halves of the planes.
+// Two neighbouring elements as halves of the planes. The second plane is 2^11 times what the first has left, so that it has all its bits wherever
+// the first has, down to 2^-28 of the row's largest; products with it are added up by themselves and divided by 2^11.
 __device__ __forceinline__ void planes2(float x, float y, uint32_t* hi, uint32_t* lo) {
   const __half2 h = __floats2half2_rn(x, y);
   const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+  const __half2 l = __floats2half2_rn((x - f.x) * kLoUp, (y - f.y) * kLoUp);
   *hi = *reinterpret_cast<const uint32_t*>(&h);
   *lo = *reinterpret_cast<const uint32_t*>(&l);
 }
+
+// Two magnitudes as far as their scales depend on them, in one word: fp32 numbers order like their upper halves do as whole numbers. (No number: none.)
+__device__ __forceinline__ uint32_t pack_most(float a, float b) { return __byte_perm(__float_as_uint(fmaxf(a, 0.f)), __float_as_uint(fmaxf(b, 0.f)), 0x7632); }
+__device__ __forceinline__ float first_of(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float second_of(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
 
 // ROUNDED: the output leaves as its two tf32 planes.
 template <int WR, bool ROUNDED>
@@ -62,7 +70,6 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
                      long long mask_row, int causal, float scale, float* __restrict__ out, float* __restrict__ out_lo) {
   constexpr int WK = kWarps / WR, kRows = 16 * WR, kMine = kKeys / WK, NT = kMine / 8;  // keys of a tile for a warp, in eights
   __shared__ __align__(16) Shared sm;
-  __shared__ int v_most[2];
   pdl_trigger();
   pdl_wait();
   const int b = blockIdx.z, h = blockIdx.y, q0 = blockIdx.x * kRows;
@@ -100,15 +107,13 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
 #pragma unroll
       for (int e = 0; e < 4; ++e) planes2(x[s][e].x * up[e & 1], x[s][e].y * up[e & 1], &qh[s][e], &ql[s][e]);
   }
-  if (tid < 2) v_most[tid] = 0;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[8][4];
 #pragma unroll
   for (int n = 0; n < 8; ++n)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
   const int keys = causal ? min(len, q0 + kRows) : len;
-  int turn = 0;
-  for (int j0 = 0; j0 < keys; j0 += kKeys, turn ^= 1) {
+  for (int j0 = 0; j0 < keys; j0 += kKeys) {
     // a thread's keys and values: four elements of rows (tid / 16), + 8, ...
     const int col = (tid & 15) * 4, first = tid >> 4;
     float4 k[8], v[8];
@@ -122,33 +127,24 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
       }
     }
     __syncthreads();  // the tile before has been read
-    float most = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float top = fmaxf(fmaxf(fabsf(k[i].x), fabsf(k[i].y)), fmaxf(fabsf(k[i].z), fabsf(k[i].w)));
+      uint32_t top = pack_most(fmaxf(fmaxf(fabsf(k[i].x), fabsf(k[i].y)), fmaxf(fabsf(k[i].z), fabsf(k[i].w))),
+                               fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
 #pragma unroll
-      for (int o = 1; o < 16; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      float up;
-      const float down = f16_planes_scale(top, &up);
+      for (int o = 1; o < 16; o <<= 1) top = __vmaxs2(top, __shfl_xor_sync(0xffffffffu, top, o));
+      float k_up, v_up;
+      const float k_down = f16_planes_scale(first_of(top), &k_up), v_down = f16_planes_scale(second_of(top), &v_up);
       const int r = first + i * 8;
-      if (col == 0) sm.t.k_scale[r] = down * scale;
+      if (col == 0) {
+        sm.t.k_scale[r] = k_down * scale;
+        sm.t.v_scale[r] = v_down;
+      }
       uint2 hi, lo;
-      planes2(k[i].x * up, k[i].y * up, &hi.x, &lo.x);
-      planes2(k[i].z * up, k[i].w * up, &hi.y, &lo.y);
+      planes2(k[i].x * k_up, k[i].y * k_up, &hi.x, &lo.x);
+      planes2(k[i].z * k_up, k[i].w * k_up, &hi.y, &lo.y);
       *reinterpret_cast<uint2*>(&sm.t.k[0][r * kPitch + col]) = hi;
       *reinterpret_cast<uint2*>(&sm.t.k[1][r * kPitch + col]) = lo;
-      most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
-    }
-    most = warp_max(most);
-    if (lane == 0) atomicMax(&v_most[turn], __float_as_int(most));  // (non-negative floats order like their bits)
-    __syncthreads();
-    float v_up;
-    const float v_down = f16_planes_scale(__int_as_float(v_most[turn]), &v_up);
-    if (tid == 0) v_most[turn ^ 1] = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = first + i * 8;
-      uint2 hi, lo;
       planes2(v[i].x * v_up, v[i].y * v_up, &hi.x, &lo.x);
       planes2(v[i].z * v_up, v[i].w * v_up, &hi.y, &lo.y);
       *reinterpret_cast<uint2*>(&sm.t.v[0][r * kPitch + col]) = hi;
@@ -179,6 +175,10 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
         }
       }
 #pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n + u][e] *= kLoDown;
+#pragma unroll
       for (int d = 0; d < 4; ++d)
 #pragma unroll
         for (int u = 0; u < 2; ++u) mma16816(s[n + u], qh[d], kh[d][2 * u], kh[d][2 * u + 1]);
@@ -205,16 +205,31 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
       m[r] = top[r];
       l[r] *= keep[r];
     }
-    uint32_t ph[NT / 2][4], pl[NT / 2][4];
+    // The probabilities, and those times the values' scales as planes, scaled by the largest of the row: a key that a row does not see leaves no
+    // trace in it, however large its values.
+    float most[2] = {0.f, 0.f};
 #pragma unroll
-    for (int n = 0; n < NT; ++n)
+    for (int n = 0; n < NT; ++n) {
+      const float2 vs = *reinterpret_cast<const float2*>(&sm.t.v_scale[mine + n * 8 + t * 2]);
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const float x = expf(s[n][r * 2] - centre[r]), y = expf(s[n][r * 2 + 1] - centre[r]);
         l[r] += x + y;
-        planes2(x * kProbScale, y * kProbScale, &ph[n / 2][(n & 1) * 2 + r], &pl[n / 2][(n & 1) * 2 + r]);
+        s[n][r * 2] = x * vs.x;
+        s[n][r * 2 + 1] = y * vs.y;
+        most[r] = fmaxf(most[r], fmaxf(s[n][r * 2], s[n][r * 2 + 1]));
       }
-    const float factor = v_down * (1.f / kProbScale);
+    }
+    uint32_t both = pack_most(most[0], most[1]);
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) both = __vmaxs2(both, __shfl_xor_sync(0xffffffffu, both, o));
+    float p_up[2];
+    const float factor[2] = {f16_planes_scale(first_of(both), &p_up[0]), f16_planes_scale(second_of(both), &p_up[1])};
+    uint32_t ph[NT / 2][4], pl[NT / 2][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) planes2(s[n][r * 2] * p_up[r], s[n][r * 2 + 1] * p_up[r], &ph[n / 2][(n & 1) * 2 + r], &pl[n / 2][(n & 1) * 2 + r]);
 #pragma unroll
     for (int d = 0; d < 4; ++d) {  // sixteen dimensions
       float o[2][4];
@@ -236,13 +251,17 @@ attention_f32_kernel(const float* __restrict__ qkv, const int32_t* __restrict__ 
         }
       }
 #pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[u][e] *= kLoDown;
+#pragma unroll
       for (int n = 0; n < NT / 2; ++n)
 #pragma unroll
         for (int u = 0; u < 2; ++u) mma16816(o[u], ph[n], vh[n][2 * u], vh[n][2 * u + 1]);
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[d * 2 + u][e] = fmaf(o[u][e], factor, acc[d * 2 + u][e] * keep[e >> 1]);
+        for (int e = 0; e < 4; ++e) acc[d * 2 + u][e] = fmaf(o[u][e], factor[e >> 1], acc[d * 2 + u][e] * keep[e >> 1]);
     }
   }
   __syncthreads();  // the last tile has been read: the warps' results take its place
