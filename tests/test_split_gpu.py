@@ -74,6 +74,19 @@ def test_product(ctx, M, N, K):
     assert ctx.device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 768, 768), (128, 768, 768), (17, 512, 512), (128, 384, 384), (250, 512, 512), (128, 1024, 1024), (100, 768, 3072), (300, 2304, 768)])
+def test_no_further_off_than_tf32_planes(ctx, M, N, K):
+    """Few rows, whose products are split along K: an accumulator adds up no more than with tf32 planes."""
+    x, w, tf32 = randn(M, K), randn(N, K, seed=2, scale=K ** -0.5), torch.zeros(M, N, device=DEV)
+    exact = x.double() @ w.double().T
+    xp, wp = torch.zeros(2, M, K, device=DEV), torch.zeros(2, N, K, device=DEV)
+    ctx.call("split_tf32", x, M * K, xp[0], xp[1])
+    ctx.call("split_tf32", w, N * K, wp[0], wp[1])
+    ctx.linear_ex(_capi.F32, _capi.F32, xp[0], wp[0], M, N, K, _capi.EPI_NONE, tf32, A2=xp[1], W2=wp[1])
+    # (both are mostly what the accumulators cut off, which is the same but for the inputs' noise where as much is added up)
+    assert err(product(ctx, split(ctx, x), split(ctx, w), N, K, _capi.EPI_NONE), exact) < 1.1 * err(tf32, exact)
+
+
 @pytest.mark.parametrize("M", [5, 300])
 def test_product_over_the_range_of_scales(ctx, M):
     """Rows and columns many powers of two apart, and a row's own elements too: every element is as close to its own terms as in tf32 planes, whose exponent is fp32's."""

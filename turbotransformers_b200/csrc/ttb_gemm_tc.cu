@@ -18,10 +18,11 @@
 //   bf16 activations kept as hi + lo planes :  A_hi.W + A_lo.W                       (2 passes)
 //   fp32 as three tf32 products             :  A_hi.W_hi + A_lo.W_hi + A_hi.W_lo     (3 passes)
 //   fp32 as three fp16 products             :  the same, of rows that are scaled into fp16's range; the epilogue takes the scales out again
-// fp16 planes hold as many bits as tf32 ones (an element to 2^-23, or to 2^-40 of its row's largest) at half the bytes and twice the rate, and a sum is
-// half as many instructions, each of which truncates it: us, tf32 / fp16 planes, and error against 64 bits: 128 x 2304 x 768 11.6 / 10.2, 527 x 768 x 3072 33.8 /
-// 19.6, 1.1e-5 / 5.6e-6; 3000 x 2304 x 768 44.7 / 27.7, 2.8e-6 / 1.5e-6; 3000 x 768 x 3072 63.1 / 32.1. (128 x 768 x 768 9.5 / 10.2, 8.3e-7 / 1.5e-6: there
-// is less to split along K.) BERT-base fp32: 1 x 128 1085 -> 941, 7.5e-6 -> 4.8e-6; 8 ragged requests 1748 -> 1277, 1.7e-5 -> 8.6e-6.
+// fp16 planes hold as many bits as tf32 ones (an element to 2^-23, or to 2^-39 of its row's largest) at half the bytes and twice the rate, and a sum is
+// half as many instructions, each of which truncates it: us, tf32 / fp16 planes, and error against 64 bits: 128 x 768 x 768 8.9 / 8.0, 8.3e-7 / 6.2e-7; 128 x 2304 x
+// 768 11.3 / 7.9, 1.5e-6 both; 527 x 768 x 3072 33.9 / 19.6, 1.1e-5 / 5.6e-6; 3000 x 2304 x 768 45.0 / 27.8, 2.8e-6 / 1.5e-6; 3000 x 768 x 3072 63.9 / 32.2. With a row's
+// elements up to 2^20 apart, and the weights' as far the other way, the errors stay so; beyond, where fp16 planes have fewer bits of the small ones, tf32 planes are
+// closer (2^24 apart: 128 x 768 x 768 8.3e-7 / 1.1e-5).
 // Products of few tiles with a long K are split along K over the CTAs of a cluster: every CTA accumulates its K range
 // in its own TMEM, the others hand their partial tile to the first CTA through distributed shared memory, and that CTA
 // adds them in rank order and runs the epilogue, so the result does not depend on timing.
@@ -1375,12 +1376,22 @@ TilePlan choose_tile(ttb_ctx* ctx, int64_t M, int64_t N, int64_t K, int npass, b
   consider({64, 1, false, tiles(64), sms}, kCost64.fixed, kCost64, products, narrow_kb);
   const int64_t t32 = tiles(32);
   consider({32, 1, false, t32, sms}, kCost32.fixed, kCost32, products, narrow_kb);
+  auto splits = [&](int s) { return t32 * s <= sms && s <= narrow_kb / 2 && t32 <= max_resident_clusters<KIND, OutT, VAR>(ctx, s); };
   // Few 128 x 32 tiles: the CTAs of a cluster may share each tile's K range, two k-blocks or more each, so that the weights
   // stream through (nearly) all SMs instead of a few. At M = 128, K = 3072 (48 k-blocks): 15.6 us in one CTA per tile, 8.7 split
   // four ways. All clusters must be resident at once (one wave): how many the device holds depends on how they pack into its GPCs.
   for (int s = splitk_cap(); s >= 2; --s) {
-    if (t32 * s > sms || s > narrow_kb / 2 || t32 > max_resident_clusters<KIND, OutT, VAR>(ctx, s)) continue;
-    consider({32, s, false, t32, t32}, kCostSplit + kCostSplitCta * (s - 1), kCost32, products, (narrow_kb + s - 1) / s);
+    if (splits(s)) consider({32, s, false, t32, t32}, kCostSplit + kCostSplitCta * (s - 1), kCost32, products, (narrow_kb + s - 1) / s);
+  }
+  // fp32 as fp16 planes: where tf32 planes, with twice the k-blocks, pay for three CTAs along K and more, one less here, so that no accumulator adds up more
+  // products than with those (the tensor core truncates each sum). us and error, tf32 / fp16 in one CTA / in three: 128 x 768 x 768 8.9, 8.3e-7 / 7.6, 1.5e-6 /
+  // 8.0, 6.2e-7; 64 x 512 x 512 6.9, 6.0e-7 / 6.0, 1.1e-6 / 6.6, 5.2e-7. (For two tf32 CTAs and one of fp16 the errors are the same.)
+  if constexpr (VAR == VAR_SPLIT) {
+    int s = choose_tile<KIND_TF32, OutT, VAR_PLAIN>(ctx, M, N, K, npass, words).split_k - 1;
+    if (s >= 2 && best.split_k < s) {
+      while (s >= 2 && !splits(s)) --s;
+      if (s >= 2 && best.split_k < s) return {32, s, false, t32, t32};
+    }
   }
   return best;
 }
