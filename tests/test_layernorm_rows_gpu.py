@@ -16,8 +16,8 @@ def _rows(M, N, dtype):
     return x, *(torch.randn(N, generator=g, device=DEV).to(dtype) for _ in range(2))
 
 
-@pytest.mark.parametrize("N", [8, 776, 1024, 1032])
-@pytest.mark.parametrize("waves,more", [(0, 1), (0, 3), (64, 0), (64, 1)])
+@pytest.mark.parametrize("N", [8, 256, 776, 1024, 1032])
+@pytest.mark.parametrize("waves,more", [(0, 1), (0, 3), (5, 1), (8, 0), (30, 0), (30, 1), (64, 0), (64, 1)])
 def test_planes_of_many_rows_are_those_of_few(ctx, N, waves, more):
     M = waves * torch.cuda.get_device_properties(0).multi_processor_count + more
     x, gamma, beta = _rows(M, N, torch.bfloat16)
@@ -46,3 +46,19 @@ def test_int8_form_is_that_of_the_two_kernels(ctx, dtype, N, waves, more):
     ctx.call("layernorm", code, x, out2, gamma, beta, M, N, 1e-12)
     ctx.call("quantize_rows_int8", code, out2, M, N, q2, s2)
     assert torch.equal(out, out2) and torch.equal(q, q2) and torch.equal(s, s2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("N", [8, 256, 264, 1024])
+@pytest.mark.parametrize("waves,more", [(5, 1), (8, 0), (30, 1), (30, 2), (56, 0), (56, 1)])
+def test_sums_of_many_rows_are_those_of_few(ctx, dtype, N, waves, more):
+    M = waves * torch.cuda.get_device_properties(0).multi_processor_count + more
+    y, gamma, beta = _rows(M, N, dtype)
+    y, bias, out, code = y.to(dtype), beta * 3, (y * 0.5 + 1).to(dtype), _capi.dtype_code(dtype)
+    last = out[-3:].clone()
+    want = torch.nn.functional.layer_norm(out.double() + y.double() + bias.double(), (N,), gamma.double(), beta.double(), 1e-12)
+    ctx.call("add_bias_layernorm", code, out, y, bias, gamma, beta, M, N, 1e-12)
+    tolerance = (N / 32 + 16) * 2.0 ** -23 if dtype == torch.float32 else 2.0 ** -10
+    assert float((out.double() - want).abs().max()) <= tolerance * float(want.abs().max())
+    ctx.call("add_bias_layernorm", code, last, y[-3:].contiguous(), bias, gamma, beta, 3, N, 1e-12)
+    assert torch.equal(last, out[-3:])

@@ -19,58 +19,55 @@ inline int grid_for(int64_t work, int per_block, int sm_count) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// LayerNorm: out = LN(x [+ residual + bias]) * gamma + beta. One warp per pair of rows, both rows cached in registers
-// and all of their loads issued before the first reduction, so that a warp keeps 2 x N elements in flight.
+// LayerNorm: out = LN(x [+ residual + bias]) * gamma + beta. A warp has ROWS rows in registers, all of whose loads are issued before the first reduction.
 // ITERS vectors of 8 elements per lane and row: N % 8 == 0 and N <= 256*ITERS. x may be out (no __restrict__ on them).
 // TIn is the type of x / residual, TOut of gamma / beta / bias / out. EXTRA adds two optional outputs for models that
 // carry more precision than TOut between layers: out_lo = what rounding to TOut dropped, out_f32 = the fp32 value.
+// AHEAD: the norm's weights are sent for right behind the row, not behind its sums.
 // ------------------------------------------------------------------------------------------------
 constexpr int kLnWarps = 8;
-// A warp has a row, and two warps are a CTA, whatever the rows: sixteen rows a CTA left most SMs without one while the rest moved 200 KB each, and two rows a warp
-// leave no registers for the norm's weights, which are then fetched behind the sums. us a launch, fp32 rows of 768 to bf16 and its planes, eight warps of two rows / now:
-// 128 rows 2.7 / 2.2, 800 6.1 / 3.8, 2048 7.0 / 4.3, 3200 7.2 / 5.6, 8192 12.5 / 10.5, 18424 29.4 / 28.2; slower for
-// narrow fp32 rows alone, 18424 x 256 7.1 / 8.5. (The former up to 1184 rows: two warps of a row each. With the norm's weights ahead of the row: 800 rows 4.8, 3200 6.8.)
-// BERT-base bf16, 16 x 200: 1924 -> 1866.
-constexpr int kLnRowWarps = 2;
 
 // EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
 // same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
 // other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099).
-template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA>
-__global__ void __launch_bounds__(kLnRowWarps * 32)
+template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS, bool AHEAD>
+__global__ void __launch_bounds__(WARPS * 32)
 layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut* __restrict__ bias, const TOut* __restrict__ gamma,
                       const TOut* __restrict__ beta, TOut* out, TOut* __restrict__ out_lo, float* __restrict__ out_f32, int64_t M, int N,
                       float eps) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
-  for (int64_t row = (int64_t)blockIdx.x * kLnRowWarps + (threadIdx.x >> 5); row < M; row += (int64_t)gridDim.x * kLnRowWarps) {
-    float v[ITERS][8];
-    float sum = 0.f;
+  for (int64_t row0 = ((int64_t)blockIdx.x * WARPS + (threadIdx.x >> 5)) * ROWS; row0 < M; row0 += (int64_t)gridDim.x * WARPS * ROWS) {
+    float v[ROWS][ITERS][8], sum[ROWS];
 #pragma unroll
-    for (int it = 0; it < ITERS; ++it) {
-      const int col = (it * 32 + lane) * 8;
-      if (col < N) {
-        Vec8<TIn> a;
-        a.load(x + row * N + col);
-        if (ADD) {
-          Vec8<TIn> rs;
-          Vec8<TOut> add;
-          rs.load(residual + row * N + col);
-          add.load(bias + col);
+    for (int r = 0; r < ROWS; ++r) {
+      sum[r] = 0.f;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) a.v[j] = a.v[j] + rs.v[j] + add.v[j];
+      for (int it = 0; it < ITERS; ++it) {
+        const int col = (it * 32 + lane) * 8;
+        if ((ROWS == 1 || row0 + r < M) && col < N) {
+          const int64_t at = (row0 + r) * N + col;
+          Vec8<TIn> a;
+          a.load(x + at);
+          if (ADD) {
+            Vec8<TIn> rs;
+            Vec8<TOut> add;
+            rs.load(residual + at);
+            add.load(bias + col);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a.v[j] = a.v[j] + rs.v[j] + add.v[j];
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { v[r][it][j] = a.v[j]; sum[r] += a.v[j]; }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[r][it][j] = 0.f;
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { v[it][j] = a.v[j]; sum += a.v[j]; }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[it][j] = 0.f;
       }
     }
-    constexpr bool kAhead = ITERS <= 4;  // the norm's weights are sent for right behind the row, not behind the sums, where registers are left
-    Vec8<TOut> g[kAhead ? ITERS : 1], b[kAhead ? ITERS : 1];
-    if (kAhead) {
+    Vec8<TOut> g[AHEAD ? ITERS : 1], b[AHEAD ? ITERS : 1];
+    if (AHEAD) {
 #pragma unroll
       for (int it = 0; it < ITERS; ++it) {
         const int col = (it * 32 + lane) * 8;
@@ -80,64 +77,100 @@ layernorm_rows_kernel(const TIn* x, const TIn* __restrict__ residual, const TOut
         }
       }
     }
-    const float mean = warp_sum(sum) / (float)N;
-    float sq = 0.f;
+    float mean[ROWS], rstd[ROWS];
 #pragma unroll
-    for (int it = 0; it < ITERS; ++it) {
-      const int col = (it * 32 + lane) * 8;
-      if (col < N) {
+    for (int r = 0; r < ROWS; ++r) mean[r] = warp_sum(sum[r]) / (float)N;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { float d = v[it][j] - mean; sq += d * d; }
+    for (int r = 0; r < ROWS; ++r) {
+      float sq = 0.f;
+#pragma unroll
+      for (int it = 0; it < ITERS; ++it) {
+        const int col = (it * 32 + lane) * 8;
+        if (col < N) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) { float d = v[r][it][j] - mean[r]; sq += d * d; }
+        }
       }
+      rstd[r] = rsqrtf(warp_sum(sq) / (float)N + eps);
     }
-    const float rstd = rsqrtf(warp_sum(sq) / (float)N + eps);
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int col = (it * 32 + lane) * 8;
       if (col < N) {
-        const int w = kAhead ? it : 0;
-        if (!kAhead) {
+        const int w = AHEAD ? it : 0;
+        if (!AHEAD) {
           g[0].load(gamma + col);
           b[0].load(beta + col);
         }
-        Vec8<TOut> o;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o.v[j] = b[w].v[j] + g[w].v[j] * rstd * (v[it][j] - mean);
-        if (EXTRA == 3 && (it + 1) * 256 <= N) {
+        for (int r = 0; r < ROWS; ++r) {
+          const int64_t row = row0 + r;
+          if (ROWS > 1 && row >= M) continue;
+          Vec8<TOut> o;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float word[4];
+          for (int j = 0; j < 8; ++j) o.v[j] = b[w].v[j] + g[w].v[j] * rstd[r] * (v[r][it][j] - mean[r]);
+          if (EXTRA == 3 && (it + 1) * 256 <= N) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float first = __shfl_sync(0xffffffffu, o.v[j], h * 16 + (lane >> 1)), second = __shfl_sync(0xffffffffu, o.v[4 + j], h * 16 + (lane >> 1));
-              word[j] = (lane & 1) ? second : first;
+            for (int h = 0; h < 2; ++h) {
+              float word[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float first = __shfl_sync(0xffffffffu, o.v[j], h * 16 + (lane >> 1)), second = __shfl_sync(0xffffffffu, o.v[4 + j], h * 16 + (lane >> 1));
+                word[j] = (lane & 1) ? second : first;
+              }
+              const int64_t at = row * N + it * 256 + h * 128 + lane * 4;
+              *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = make_float4(word[0], word[1], word[2], word[3]);
+              *reinterpret_cast<float4*>(out_f32 + at) = make_float4(tf32_hi(word[0]), tf32_hi(word[1]), tf32_hi(word[2]), tf32_hi(word[3]));
+              *reinterpret_cast<float4*>(reinterpret_cast<float*>(out_lo) + at) =
+                  make_float4(tf32_lo(word[0], true), tf32_lo(word[1], true), tf32_lo(word[2], true), tf32_lo(word[3], true));
             }
-            const int64_t at = row * N + it * 256 + h * 128 + lane * 4;
-            *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = make_float4(word[0], word[1], word[2], word[3]);
-            *reinterpret_cast<float4*>(out_f32 + at) = make_float4(tf32_hi(word[0]), tf32_hi(word[1]), tf32_hi(word[2]), tf32_hi(word[3]));
-            *reinterpret_cast<float4*>(reinterpret_cast<float*>(out_lo) + at) =
-                make_float4(tf32_lo(word[0], true), tf32_lo(word[1], true), tf32_lo(word[2], true), tf32_lo(word[3], true));
+            continue;
           }
-          continue;
-        }
-        o.store(out + row * N + col);
-        if (EXTRA) {
-          if (EXTRA >= 2 || out_f32) {
-            Vec8<float> f;
+          o.store(out + row * N + col);
+          if (EXTRA) {
+            if (EXTRA >= 2 || out_f32) {
+              Vec8<float> f;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f.v[j] = EXTRA >= 2 ? tf32_hi(o.v[j]) : o.v[j];
-            f.store(out_f32 + row * N + col);
-          }
-          if (EXTRA >= 2 || out_lo) {
-            Vec8<TOut> l;
+              for (int j = 0; j < 8; ++j) f.v[j] = EXTRA >= 2 ? tf32_hi(o.v[j]) : o.v[j];
+              f.store(out_f32 + row * N + col);
+            }
+            if (EXTRA >= 2 || out_lo) {
+              Vec8<TOut> l;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j], EXTRA >= 2);
-            l.store(out_lo + row * N + col);
+              for (int j = 0; j < 8; ++j) l.v[j] = rest_of<TOut>(o.v[j], EXTRA >= 2);
+              l.store(out_lo + row * N + col);
+            }
           }
         }
       }
     }
   }
+}
+
+// How many rows a warp and warps a CTA have. A row a warp and two warps a CTA: sixteen rows a CTA left most SMs without one while the rest moved 200 KB
+// each, and two rows a warp leave no registers for the norm's weights, which are then fetched behind the sums. us a launch, fp32 rows of 768 to bf16 and its planes,
+// eight warps of two rows / so: 128 rows 2.7 / 2.2, 800 6.1 / 3.8, 2048 7.0 / 4.3, 3200 7.2 / 5.6, 8192 12.5 / 10.5, 18424 29.4 / 28.2. (With the norm's weights ahead of
+// the row: 800 rows 4.8, 3200 6.8.) BERT-base bf16, 16 x 200: 1924 -> 1866. Where that is not the fastest:
+//   Rows of up to 256 columns, an access or two a lane, beyond 30 rows an SM: eight warps of two rows, fewer CTAs to start (fp32 9000 x 256 6.4 -> 4.5, 18424 x 256
+//   8.7 -> 7.3, 40000 x 256 with a residual 20.7 -> 18.5). From 5 to 8 rows an SM, and with planes up to there: weights behind the sums (1184 x 256 2.8 -> 2.3,
+//   740 with planes 2.28 -> 2.21).
+//   fp32 rows with a residual beyond 56 rows an SM, bound by how many rows are on their way: the weights' registers for another CTA (18424 x 1024 52.4 -> 39.6; two rows
+//   a warp 49.8; 18424 x 768 32.9 -> 26.8).
+template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA>
+void launch_layernorm_rows(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut* bias, const TOut* gamma, const TOut* beta, TOut* out, TOut* out_lo,
+                           float* out_f32, int64_t M, int64_t N, float eps) {
+  auto launch = [&](auto kernel, int warps, int rows) {
+    launch_pdl(kernel, dim3(grid_for((M + rows - 1) / rows, warps, ctx->sm_count)), dim3(warps * 32), 0, ctx->stream, x, residual, bias, gamma, beta, out, out_lo, out_f32, M,
+               (int)N, eps);
+  };
+  const int64_t sms = ctx->sm_count;
+  if constexpr (ITERS == 1 && EXTRA <= 1) {
+    if (M > 30 * sms) return launch(layernorm_rows_kernel<TIn, TOut, ITERS, ADD, EXTRA, kLnWarps, 2, false>, kLnWarps, 2);
+    if (M <= 8 * sms && (EXTRA || M > 5 * sms)) return launch(layernorm_rows_kernel<TIn, TOut, ITERS, ADD, EXTRA, 2, 1, false>, 2, 1);
+  } else if constexpr (ITERS <= 4 && EXTRA == 0 && ADD && std::is_same<TOut, float>::value) {
+    if (M > 56 * sms) return launch(layernorm_rows_kernel<TIn, TOut, ITERS, ADD, EXTRA, 2, 1, false>, 2, 1);
+  }
+  launch(layernorm_rows_kernel<TIn, TOut, ITERS, ADD, EXTRA, 2, 1, (ITERS <= 4)>, 2, 1);  // (wider rows leave no registers for the weights)
 }
 
 // The same for 16-bit rows without the residual form (the 16-bit models' hot case), as a streaming kernel: a grid that
@@ -590,10 +623,7 @@ int launch_layernorm(ttb_ctx* ctx, const TIn* x, const TIn* residual, const TOut
   constexpr bool kFloat = std::is_same<TOut, float>::value;  // fp32 with both extras: its planes
   constexpr int kPlanes = kFloat ? 2 : 1, kPlanesTraded = kFloat ? 3 : 1;
   const bool planes = kFloat && out_lo && out_f32, traded = planes && M > (int64_t)ctx->sm_count;
-  const int row_grid = grid_for(M, kLnRowWarps, ctx->sm_count);
-#define LN_ROWS(IT, EXTRA)                                                                                                                          \
-  launch_pdl(layernorm_rows_kernel<TIn, TOut, IT, ADD, EXTRA>, dim3(row_grid), dim3(kLnRowWarps * 32), 0, ctx->stream, x, residual, bias, gamma, beta, \
-             out, out_lo, out_f32, M, (int)N, eps)
+#define LN_ROWS(IT, EXTRA) launch_layernorm_rows<TIn, TOut, IT, ADD, EXTRA>(ctx, x, residual, bias, gamma, beta, out, out_lo, out_f32, M, N, eps)
 #define LN_CASE(IT)                                  \
   do {                                               \
     if (traded) LN_ROWS(IT, kPlanesTraded);          \
