@@ -112,7 +112,7 @@ def test_layer_norm_leaves_the_planes_of_its_output(ctx, M, N):
 
 
 def test_embedding_leaves_the_planes_of_its_output(ctx):
-    for hidden in (768, 128, 1000):
+    for hidden in (768, 128, 1000, 8, 264, 520, 1024, 1032, 2048, 2056):
         ids, out = torch.randint(0, 100, (3, 7), generator=torch.Generator(device=DEV).manual_seed(1), device=DEV), torch.zeros(21, hidden, device=DEV)
         planes, scale, plain = torch.zeros(2, 21, hidden, device=DEV).half(), torch.zeros(21, device=DEV), torch.zeros(21, hidden, device=DEV)
         tables = (randn(100, hidden), randn(16, hidden, seed=2), randn(2, hidden, seed=3), randn(hidden, seed=4), randn(hidden, seed=5))

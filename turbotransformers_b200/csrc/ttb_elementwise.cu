@@ -826,6 +826,25 @@ __device__ __forceinline__ int find_sequence(const int32_t* cu, int B, int token
   return lo;
 }
 
+// Token t's rows of the three tables. One that is out of range is reported, and the nearest taken. All lanes of a warp call it.
+struct Looked {
+  int64_t id, pos, type;
+};
+__device__ __forceinline__ Looked look_up(const int64_t* ids, const int64_t* pos_ids, const int64_t* type_ids, const int32_t* cu, int B, int seq_len, int64_t t,
+                                          int64_t vocab, int64_t n_pos, int64_t n_types, int* status) {
+  Looked at;
+  at.id = ids[t];
+  at.pos = pos_ids ? pos_ids[t] : (cu ? (int64_t)t - cu[find_sequence(cu, B, (int)t)] : (t % seq_len));
+  at.type = type_ids ? type_ids[t] : 0;
+  if (at.id < 0 || at.id >= vocab || at.pos < 0 || at.pos >= n_pos || at.type < 0 || at.type >= n_types) {
+    if ((threadIdx.x & 31) == 0) atomicExch(status, (int)TTB_ERR_BAD_INDEX);
+    at.id = at.id < 0 ? 0 : (at.id >= vocab ? vocab - 1 : at.id);
+    at.pos = at.pos < 0 ? 0 : (at.pos >= n_pos ? n_pos - 1 : at.pos);
+    at.type = at.type < 0 ? 0 : (at.type >= n_types ? n_types - 1 : at.type);
+  }
+  return at;
+}
+
 // word[id] + position[pos] + token_type[tt] -> LayerNorm, one warp per token, any hidden size.
 template <typename T>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
@@ -840,19 +859,10 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
   const int lane = threadIdx.x & 31;
   const int warps_total = gridDim.x * kRowsPerBlock;
   for (int64_t t = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); t < n_tokens; t += warps_total) {
-    int64_t id = ids[t];
-    int64_t pos = pos_ids ? pos_ids[t] : (cu ? (int64_t)t - cu[find_sequence(cu, B, (int)t)] : (t % seq_len));
-    int64_t tt = type_ids ? type_ids[t] : 0;
-    bool bad = id < 0 || id >= vocab || pos < 0 || pos >= n_pos || tt < 0 || tt >= n_types;
-    if (bad) {
-      if (lane == 0) atomicExch(status, (int)TTB_ERR_BAD_INDEX);
-      id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
-      pos = pos < 0 ? 0 : (pos >= n_pos ? n_pos - 1 : pos);
-      tt = tt < 0 ? 0 : (tt >= n_types ? n_types - 1 : tt);
-    }
-    const T* w = word + id * hidden;
-    const T* p = position + pos * hidden;
-    const T* y = token_type + tt * hidden;
+    const Looked at = look_up(ids, pos_ids, type_ids, cu, B, seq_len, t, vocab, n_pos, n_types, status);
+    const T* w = word + at.id * hidden;
+    const T* p = position + at.pos * hidden;
+    const T* y = token_type + at.type * hidden;
     // same accumulation order as the reference: word, then token type, then position
     auto val = [&](int c) { return (to_f(w[c]) + to_f(y[c])) + to_f(p[c]); };
     float sum = 0.f;
@@ -900,6 +910,66 @@ embedding_ln_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__
   }
 }
 
+// The same in fp32 with the output's fp16 planes and their scales (ttb_split_f16), hidden <= 32 * NI: the sum is held in registers, in the order of the kernel above
+// (whose output this one's is bit for bit). Bound by latency, of the tables' rows and of the three sums and maxima over a row: two warps a CTA.
+// us a launch of 768 columns, the kernel above with a pass over the tables for each of them / now: 128 rows 10.5 / 4.2, 527 10.3 / 5.4, 3000 17.4 / 9.3.
+constexpr int kEmbeddingWarps = 2;
+template <int NI>
+__global__ void __launch_bounds__(kEmbeddingWarps * 32)
+embedding_ln_split_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ pos_ids, const int64_t* __restrict__ type_ids,
+                          const int32_t* __restrict__ cu, int B, int seq_len, int64_t n_tokens, const float* __restrict__ word,
+                          const float* __restrict__ position, const float* __restrict__ token_type, const float* __restrict__ gamma,
+                          const float* __restrict__ beta, int hidden, int64_t vocab, int64_t n_pos, int64_t n_types, float eps, float* __restrict__ out,
+                          __half* __restrict__ hi, __half* __restrict__ lo, float* __restrict__ scale, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  for (int64_t t = (int64_t)blockIdx.x * kEmbeddingWarps + (threadIdx.x >> 5); t < n_tokens; t += (int64_t)gridDim.x * kEmbeddingWarps) {
+    const Looked at = look_up(ids, pos_ids, type_ids, cu, B, seq_len, t, vocab, n_pos, n_types, status);
+    const float* w = word + at.id * hidden;
+    const float* p = position + at.pos * hidden;
+    const float* y = token_type + at.type * hidden;
+    float v[NI], sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = i * 32 + lane;
+      v[i] = c < hidden ? (w[c] + y[c]) + p[c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (i * 32 + lane < hidden) sum += v[i];
+    const float mean = warp_sum(sum) / (float)hidden;
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (i * 32 + lane < hidden) { const float d = v[i] - mean; sq += d * d; }
+    const float rstd = rsqrtf(warp_sum(sq) / (float)hidden + eps);
+    float top = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = i * 32 + lane;
+      if (c < hidden) {
+        v[i] = beta[c] + gamma[c] * rstd * (v[i] - mean);
+        out[t * hidden + c] = v[i];
+        top = fmaxf(top, fabsf(v[i]));
+      }
+    }
+    float up;
+    const float down = f16_planes_scale(warp_max(top), &up);
+    if (lane == 0) scale[t] = down;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int c = i * 32 + lane;
+      if (c < hidden) {
+        const float x = v[i] * up;
+        const __half h = __float2half_rn(x);
+        hi[t * hidden + c] = h;
+        lo[t * hidden + c] = __float2half_rn(x - __half2float(h));
+      }
+    }
+  }
+}
+
 // The same for 16-bit tables with hidden % 8 == 0 and hidden <= 256 * ITERS: 16-byte loads of the three rows, the sum held
 // in registers for the two passes of the statistics and the output.
 template <typename T, int ITERS>
@@ -914,19 +984,10 @@ embedding_ln16_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict
   const int lane = threadIdx.x & 31;
   const int warps_total = gridDim.x * kRowsPerBlock;
   for (int64_t t = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); t < n_tokens; t += warps_total) {
-    int64_t id = ids[t];
-    int64_t pos = pos_ids ? pos_ids[t] : (cu ? (int64_t)t - cu[find_sequence(cu, B, (int)t)] : (t % seq_len));
-    int64_t tt = type_ids ? type_ids[t] : 0;
-    const bool bad = id < 0 || id >= vocab || pos < 0 || pos >= n_pos || tt < 0 || tt >= n_types;
-    if (bad) {
-      if (lane == 0) atomicExch(status, (int)TTB_ERR_BAD_INDEX);
-      id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
-      pos = pos < 0 ? 0 : (pos >= n_pos ? n_pos - 1 : pos);
-      tt = tt < 0 ? 0 : (tt >= n_types ? n_types - 1 : tt);
-    }
-    const T* w = word + id * hidden;
-    const T* p = position + pos * hidden;
-    const T* y = token_type + tt * hidden;
+    const Looked at = look_up(ids, pos_ids, type_ids, cu, B, seq_len, t, vocab, n_pos, n_types, status);
+    const T* w = word + at.id * hidden;
+    const T* p = position + at.pos * hidden;
+    const T* y = token_type + at.type * hidden;
     float v[ITERS][8];
     float sum = 0.f;
 #pragma unroll
@@ -1652,6 +1713,19 @@ static int embedding_ln(ttb_ctx* ctx, int dtype, const int64_t* ids, const int64
     else EMB16_PICK(__nv_bfloat16);
 #undef EMB16_PICK
 #undef EMB16
+    return launched(ctx, "embedding_ln");
+  }
+  if (out_scale && hidden <= 2048) {
+    auto launch = [&](auto kernel) {
+      launch_pdl(kernel, dim3(grid_for(n_tokens, kEmbeddingWarps, ctx->sm_count)), dim3(kEmbeddingWarps * 32), 0, ctx->stream, ids, position_ids, token_type_ids, cu_seqlens,
+                 (int)B, (int)(seq_len > 0 ? seq_len : 1), n_tokens, (const float*)word, (const float*)position, (const float*)token_type, (const float*)gamma,
+                 (const float*)beta, (int)hidden, vocab, n_positions, n_types, eps, (float*)out, reinterpret_cast<__half*>(out_f32), (__half*)out_lo, out_scale, ctx->d_status);
+    };
+    if (hidden <= 256) launch(embedding_ln_split_kernel<8>);
+    else if (hidden <= 512) launch(embedding_ln_split_kernel<16>);
+    else if (hidden <= 768) launch(embedding_ln_split_kernel<24>);
+    else if (hidden <= 1024) launch(embedding_ln_split_kernel<32>);
+    else launch(embedding_ln_split_kernel<64>);
     return launched(ctx, "embedding_ln");
   }
   TTB_DISPATCH_FLOAT(ctx, dtype, T,
