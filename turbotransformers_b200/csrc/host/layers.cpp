@@ -278,7 +278,7 @@ void PackedLinear::Forward(const Tensor& x, int64_t M, int epilogue, const void*
     return;
   }
   if (dt == TTB_F32 && (core::Fp32TensorCores() || (x.lo() && !x.hi())) && K % 4 == 0 && M > 0) {
-    // the same with tf32 planes, for widths that are no multiple of eight
+    // the same with tf32 planes, for widths that are no multiple of eight and activations that come as such planes, as from a layer norm wider than 2048
     Tensor planes(nullptr);
     const float* w = PackedTf32(is_trans);
     ttb_linear_args args{};

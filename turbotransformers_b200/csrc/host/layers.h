@@ -32,7 +32,8 @@ class PackedLinear {
   int64_t out_dim(bool is_trans) const { return weight_.shape(is_trans ? 0 : 1); }
   // K-major [N,K] copy in the weight's own 16-bit dtype (built on first use).
   const void* Packed(bool is_trans) const;
-  // fp32 weights as two tf32 planes [2][N,K] (hi, then lo), for the three-product tensor-core GEMM of widths that are no multiple of eight.
+  // fp32 weights as two tf32 planes [2][N,K] (hi, then lo), for the three-product tensor-core GEMM of widths that are no multiple of eight and of
+  // activations that come as such planes.
   const float* PackedTf32(bool is_trans) const;
   // fp32 weights as two fp16 planes [N,K] with a scale for each row (ttb_split_f16).
   struct Split {

@@ -8,7 +8,7 @@
 //     (TTB_CHAIN_UNWRITTEN); a reader asks for the words that it needs until they are others. A barrier over the grid was a flush, an atomic and a poll, 1.0
 //     us, and the rows' way from L2 behind it as much again: 278 us a step then, 235 with nothing else changed. (ttb_chain_forward, whose callers place
 //     results as they like, still has them.)
-//   * Nothing is spilled. With 227 KB of shared memory a spill does not stay in L1: 200 us with 320 bytes of them, 175 without. A third warpgroup, of which one
+//   * Nothing is spilled (but 20 bytes by the kernel for 64 rows and depths that are no whole number of steps). With 227 KB of shared memory a spill does not stay in L1: 200 us with 320 bytes of them, 175 without. A third warpgroup, of which one
 //     warp sends for weights, gives its registers to the two that compute.
 //   * Few instructions. Every operation runs through its own once, behind all those of the others, so that fetching them counts: 1 to 3 cycles each
 //     while a layer's fit in 32 KB, 6 and more beyond (measured on straight code), and a jump 30 to 100. One function for all products, steps of K that are jumped

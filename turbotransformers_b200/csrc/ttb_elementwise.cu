@@ -27,8 +27,8 @@ inline int grid_for(int64_t work, int per_block, int sm_count) {
 // ------------------------------------------------------------------------------------------------
 constexpr int kLnWarps = 8;
 
-// EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two planes of its output, out_f32 and out_lo; 3, the
-// same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
+// EXTRA: 0, the output alone; 1, out_lo and out_f32 where they are given; 2, fp32 with the two tf32 planes of its output, out_f32 and out_lo (the C call's: layers of
+// such widths take layernorm_split_kernel, wider ones the generic kernel); 3, the same with the lanes trading places before they store (more rows than SMs: bound by the stores, which write 512 bytes in a row then, not every
 // other 16 of 1024: BERT-base fp32, 527 rows, 1800 -> 1728 us, 256 1542 -> 1522, 150 the same; with 128 rows the exchange is latency, 1084 -> 1099).
 template <typename TIn, typename TOut, int ITERS, bool ADD, int EXTRA, int WARPS, int ROWS, bool AHEAD>
 __global__ void __launch_bounds__(WARPS * 32)

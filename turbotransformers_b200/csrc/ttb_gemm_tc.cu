@@ -1330,7 +1330,8 @@ struct TileCost {
 // a vocabulary, in fp16, int8, bf16 as two products (16-bit, two-plane and fp32 outputs) and fp32 as three: 1914 shapes. The kernel
 // chosen is on average 0.3 % slower than the best one; the widest tile that still gives every SM one would be 5 % slower.
 // (Constants fitted to single products of BERT-base widths alone took the narrow tiles' shared slots to be cheaper than they are:
-// bf16 4096 x 3072 x 768 37.7 us, 33.3 in pairs; fp32 4096 x 2304 x 768 63.3, 56.1.)
+// bf16 4096 x 3072 x 768 37.7 us, 33.3 in pairs; fp32 4096 x 2304 x 768 63.3, 56.1.) fp32 as three products of fp16 planes, which came later, on M = 1 .. 6000 by 15
+// pairs (N, K) from 256 x 256 to 1024 x 4096: on average 0.2 % slower than the best one, 8 to 10 % where pairs would just pay (3000 x 3072 x 768 36.4, 33.6 us in pairs).
 constexpr TileCost kCostPair = {8900, {265, 0, 0}, {1050, 3700}, 500, 230, 32};
 constexpr TileCost kCost256 = {5150, {385, 0, 0}, {2950, 6750}, 1000, 240, 32};
 constexpr TileCost kCost128 = {2750, {255, 430, 520}, {2250, 3500}, 1200, 110, 32};
