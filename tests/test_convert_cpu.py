@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from turbotransformers_b200._cxx import cxx
-from turbotransformers_b200.layers.utils import convert2tt_tensor, try_convert
+from turbotransformers_b200.layers.utils import convert2tt_tensor, lend, try_convert
 
 
 def other_data(t):
@@ -36,3 +36,12 @@ def test_keeps_its_shape_where_the_memory_grows():
     kept = convert2tt_tensor(t)
     t.resize_(40, 50)
     assert [kept.shape(i) for i in range(kept.n_dim())] == [2, 3] and kept.numel() == 6
+
+
+def test_lent_for_a_call():
+    """For as long as the tensor is left alone the alias is that of try_convert, and what is no plain tensor goes the usual way."""
+    t = torch.arange(6.0).reshape(2, 3)
+    for given in (t, t.clone().requires_grad_(), torch.nn.Parameter(t.clone())):
+        lent = lend(given)
+        assert [lent.shape(i) for i in range(lent.n_dim())] == [2, 3] and (cxx.tensor2nparrayf(lent) == t.numpy()).all()
+    assert lend(None) is None and lend(lent) is lent

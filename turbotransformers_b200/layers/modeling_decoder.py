@@ -17,7 +17,7 @@ import torch
 from .._cxx import cxx
 from .modules import MultiHeadedAttention, PositionwiseFeedForward, _empty
 from .return_type import ReturnType, convert_returns_as_type
-from .utils import AnyTensor, try_convert, use_current_stream
+from .utils import AnyTensor, lend, try_convert, use_current_stream
 
 __all__ = ['TransformerDecoderLayer', 'TransformerDecoder']
 
@@ -79,8 +79,8 @@ class TransformerDecoderLayer:
         return TransformerDecoderLayer(self_attn, context_attn, feed_forward)
 
 
-_CACHE_NAMES = ("self_keys", "self_values", "memory_keys", "memory_values")
-_CACHED = set(_CACHE_NAMES)
+_CACHE = (("self_keys", try_convert), ("self_values", try_convert), ("memory_keys", lend), ("memory_values", lend))
+_CACHED = {name for name, _ in _CACHE}
 
 
 def _unmodified(layer) -> bool:
@@ -158,7 +158,7 @@ class TransformerDecoder:
             return None
         first, keys = self.transformer_layers[0], self.state["cache"]["layer_0"].get("self_keys")
         use_current_stream(x)
-        x = try_convert(x)
+        x = lend(x)
         past = 0 if keys is None or not isinstance(keys, cxx.Tensor) or keys.is_null() else keys.shape(0)
         if not (isinstance(first.self_attn, cxx.MultiHeadedAttention) and isinstance(first.feed_forward, cxx.PositionwiseFeedForward) and
                 cxx.decoder_chain_takes(first.self_attn, first.feed_forward, first._ffn_trans, x, past, src_pad_mask.size(-1),
@@ -169,14 +169,15 @@ class TransformerDecoder:
         for (s, c, f), cache in zip(parts, caches):
             if set(cache) != _CACHED or type(s) is not MultiHeadedAttention or type(c) is not MultiHeadedAttention or type(f) is not PositionwiseFeedForward:
                 return None
-        held = [tuple([_empty() if c[k] is None else try_convert(c[k]) for k in _CACHE_NAMES]) for c in caches]
+        # (the keys and values of the layers' own stay with the cache; what is given of the memory, and x and the mask, are read by this call alone)
+        held = [tuple([_empty() if c[k] is None else convert(c[k]) for k, convert in _CACHE]) for c in caches]
         # a memory entry is only read where both of a layer are filled; otherwise both are projected, whichever was given
         projected = [h[2].is_null() or h[3].is_null() for h in held]
         memory = memory_bank.transpose(0, 1).contiguous() if any(projected) else None
         src_mask = (src_pad_mask.float() * -1e18).contiguous()
         out, attn = _empty(), _empty()
-        if not cxx.decoder_chain(parts, held, x, False, first._ffn_trans, None, None, try_convert(memory),
-                                 try_convert(src_mask), out, None, attn):
+        if not cxx.decoder_chain(parts, held, x, False, first._ffn_trans, None, None, lend(memory),
+                                 lend(src_mask), out, None, attn):
             return None
         use_current_stream(src_mask)  # torch reads the results on the caller's stream, wherever another thread has pointed the runtime meanwhile
         for c, h, fresh in zip(caches, held, projected):
